@@ -94,7 +94,7 @@ static void destroy(Ctx *c) {
                   c->ktile_sys, c->ftile_sys, c->k_sys, c->kf_part, c->ered, c->ered_done, c->sys_items, c->ftab_lj2, c->rb_scan,
                   c->fxr, c->intra_buf, c->ithm, c->nhc, c->cwl, c->cwn, c->cw_tf, c->cw_tg, c->cw_tl,
                   c->cw_part, c->nvt_kin, c->nvt_chsum, c->th_atoms, c->th_choff, c->th_chunk,
-                  c->cw_sys, c->cw_sitems, c->cw_items, c->cw_gidx, c->cw_scan, c->grp_work};
+                  c->cw_sys, c->cw_sitems, c->cw_items, c->cw_gidx, c->cw_scan, c->grp_work, c->smeta, c->xspan};
   cw_destroy(c);
   for (void *p : ptrs)
     if (p) cudaFree(p);
@@ -447,6 +447,27 @@ static int create(const cm3d_nb_system *systems, int nsys, const cm3d_nb_options
   if ((rc = upload(&c->cexcl_off, coff.data(), coff.size()))) return rc;
   if ((rc = upload(&c->cexcl_idx, cidx.data(), cidx.size()))) return rc;
   if ((rc = upload(&c->icharge, ich.data(), ich.size()))) return rc;
+  // the span of the atoms excluded from each atom (an entry sits at the
+  // lower index; the list kernels look a pair up only inside the span)
+  {
+    std::vector<int2> span((size_t)n, make_int2(n, -1));
+    auto widen = [&](const std::vector<int> &off, const std::vector<int> &idx) {
+      for (int i = 0; i < n; i++)
+        for (int k = off[i]; k < off[i + 1]; k++) {
+          const int j = idx[k];
+          if (j <= i || j >= n) continue;
+          span[i].x = std::min(span[i].x, j);
+          span[i].y = std::max(span[i].y, j);
+          span[j].x = std::min(span[j].x, i);
+          span[j].y = std::max(span[j].y, i);
+        }
+    };
+    widen(eoff, eidx);
+    widen(coff, cidx);
+    // as {lowest, highest - lowest}; none: a span that holds no atom
+    for (int2 &x : span) x = x.y < 0 ? make_int2(0x7fffffff, 0) : make_int2(x.x, x.y - x.x);
+    if ((rc = upload(&c->xspan, span.data(), span.size()))) return rc;
+  }
   // accumulators: per system ACC_COUNT sums + device copies of hmati and hmat
   std::vector<double> acc0((size_t)nsys * ACC_STRIDE, 0.0);
   for (int sy = 0; sy < nsys; sy++)

@@ -77,6 +77,8 @@ struct SysP {
   int ftile0, ftiles;        // reciprocal-force tiles (global tile ids)
   long long spart0;          // first per-tile partial S(k) of the system
   float lim2;                // FP32 list prefilter radius^2 (inf = off)
+  float lim2_image;          //   and that of a minimum-image distance (grids of fewer than 3 cells)
+  int image_ok;              // the grid allows FP32 minimum images in the list tests
   float rc2_el, dx2c, offc, tablast_e;
   float hF[9], hiF[9];
   double h[9], hi[9];
@@ -234,6 +236,8 @@ struct Ctx {
   double *ered = nullptr;              // k_ereduce: per-block partial sums of one large system
   unsigned *ered_done = nullptr;       // k_ereduce: blocks finished per quantity
   int lw_cap = 0;                      // staged list build: neighbourhood atoms per block (0: off)
+  int list_tile = 0;                   // tiled list build: every system has 3 or more cells per axis
+  int lw_atoms = 1;                    //   and atoms of its fullest cell (mean count + 25%)
   int *grp_work = nullptr;             // groups with ecorr pairs, bonds or bends (device)
   int ngwork = 0;
   int *rb_scan = nullptr;              // staged list build: cells rebuilt before each system (nsys + 1)
@@ -379,6 +383,8 @@ struct Ctx {
   float *epart = nullptr;               // mixed: per-atom energy/virial partials
   int *styp = nullptr;                  // sorted type
   int *sorig = nullptr;                 // sorted -> original (== cell_atoms)
+  int2 *smeta = nullptr;                // sorted: {atom index, 2 type + charged}
+  int2 *xspan = nullptr;                // per atom: {lowest atom index excluded from it, highest - lowest}
   float4 *shift = nullptr;              // 27 FP32 cell-shift vectors
   double *corner = nullptr;             // per sorted atom cell-origin offset (3n FP64)
   int4 *cimg = nullptr;                 // per atom: packed cell coords | periodic image
@@ -520,6 +526,25 @@ constexpr int CM3D_CS_THREADS = 512;            // k_pair_cs block: four groups 
 int cw_set_row(Ctx *c, int row);
 int host_outputs_tail(Ctx *c);                  // nb_step.cu: end of a step with registered host outputs                // nb_cwin.cu: a batch's list layout, 32 or 8 lanes per atom
 int cw_convert(Ctx *c, bool device_flag, bool all);   // nb_cwin.cu: master list -> compact list
+int cw_check(Ctx *c, bool device_flag);         // nb_cwin.cu: did every window fit? (after a list build)
+// The compact list of one system as the list kernel writes it directly: a
+// slot of `words` 8-byte words per sorted atom in `blocks` blocks of
+// COMPACT_BLOCK 16-bit entries, the LJ segment from the first block up and
+// the electrostatics-only segment from the last block down (see nb_cwin.cu).
+constexpr int COMPACT_BLOCK = 4 * CM3D_CW_ROW;
+constexpr unsigned COMPACT_EL = 0x4000u;        // an LJ-segment entry that is also in the te list
+struct CompactOut {
+  uint2 *list;
+  int2 *len;
+  int words, blocks, cap;
+};
+// 16-bit index of entry k of a segment inside its slot: block, lane's 8-byte
+// word, entry of the word
+__device__ __forceinline__ int compact_place(int k, bool front, int blocks) {
+  const int b0 = k & ~(COMPACT_BLOCK - 1);
+  return (front ? b0 : (blocks - 1) * COMPACT_BLOCK - b0) + ((k & (CM3D_CW_ROW - 1)) << 2) + ((k / CM3D_CW_ROW) & 3);
+}
+bool cw_direct(Ctx *c, bool device_flag, CompactOut *W, int *rc);   // nb_cwin.cu
 void cw_destroy(Ctx *c);                        // nb_cwin.cu: host-side group data
 bool cw_applies(Ctx *c, int iflg, bool ns);     // nb_cwin.cu
 int cw_pairs(Ctx *c, int mask, double *fout);   // nb_cwin.cu: pair kernel launch

@@ -54,7 +54,7 @@ constexpr int CW_THREADS_WIDE = 640;       // 20 warps at 96 registers: the auto
 constexpr int CW_ROW = CM3D_CW_ROW;         // interleave width (entries per pass of a block)
 constexpr int CW_BLOCK = 4 * CW_ROW;        // entries per block: one 8-byte word per lane
 constexpr uint32_t CW_IDX = 0x3FFFu;        // window index bits of an entry
-constexpr uint32_t CW_EL = 0x4000u;         // LJ-segment entry: the pair is also in CM3D's te list
+constexpr uint32_t CW_EL = COMPACT_EL;      // LJ-segment entry: the pair is also in CM3D's te list
 constexpr int CW_MAX_CAP = 16382;           // window slots (the dummy slot `cap` must fit 14 bits)
 constexpr float CW_MAGIC = 12582912.0f;     // 1.5 * 2^23: p + MAGIC rounded toward zero holds floor(p)
 constexpr unsigned CW_MAGIC_BITS = 0x4B400000u;
@@ -78,7 +78,11 @@ struct CwP {
 };
 
 // ------------------------------------------------------------------
-// Master list -> compact list.  Warp per cell-sorted atom t (one system:
+// Master list -> compact list, in list order, where the list kernel has not
+// written it itself (k_list_tile).  (Entries re-ordered so that a quarter-warp
+// reads eight bank groups made the pair kernel of 331,776 water atoms 0.75 ms
+// instead of 0.92, but cost this pass 4 ms per rebuild, a rebuild every three
+// or four steps.)  Warp per cell-sorted atom t (one system:
 // every atom; a batch: the atoms of the compact systems being rebuilt): the 27-cell
 // window layout of t's cell (stencil cell w = shift code, j-cell = i-cell -
 // k_w, cells in code order) gives delta[w] = window offset - first sorted
@@ -122,161 +126,42 @@ __device__ __forceinline__ void cw_convert_atom(const int t, const int lane, int
     atomicAdd((unsigned long long *)(stat + ST_CWIN), 1ull);
     if (halt) *halt = 1;
   }
-  {
-    {
-      const int na = fits ? nlen[t] : 0, nb = fits ? nlen[n + t] : 0;
-      const uint32_t *src = nbr + (size_t)t * stride;
-      uint2 *dst = cwl + (size_t)t * words;
-      // blocks of 4 row entries: row 32 lanes per atom (k_pair_cw) or 8 (k_pair_cs)
-      const int blk = 4 * row;
-      const int nba = (na + blk - 1) / blk, nbb = (nb + blk - 1) / blk;
-      // padding first: every slot of the atom's blocks holds the dummy
-      for (int w = lane; w < (nba + nbb) * row; w += 32)
-        dst[w] = make_uint2(dummy | (dummy << 16), dummy | (dummy << 16));
-      __syncwarp();
-      for (int sg = 0; sg < 2; sg++) {
-        const bool front = sg == 0;
-        const int m = front ? na : nb;
-        const uint32_t *in = front ? src : src + (stride - nb);   // the back segment ends at the slot's end
-        unsigned short *out = reinterpret_cast<unsigned short *>(dst + (front ? 0 : nba * row));
-        // every lane calls it (the delta comes by shuffle); -1 past the end
-        auto window_index_of = [&](bool v, uint32_t en, uint32_t &o) -> int {
-          const int code = (en >> ENT_CODE_SHIFT) & 31;
-          const int wi = (int)(en & ENT_JMASK) + __shfl_sync(0xffffffffu, delta, code);
-          // inside the window by construction (a pair's shift code names
-          // j's stencil cell); anything else would index past the staged
-          // atoms, so it becomes the dummy
-          o = wi >= 0 && wi < tot ? (uint32_t)wi : dummy;
-          if (front && (en & ENT_EL) && o != dummy) o |= CW_EL;
-          return v ? (int)(o & 7u) : -1;
-        };
-        auto window_index = [&](int e, uint32_t &o) -> int {
-          const bool v = e < m;
-          return window_index_of(v, v ? in[e] : 0u, o);
-        };
-        // bank classes: the window slot mod 8 (the 16-byte bank group of
-        // the staged position).  Position j of the segment is read by lane
-        // j % row (of the atom's lanes), so putting a class-(j % 8) entry at
-        // j gives the 8 lanes of each quarter-warp 8 different bank groups;
-        // the entries that do not fit their own class's positions fill the
-        // rest.  Ranks within a class go lane by lane (lane l's entries l,
-        // l + 32, ... after those of the lanes before it): each lane counts
-        // its classes in 16-bit fields (classes 0-3 in c03, 4-7 in c47), one
-        // warp scan gives the bases -- no warp vote per entry.
-        // a segment of up to CW_KEEP x 32 entries keeps its window indices
-        // in registers between the passes (16 bits each, two per register;
-        // 0xFFFF past the segment's end), with every entry's load issued
-        // up front; longer segments read the master list twice
-        constexpr int CW_KEEP = 24;
-        const bool kept = m <= 32 * CW_KEEP;
-        unsigned pk[CW_KEEP / 2];
-        unsigned long long c03 = 0ull, c47 = 0ull;
-        auto count = [&](int cl) {
-          if (cl < 4) c03 += 1ull << (16 * cl);
-          else c47 += 1ull << (16 * (cl - 4));
-        };
-        if (kept) {
-          uint32_t en[CW_KEEP];
+  const int na = fits ? nlen[t] : 0, nb = fits ? nlen[n + t] : 0;
+  const uint32_t *src = nbr + (size_t)t * stride;
+  uint2 *dst = cwl + (size_t)t * words;
+  // blocks of 4 row entries: row 32 lanes per atom (k_pair_cw) or 8
+  // (k_pair_cs).  With 32 the electrostatic segment's blocks lie from the
+  // slot's end down (CompactOut), with 8 they follow the LJ segment's.
+  const int blk = 4 * row, nba = (na + blk - 1) / blk;
+  const int last = words / row - 1;
+  for (int sg = 0; sg < 2; sg++) {
+    const bool front = sg == 0;
+    const int m = front ? na : nb;
+    const uint32_t *in = front ? src : src + stride - 1;      // the back segment runs down from the slot's end
+    // lane l makes the 8-byte word l % row of block l / row: entries r,
+    // r + row, r + 2 row, r + 3 row of it, in list order
+    for (int b0 = 0; b0 * blk < m; b0 += 32 / row) {
+      const int b = b0 + lane / row, r = lane & (row - 1);
+      unsigned o[4];
 #pragma unroll
-          for (int k = 0; k < CW_KEEP; k++) en[k] = k * 32 + lane < m ? in[k * 32 + lane] : 0u;
-#pragma unroll
-          for (int k = 0; k < CW_KEEP; k++) {
-            unsigned ok = 0xFFFFu;
-            if (k * 32 < m) {
-              uint32_t o;
-              const int cl = window_index_of(k * 32 + lane < m, en[k], o);
-              if (cl >= 0) {
-                ok = o;
-                count(cl);
-              }
-            }
-            if (k & 1) pk[k >> 1] |= ok << 16;
-            else pk[k >> 1] = ok;
-          }
-        } else {
-          for (int e0 = 0; e0 < m; e0 += 32) {
-            uint32_t o;
-            const int cl = window_index(e0 + lane, o);
-            if (cl >= 0) count(cl);
-          }
-        }
-        unsigned long long i03 = c03, i47 = c47;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const unsigned long long a = __shfl_up_sync(0xffffffffu, i03, o);
-          const unsigned long long b = __shfl_up_sync(0xffffffffu, i47, o);
-          if (lane >= o) {
-            i03 += a;
-            i47 += b;
-          }
-        }
-        const unsigned long long t03 = __shfl_sync(0xffffffffu, i03, 31), t47 = __shfl_sync(0xffffffffu, i47, 31);
-        int cnt[8];
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-          cnt[q] = (int)((t03 >> (16 * q)) & 0xFFFFull);
-          cnt[q + 4] = (int)((t47 >> (16 * q)) & 0xFFFFull);
-        }
-        const int Q = m >> 3;
-        // running ranks: this lane's bases, advanced per entry
-        unsigned long long r03 = i03 - c03, r47 = i47 - c47;
-        auto place = [&](int cl, uint32_t o) {
-          int rank;
-          if (cl < 4) {
-            rank = (int)((r03 >> (16 * cl)) & 0xFFFFull);
-            r03 += 1ull << (16 * cl);
-          } else {
-            rank = (int)((r47 >> (16 * (cl - 4))) & 0xFFFFull);
-            r47 += 1ull << (16 * (cl - 4));
-          }
-          int pos;
-          if (rank < Q) {
-            pos = cl + 8 * rank;
-          } else {
-            // the L-th free position: the unused class positions of the
-            // classes short of Q entries, in class order, then the tail
-            int L = rank - Q;
-#pragma unroll
-            for (int q = 0; q < 8; q++)
-              if (q < cl) L += max(0, cnt[q] - Q);
-            pos = -1;
-#pragma unroll
-            for (int q = 0; q < 8; q++) {
-              const int d = max(0, Q - cnt[q]);
-              if (pos < 0) {
-                if (L < d) pos = q + 8 * (cnt[q] + L);
-                else L -= d;
-              }
-            }
-            if (pos < 0) pos = 8 * Q + L;
-          }
-          // position -> (block, lane, k): 16-bit entry k of the block's
-          // word for lane r % row (row is 8 or 32: a power of two)
-          const int bb = pos / blk, r = pos - bb * blk;
-          out[(bb * row + (r & (row - 1))) * 4 + r / row] = (unsigned short)o;
-        };
-        if (kept) {
-#pragma unroll
-          for (int k = 0; k < CW_KEEP; k++) {
-            if (k * 32 < m) {
-              const unsigned o = (k & 1) ? pk[k >> 1] >> 16 : pk[k >> 1] & 0xFFFFu;
-              if (o != 0xFFFFu) place((int)(o & 7u), o);
-            }
-          }
-        } else {
-          for (int e0 = 0; e0 < m; e0 += 32) {
-            uint32_t o = dummy;
-            const int cl = window_index(e0 + lane, o);
-            if (cl >= 0) place(cl, o);
-          }
-        }
+      for (int k = 0; k < 4; k++) {
+        const int e = b * blk + k * row + r;
+        const uint32_t en = e < m ? (front ? in[e] : in[-e]) : 0u;
+        const int wi = (int)(en & ENT_JMASK) + __shfl_sync(0xffffffffu, delta, (en >> ENT_CODE_SHIFT) & 31);
+        // inside the window by construction (a pair's shift code names j's
+        // stencil cell); anything else would index past the staged atoms, so
+        // it becomes the dummy, which also pads the segment's last block
+        o[k] = e < m && wi >= 0 && wi < tot ? (unsigned)wi | (front && (en & ENT_EL) ? CW_EL : 0u) : dummy;
       }
-      if (lane == 0) cwn[t] = make_int2(na, nb);
+      if (b * blk < m)
+        dst[(front ? b : (row == CW_ROW ? last - b : nba + b)) * row + r] =
+            make_uint2(o[0] | o[1] << 16, o[2] | o[3] << 16);
     }
   }
+  if (lane == 0) cwn[t] = make_int2(na, nb);
 }
 
-__global__ void __launch_bounds__(256, 2) k_cw_convert(int ncx, int ncy, int ncz, int cap, int n, int words, int row,
+__global__ void __launch_bounds__(256) k_cw_convert(int ncx, int ncy, int ncz, int cap, int n, int words, int row,
                                                     const int *__restrict__ cell_start,
                                                     const int *__restrict__ cell_of,
                                                     const int *__restrict__ sorig,
@@ -335,7 +220,7 @@ __global__ void __launch_bounds__(1024) k_cw_scan(int nsys, const SysP *__restri
 // A batch: warps walk the scanned range (a fixed grid, so that a captured
 // step converts whatever the device-side rebuild flags select); atom v of the
 // range lies in the last system s with scan[s] <= v, each on its own grid.
-__global__ void __launch_bounds__(256, 2) k_cw_convert_sys(int nsys, const int *__restrict__ scan,
+__global__ void __launch_bounds__(256) k_cw_convert_sys(int nsys, const int *__restrict__ scan,
                                                         const SysP *__restrict__ sp, int cap, int n, int words,
                                                         int row, const int *__restrict__ cell_start,
                                                         const int *__restrict__ cell_of,
@@ -669,29 +554,38 @@ __global__ void __launch_bounds__(NT, 1) k_pair_cw(
     // next atom's lengths and first two list words are loaded while this
     // one is evaluated (every slot holds at least two blocks)
     const int astep = nsplit * NWARP;
-    int2 nn_nx = make_int2(0, 0);
+    // block b of an atom's list: its LJ segment's blocks, then the
+    // electrostatic ones, which lie from the slot's end down
+    const int lastb = P.words / CW_ROW - 1;
+    auto block_at = [&](int b, int nba) { return b < nba ? b : lastb - (b - nba); };
+    auto blocks_of = [&](int m) { return (m + CW_BLOCK - 1) / CW_BLOCK; };
+    int2 nn_nx = make_int2(0, 0), nn_nx2 = nn_nx;          // lengths of the next atom and of the one after it
     uint2 p0 = make_uint2(0u, 0u), p1 = make_uint2(0u, 0u);
     if (staged && part * NWARP + warp < cin) {
       const int tn = ci0 + part * NWARP + warp;
       nn_nx = cwn[tn];
-      p0 = __ldg(cwl + (size_t)tn * P.words + lane);
-      p1 = __ldg(cwl + (size_t)tn * P.words + CW_ROW + lane);
+      if (part * NWARP + warp + astep < cin) nn_nx2 = cwn[tn + astep];
+      const int nba = blocks_of(nn_nx.x);
+      p0 = __ldg(cwl + (size_t)tn * P.words + block_at(0, nba) * CW_ROW + lane);
+      p1 = __ldg(cwl + (size_t)tn * P.words + block_at(1, nba) * CW_ROW + lane);
     }
     for (int a = part * NWARP + warp; staged && a < cin; a += astep) {
       const int t = ci0 + a;
       const int2 nn = nn_nx;
       uint2 w0 = p0, w1 = p1;
+      nn_nx = nn_nx2;
       if (a + astep < cin) {
         const int tn = t + astep;
-        nn_nx = cwn[tn];
-        p0 = __ldg(cwl + (size_t)tn * P.words + lane);
-        p1 = __ldg(cwl + (size_t)tn * P.words + CW_ROW + lane);
+        if (a + 2 * astep < cin) nn_nx2 = cwn[tn + astep];
+        const int nba = blocks_of(nn_nx.x);
+        p0 = __ldg(cwl + (size_t)tn * P.words + block_at(0, nba) * CW_ROW + lane);
+        p1 = __ldg(cwl + (size_t)tn * P.words + block_at(1, nba) * CW_ROW + lane);
       }
       CwAcc A;
       cw_zero(A);
       const float4 xi = wx[ioff + a];
       const int ti = LJM == 2 ? wt[ioff + a] : 0;
-      const int nba = (nn.x + CW_BLOCK - 1) / CW_BLOCK, nbt = nba + (nn.y + CW_BLOCK - 1) / CW_BLOCK;
+      const int nba = blocks_of(nn.x), nbt = nba + blocks_of(nn.y);
       const uint2 *words = cwl + (size_t)t * P.words + lane;
       auto geom = [&](uint32_t e, float4 &xj, float &dx, float &dy, float &dz) {
         xj = lds_f4(wxb + ((e & CW_IDX) << 4));
@@ -732,7 +626,7 @@ __global__ void __launch_bounds__(NT, 1) k_pair_cw(
       const uint2 pad = make_uint2((uint32_t)P.cap | ((uint32_t)P.cap << 16), (uint32_t)P.cap | ((uint32_t)P.cap << 16));
       if (nbt < 2) w1 = pad;
       for (int b = 0; b < nbt; b++) {
-        const uint2 w2 = b + 2 < nbt ? __ldg(words + (b + 2) * CW_ROW) : pad;
+        const uint2 w2 = b + 2 < nbt ? __ldg(words + block_at(b + 2, nba) * CW_ROW) : pad;
         const bool front = b < nba;
         const int m = front ? min(CW_BLOCK, nn.x - b * CW_BLOCK) : min(CW_BLOCK, nn.y - (b - nba) * CW_BLOCK);
         const uint32_t e[4] = {w0.x & 0xFFFFu, w0.x >> 16, w0.y & 0xFFFFu, w0.y >> 16};
@@ -763,7 +657,7 @@ __global__ void __launch_bounds__(NT, 1) k_pair_cw(
       if (__any_sync(0xffffffffu, (HAS_EL && A.r2min < P.r2under) || (LJM && A.pminl < 1.f))) {
         unsigned cnt = 0;
         for (int b = 0; b < nbt; b++) {
-          const uint2 w = __ldg(words + b * CW_ROW);
+          const uint2 w = __ldg(words + block_at(b, nba) * CW_ROW);
           const uint32_t e[4] = {w.x & 0xFFFFu, w.x >> 16, w.y & 0xFFFFu, w.y >> 16};
           const bool front = b < nba;
 #pragma unroll
@@ -1666,27 +1560,64 @@ int cw_set_row(Ctx *c, int row) {
   return cw_convert(c, false, true);
 }
 
+// the master slots widen on overflow (host-driven builds only): so do the
+// compact list's; *grown: every atom's list has to be written again
+static int cw_fit_words(Ctx *c, bool *grown) {
+  *grown = false;
+  if (cw_words_row(c->nbr_stride, c->cw_row) <= c->cw_words) return CM3D_NB_OK;
+  const int words = cw_words_for(c->nbr_stride);
+  DevLock lock(device_mutex());
+  CK(cudaStreamSynchronize(c->st));
+  cudaFree(c->cwl);
+  c->cwl = nullptr;
+  CK(cudaMalloc(&c->cwl, sizeof(uint2) * (size_t)c->n * (size_t)words));
+  c->cw_words = words;
+  *grown = true;
+  if (c->graph) {
+    cudaGraphExecDestroy(c->graph);
+    c->graph = nullptr;
+  }
+  return CM3D_NB_OK;
+}
+
+// Whether the list kernel writes the compact list itself (one system on the
+// compact path, 32 lanes per atom), and where
+bool cw_direct(Ctx *c, bool device_flag, CompactOut *W, int *rc) {
+  *rc = CM3D_NB_OK;
+  if (!c->cw_ok || !c->cw_use || c->cw_batch || c->cw_row != CW_ROW) return false;
+  if (!device_flag) {
+    bool grown;
+    if ((*rc = cw_fit_words(c, &grown))) return false;
+  }
+  *W = {c->cwl, c->cwn, c->cw_words, c->cw_words / CW_ROW, c->cw_cap};
+  return true;
+}
+
+// a host-driven build: a window that did not fit turns the compact path off
+// for this context (the gather/window kernels read the master list)
+int cw_check(Ctx *c, bool device_flag) {
+  if (device_flag) return CM3D_NB_OK;
+  CK(cudaMemcpyAsync(c->h_stat, c->stat, sizeof(long long) * ST_COUNT, cudaMemcpyDeviceToHost, c->st));
+  CK(cudaStreamSynchronize(c->st));
+  if (c->h_stat[ST_CWIN] > 0) {
+    c->cw_ok = 0;
+    c->cw_use = 0;
+    long long zero = 0;
+    CK(cudaMemcpy(c->stat + ST_CWIN, &zero, sizeof(long long), cudaMemcpyHostToDevice));
+  }
+  return CM3D_NB_OK;
+}
+
 // after a (gated) rebuild of the master list: the compact list (a batch:
 // of the compact systems being rebuilt, or of all after the slots widened)
 int cw_convert(Ctx *c, bool device_flag, bool all) {
   // (a context whose autotuner chose another kernel keeps no compact lists;
   // the autotuner converts them all before it times the compact path)
   if (!c->cw_ok || !c->cw_use) return CM3D_NB_OK;
-  // the master slots widen on overflow (host-driven builds only): so do ours
-  if (cw_words_row(c->nbr_stride, c->cw_row) > c->cw_words) {
-    const int words = cw_words_for(c->nbr_stride);
-    DevLock lock(device_mutex());
-    CK(cudaStreamSynchronize(c->st));
-    cudaFree(c->cwl);
-    c->cwl = nullptr;
-    CK(cudaMalloc(&c->cwl, sizeof(uint2) * (size_t)c->n * (size_t)words));
-    c->cw_words = words;
-    all = true;
-    if (c->graph) {
-      cudaGraphExecDestroy(c->graph);
-      c->graph = nullptr;
-    }
-  }
+  bool grown;
+  int rc = cw_fit_words(c, &grown);
+  if (rc) return rc;
+  all = all || grown;
   const int *gate = device_flag ? c->istate : nullptr;
   int *halt = device_flag ? c->istate + IS_HALT : nullptr;
   if (c->cw_batch) {
@@ -1703,19 +1634,7 @@ int cw_convert(Ctx *c, bool device_flag, bool all) {
     c->launches++;
   }
   CKL(c);
-  if (!device_flag) {
-    // a host-driven build: a window that did not fit turns the compact path
-    // off for this context (the gather/window kernels read the master list)
-    CK(cudaMemcpyAsync(c->h_stat, c->stat, sizeof(long long) * ST_COUNT, cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
-    if (c->h_stat[ST_CWIN] > 0) {
-      c->cw_ok = 0;
-      c->cw_use = 0;
-      long long zero = 0;
-      CK(cudaMemcpy(c->stat + ST_CWIN, &zero, sizeof(long long), cudaMemcpyHostToDevice));
-    }
-  }
-  return CM3D_NB_OK;
+  return cw_check(c, device_flag);
 }
 
 template <bool EL, int LJM, bool BATCH, int NT>

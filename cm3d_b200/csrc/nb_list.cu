@@ -216,19 +216,38 @@ __global__ void __launch_bounds__(SORT_THREADS) k_cell_sort(int ncells, int per_
   }
 }
 
+// What the list kernels read: atoms, cells, parameters and exclusions.
+struct ListK {
+  int n;
+  const int *cell_atoms, *cell_start, *cell_of;
+  const float4 *xq;
+  const double *pos;
+  const int *itype, *map;
+  const double *icut, *q;
+  const int *excl_off, *excl_idx, *cexcl_off, *cexcl_idx;
+  const int4 *cimg;
+  const int2 *smeta, *xspan;
+};
+
 // Exact membership test of one candidate pair, in CM3D's FP64 operation
-// order.  Returns flags (bit0 t, bit1 s, bit2 te, bit3 se, bit4 bad shift)
-// and the cell-shift code of the pair for the full list.
-__device__ __forceinline__ int exact_flags(const SysP &P, int n, int i, int j, int4 ci,
-                                           const double *__restrict__ pos, double xi, double yi, double zi, int ti,
-                                           bool qi, const int *__restrict__ itype, const int *__restrict__ map,
-                                           const double *__restrict__ icut, const double *__restrict__ q,
-                                           const int *__restrict__ excl_off, const int *__restrict__ excl_idx,
-                                           const int *__restrict__ cexcl_off, const int *__restrict__ cexcl_idx,
-                                           const int4 *__restrict__ cimg, int &code) {
-  const int intr = map[P.map0 + ti * P.ntypes + itype[j]];
+// order.  Returns the pair's full-list entry without j: its list flags
+// (ENT_LJ t, ENT_LJS s, ENT_EL te, ENT_ELS se), near-image bit and cell-shift
+// code, and EXACT_BAD where the code does not exist; 0 for a pair in no list.
+// Not inlined: the few pairs that FP32 cannot decide would otherwise cost
+// every list kernel its registers.
+constexpr uint32_t EXACT_BAD = 1u;
+constexpr uint32_t ENT_FLAGS = ENT_LJ | ENT_EL | ENT_LJS | ENT_ELS;
+__device__ __noinline__ uint32_t exact_entry(const SysP &P, const ListK &K, int i, int j) {
+  const int n = K.n;
+  const double *__restrict__ pos = K.pos;
+  const int ti = K.itype[i];
+  const int4 ci = K.cimg[i];
+  const bool qi = K.q[i] != 0.0;
+  const double xi = pos[i], yi = pos[n + i], zi = pos[2 * n + i];
+  const double *__restrict__ icut = K.icut;
+  const int intr = K.map[P.map0 + ti * P.ntypes + K.itype[j]];
   const bool lj_ok = intr >= 0;
-  const bool el_ok = qi && q[j] != 0.0;
+  const bool el_ok = qi && K.q[j] != 0.0;
   if (!lj_ok && !el_ok) return 0;
   double dx = xi - pos[j], dy = yi - pos[n + j], dz = zi - pos[2 * n + j];
   double sx = __dadd_rn(__dadd_rn(__dmul_rn(dx, P.hi[0]), __dmul_rn(dy, P.hi[1])), __dmul_rn(dz, P.hi[2]));
@@ -242,34 +261,30 @@ __device__ __forceinline__ int exact_flags(const SysP &P, int n, int i, int j, i
   const double ey = __dadd_rn(__dadd_rn(__dmul_rn(sx, P.h[3]), __dmul_rn(sy, P.h[4])), __dmul_rn(sz, P.h[5]));
   const double ez = __dadd_rn(__dadd_rn(__dmul_rn(sx, P.h[6]), __dmul_rn(sy, P.h[7])), __dmul_rn(sz, P.h[8]));
   const double r2 = r2_ref(ex, ey, ez);
-  int flags = 0;
-  if (lj_ok && r2 < icut[8 * intr + 5] && !(P.excl && excluded(i, j, excl_off, excl_idx))) {
-    flags |= 1;
-    if (r2 < icut[8 * intr + 4]) flags |= 2;
+  uint32_t en = 0;
+  if (lj_ok && r2 < icut[8 * intr + 5] && !(P.excl && excluded(i, j, K.excl_off, K.excl_idx))) {
+    en |= ENT_LJ;
+    if (r2 < icut[8 * intr + 4]) en |= ENT_LJS;
   }
-  if (el_ok && r2 < P.rmaxl_skin2_e && !(P.cexcl && excluded(i, j, cexcl_off, cexcl_idx))) {
-    flags |= 4;
-    if (r2 < P.rmaxs_skin2_e) flags |= 8;
+  if (el_ok && r2 < P.rmaxl_skin2_e && !(P.cexcl && excluded(i, j, K.cexcl_off, K.cexcl_idx))) {
+    en |= ENT_EL;
+    if (r2 < P.rmaxs_skin2_e) en |= ENT_ELS;
   }
-  if (!flags) return 0;
+  if (!en) return 0;
   // small boxes: the atoms may move skin/2 each before the next rebuild, so a
   // pair whose fractional displacement is within skin / plane spacing of 1/2
   // may change its nearest image; the pair kernel checks those pairs
-  if (P.smallbox && (fabs(sx) > P.near_s[0] || fabs(sy) > P.near_s[1] || fabs(sz) > P.near_s[2])) flags |= 32;
+  if (P.smallbox && (fabs(sx) > P.near_s[0] || fabs(sy) > P.near_s[1] || fabs(sz) > P.near_s[2])) en |= ENT_NEAR;
   // shift code: k = (n_i - n_j - m) nc + (c_i - c_j) per dimension; |k| <= 1
   // whenever r < rlist <= cell width.  Anything else means the geometry
   // assumption broke: flag it and use the zero shift rather than index past
   // the shift table.
-  const int4 cj = cimg[j];
+  const int4 cj = K.cimg[j];
   const int kx = (ci.y - cj.y - (int)mx) * P.nc[0] + ((ci.x & 1023) - (cj.x & 1023));
   const int ky = (ci.z - cj.z - (int)my) * P.nc[1] + (((ci.x >> 10) & 1023) - ((cj.x >> 10) & 1023));
   const int kz = (ci.w - cj.w - (int)mz) * P.nc[2] + (((ci.x >> 20) & 1023) - ((cj.x >> 20) & 1023));
-  code = (kx + 1) * 9 + (ky + 1) * 3 + (kz + 1);
-  if (kx < -1 || kx > 1 || ky < -1 || ky > 1 || kz < -1 || kz > 1) {
-    code = 13;
-    flags |= 16;
-  }
-  return flags;
+  if (kx < -1 || kx > 1 || ky < -1 || ky > 1 || kz < -1 || kz > 1) return en | 13u << ENT_CODE_SHIFT | EXACT_BAD;
+  return en | (uint32_t)((kx + 1) * 9 + (ky + 1) * 3 + (kz + 1)) << ENT_CODE_SHIFT;
 }
 
 // The candidate walk shared by both list kernels.  One warp owns the
@@ -282,26 +297,69 @@ __device__ __forceinline__ int exact_flags(const SysP &P, int n, int i, int j, i
 // FP64 test on them at once (`decide(first, m)`: lane l < m takes queue entry
 // first + l), so the expensive test runs on full warps.
 //
-// With qr (the full lists of a grid of 3 or more cells per axis) the queue
-// also keeps each survivor's FP32 squared distance and its stencil cell's
-// shift code (bits ENT_CODE_SHIFT and up of the queue entry), for the
-// FP32-first flags (fast_flags); with `prune` (an orthorhombic such grid of
-// cells cw wide) stencil cells wholly beyond lim2 from the atom, by the gaps
-// to their faces less 1e-3 A, are skipped -- none of their atoms would pass
-// the prefilter, so the lists are the same.
+// The queue keeps each survivor's FP32 squared distance (qr) beside its index
+// and the code of its cell shift (bits ENT_CODE_SHIFT and up), for the
+// FP32-first flags (list_flags).  In a grid of 3 or more cells per axis
+// (G_STENCIL) the stencil image is the only image in range and its code the
+// pair's; with `prune` (such a grid in an orthorhombic box, cells cw wide)
+// stencil cells wholly beyond lim2 from the atom, by the gaps to their faces
+// less 1e-3 A, are skipped -- none of their atoms would pass the prefilter, so
+// the lists are the same.  In a coarser grid (G_IMAGE) the minimum image is
+// taken in FP32 (fold), which also gives the code; a pair whose fractional
+// displacement lies so close to 1/2 (or to a small box's near-image bound)
+// that FP32 may choose another image than CM3D's FP64 arithmetic carries
+// CODE_EXACT instead, and is decided in FP64.  G_EXACT takes no FP32 decision.
 constexpr int LQ = 64;                     // queue entries per warp (> 2 * 32 - 1)
+constexpr int CODE_EXACT = 31;             // queue code: the FP64 test decides
+constexpr int QUEUE_NEAR = (int)ENT_NEAR;  // queue bit: ENT_NEAR of a small box
+enum { G_EXACT = 0, G_STENCIL = 1, G_IMAGE = 2 };
+
+__device__ __forceinline__ int grid_kind(const SysP &P) {
+  if (P.nc[0] >= 3 && P.nc[1] >= 3 && P.nc[2] >= 3) return P.smallbox ? G_EXACT : G_STENCIL;
+  return P.image_ok ? G_IMAGE : G_EXACT;
+}
+
+// Minimum image of the FP32 displacement (dx, dy, dz) to an atom of the
+// stencil cell of shift code `code`: period()'s fold in FP32.  Returns the
+// squared distance and leaves the image's shift code (CODE_EXACT where FP32
+// cannot tell, see above) and near-image bit in `code`.  The displacement is
+// a difference of coordinates no larger than a box of at most 8 list radii
+// per axis, so s carries an error of about 1e-7; 1e-5 is the margin.
+__device__ __forceinline__ float fold(const SysP &P, float dx, float dy, float dz, int &code) {
+  const float sx = P.hiF[0] * dx + P.hiF[1] * dy + P.hiF[2] * dz;
+  const float sy = P.hiF[3] * dx + P.hiF[4] * dy + P.hiF[5] * dz;
+  const float sz = P.hiF[6] * dx + P.hiF[7] * dy + P.hiF[8] * dz;
+  const float mx = rintf(sx), my = rintf(sy), mz = rintf(sz);
+  dx -= P.hF[0] * mx + P.hF[1] * my + P.hF[2] * mz;
+  dy -= P.hF[3] * mx + P.hF[4] * my + P.hF[5] * mz;
+  dz -= P.hF[6] * mx + P.hF[7] * my + P.hF[8] * mz;
+  const float ax = fabsf(sx - mx), ay = fabsf(sy - my), az = fabsf(sz - mz);
+  constexpr float EPS = 1e-5f;
+  bool exact = ax > 0.5f - EPS || ay > 0.5f - EPS || az > 0.5f - EPS;
+  int near = 0;
+  if (P.smallbox) {
+    const float nx = (float)P.near_s[0], ny = (float)P.near_s[1], nz = (float)P.near_s[2];
+    exact |= fabsf(ax - nx) < EPS || fabsf(ay - ny) < EPS || fabsf(az - nz) < EPS;
+    if (ax > nx || ay > ny || az > nz) near = QUEUE_NEAR;
+  }
+  const int kx = code / 9 - 1 - (int)mx * P.nc[0], ky = (code / 3) % 3 - 1 - (int)my * P.nc[1],
+            kz = code % 3 - 1 - (int)mz * P.nc[2];
+  exact |= kx < -1 || kx > 1 || ky < -1 || ky > 1 || kz < -1 || kz > 1;
+  code = exact ? CODE_EXACT << ENT_CODE_SHIFT : ((kx + 1) * 9 + (ky + 1) * 3 + (kz + 1)) << ENT_CODE_SHIFT | near;
+  return fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+}
 
 template <class Decide>
-__device__ __forceinline__ void walk_candidates(const SysP &P, int i, int4 ci, float4 xi4, bool half_only,
-                                                const int *__restrict__ cell_atoms,
-                                                const int *__restrict__ cell_start,
-                                                const float4 *__restrict__ xq, int *qbuf, Decide &decide,
-                                                float *qr = nullptr, bool prune = false,
-                                                float3 cw = make_float3(0.f, 0.f, 0.f), int t = -1) {
+__device__ __forceinline__ void walk_candidates(const SysP &P, const ListK &K, int i, bool half_only, int *qbuf,
+                                                float *qr, Decide &decide, int kind, bool prune, float3 cw, int t) {
+  const int *__restrict__ cell_start = K.cell_start;
+  const float4 *__restrict__ xq = K.xq;
+  const int4 ci = K.cimg[i];
+  const float4 xi4 = xq[t];
   const int lane = threadIdx.x & 31;
   const unsigned lt_mask = (1u << lane) - 1u;
   const int cx = ci.x & 1023, cy = (ci.x >> 10) & 1023, cz = (ci.x >> 20) & 1023;
-  const float lim2 = P.lim2;
+  const float lim2 = kind == G_IMAGE ? P.lim2_image : P.lim2;
   // the stencil cells in walk order (x offsets outermost), one per lane:
   // their sorted-atom ranges (empty where pruned) and shift codes, loaded
   // together up front
@@ -359,25 +417,26 @@ __device__ __forceinline__ void walk_candidates(const SysP &P, int i, int4 ci, f
     if (w >= 0 && u0 + lane < hi) xn = xq[u0 + lane];
     bool keep = false;
     float r2f = 0.f;
+    int qc = ccur << ENT_CODE_SHIFT;
     if (u < hcur) {
       const float dx = (xi4.x - xj.x) + Sc.x, dy = (xi4.y - xj.y) + Sc.y, dz = (xi4.z - xj.z) + Sc.z;
-      r2f = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-      keep = r2f < lim2;
-      if (keep) {
-        // the atom itself (sorted index t when given); half lists: j > i
-        if (half_only || t < 0) {
-          const int j = cell_atoms[u];
-          keep = j != i && (!half_only || j > i);
-        } else {
-          keep = u != t;
-        }
+      if (kind == G_IMAGE) {
+        qc = ccur;
+        r2f = fold(P, dx, dy, dz, qc);
+      } else {
+        r2f = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+        if (kind == G_EXACT) qc = CODE_EXACT << ENT_CODE_SHIFT;
       }
+      // the atom itself; half lists: j > i
+      keep = r2f < lim2 && (half_only ? K.cell_atoms[u] > i : u != t);
     }
     const unsigned bk = __ballot_sync(0xffffffffu, keep);
     if (keep) {
       const int slot = (tail + __popc(bk & lt_mask)) & (LQ - 1);
-      qbuf[slot] = qr ? (u | (ccur << ENT_CODE_SHIFT)) : u;
-      if (qr) qr[slot] = r2f;
+      // half lists need no code, only whether FP32 may decide (the plain
+      // engine's sorted indices can need more than ENT_JBITS bits)
+      qbuf[slot] = half_only ? u : u | qc;
+      qr[slot] = half_only && ((qc >> ENT_CODE_SHIFT) & 31) == CODE_EXACT ? -1.f : r2f;
     }
     tail += __popc(bk);
     __syncwarp();
@@ -394,6 +453,116 @@ __device__ __forceinline__ void walk_candidates(const SysP &P, int i, int4 ci, f
   }
 }
 
+// What an atom's list flags need of the atom itself, loaded once per warp:
+// its types' list radii (lane tj: the LJ radii of the interaction with type
+// tj, FP32, -1 for none; read by shuffle -- no table load per pair), its
+// charge's, and the span of the atom indices excluded from it (a pair outside
+// it needs no look-up of the exclusion lists).
+struct ListAtom {
+  int ti;
+  bool rows;                               // the types fit the lanes
+  float rl, rs;                            // lane tj: LJ list radii^2 (t, s)
+  float el, es;                            // electrostatic list radii^2 (te, se), -1 without charge
+  float near;                              // FP32 decides beyond this distance from every radius^2
+  int xlo;
+  unsigned xw;                             // excluded from it: atoms among xlo .. xlo + xw
+};
+
+__device__ __forceinline__ ListAtom list_atom(const SysP &P, const ListK &K, int2 meta) {
+  const int lane = threadIdx.x & 31;
+  ListAtom A;
+  A.ti = meta.y >> 1;
+  A.rows = P.ntypes <= 32;
+  A.rl = A.rs = A.el = A.es = -1.f;
+  if (A.rows && lane < P.ntypes) {
+    const int intr = K.map[P.map0 + A.ti * P.ntypes + lane];
+    if (intr >= 0) {
+      A.rl = (float)K.icut[8 * intr + 5];
+      A.rs = (float)K.icut[8 * intr + 4];
+    }
+  }
+  if (meta.y & 1) {
+    A.el = (float)P.rmaxl_skin2_e;
+    A.es = (float)P.rmaxs_skin2_e;
+  }
+  A.near = fmaf(4e-5f, P.lim2_image, 2e-3f);
+  const int2 x = K.xspan[meta.x];
+  A.xlo = x.x;
+  A.xw = (unsigned)x.y;
+  return A;
+}
+
+// r2f against the LJ and electrostatic list radii^2 (-1: no such list);
+// *near: within `margin` of one of them
+__device__ __forceinline__ uint32_t radii_flags(float r2f, float rl, float rs, float el, float es, float margin,
+                                                bool *near) {
+  *near = fminf(fminf(fabsf(r2f - rl), fabsf(r2f - rs)), fminf(fabsf(r2f - el), fabsf(r2f - es))) < margin;
+  uint32_t fl = r2f < rl ? (r2f < rs ? ENT_LJ | ENT_LJS : ENT_LJ) : 0u;
+  if (r2f < el) fl |= r2f < es ? ENT_EL | ENT_ELS : ENT_EL;
+  return fl;
+}
+
+__device__ __forceinline__ uint32_t strike_excluded(const SysP &P, const ListK &K, uint32_t fl, int i, int j) {
+  if (P.excl && excluded(i, j, K.excl_off, K.excl_idx)) fl &= ~(ENT_LJ | ENT_LJS);
+  if (P.cexcl && excluded(i, j, K.cexcl_off, K.cexcl_idx)) fl &= ~(ENT_EL | ENT_ELS);
+  return fl;
+}
+
+// List flags (ENT_*) of a pair from its FP32 squared distance: the tests of
+// exact_entry.  Each comparison with a list radius R^2 matches CM3D's FP64 one
+// unless the FP32 value lies within 4e-5 R^2 + 2e-3 A^2 of R^2 -- a margin ten
+// times the FP32 error of a squared distance formed from cell-relative
+// coordinates (cells are narrower than two list radii); the largest R^2 of
+// the system gives the margin for all of them -- and then *exact is set and
+// the caller decides in FP64 (exact_entry).  Called by the whole warp (the
+// radii come by shuffle); `on`: this lane has a pair.
+__device__ __forceinline__ uint32_t list_flags(const SysP &P, const ListK &K, const ListAtom &A, bool on, int i,
+                                               int2 mj, float r2f, bool *exact) {
+  const int j = mj.x, tj = mj.y >> 1;
+  float rl, rs;
+  if (A.rows) {
+    rl = __shfl_sync(0xffffffffu, A.rl, tj & 31);
+    rs = __shfl_sync(0xffffffffu, A.rs, tj & 31);
+  } else {
+    rl = rs = -1.f;
+    const int intr = on ? K.map[P.map0 + A.ti * P.ntypes + tj] : -1;
+    if (intr >= 0) {
+      rl = (float)K.icut[8 * intr + 5];
+      rs = (float)K.icut[8 * intr + 4];
+    }
+  }
+  const bool qj = (mj.y & 1) != 0;
+  bool near;
+  uint32_t fl = radii_flags(r2f, rl, rs, qj ? A.el : -1.f, qj ? A.es : -1.f, A.near, &near);
+  *exact = on && near;
+  if (!on) fl = 0u;
+  if (fl && (unsigned)(j - A.xlo) <= A.xw) fl = strike_excluded(P, K, fl, i, j);
+  return fl;
+}
+
+// Appends a warp's entries to an atom's slot (na, nb: its segments so far):
+// the pairs in an LJ list from the front, the electrostatics-only ones from
+// the back.  Every write lands inside the slot; once the two segments meet (an
+// overflow) the slot's contents no longer matter: the lengths are set to zero
+// at the end and the list is built again with wider slots.
+__device__ __forceinline__ void append(uint32_t *__restrict__ out, int stride, uint32_t en, int &na, int &nb) {
+  const unsigned lt_mask = (1u << (threadIdx.x & 31)) - 1u;
+  const bool fa = (en & (ENT_LJ | ENT_LJS)) != 0, any = (en & ENT_FLAGS) != 0;
+  const unsigned ba = __ballot_sync(0xffffffffu, fa), bb = __ballot_sync(0xffffffffu, any && !fa);
+  const int at = fa ? na + __popc(ba & lt_mask) : stride - 1 - (nb + __popc(bb & lt_mask));
+  if (any && (fa ? at < stride - nb : at >= na)) out[at] = en;
+  na += __popc(ba);
+  nb += __popc(bb);
+}
+
+__device__ __forceinline__ bool ortho(const SysP &P) {
+  return P.h[1] == 0. && P.h[2] == 0. && P.h[3] == 0. && P.h[5] == 0. && P.h[6] == 0. && P.h[7] == 0.;
+}
+// edges of an orthorhombic box's cells
+__device__ __forceinline__ float3 cell_width(const SysP &P) {
+  return make_float3(P.hF[0] / (float)P.nc[0], P.hF[4] / (float)P.nc[1], P.hF[8] / (float)P.nc[2]);
+}
+
 struct ListCaps {
   long long cap[4];
 };
@@ -404,16 +573,14 @@ struct ListCaps {
 // every system (host-driven builds and the single-system plain engine).
 template <bool FILL>
 __global__ void __launch_bounds__(256) k_list_half(
-    int n, const SysP *__restrict__ sp, const int *__restrict__ sys_of, ListCaps C,
-    const int *__restrict__ cell_atoms, const int *__restrict__ cell_start, const float4 *__restrict__ xq,
-    const double *__restrict__ pos, const int *__restrict__ itype, const int *__restrict__ map,
-    const double *__restrict__ icut, const double *__restrict__ q, const int *__restrict__ excl_off,
-    const int *__restrict__ excl_idx, const int *__restrict__ cexcl_off, const int *__restrict__ cexcl_idx,
-    const int4 *__restrict__ cimg, int *__restrict__ cnt, const long long *__restrict__ off,
+    const __grid_constant__ ListK K, const SysP *__restrict__ sp, const int *__restrict__ sys_of, ListCaps C,
+    int *__restrict__ cnt, const long long *__restrict__ off,
     const long long *__restrict__ tot, int2 *__restrict__ l0, int2 *__restrict__ l1, int2 *__restrict__ l2,
     int2 *__restrict__ l3, long long *__restrict__ stat, int *__restrict__ halt, const int *__restrict__ gate) {
   if (gated_off(gate, 1)) return;
   __shared__ int qs[256 / 32][LQ];
+  __shared__ float qrs[256 / 32][LQ];
+  const int n = K.n;
   const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (t >= n) return;                                     // whole warps
@@ -436,36 +603,38 @@ __global__ void __launch_bounds__(256) k_list_half(
     }
   }
   int *qbuf = qs[threadIdx.x >> 5];
+  float *qr = qrs[threadIdx.x >> 5];
   const SysP &P = sp[sys_of[t]];
-  const int i = cell_atoms[t];
-  const int4 ci = cimg[i];
-  const double xi = pos[i], yi = pos[n + i], zi = pos[2 * n + i];
-  const int ti = itype[i];
-  const bool qi = q[i] != 0.0;
+  const int2 mi = K.smeta[t];
+  const int i = mi.x;
+  const ListAtom A = list_atom(P, K, mi);
   int c[4] = {0, 0, 0, 0};
   unsigned bad = 0;
   auto decide = [&](int first, int m) {
-    int fl = 0, code = 13, j = -1;
-    if (lane < m) {
-      j = cell_atoms[qbuf[(first + lane) & (LQ - 1)]];
-      fl = exact_flags(P, n, i, j, ci, pos, xi, yi, zi, ti, qi, itype, map, icut, q, excl_off, excl_idx,
-                       cexcl_off, cexcl_idx, cimg, code);
-    }
-    bad |= (fl >> 4) & 1;
-    const unsigned b0 = __ballot_sync(0xffffffffu, fl & 1), b1 = __ballot_sync(0xffffffffu, fl & 2);
-    const unsigned b2 = __ballot_sync(0xffffffffu, fl & 4), b3 = __ballot_sync(0xffffffffu, fl & 8);
+    const bool on = lane < m;
+    const int slot = (first + lane) & (LQ - 1);
+    const int2 mj = on ? K.smeta[qbuf[slot]] : make_int2(-1, 0);
+    const float r2f = qr[slot];
+    const int j = mj.x;
+    const bool exact = r2f < 0.f;
+    bool near;
+    uint32_t fl = list_flags(P, K, A, on && !exact, i, mj, r2f, &near);
+    if (on && (exact || near)) fl = exact_entry(P, K, i, j);
+    bad |= fl & EXACT_BAD;
+    const unsigned b0 = __ballot_sync(0xffffffffu, fl & ENT_LJ), b1 = __ballot_sync(0xffffffffu, fl & ENT_LJS);
+    const unsigned b2 = __ballot_sync(0xffffffffu, fl & ENT_EL), b3 = __ballot_sync(0xffffffffu, fl & ENT_ELS);
     if (!FILL) {
       c[0] += __popc(b0); c[1] += __popc(b1); c[2] += __popc(b2); c[3] += __popc(b3);
     } else {
       const int2 pr = make_int2(i, j);
-      if (fl & 1) l0[p[0] + __popc(b0 & lt_mask)] = pr;
-      if (fl & 2) l1[p[1] + __popc(b1 & lt_mask)] = pr;
-      if (fl & 4) l2[p[2] + __popc(b2 & lt_mask)] = pr;
-      if (fl & 8) l3[p[3] + __popc(b3 & lt_mask)] = pr;
+      if (fl & ENT_LJ) l0[p[0] + __popc(b0 & lt_mask)] = pr;
+      if (fl & ENT_LJS) l1[p[1] + __popc(b1 & lt_mask)] = pr;
+      if (fl & ENT_EL) l2[p[2] + __popc(b2 & lt_mask)] = pr;
+      if (fl & ENT_ELS) l3[p[3] + __popc(b3 & lt_mask)] = pr;
       p[0] += __popc(b0); p[1] += __popc(b1); p[2] += __popc(b2); p[3] += __popc(b3);
     }
   };
-  walk_candidates(P, i, ci, xq[t], true, cell_atoms, cell_start, xq, qbuf, decide);
+  walk_candidates(P, K, i, true, qbuf, qr, decide, grid_kind(P), false, make_float3(0.f, 0.f, 0.f), t);
   if (FILL) {
     if (bad && lane == 0) atomicAdd((unsigned long long *)(stat + ST_BADSHIFT), 1ull);
   } else if (lane == 0) {
@@ -477,7 +646,7 @@ __global__ void __launch_bounds__(256) k_list_half(
 // positions moved by their cell's shift into the frame of atom t's cell
 // (s_x) and their sorted indices (s_u, low ENT_JBITS bits), walked 32 at a
 // time with the same prefilter and in the same order as walk_candidates.  The
-// queue holds the staged index, and qr its FP32 squared distance.
+// queue holds the staged index and the code, qr the FP32 squared distance.
 //
 // With `prune` (an orthorhombic cell grid of three or more cells per axis,
 // cells cw wide), the lanes first bound atom t's distance from each stencil
@@ -486,10 +655,11 @@ __global__ void __launch_bounds__(256) k_list_half(
 // the prefilter, and the others keep their order, so the lists are the same.
 // s_off holds the stencil cells' first staged index, s_code their shift code.
 template <class Decide>
-__device__ __forceinline__ void walk_staged(int t, float4 xi4, float lim2, const float4 *s_x, const int *s_u,
+__device__ __forceinline__ void walk_staged(const SysP &P, int t, float4 xi4, const float4 *s_x, const int *s_u,
                                             int cnt, int *qbuf, float *qr, Decide &decide, const int *s_off,
-                                            const int *s_code, int nw, bool prune, float3 cw) {
+                                            const int *s_code, int nw, int kind, bool prune, float3 cw) {
   const int lane = threadIdx.x & 31;
+  const float lim2 = kind == G_IMAGE ? P.lim2_image : P.lim2;
   const unsigned lt_mask = (1u << lane) - 1u;
   unsigned vis = nw >= 32 ? 0xffffffffu : (1u << nw) - 1u;
   if (prune) {
@@ -519,17 +689,25 @@ __device__ __forceinline__ void walk_staged(int t, float4 xi4, float lim2, const
     const int k = k0 + lane;
     bool keep = false;
     float r2f = 0.f;
+    int qc = 0;
     if (k < b) {
       const float4 xs = s_x[k];
-      const int u = s_u[k] & (int)ENT_JMASK;
+      const unsigned uc = (unsigned)s_u[k];
+      const int u = (int)(uc & ENT_JMASK);
       const float dx = xi4.x - xs.x, dy = xi4.y - xs.y, dz = xi4.z - xs.z;
-      r2f = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+      if (kind == G_IMAGE) {
+        qc = (int)(uc >> ENT_CODE_SHIFT);
+        r2f = fold(P, dx, dy, dz, qc);
+      } else {
+        r2f = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+        qc = kind == G_EXACT ? CODE_EXACT << ENT_CODE_SHIFT : (int)(uc & ~ENT_JMASK);
+      }
       keep = u != t && r2f < lim2;
     }
     const unsigned bk = __ballot_sync(0xffffffffu, keep);
     if (keep) {
       const int slot = (tail + __popc(bk & lt_mask)) & (LQ - 1);
-      qbuf[slot] = k;
+      qbuf[slot] = k | qc;
       qr[slot] = r2f;
     }
     tail += __popc(bk);
@@ -548,42 +726,6 @@ __device__ __forceinline__ void walk_staged(int t, float4 xi4, float lim2, const
   }
 }
 
-// List flags from the FP32 squared distance of a staged pair (cell grid of 3
-// or more cells per axis, where the stencil image is the only image within
-// the list radius and its shift code the pair's).  Each comparison with a
-// list radius R^2 matches CM3D's FP64 one unless the FP32 value lies within
-// 4e-5 R^2 + 2e-3 A^2 of R^2 -- a margin ten times the FP32 error of a
-// squared distance formed from cell-relative coordinates (cells are narrower
-// than two list radii) -- and then *exact is set and the caller decides in
-// FP64 (exact_flags).  Same tests, same order as exact_flags.
-__device__ __forceinline__ int fast_flags(const SysP &P, int i, int j, int ti, int tj, bool qi, bool qj,
-                                          float r2f, const int *__restrict__ map, const double *__restrict__ icut,
-                                          const int *__restrict__ excl_off, const int *__restrict__ excl_idx,
-                                          const int *__restrict__ cexcl_off, const int *__restrict__ cexcl_idx,
-                                          bool *exact) {
-  const int intr = map[P.map0 + ti * P.ntypes + tj];
-  const bool lj_ok = intr >= 0;
-  const bool el_ok = qi && qj;
-  if (!lj_ok && !el_ok) return 0;
-  bool near = false;
-  auto below = [&](double R2d) {
-    const float R2 = (float)R2d;
-    near |= fabsf(r2f - R2) < fmaf(4e-5f, R2, 2e-3f);
-    return r2f < R2;
-  };
-  int flags = 0;
-  if (lj_ok && below(icut[8 * intr + 5]) && !(P.excl && excluded(i, j, excl_off, excl_idx))) {
-    flags |= 1;
-    if (below(icut[8 * intr + 4])) flags |= 2;
-  }
-  if (el_ok && below(P.rmaxl_skin2_e) && !(P.cexcl && excluded(i, j, cexcl_off, cexcl_idx))) {
-    flags |= 4;
-    if (below(P.rmaxs_skin2_e)) flags |= 8;
-  }
-  *exact = near;
-  return flags;
-}
-
 // The full list of sorted atom t (mixed mode; one warp): both directions,
 // every pair in CM3D's t or te list, written straight into its fixed slot
 // nbr[t * stride ...] in two segments, each in candidate order: the pairs in
@@ -597,87 +739,43 @@ __device__ __forceinline__ int fast_flags(const SysP &P, int i, int j, int ti, i
 // otherwise from global memory through the stencil walk.
 template <bool STAGED>
 __device__ __forceinline__ void full_list_atom(
-    const SysP &P, int n, int t, int stride, const int *__restrict__ cell_atoms,
-    const int *__restrict__ cell_start, const float4 *__restrict__ xq, const double *__restrict__ pos,
-    const int *__restrict__ itype, const int *__restrict__ map, const double *__restrict__ icut,
-    const double *__restrict__ q, const int *__restrict__ excl_off, const int *__restrict__ excl_idx,
-    const int *__restrict__ cexcl_off, const int *__restrict__ cexcl_idx, const int4 *__restrict__ cimg,
-    uint32_t *__restrict__ nbr, int *__restrict__ nlen, long long *__restrict__ stat, int *__restrict__ halt,
-    int *qbuf, float *qr, const float4 *s_x, const int *s_u, const int *s_j, int scnt,
-    bool fast, const int *s_off = nullptr, const int *s_code = nullptr, int nw = 0, bool prune = false,
-    float3 cw = make_float3(0.f, 0.f, 0.f)) {
+    const SysP &P, const ListK &K, int t, int stride, uint32_t *__restrict__ nbr, int *__restrict__ nlen,
+    long long *__restrict__ stat, int *__restrict__ halt,
+    int *qbuf, float *qr, int kind, bool prune, float3 cw, const float4 *s_x = nullptr, const int *s_u = nullptr,
+    const int *s_j = nullptr, int scnt = 0, const int *s_off = nullptr, const int *s_code = nullptr, int nw = 0) {
   const int lane = threadIdx.x & 31;
   const unsigned lt_mask = (1u << lane) - 1u;
-  const int i = cell_atoms[t];
-  const int4 ci = cimg[i];
-  const double xi = pos[i], yi = pos[n + i], zi = pos[2 * n + i];
-  const int ti = itype[i];
-  const bool qi = q[i] != 0.0;
+  const int n = K.n;
+  const int2 mi = K.smeta[t];
+  const int i = mi.x;
+  const ListAtom A = list_atom(P, K, mi);
   uint32_t *out = nbr + (size_t)t * stride;
   int na = 0, nb = 0;
   unsigned bad = 0;
   auto decide = [&](int first, int m) {
-    int fl = 0, code = 13, u = 0;
-    if (lane < m) {
-      const int slot = (first + lane) & (LQ - 1);
+    const bool on = lane < m;
+    const int slot = (first + lane) & (LQ - 1);
+    const int e = on ? qbuf[slot] : CODE_EXACT << ENT_CODE_SHIFT;
+    int u = e & (int)ENT_JMASK;
+    const int code = (e >> ENT_CODE_SHIFT) & 31;
+    int2 mj = make_int2(-1, 0);
+    if (on) {
       if (STAGED) {
-        const int k = qbuf[slot];
-        const int uc = s_u[k];
-        u = uc & (int)ENT_JMASK;
-        const int j = s_j[k];
-        bool exact = !fast;
-        if (fast) {
-          const int meta = __float_as_int(s_x[k].w);
-          fl = fast_flags(P, i, j, ti, meta >> 1, qi, (meta & 1) != 0, qr[slot], map, icut, excl_off, excl_idx,
-                          cexcl_off, cexcl_idx, &exact);
-          code = (int)((unsigned)uc >> ENT_CODE_SHIFT);
-        }
-        if (exact)
-          fl = exact_flags(P, n, i, j, ci, pos, xi, yi, zi, ti, qi, itype, map, icut, q, excl_off, excl_idx,
-                           cexcl_off, cexcl_idx, cimg, code);
+        mj = make_int2(s_j[u], __float_as_int(s_x[u].w));
+        u = s_u[u] & (int)ENT_JMASK;
       } else {
-        const int uc = qbuf[slot];
-        u = fast ? (uc & (int)ENT_JMASK) : uc;
-        const int j = cell_atoms[u];
-        bool exact = !fast;
-        if (fast) {
-          fl = fast_flags(P, i, j, ti, itype[j], qi, q[j] != 0.0, qr[slot], map, icut, excl_off, excl_idx,
-                          cexcl_off, cexcl_idx, &exact);
-          code = (int)((unsigned)uc >> ENT_CODE_SHIFT);
-        }
-        if (exact)
-          fl = exact_flags(P, n, i, j, ci, pos, xi, yi, zi, ti, qi, itype, map, icut, q, excl_off, excl_idx,
-                           cexcl_off, cexcl_idx, cimg, code);
+        mj = K.smeta[u];
       }
     }
-    bad |= (fl >> 4) & 1;
-    const bool fa = (fl & 3) != 0;                   // in an LJ list: front segment
-    const bool fb = !fa && (fl & 12) != 0;           // electrostatics only: back segment
-    const unsigned ba = __ballot_sync(0xffffffffu, fa), bb = __ballot_sync(0xffffffffu, fb);
-    if (fa || fb) {
-      uint32_t e = (uint32_t)u | ((uint32_t)code << ENT_CODE_SHIFT);
-      if (fl & 1) e |= ENT_LJ;
-      if (fl & 2) e |= ENT_LJS;
-      if (fl & 4) e |= ENT_EL;
-      if (fl & 8) e |= ENT_ELS;
-      if (fl & 32) e |= ENT_NEAR;
-      // every write lands inside the slot; once the two segments meet (an
-      // overflow) the slot's contents no longer matter: the lengths are set
-      // to zero below and the list is built again with wider slots
-      if (fa) {
-        const int slot = na + __popc(ba & lt_mask);
-        if (slot < stride - nb) out[slot] = e;
-      } else {
-        const int slot = nb + __popc(bb & lt_mask);
-        if (slot < stride - na) out[stride - 1 - slot] = e;
-      }
-    }
-    na += __popc(ba);
-    nb += __popc(bb);
+    bool near;
+    uint32_t en = list_flags(P, K, A, on && code != CODE_EXACT, i, mj, qr[slot], &near);
+    if (en) en |= (uint32_t)code << ENT_CODE_SHIFT | (uint32_t)(e & QUEUE_NEAR);
+    if (on && (near || code == CODE_EXACT)) en = exact_entry(P, K, i, mj.x);
+    bad |= en & EXACT_BAD;
+    append(out, stride, (en & ~EXACT_BAD) | (uint32_t)u, na, nb);
   };
-  if (STAGED) walk_staged(t, xq[t], P.lim2, s_x, s_u, scnt, qbuf, qr, decide, s_off, s_code, nw, prune, cw);
-  else walk_candidates(P, i, ci, xq[t], false, cell_atoms, cell_start, xq, qbuf, decide, fast ? qr : nullptr,
-                       prune, cw, t);
+  if (STAGED) walk_staged(P, t, K.xq[t], s_x, s_u, scnt, qbuf, qr, decide, s_off, s_code, nw, kind, prune, cw);
+  else walk_candidates(P, K, i, false, qbuf, qr, decide, kind, prune, cw, t);
   const int count = na + nb;
   if (lane == 0) {
     if (count <= stride) {
@@ -701,30 +799,302 @@ __device__ __forceinline__ void full_list_atom(
 // Mixed mode, warp per atom over every atom (the candidates walked in global
 // memory): the fallback of k_list_win.
 __global__ void __launch_bounds__(256, 3) k_list_full(
-    int n, const SysP *__restrict__ sp, const int *__restrict__ sys_of, const int *__restrict__ sreb, int all,
-    int stride, const int *__restrict__ cell_atoms, const int *__restrict__ cell_start,
-    const float4 *__restrict__ xq, const double *__restrict__ pos, const int *__restrict__ itype,
-    const int *__restrict__ map, const double *__restrict__ icut, const double *__restrict__ q,
-    const int *__restrict__ excl_off, const int *__restrict__ excl_idx, const int *__restrict__ cexcl_off,
-    const int *__restrict__ cexcl_idx, const int4 *__restrict__ cimg, uint32_t *__restrict__ nbr,
-    int *__restrict__ nlen, long long *__restrict__ stat, int *__restrict__ halt, const int *__restrict__ gate) {
+    const __grid_constant__ ListK K, const SysP *__restrict__ sp, const int *__restrict__ sys_of,
+    const int *__restrict__ sreb, int all, int stride, uint32_t *__restrict__ nbr, int *__restrict__ nlen,
+    long long *__restrict__ stat, int *__restrict__ halt, const int *__restrict__ gate) {
   if (gated_off(gate, 1)) return;
   __shared__ int qs[256 / 32][LQ];
   __shared__ float qrs[256 / 32][LQ];
   const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (t >= n) return;                                     // whole warps
+  if (t >= K.n) return;                                   // whole warps
   const int s = sys_of[t];
   if (sys_skip(s, sreb, all)) return;                     // whole warps
-  // FP32-first flags and stencil pruning where the grid allows them (as in
-  // k_list_win: 3 or more cells per axis, no near-image pairs)
   const SysP &P = sp[s];
-  const bool fast = P.nc[0] >= 3 && P.nc[1] >= 3 && P.nc[2] >= 3 && !P.smallbox;
-  const bool ortho = P.h[1] == 0. && P.h[2] == 0. && P.h[3] == 0. && P.h[5] == 0. && P.h[6] == 0. && P.h[7] == 0.;
-  const float3 cw = make_float3(P.hF[0] / (float)P.nc[0], P.hF[4] / (float)P.nc[1], P.hF[8] / (float)P.nc[2]);
-  full_list_atom<false>(P, n, t, stride, cell_atoms, cell_start, xq, pos, itype, map, icut, q, excl_off,
-                        excl_idx, cexcl_off, cexcl_idx, cimg, nbr, nlen, stat, halt, qs[threadIdx.x >> 5],
-                        qrs[threadIdx.x >> 5], nullptr, nullptr, nullptr, 0, fast, nullptr, nullptr, 0,
-                        fast && ortho, cw);
+  const int kind = grid_kind(P);
+  full_list_atom<false>(P, K, t, stride, nbr, nlen, stat, halt, qs[threadIdx.x >> 5], qrs[threadIdx.x >> 5], kind,
+                        kind == G_STENCIL && ortho(P), cell_width(P));
+}
+
+// Mixed mode, grids of 3 or more cells per axis whose neighbourhoods hold
+// thousands of atoms.  A block takes up to 32 (`group`) atoms of one cell, one per lane,
+// and its warps share the chunks of 32 candidates of the cell's stencil.  A
+// candidate, staged as (x, y, z, |x|^2) in the cell's frame, is read by all
+// lanes at once and tested against all 32 atoms by three FMAs and a
+// comparison (|xj|^2 - 2 xi.xj against lim2 - |xi|^2); a lane that keeps it
+// appends one byte to its atom's row of survivors.  After LT_C chunks the
+// warps take the atoms in turn, 32 survivors at a time: FP32 distance, list
+// flags (list_flags' tests), the master list entry and, for a system on the
+// compact pair path (CW), its 16-bit window entry, which needs no conversion
+// pass.  Candidate order is that of the other list kernels, so are the lists.
+//
+// Bound by instruction issue (8 instructions per candidate and 32 atoms, some
+// 150 per 32 survivors).  41,472 water atoms (485 neighbours each): both lists
+// in 0.35 ms; one atom per warp (k_list_full) and the conversion pass took
+// 0.53 + 0.37 ms.
+constexpr int LT_C = 32;                   // chunks between decisions
+constexpr int LT_WARPS = 4;
+constexpr int LT_WC = LT_C / LT_WARPS;     // chunks per warp (their candidates fit a byte)
+constexpr int LT_TYPES = 8;                // types whose radii are held in shared memory
+
+struct TileSmem {
+  unsigned char kept[LT_WARPS][32][LT_WC * 32 + 4];   // per warp and atom: survivors, chunk of the warp << 5 | place
+  float4 cand[LT_WARPS][2][32];            // candidates being tested
+  int count[LT_WARPS][32];                 // survivors
+  uint2 chunk[LT_C];                       // {first candidate | shift code << ENT_CODE_SHIFT, its window index}
+  unsigned char valid[LT_C];               // candidates of the chunk
+  float4 shift[27];
+  int lo[27], cells[27], first[28], woff[27];   // stencil cells in walk order: first atom, count, first chunk, window offset
+  float4 xi[32];
+  int4 atom[32];                           // {atom, 2 type + charged, lowest excluded, span}
+  int na[32], nb[32];                      // segment lengths so far
+  float2 radii[LT_TYPES * LT_TYPES];       // LJ list radii^2 (t, s), -1: none
+};
+
+// appends byte `v` at shared address `at` where d < limit: two predicated
+// instructions (a branch per candidate cost three times the test itself)
+__device__ __forceinline__ void keep_if(float d, float limit, unsigned &at, unsigned v) {
+  asm volatile("{\n .reg .pred p;\n setp.lt.f32 p, %1, %2;\n @p st.shared.u8 [%0], %3;\n @p add.u32 %0, %0, 1;\n}"
+               : "+r"(at)
+               : "f"(d), "f"(limit), "r"(v)
+               : "memory");
+}
+
+template <bool CW>
+__global__ void __launch_bounds__(LT_WARPS * 32, 5) k_list_tile(
+    const __grid_constant__ ListK K, int group, int parts, const SysP *__restrict__ sp,
+    const int *__restrict__ cell_sys, const int *__restrict__ sreb, int all, int stride, uint32_t *__restrict__ nbr,
+    int *__restrict__ nlen, const __grid_constant__ CompactOut W, long long *__restrict__ stat,
+    int *__restrict__ halt, const int *__restrict__ gate) {
+  if (gated_off(gate, 1)) return;
+  __shared__ TileSmem M;
+  const int cell = blockIdx.x / parts, part = blockIdx.x - cell * parts;
+  const int sy = cell_sys[cell];
+  if (sys_skip(sy, sreb, all)) return;
+  const SysP &P = sp[sy];
+  const int hi = K.cell_start[cell + 1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = K.n;
+  const unsigned lt_mask = (1u << lane) - 1u;
+  const float4 *__restrict__ xq = K.xq;
+  const int first_atom = K.cell_start[cell];
+  if (first_atom + part * group >= hi) return;
+  const int ntypes = P.ntypes;
+  const bool rows = ntypes <= LT_TYPES;
+  if (warp == 0) {
+    // the stencil in walk_candidates' order (x offsets outermost): shift
+    // codes 26 down to 0; the compact window holds the cells in code order
+    const int lc = cell - P.c0;
+    const int cz = lc % P.nc[2], cy = (lc / P.nc[2]) % P.nc[1], cx = lc / (P.nc[2] * P.nc[1]);
+    int lo = 0, cnt = 0;
+    if (lane < 27) {
+      int jx = cx + lane / 9 - 1, jy = cy + (lane / 3) % 3 - 1, jz = cz + lane % 3 - 1;
+      jx = jx < 0 ? jx + P.nc[0] : (jx >= P.nc[0] ? jx - P.nc[0] : jx);
+      jy = jy < 0 ? jy + P.nc[1] : (jy >= P.nc[1] ? jy - P.nc[1] : jy);
+      jz = jz < 0 ? jz + P.nc[2] : (jz >= P.nc[2] ? jz - P.nc[2] : jz);
+      const int jc = P.c0 + (jx * P.nc[1] + jy) * P.nc[2] + jz;
+      lo = K.cell_start[jc];
+      cnt = K.cell_start[jc + 1] - lo;
+      M.shift[lane] = P.shift[lane];
+      M.lo[lane] = lo;
+      M.cells[lane] = cnt;
+    }
+    int chunks = (cnt + 31) >> 5, atoms = cnt;
+    const int mine = chunks;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, chunks, o), u = __shfl_up_sync(0xffffffffu, atoms, o);
+      if (lane >= o) {
+        chunks += v;
+        atoms += u;
+      }
+    }
+    const int tot = __shfl_sync(0xffffffffu, atoms, 31);
+    if (lane < 27) {
+      M.first[lane] = chunks - mine;
+      M.woff[lane] = tot - atoms;                          // the atoms of the cells after it
+    }
+    if (lane == 26) M.first[27] = chunks;
+  }
+  if (rows)
+    for (int k = threadIdx.x; k < ntypes * ntypes; k += LT_WARPS * 32) {
+      const int intr = K.map[P.map0 + k];
+      M.radii[k] = intr >= 0 ? make_float2((float)K.icut[8 * intr + 5], (float)K.icut[8 * intr + 4])
+                             : make_float2(-1.f, -1.f);
+    }
+  __syncthreads();
+  const int nchunks = M.first[27], window = M.woff[0] + M.cells[0];
+  const bool fits = !CW || window <= W.cap;
+  if (CW && !fits && part == 0 && threadIdx.x == 0) {
+    atomicAdd((unsigned long long *)(stat + ST_CWIN), 1ull);
+    if (halt) *halt = 1;
+  }
+  const float near_r = fmaf(4e-5f, P.lim2_image, 2e-3f);
+  const float el_r = (float)P.rmaxl_skin2_e, es_r = (float)P.rmaxs_skin2_e;
+  // the threshold's room for the rounding of the larger terms (coordinates of
+  // up to two cells); the survivors' distances are formed anew
+  float lim;
+  {
+    float ext = 0.f;
+#pragma unroll
+    for (int k = 0; k < 9; k++) ext += fabsf(P.hF[k]) / (float)P.nc[k % 3];
+    lim = fmaf(2e-5f * ext, ext, P.lim2);
+  }
+  unsigned bad = 0;
+  for (int t0 = first_atom + part * group; t0 < hi; t0 += parts * group) {
+    const int nseg = min(group, hi - t0);
+    __syncthreads();                                       // the previous atoms' arrays are no longer read
+    const float4 x = xq[t0 + min(lane, nseg - 1)];
+    const float X = -2.f * x.x, Y = -2.f * x.y, Z = -2.f * x.z;
+    const float T = lane < nseg ? lim - fmaf(x.z, x.z, fmaf(x.y, x.y, x.x * x.x)) : -3.0e38f;
+    if (threadIdx.x < nseg) {
+      const int2 mi = K.smeta[t0 + threadIdx.x];
+      const int2 xs = K.xspan[mi.x];
+      M.atom[threadIdx.x] = make_int4(mi.x, mi.y, xs.x, xs.y);
+      M.xi[threadIdx.x] = x;
+      M.na[threadIdx.x] = M.nb[threadIdx.x] = 0;
+    }
+    for (int c0 = 0; c0 < nchunks; c0 += LT_C) {
+      const int nc = min(LT_C, nchunks - c0);
+      __syncthreads();                                     // the last decisions are made
+      if (threadIdx.x < nc) {
+        const int c = c0 + threadIdx.x;
+        int wa = 0, wb = 27;                               // the last cell with first <= c
+        while (wb - wa > 1) {
+          const int mid = (wa + wb) >> 1;
+          if (M.first[mid] <= c) wa = mid;
+          else wb = mid;
+        }
+        const int k = (c - M.first[wa]) * 32;
+        M.chunk[threadIdx.x] = make_uint2((unsigned)(M.lo[wa] + k) | (unsigned)(26 - wa) << ENT_CODE_SHIFT,
+                                          (unsigned)(M.woff[wa] + k));
+        M.valid[threadIdx.x] = (unsigned char)min(32, M.cells[wa] - k);
+      }
+      __syncthreads();
+      // test: this warp's chunks
+      {
+        const unsigned kept0 = (unsigned)__cvta_generic_to_shared(M.kept[warp][lane]);
+        unsigned kept = kept0;
+        const int ca = warp * LT_WC, cb = min(nc, ca + LT_WC);
+        float4 xn = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (ca < cb && lane < M.valid[ca]) xn = xq[(M.chunk[ca].x & ENT_JMASK) + lane];
+        for (int c = ca; c < cb; c++) {
+          const float4 S = M.shift[M.chunk[c].x >> ENT_CODE_SHIFT];
+          const float px = xn.x - S.x, py = xn.y - S.y, pz = xn.z - S.z;
+          const int nv = M.valid[c];
+          float4 *cand = M.cand[warp][c & 1];
+          cand[lane] = make_float4(px, py, pz, lane < nv ? fmaf(pz, pz, fmaf(py, py, px * px)) : 3.0e38f);
+          __syncwarp();
+          if (c + 1 < cb && lane < M.valid[c + 1]) xn = xq[(M.chunk[c + 1].x & ENT_JMASK) + lane];
+          const unsigned base = (unsigned)(c - ca) << 5;
+#pragma unroll 8
+          for (int k = 0; k < 32; k++) {
+            const float4 p = cand[k];
+            keep_if(fmaf(X, p.x, fmaf(Y, p.y, fmaf(Z, p.z, p.w))), T, kept, base + k);
+          }
+        }
+        M.count[warp][lane] = (int)(kept - kept0);
+      }
+      __syncthreads();
+      // decide: this warp's atoms
+      for (int a = warp; a < nseg; a += LT_WARPS) {
+        const int n0 = M.count[0][a], n1 = n0 + M.count[1][a], n2 = n1 + M.count[2][a], total = n2 + M.count[3][a];
+        const int t = t0 + a;
+        const float4 xi = M.xi[a];
+        const int4 at = M.atom[a];
+        uint32_t *out = nbr + (size_t)t * stride;
+        unsigned short *cout = CW ? reinterpret_cast<unsigned short *>(W.list + (size_t)t * W.words) : nullptr;
+        int na = M.na[a], nb = M.nb[a];
+        const bool qi = (at.y & 1) != 0;
+        const float2 *row = M.radii + (at.y >> 1) * ntypes;
+        for (int h = 0; h < total; h += 32) {
+          const int k = h + lane;
+          const int p = (k >= n0) + (k >= n1) + (k >= n2);
+          const int k0 = p == 0 ? 0 : (p == 1 ? n0 : (p == 2 ? n1 : n2));
+          const bool in = k < total;
+          const int e = in ? M.kept[p][a][k - k0] : 0;
+          const uint2 cu = M.chunk[in ? p * LT_WC + (e >> 5) : 0];
+          const int u = (int)(cu.x & ENT_JMASK) + (e & 31);
+          const unsigned code = cu.x >> ENT_CODE_SHIFT;
+          const bool on = in && u != t;
+          float r2f = 3.0e38f;
+          int2 mj = make_int2(-1, 0);
+          if (on) {
+            const float4 xj = xq[u], Sc = M.shift[code];
+            mj = K.smeta[u];
+            const float dx = (xi.x - xj.x) + Sc.x, dy = (xi.y - xj.y) + Sc.y, dz = (xi.z - xj.z) + Sc.z;
+            r2f = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+          }
+          float rl = -1.f, rs = -1.f;
+          if (rows) {
+            const float2 r = row[mj.y >> 1];
+            rl = r.x;
+            rs = r.y;
+          } else if (on) {
+            const int intr = K.map[P.map0 + (at.y >> 1) * ntypes + (mj.y >> 1)];
+            if (intr >= 0) {
+              rl = (float)K.icut[8 * intr + 5];
+              rs = (float)K.icut[8 * intr + 4];
+            }
+          }
+          const bool qq = qi && (mj.y & 1);
+          bool near;
+          uint32_t en = radii_flags(r2f, rl, rs, qq ? el_r : -1.f, qq ? es_r : -1.f, near_r, &near);
+          if (en && (unsigned)(mj.x - at.z) <= (unsigned)at.w) en = strike_excluded(P, K, en, at.x, mj.x);
+          en |= code << ENT_CODE_SHIFT;
+          if (on && near) en = exact_entry(P, K, at.x, mj.x);
+          bad |= en & EXACT_BAD;
+          // append (see append()), to both lists
+          const bool fa = (en & (ENT_LJ | ENT_LJS)) != 0, any = (en & ENT_FLAGS) != 0;
+          const unsigned ba = __ballot_sync(0xffffffffu, fa), bb = __ballot_sync(0xffffffffu, any && !fa);
+          const int place = fa ? na + __popc(ba & lt_mask) : nb + __popc(bb & lt_mask);
+          if (any && place < stride - (fa ? nb : na)) {
+            out[fa ? place : stride - 1 - place] = (en & ~EXACT_BAD) | (uint32_t)u;
+            if (CW && fits) {
+              // (a code other than the candidate's own names no window slot:
+              // bad geometry, reported by ST_BADSHIFT)
+              const unsigned o = cu.y + (unsigned)(e & 31);
+              cout[compact_place(place, fa, W.blocks)] = (unsigned short)(fa && (en & ENT_EL) ? o | COMPACT_EL : o);
+            }
+          }
+          na += __popc(ba);
+          nb += __popc(bb);
+        }
+        if (lane == 0) {
+          M.na[a] = na;
+          M.nb[a] = nb;
+        }
+      }
+    }
+    __syncthreads();
+    for (int a = warp; a < nseg; a += LT_WARPS) {
+      const int t = t0 + a;
+      int na = M.na[a], nb = M.nb[a];
+      if (na + nb > stride) {
+        if (lane == 0) {
+          atomicMax((unsigned long long *)(stat + ST_NEED_STRIDE), (unsigned long long)(na + nb));
+          if (halt) {
+            atomicAdd((unsigned long long *)(stat + ST_OVERFLOW), 1ull);
+            *halt = 1;
+          }
+        }
+        na = nb = 0;
+      }
+      if (lane == 0) {
+        nlen[t] = na;
+        nlen[n + t] = nb;
+      }
+      if (CW) {
+        if (!fits) na = nb = 0;
+        // the unused places of each segment's last block name the dummy slot
+        unsigned short *cout = reinterpret_cast<unsigned short *>(W.list + (size_t)t * W.words);
+        const int ea = (na + COMPACT_BLOCK - 1) / COMPACT_BLOCK * COMPACT_BLOCK,
+                  eb = (nb + COMPACT_BLOCK - 1) / COMPACT_BLOCK * COMPACT_BLOCK;
+        for (int k = na + lane; k < ea; k += 32) cout[compact_place(k, true, W.blocks)] = (unsigned short)W.cap;
+        for (int k = nb + lane; k < eb; k += 32) cout[compact_place(k, false, W.blocks)] = (unsigned short)W.cap;
+        if (lane == 0) W.len[t] = make_int2(na, nb);
+      }
+    }
+  }
+  if (__any_sync(0xffffffffu, bad) && lane == 0) atomicAdd((unsigned long long *)(stat + ST_BADSHIFT), 1ull);
 }
 
 // The cells of the systems being rebuilt, as one index range: rb_scan[s] is
@@ -784,14 +1154,10 @@ constexpr int LW_THREADS = 256;
 constexpr size_t LW_BYTES_PER_ATOM = sizeof(float4) + 2 * sizeof(int);   // s_x (w: type, charge), s_u, s_j
 constexpr long long LW_MAX_CAP = 2048;     // largest staged neighbourhood (48 KB)
 
-__global__ void __launch_bounds__(LW_THREADS) k_list_win(
-    int nsys, const int *__restrict__ rb_scan, const SysP *__restrict__ sp, int n, int stride, int cap,
-    const int *__restrict__ cell_atoms, const int *__restrict__ cell_start,
-    const float4 *__restrict__ xq, const double *__restrict__ pos, const int *__restrict__ itype,
-    const int *__restrict__ map, const double *__restrict__ icut, const double *__restrict__ q,
-    const int *__restrict__ excl_off, const int *__restrict__ excl_idx, const int *__restrict__ cexcl_off,
-    const int *__restrict__ cexcl_idx, const int4 *__restrict__ cimg, uint32_t *__restrict__ nbr,
-    int *__restrict__ nlen, long long *__restrict__ stat, int *__restrict__ halt, const int *__restrict__ gate) {
+__global__ void __launch_bounds__(LW_THREADS, 3) k_list_win(
+    const __grid_constant__ ListK K, int nsys, const int *__restrict__ rb_scan, const SysP *__restrict__ sp,
+    int stride, int cap, int parts, uint32_t *__restrict__ nbr, int *__restrict__ nlen,
+    long long *__restrict__ stat, int *__restrict__ halt, const int *__restrict__ gate) {
   if (gated_off(gate, 1)) return;
   extern __shared__ float4 s_x[];                        // cap
   int *s_u = reinterpret_cast<int *>(s_x + cap);         // cap: sorted index | shift code << ENT_CODE_SHIFT
@@ -801,8 +1167,10 @@ __global__ void __launch_bounds__(LW_THREADS) k_list_win(
   __shared__ int s_cs[27], s_off[27], s_code[27], s_tot, s_nw;
   __shared__ float4 s_sh[27];
   const int warp = threadIdx.x >> 5;
-  const int total = rb_scan[nsys];
-  for (int v = blockIdx.x; v < total; v += gridDim.x) {
+  const int total = rb_scan[nsys] * parts;
+  for (int item = blockIdx.x; item < total; item += gridDim.x) {
+    // rebuilt cell v, every parts-th round of its atoms from `part` on
+    const int v = item / parts, part = item - v * parts;
     // the system of rebuilt cell v: the last s with rb_scan[s] <= v (systems
     // without rebuilt cells share their successor's value and are passed)
     int sa = 0, sb = nsys;
@@ -831,8 +1199,8 @@ __global__ void __launch_bounds__(LW_THREADS) k_list_win(
         jy = jy < 0 ? jy + P.nc[1] : (jy >= P.nc[1] ? jy - P.nc[1] : jy);
         jz = jz < 0 ? jz + P.nc[2] : (jz >= P.nc[2] ? jz - P.nc[2] : jz);
         const int cell = P.c0 + (jx * P.nc[1] + jy) * P.nc[2] + jz;
-        const int cs = cell_start[cell];
-        cn = cell_start[cell + 1] - cs;
+        const int cs = K.cell_start[cell];
+        cn = K.cell_start[cell + 1] - cs;
         s_cs[w] = cs;
         s_code[w] = (1 - ox) * 9 + (1 - oy) * 3 + (1 - oz);
         s_sh[w] = P.shift[s_code[w]];
@@ -864,28 +1232,25 @@ __global__ void __launch_bounds__(LW_THREADS) k_list_win(
           else wb = mid;
         }
         const int u = s_cs[wa] + (g - s_off[wa]);
-        const float4 x = xq[u];
-        const int j = cell_atoms[u];
+        const float4 x = K.xq[u];
+        const int2 mj = K.smeta[u];
         const float4 sh = s_sh[wa];
-        s_x[g] = make_float4(x.x - sh.x, x.y - sh.y, x.z - sh.z, __int_as_float(itype[j] * 2 + (q[j] != 0.0 ? 1 : 0)));
+        s_x[g] = make_float4(x.x - sh.x, x.y - sh.y, x.z - sh.z, __int_as_float(mj.y));
         s_u[g] = u | (s_code[wa] << ENT_CODE_SHIFT);
-        s_j[g] = j;
+        s_j[g] = mj.x;
       }
     }
     __syncthreads();
-    const int lo = cell_start[c], hi = cell_start[c + 1];
-    const bool fast = P.nc[0] >= 3 && P.nc[1] >= 3 && P.nc[2] >= 3 && !P.smallbox;
-    const bool ortho = P.h[1] == 0. && P.h[2] == 0. && P.h[3] == 0. && P.h[5] == 0. && P.h[6] == 0. && P.h[7] == 0.;
-    const float3 cw = make_float3(P.hF[0] / (float)P.nc[0], P.hF[4] / (float)P.nc[1], P.hF[8] / (float)P.nc[2]);
-    for (int t = lo + warp; t < hi; t += LW_THREADS / 32) {
+    const int lo = K.cell_start[c], hi = K.cell_start[c + 1];
+    const int kind = grid_kind(P);
+    const bool prune = kind == G_STENCIL && ortho(P);
+    const float3 cw = cell_width(P);
+    for (int t = lo + part * (LW_THREADS / 32) + warp; t < hi; t += parts * (LW_THREADS / 32)) {
       if (staged)
-        full_list_atom<true>(P, n, t, stride, cell_atoms, cell_start, xq, pos, itype, map, icut, q, excl_off,
-                             excl_idx, cexcl_off, cexcl_idx, cimg, nbr, nlen, stat, halt, qs[warp], qrs[warp], s_x,
-                             s_u, s_j, tot, fast, s_off, s_code, nw, fast && ortho && nw == 27, cw);
+        full_list_atom<true>(P, K, t, stride, nbr, nlen, stat, halt, qs[warp], qrs[warp], kind, prune && nw == 27, cw,
+                             s_x, s_u, s_j, tot, s_off, s_code, nw);
       else
-        full_list_atom<false>(P, n, t, stride, cell_atoms, cell_start, xq, pos, itype, map, icut, q, excl_off,
-                              excl_idx, cexcl_off, cexcl_idx, cimg, nbr, nlen, stat, halt, qs[warp], nullptr,
-                              nullptr, nullptr, nullptr, 0, false);
+        full_list_atom<false>(P, K, t, stride, nbr, nlen, stat, halt, qs[warp], qrs[warp], kind, prune, cw);
     }
   }
 }
@@ -896,7 +1261,8 @@ __global__ void k_sorted_init(int n, const SysP *__restrict__ sp, const int *__r
                               const int *__restrict__ sreb, int all, const int *__restrict__ cell_atoms,
                               const int4 *__restrict__ cimg, const int *__restrict__ itype,
                               const double *__restrict__ pos, const double *__restrict__ q, int *__restrict__ rank,
-                              int *__restrict__ styp, double *__restrict__ corner, float4 *__restrict__ xq,
+                              int *__restrict__ styp, int2 *__restrict__ smeta, double *__restrict__ corner,
+                              float4 *__restrict__ xq,
                               const int *__restrict__ gate) {
   if (gated_off(gate, 1)) return;
   int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -919,6 +1285,7 @@ __global__ void k_sorted_init(int n, const SysP *__restrict__ sp, const int *__r
   xq[t] = make_float4((float)(pos[i] - c0), (float)(pos[n + i] - c1), (float)(pos[2 * n + i] - c2), (float)q[i]);
   rank[i] = t;
   styp[t] = itype[i];
+  smeta[t] = make_int2(i, itype[i] * 2 + (q[i] != 0.0 ? 1 : 0));
 }
 
 // The cell corners (and FP32 cell-relative positions) under a new box: every
@@ -928,7 +1295,7 @@ int refresh_corners(Ctx *c) {
   if (c->mode != CM3D_NB_MIXED || !c->lists_built) return CM3D_NB_OK;
   k_sorted_init<<<grid_for(c->n, 256), 256, 0, c->st>>>(c->n, c->sp, c->sys_of, c->sreb, 1, c->cell_atoms,
                                                         c->cimg, c->itype, c->pos, c->q, c->rank, c->styp,
-                                                        c->corner, c->xq, nullptr);
+                                                        c->smeta, c->corner, c->xq, nullptr);
   c->launches++;
   CKL(c);
   return CM3D_NB_OK;
@@ -986,6 +1353,14 @@ void cell_shifts(SysP &P, const SysH &H) {
         P.shift_lo[k] = make_float4((float)(v0 - (double)(float)v0), (float)(v1 - (double)(float)v1),
                                     (float)(v2 - (double)(float)v2), 0.f);
       }
+  // FP32 minimum images in the list tests of a coarse grid: candidates lie
+  // within two cells, so cells of at most 4 list radii bound the displacement
+  P.image_ok = 1;
+  for (int d = 0; d < 3; d++) {
+    const double w = 1.0 / sqrt(H.hmati[3 * d] * H.hmati[3 * d] + H.hmati[3 * d + 1] * H.hmati[3 * d + 1] +
+                                H.hmati[3 * d + 2] * H.hmati[3 * d + 2]);
+    if (!(w / P.nc[d] <= 4.0 * H.rlist)) P.image_ok = 0;
+  }
 }
 
 int list_setup(Ctx *c) {
@@ -1011,11 +1386,12 @@ int list_setup(Ctx *c) {
     stencil(P.nc[2], P.sz, &P.nsz);
     // with three or more cells per direction the stencil neighbour's image
     // is the minimum image of every pair in range, so the FP32 prefilter is
-    // exact up to rounding; with fewer cells every candidate goes to the
-    // FP64 test
+    // exact up to rounding; with fewer cells the minimum image is taken first
+    // (lim2_image), or every candidate goes to the FP64 test
     const bool pre = P.nc[0] >= 3 && P.nc[1] >= 3 && P.nc[2] >= 3;
     const double rl = H.rlist + 1e-3;
     P.lim2 = pre ? (float)(rl * rl) : INFINITY;
+    P.lim2_image = (float)(rl * rl);
     cell_shifts(P, H);
     // first guess of the full-list slot: 1.3 x the mean number of atoms in
     // a list sphere, plus 64
@@ -1047,6 +1423,7 @@ int list_setup(Ctx *c) {
   CK(cudaMalloc(&c->ltot, sizeof(long long) * LT_COUNT));
   CK(cudaMallocHost(&c->h_ltot, sizeof(long long) * LT_COUNT));
   CK(cudaMalloc(&c->styp, sizeof(int) * (size_t)c->n));
+  CK(cudaMalloc(&c->smeta, sizeof(int2) * (size_t)c->n));
   CK(cudaMalloc(&c->corner, sizeof(double) * 3 * (size_t)c->n));
   CK(cudaMalloc(&c->xq, sizeof(float4) * (size_t)c->n));
   CK(cudaMalloc(&c->cimg, sizeof(int4) * (size_t)c->n));
@@ -1062,6 +1439,7 @@ int list_setup(Ctx *c) {
       const SysP &S = c->h_sp[sy];
       const double per_cell = (double)S.n / (double)(S.ncells > 0 ? S.ncells : 1);
       nb_max = std::max(nb_max, per_cell * S.nsx * S.nsy * S.nsz);
+      c->lw_atoms = std::max(c->lw_atoms, (int)(1.25 * per_cell) + 1);
     }
     c->lw_smem_max = c->smem_optin > 8192 ? c->smem_optin - 8192 : 0;
     long long cap = (long long)(1.6 * nb_max) + 64;
@@ -1072,6 +1450,11 @@ int list_setup(Ctx *c) {
     if (c->lw_cap < 64 || cap > LW_MAX_CAP) c->lw_cap = 0;
     const char *lk = getenv("CM3D_NB_LIST_KERNEL");
     if (lk && strcmp(lk, "walk") == 0) c->lw_cap = 0;
+    c->list_tile = 1;
+    for (int sy = 0; sy < c->nsys; sy++)
+      for (int d = 0; d < 3; d++)
+        if (c->h_sp[sy].nc[d] < 3) c->list_tile = 0;
+    if (lk && strcmp(lk, "walk") == 0) c->list_tile = 0;
     CK(cudaMalloc(&c->rb_scan, sizeof(int) * ((size_t)c->nsys + 1)));
     CK(cudaMalloc(&c->nlen, sizeof(int) * 2 * (size_t)c->n));
     CK(cudaMemset(c->nlen, 0, sizeof(int) * 2 * (size_t)c->n));
@@ -1176,11 +1559,16 @@ int build_lists(Ctx *c, bool device_flag, bool all) {
         c->ncells, per_block, c->cell_sys, c->sreb, al, c->cell_start, c->itype, c->cell_atoms, gate);
   }
   k_sorted_init<<<grid_for(n, B), B, 0, c->st>>>(n, c->sp, c->sys_of, c->sreb, al, c->cell_atoms, cimg, c->itype,
-                                                  c->pos, c->q, c->rank, c->styp, c->corner, c->xq, gate);
+                                                  c->pos, c->q, c->rank, c->styp, c->smeta, c->corner, c->xq, gate);
   c->launches += 6;
   const long long warps_threads = 32LL * n;
+  int *halt = device_flag ? c->istate + IS_HALT : nullptr;
+  const ListK K = {n, c->cell_atoms, c->cell_start, c->cell_of, c->xq, c->pos, c->itype, c->map, c->icut, c->q,
+                   c->excl_off, c->excl_idx, c->cexcl_off, c->cexcl_idx, cimg, c->smeta, c->xspan};
+  bool direct = false;                       // the list kernel wrote the compact lists as well
   if (c->mode == CM3D_NB_MIXED) {
     for (;;) {
+      CompactOut W = {nullptr, nullptr, 0, 0, 0};
       if (c->lw_cap > 0) {
         // block per cell over the cells of the systems being rebuilt, the
         // stencil neighbourhood staged in shared memory
@@ -1193,18 +1581,34 @@ int build_lists(Ctx *c, bool device_flag, bool all) {
         int per_sm = 1;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_list_win, LW_THREADS, smem);
         long long grid = (long long)c->num_sms * (per_sm > 0 ? per_sm : 1);
-        if (grid > c->ncells) grid = c->ncells;
+        // a grid of few cells is split into parts of the cells' atoms until
+        // the resident blocks all have work (8 cells of 81 water atoms run on
+        // 8 of the 148 SMs: 135 us, split and with FP32 minimum images 9 us)
+        int parts = 1;
+        while ((long long)c->ncells * parts < grid && parts * (LW_THREADS / 32) < c->lw_atoms) parts++;
+        if (grid > (long long)c->ncells * parts) grid = (long long)c->ncells * parts;
         k_rebuild_cells<<<1, 1024, 0, c->st>>>(c->nsys, c->sp, c->sreb, al, c->rb_scan, gate);
-        k_list_win<<<(int)grid, LW_THREADS, smem, c->st>>>(
-            c->nsys, c->rb_scan, c->sp, n, c->nbr_stride, c->lw_cap, c->cell_atoms, c->cell_start, c->xq, c->pos,
-            c->itype, c->map, c->icut, c->q, c->excl_off, c->excl_idx, c->cexcl_off, c->cexcl_idx, cimg, c->nbr,
-            c->nlen, c->stat, device_flag ? c->istate + IS_HALT : nullptr, gate);
+        k_list_win<<<(int)grid, LW_THREADS, smem, c->st>>>(K, c->nsys, c->rb_scan, c->sp, c->nbr_stride, c->lw_cap,
+                                                           parts, c->nbr, c->nlen, c->stat, halt, gate);
         c->launches++;
+      } else if (c->list_tile) {
+        int rc = CM3D_NB_OK;
+        const bool compact = cw_direct(c, device_flag, &W, &rc);
+        if (rc) return rc;
+        // fewer atoms per block where blocks of 32 would leave SMs idle: the
+        // tests then run on fewer lanes, but a block's decisions, one atom
+        // after another, are what a small system waits for (3993 atoms: 169 us
+        // with 32 atoms per block, 102 with 8; 12,288: 212 with 32, 277 with 16)
+        int group = 32;
+        while (group > 8 && (long long)n / group < 2LL * c->num_sms) group /= 2;
+        const int parts = (c->lw_atoms + group - 1) / group;
+        const auto kern = compact ? k_list_tile<true> : k_list_tile<false>;
+        kern<<<c->ncells * parts, LT_WARPS * 32, 0, c->st>>>(K, group, parts, c->sp, c->cell_sys, c->sreb, al,
+                                                             c->nbr_stride, c->nbr, c->nlen, W, c->stat, halt, gate);
+        direct = compact;
       } else {
-        k_list_full<<<grid_for(warps_threads, 256), 256, 0, c->st>>>(
-            n, c->sp, c->sys_of, c->sreb, al, c->nbr_stride, c->cell_atoms, c->cell_start, c->xq, c->pos,
-            c->itype, c->map, c->icut, c->q, c->excl_off, c->excl_idx, c->cexcl_off, c->cexcl_idx, cimg, c->nbr,
-            c->nlen, c->stat, device_flag ? c->istate + IS_HALT : nullptr, gate);
+        k_list_full<<<grid_for(warps_threads, 256), 256, 0, c->st>>>(K, c->sp, c->sys_of, c->sreb, al, c->nbr_stride,
+                                                                     c->nbr, c->nlen, c->stat, halt, gate);
       }
       c->launches++;
       CKL(c);
@@ -1218,14 +1622,13 @@ int build_lists(Ctx *c, bool device_flag, bool all) {
     }
   }
   if (c->mode == CM3D_NB_MIXED) {
-    int rc = cw_convert(c, device_flag, all);
+    int rc = direct ? cw_check(c, device_flag) : cw_convert(c, device_flag, all);
     if (rc) return rc;
   }
   if (want_half) {
     k_list_half<false><<<grid_for(warps_threads, 256), 256, 0, c->st>>>(
-        n, c->sp, c->sys_of, caps(c), c->cell_atoms, c->cell_start, c->xq, c->pos, c->itype, c->map, c->icut,
-        c->q, c->excl_off, c->excl_idx, c->cexcl_off, c->cexcl_idx, cimg, c->cnt, nullptr, nullptr, nullptr,
-        nullptr, nullptr, nullptr, c->stat, nullptr, gate);
+        K, c->sp, c->sys_of, caps(c), c->cnt, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, c->stat, nullptr,
+        gate);
     k_scan<int, long long><<<dim3(1, 4), 1024, 0, c->st>>>(c->cnt, c->off, c->ltot, n, gate);
     c->launches += 2;
     CKL(c);
@@ -1239,9 +1642,8 @@ int build_lists(Ctx *c, bool device_flag, bool all) {
       }
     }
     k_list_half<true><<<grid_for(warps_threads, 256), 256, 0, c->st>>>(
-        n, c->sp, c->sys_of, caps(c), c->cell_atoms, c->cell_start, c->xq, c->pos, c->itype, c->map, c->icut,
-        c->q, c->excl_off, c->excl_idx, c->cexcl_off, c->cexcl_idx, cimg, nullptr, c->off, c->ltot, c->lst[0],
-        c->lst[1], c->lst[2], c->lst[3], c->stat, device_flag ? c->istate + IS_HALT : nullptr, gate);
+        K, c->sp, c->sys_of, caps(c), c->cnt, c->off, c->ltot, c->lst[0], c->lst[1], c->lst[2], c->lst[3], c->stat,
+        halt, gate);
     c->launches++;
   }
   if (!c->no_snapshot) {
