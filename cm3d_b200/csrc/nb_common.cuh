@@ -124,29 +124,54 @@ __device__ __forceinline__ bool gated_off(const int *gs, int need_rebuild) {
 // per-system counters (sstat[s * SS_COUNT + ...])
 enum { SS_REBUILDS = 0, SS_RESETS = 1, SS_COUNT = 2 };
 
-// Sum NV per-thread values into the accumulators of each thread's system
-// (acc + sys * ACC_STRIDE + slots[k]).  A warp whose threads all belong to
-// one system reduces first and adds once; a mixed warp adds per thread.
-// Threads with sys < 0 contribute nothing.  Every thread of the warp calls it.
+// Warp totals of NV per-lane values at once: halves of the value set are
+// exchanged while the set is larger than one, so lane l < P (P: NV rounded up
+// to a power of two) returns the total of v[l] after about NV + 5 shuffles,
+// where a butterfly per value takes 5 NV.  Every thread of the warp calls it.
 template <int NV>
-__device__ __forceinline__ void sys_acc(double (&v)[NV], int sys, double *acc, const int *slots) {
+__device__ __forceinline__ double warp_totals(const double (&v)[NV]) {
+  constexpr int P = NV <= 2 ? 2 : NV <= 4 ? 4 : NV <= 8 ? 8 : NV <= 16 ? 16 : 32;
+  static_assert(NV <= 32, "one value per lane");
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  double x[P];
+#pragma unroll
+  for (int k = 0; k < P; k++) x[k] = k < NV ? v[k < NV ? k : 0] : 0.0;
+#pragma unroll
+  for (int h = P / 2; h >= 1; h >>= 1) {
+    const bool hi = (lane & h) != 0;
+#pragma unroll
+    for (int i = 0; i < h; i++) {
+      const double snd = hi ? x[i] : x[i + h], kp = hi ? x[i + h] : x[i];
+      x[i] = kp + __shfl_xor_sync(full, snd, h);
+    }
+  }
+#pragma unroll
+  for (int o = P; o < 32; o <<= 1) x[0] += __shfl_xor_sync(full, x[0], o);
+  return x[0];
+}
+
+// Sum NV <= 32 per-thread values into the accumulators of each thread's system
+// (acc + sys * ACC_STRIDE + slot(k)).  A warp whose threads all belong to
+// one system reduces first, and lane k adds value k; a mixed warp adds per
+// thread.  Threads with sys < 0 contribute nothing.  Every thread of the warp
+// calls it.
+template <int NV, class Slot>
+__device__ __forceinline__ void sys_acc(double (&v)[NV], int sys, double *acc, Slot slot) {
   const unsigned full = 0xffffffffu;
   const int s0 = __shfl_sync(full, sys, 0);
   if (__all_sync(full, sys == s0 || sys < 0)) {
+    if (sys < 0) {
 #pragma unroll
-    for (int k = 0; k < NV; k++) {
-      // a quantity that is zero on every thread (e.g. no bonds in an LJ
-      // system) costs one vote, not a reduction
-      if (!__any_sync(full, sys >= 0 && v[k] != 0.0)) continue;
-      double s = sys < 0 ? 0.0 : v[k];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(full, s, o);
-      if ((threadIdx.x & 31) == 0 && s != 0.0 && s0 >= 0) atomicAdd(acc + (size_t)s0 * ACC_STRIDE + slots[k], s);
+      for (int k = 0; k < NV; k++) v[k] = 0.0;
     }
+    const double s = warp_totals<NV>(v);
+    const int lane = threadIdx.x & 31;
+    if (lane < NV && s != 0.0 && s0 >= 0) atomicAdd(acc + (size_t)s0 * ACC_STRIDE + slot(lane), s);
   } else if (sys >= 0) {
 #pragma unroll
     for (int k = 0; k < NV; k++)
-      if (v[k] != 0.0) atomicAdd(acc + (size_t)sys * ACC_STRIDE + slots[k], v[k]);
+      if (v[k] != 0.0) atomicAdd(acc + (size_t)sys * ACC_STRIDE + slot(k), v[k]);
   }
 }
 
@@ -342,6 +367,9 @@ struct Ctx {
   int2 *ecorr_pairs = nullptr;          // CM3D's iecorr/jecorr order
   // ---- bonded groups (connected components of bonds/bends/ecorr)
   int ngroups = 0;
+  int *qidx = nullptr;                  // per atom: its place in icharge, -1 uncharged (small_mol 3)
+  bool ecorr_side = false;              // force(1)'s molecule terms run beside the k-space (all ecorr atoms charged)
+  int small_mol = 0;                    // every molecule has at most this many atoms (1, 3; 0: more) and simple terms
   int *grp_atom_off = nullptr, *grp_atoms = nullptr;
   int *grp_bond_off = nullptr, *grp_bend_off = nullptr, *grp_ecorr_off = nullptr;
   int4 *bond_ij = nullptr;              // {i, j, -, -} grouped order
@@ -476,27 +504,23 @@ __device__ __forceinline__ T warp_sum(T v) {
   return v;
 }
 
-// block-wide sum of NV doubles into acc[slot..slot+NV) with one atomic per
-// value per block; all threads of the block must call it
-template <int NV>
-__device__ __forceinline__ void block_acc(double (&v)[NV], double *acc, const int *slots) {
+// the six stored elements of a symmetric 3 x 3 tensor: 0 1 2 4 5 8
+__device__ __forceinline__ int sym6(int k) { return k + (k >= 3 ? 1 : 0) + (k >= 5 ? 2 : 0); }
+
+// block-wide sum of NV doubles into acc[slot(k)] with one atomic per value per
+// block; all threads of the block must call it
+template <int NV, class Slot>
+__device__ __forceinline__ void block_acc(double (&v)[NV], double *acc, Slot slot) {
   __shared__ double red[32][NV];
-  int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-#pragma unroll
-  for (int k = 0; k < NV; k++) v[k] = warp_sum(v[k]);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+  const double s = warp_totals<NV>(v);
   __syncthreads();
-  if (lane == 0) {
-#pragma unroll
-    for (int k = 0; k < NV; k++) red[w][k] = v[k];
-  }
+  if (lane < NV) red[w][lane] = s;
   __syncthreads();
-  if (w == 0) {
-#pragma unroll
-    for (int k = 0; k < NV; k++) {
-      double s = lane < nw ? red[lane][k] : 0.0;
-      s = warp_sum(s);
-      if (lane == 0 && s != 0.0) atomicAdd(acc + slots[k], s);
-    }
+  if (w == 0 && lane < NV) {
+    double t = 0.0;
+    for (int k = 0; k < nw; k++) t += red[k][lane];
+    if (t != 0.0) atomicAdd(acc + slot(lane), t);
   }
 }
 
@@ -553,6 +577,7 @@ int kspace_forces(Ctx *c);                      // nb_kspace.cu
 bool kspace_async_ok(const Ctx *c);             // nb_kspace.cu: force(1)'s k-space beside the lists/pairs
 int kspace_fork(Ctx *c);                        // nb_kspace.cu
 int kspace_join(Ctx *c);                        // nb_kspace.cu
+int group_terms(Ctx *c, cudaStream_t st, double *part);   // nb_step.cu: force(1)'s molecule terms
 int kspace_setup(Ctx *c);                       // nb_kspace.cu
 int step_setup(Ctx *c, const cm3d_nb_system *systems, int nsys);   // nb_step.cu
 int run_step(Ctx *c, int istep0, int nsteps);   // nb_step.cu
@@ -561,7 +586,7 @@ int finish_steps(Ctx *c);                       // nb_step.cu
 int query_steps(Ctx *c, int *done);             // nb_step.cu
 int run_force(Ctx *c, int iflg);                // nb_step.cu
 int run_bonded(Ctx *c);                         // nb_step.cu
-int group_init(Ctx *c, bool zero_fxs);          // nb_step.cu
+int group_init(Ctx *c, bool zero_fxs, bool side);   // nb_step.cu
 int finish_level1(Ctx *c, double dter, double dter1, bool kick);   // nb_step.cu
 int check_displacement(Ctx *c);                 // nb_step.cu
 int reset_positions(Ctx *c);                    // nb_step.cu

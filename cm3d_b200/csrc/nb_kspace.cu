@@ -284,10 +284,9 @@ __global__ void k_sred(int ktot, int ntiles, const double2 *__restrict__ spart, 
     if (akf) akf[k] = make_float2((float)(2. * preg * sr), (float)(2. * preg * si));
     if (akd) akd[k] = make_double2(2. * preg * sr, 2. * preg * si);
   }
-  const int slots[11] = {ACC_VK, ACC_VP, ACC_VPT + 0, ACC_VPT + 1, ACC_VPT + 2, ACC_VPT + 3,
-                         ACC_VPT + 4, ACC_VPT + 5, ACC_VPT + 6, ACC_VPT + 7, ACC_VPT + 8};
-  if (BATCH) sys_acc<11>(v, sys, acc, slots);
-  else block_acc<11>(v, acc, slots);
+  const auto slot = [](int k) { return ACC_VK + k; };       // VK, VP, VPT[9]
+  if (BATCH) sys_acc<11>(v, sys, acc, slot);
+  else block_acc<11>(v, acc, slot);
 }
 
 template <bool BATCH, int A = KF_A>
@@ -464,24 +463,28 @@ __global__ void __launch_bounds__(KS_THREADS) k_kforce_mixed(int nq, const uint4
   }
 }
 
-// the row splits' partial reciprocal forces of every charged atom, summed in
-// split order (deterministic: the same result whatever else the device runs)
+// the row splits' partial reciprocal forces of every charged atom (and the
+// molecule terms' partial, where they run beside the k-space), summed in
+// split order (deterministic: the same result whatever else the device runs);
+// eight partials' loads in flight at a time
 __global__ void k_kforce_sum(int nq, int nsplit, const double *__restrict__ part, const int *__restrict__ icharge,
                              int n, double *__restrict__ fxl, const int *__restrict__ gs) {
   if (gated_off(gs, 0)) return;
   const int jq = blockIdx.x * blockDim.x + threadIdx.x;
   if (jq >= nq) return;
+  const int i = icharge[jq];
+  const double f0 = fxl[i], f1 = fxl[n + i], f2 = fxl[2 * n + i];
   double fx = 0, fy = 0, fz = 0;
+#pragma unroll 8
   for (int y = 0; y < nsplit; y++) {
     const size_t o = ((size_t)y * nq + jq) * 3;
     fx += part[o];
     fy += part[o + 1];
     fz += part[o + 2];
   }
-  const int i = icharge[jq];
-  fxl[i] += fx;
-  fxl[n + i] += fy;
-  fxl[2 * n + i] += fz;
+  fxl[i] = f0 + fx;
+  fxl[n + i] = f1 + fy;
+  fxl[2 * n + i] = f2 + fz;
 }
 
 // ------------------------------------------------------------ plain FP64
@@ -696,8 +699,9 @@ int kspace_setup(Ctx *c) {
   if (mixed) {
     // (also with one split: the forked k-space of a step writes partials)
     // zeroed once: the charged atoms of systems without k-vectors keep zero partials
-    CK(cudaMalloc(&c->kf_part, sizeof(double) * 3 * (size_t)split * c->ncharge));
-    CK(cudaMemset(c->kf_part, 0, sizeof(double) * 3 * (size_t)split * c->ncharge));
+    // (one more for the molecule terms that run beside the k-space)
+    CK(cudaMalloc(&c->kf_part, sizeof(double) * 3 * ((size_t)split + 1) * c->ncharge));
+    CK(cudaMemset(c->kf_part, 0, sizeof(double) * 3 * ((size_t)split + 1) * c->ncharge));
   }
   return CM3D_NB_OK;
 }
@@ -836,6 +840,8 @@ int kspace_fork(Ctx *c) {
   CK(cudaStreamWaitEvent(c->st2, c->ev_fork, 0));
   int rc = kspace_run(c, c->st2, true);
   if (rc) return rc;
+  // the molecules' own terms: to a partial of their own, off the main stream
+  if (c->ecorr_side && (rc = group_terms(c, c->st2, c->kf_part + (size_t)3 * c->kf_split * c->ncharge))) return rc;
   CK(cudaEventRecord(c->ev_join, c->st2));
   return CM3D_NB_OK;
 }
@@ -844,8 +850,9 @@ int kspace_fork(Ctx *c) {
 // forces to fxl in split order (after the pair forces, as without the fork)
 int kspace_join(Ctx *c) {
   CK(cudaStreamWaitEvent(c->st, c->ev_join, 0));
-  k_kforce_sum<<<grid_for(c->ncharge, 256), 256, 0, c->st>>>(c->ncharge, c->kf_split, c->kf_part, c->icharge, c->n,
-                                                              c->fxl, c->gate);
+  const int B = c->ncharge < 256 * c->num_sms ? 64 : 256;
+  k_kforce_sum<<<grid_for(c->ncharge, B), B, 0, c->st>>>(c->ncharge, c->kf_split + (c->ecorr_side ? 1 : 0), c->kf_part,
+                                                         c->icharge, c->n, c->fxl, c->gate);
   c->launches++;
   CKL(c);
   return CM3D_NB_OK;

@@ -88,9 +88,7 @@ __global__ void k_lj_plain(const long long *__restrict__ npd, const int2 *__rest
   }
   if (under) atomicAdd((unsigned long long *)(stat + ST_UNDERFLOW), (unsigned long long)under);
   if (P.iflg == 1) {
-    const int slots[9] = {ACC_SPOTL, ACC_SPOTHL, ACC_SPRSL, ACC_SPRSLT + 0, ACC_SPRSLT + 1,
-                          ACC_SPRSLT + 2, ACC_SPRSLT + 4, ACC_SPRSLT + 5, ACC_SPRSLT + 8};
-    block_acc<9>(v, acc, slots);
+    block_acc<9>(v, acc, [](int k) { return k < 3 ? ACC_SPOTL + k : ACC_SPRSLT + sym6(k - 3); });
   }
 }
 
@@ -148,9 +146,7 @@ __global__ void k_el_plain(const long long *__restrict__ npd, const int2 *__rest
   }
   if (under) atomicAdd((unsigned long long *)(stat + ST_UNDERFLOW), (unsigned long long)under);
   if (P.iflg == 1) {
-    const int slots[9] = {ACC_SPOTE, ACC_SPOTHE, ACC_SPRSE, ACC_SPRSET + 0, ACC_SPRSET + 1,
-                          ACC_SPRSET + 2, ACC_SPRSET + 4, ACC_SPRSET + 5, ACC_SPRSET + 8};
-    block_acc<9>(v, acc, slots);
+    block_acc<9>(v, acc, [](int k) { return k < 3 ? ACC_SPOTE + k : ACC_SPRSET + sym6(k - 3); });
   }
 }
 
@@ -177,10 +173,8 @@ __global__ void k_ecorr_plain(int necorr, const int2 *__restrict__ ij, int n, co
     atomicAdd(fl + ii, xd); atomicAdd(fl + n + ii, yd); atomicAdd(fl + 2 * n + ii, zd);
     atomicAdd(fl + jj, -xd); atomicAdd(fl + n + jj, -yd); atomicAdd(fl + 2 * n + jj, -zd);
   }
-  const int slots[8] = {ACC_POT_ECORR, ACC_PRS_ECORR, ACC_PRS_ECORRT + 0, ACC_PRS_ECORRT + 1,
-                        ACC_PRS_ECORRT + 2, ACC_PRS_ECORRT + 4, ACC_PRS_ECORRT + 5, ACC_PRS_ECORRT + 8};
   double w[8] = {v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7]};
-  block_acc<8>(w, acc, slots);
+  block_acc<8>(w, acc, [](int k) { return k < 2 ? ACC_POT_ECORR + k : ACC_PRS_ECORRT + sym6(k - 2); });
 }
 
 static PlainP plain_params(Ctx *c, int iflg) {

@@ -386,6 +386,176 @@ __global__ void k_inner(StepP P, int intr, const int *__restrict__ gaoff, const 
   }
 }
 
+// k_inner for a context whose molecules all have at most NA atoms (NA 1: no
+// intramolecular term at all; 3: at most two bonds and one bend, as a
+// flexible water has), no torsion level and no frozen atom: the molecule's
+// positions, velocities and bonded accelerations stay in registers through
+// the ninrra x ninnra substeps.  The general kernel passes every one of them
+// through global memory, whose latency, not the arithmetic, is its time (4096
+// water molecules, 4 substeps: 26 us; here 9 us).  An atom's local index
+// selects among registers; the sums are k_inner's, in its order.
+struct Mol3 {
+  double p[3][3], v[3][3], f[3][3];      // [atom][component]
+};
+
+__device__ __forceinline__ double pick(const double (&a)[3][3], int l, int d) {
+  return l == 0 ? a[0][d] : (l == 1 ? a[1][d] : a[2][d]);
+}
+__device__ __forceinline__ void add_to(double (&a)[3][3], int l, int d, double x) {
+#pragma unroll
+  for (int k = 0; k < 3; k++)
+    if (l == k) a[k][d] += x;
+}
+
+// fbond of local atoms i, j
+__device__ __forceinline__ void mol_bond(Mol3 &M, int i, int j, double2 par) {
+  double x[3];
+#pragma unroll
+  for (int d = 0; d < 3; d++) x[d] = pick(M.p, i, d) - pick(M.p, j, d);
+  const double r = sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]);
+  const double fr = par.y * (r - par.x) / r;
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    add_to(M.f, i, d, -(x[d] * fr));
+    add_to(M.f, j, d, x[d] * fr);
+  }
+}
+
+// fbend of local atoms i, j (centre), k
+__device__ __forceinline__ void mol_bend(Mol3 &M, int i, int j, int k, double2 par) {
+  double a[3], b[3];
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    a[d] = pick(M.p, i, d) - pick(M.p, j, d);
+    b[d] = pick(M.p, k, d) - pick(M.p, j, d);
+  }
+  const double al = a[0] * a[0] + a[1] * a[1] + a[2] * a[2];
+  const double bl = b[0] * b[0] + b[1] * b[1] + b[2] * b[2];
+  const double r11 = 1. / sqrt(al * bl), costh = (a[0] * b[0] + a[1] * b[1] + a[2] * b[2]) * r11;
+  double dudth = 0., dthdcos = -1.;
+  if (fabs(costh) < 1.) {
+    dudth = par.y * (acos(costh) - par.x);
+    dthdcos = -1. / sqrt(1. - costh * costh);
+  }
+  const double dudcos = dudth * dthdcos;
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    const double d1 = costh * a[d] / al - b[d] * r11, d3 = costh * b[d] / bl - a[d] * r11;
+    add_to(M.f, i, d, dudcos * d1);
+    add_to(M.f, j, d, dudcos * (-d1 - d3));
+    add_to(M.f, k, d, dudcos * d3);
+  }
+}
+
+template <int NA>
+__global__ void __launch_bounds__(128) k_inner_small(
+    StepP P, int intr, const int *__restrict__ gaoff, const int *__restrict__ gatoms, double *__restrict__ pos,
+    double *__restrict__ vel, const double *__restrict__ mass, const double *__restrict__ fxl,
+    const double *__restrict__ fxs, double *__restrict__ fxa, const double *__restrict__ dxn,
+    const int *__restrict__ gboff, const int4 *__restrict__ bij, const double2 *__restrict__ bp,
+    const int *__restrict__ geoff, const int4 *__restrict__ eijk, const double2 *__restrict__ ep,
+    const SysP *__restrict__ sp, const int *__restrict__ sys_of, int *__restrict__ sreb, int *__restrict__ istate,
+    const int *__restrict__ gs) {
+  if (gated_off(gs, 0)) return;
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g == 0) istate[IS_INTR] = intr;
+  if (g >= P.ngroups) return;
+  const int n = P.n;
+  // NA 1: group g is atom gatoms[g]
+  const int a0 = NA == 1 ? g : gaoff[g], na = NA == 1 ? 1 : gaoff[g + 1] - a0;
+  int id[NA];
+#pragma unroll
+  for (int a = 0; a < NA; a++) id[a] = gatoms[a0 + (a < na ? a : 0)];
+  Mol3 M;
+  double rm[NA];
+  const int sy = sys_of[id[0]];
+  const double skin2q = sp[sy].skin2q;
+#pragma unroll
+  for (int a = 0; a < NA; a++) {
+    rm[a] = 1. / mass[id[a]];
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      const int x = d * n + id[a];
+      M.p[a][d] = pos[x];
+      M.v[a][d] = vel[x];
+      M.f[a][d] = fxa[x];
+      // long and short range intermolecular kick (md_step.c:97-103)
+      if (intr == 0) M.v[a][d] += P.dter * fxl[x] + (P.use_fxs ? P.dter1 * fxs[x] : 0.0);
+      else M.v[a][d] += P.dts2 * fxs[x];
+    }
+  }
+  // the molecule's terms as local atom indices
+  int nb = 0, ne = 0;
+  int2 b0 = make_int2(0, 0), b1 = b0;
+  int3 e0 = make_int3(0, 0, 0);
+  double2 q0 = make_double2(0., 0.), q1 = q0, qe = q0;
+  if (NA > 1) {
+    auto local = [&](int i) { return i == id[0] ? 0 : (NA > 1 && i == id[1] ? 1 : 2); };
+    const int kb = gboff[g], ke = geoff[g];
+    nb = gboff[g + 1] - kb;
+    ne = geoff[g + 1] - ke;
+    if (nb > 0) {
+      b0 = make_int2(local(bij[kb].x), local(bij[kb].y));
+      q0 = bp[kb];
+    }
+    if (nb > 1) {
+      b1 = make_int2(local(bij[kb + 1].x), local(bij[kb + 1].y));
+      q1 = bp[kb + 1];
+    }
+    if (ne > 0) {
+      e0 = make_int3(local(eijk[ke].x), local(eijk[ke].y), local(eijk[ke].z));
+      qe = ep[ke];
+    }
+  }
+  const int nsub = P.ninrra * P.ninnra;
+  for (int it = 0; it < nsub; it++) {
+#pragma unroll
+    for (int a = 0; a < NA; a++)
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        M.v[a][d] += P.dta2 * M.f[a][d];
+        M.p[a][d] += P.dta2 * M.v[a][d];
+        M.p[a][d] += P.dta2 * M.v[a][d];
+      }
+    if (NA > 1 && (nb > 0 || ne > 0)) {
+#pragma unroll
+      for (int a = 0; a < NA; a++) M.f[a][0] = M.f[a][1] = M.f[a][2] = 0.;
+      if (nb > 0) mol_bond(M, b0.x, b0.y, q0);
+      if (nb > 1) mol_bond(M, b1.x, b1.y, q1);
+      if (ne > 0) mol_bend(M, e0.x, e0.y, e0.z, qe);
+#pragma unroll
+      for (int a = 0; a < NA; a++)
+#pragma unroll
+        for (int d = 0; d < 3; d++) M.f[a][d] *= rm[a];
+    }
+#pragma unroll
+    for (int a = 0; a < NA; a++)
+#pragma unroll
+      for (int d = 0; d < 3; d++) M.v[a][d] += P.dta2 * M.f[a][d];
+  }
+  // results, and nrefsh: any |r - r_last|^2 > skin^2/4 (md_finter.c:63-71)
+  bool far = false;
+#pragma unroll
+  for (int a = 0; a < NA; a++) {
+    if (a >= na) break;
+    double c2 = 0.;
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      const int x = d * n + id[a];
+      pos[x] = M.p[a][d];
+      vel[x] = M.v[a][d];
+      if (NA > 1) fxa[x] = M.f[a][d];
+      const double c = dxn[x] - M.p[a][d];
+      c2 = d == 0 ? c * c : c2 + c * c;
+    }
+    if (c2 > skin2q) far = true;
+  }
+  if (far) {
+    sreb[sy] = 1;
+    istate[IS_REBUILD] = 1;
+  }
+}
+
 // ---- NVT: the inner level with Nose-Hoover chains (intnhc_new,
 // integrate/md_therm.new.c:278-333, called between the two half drifts of
 // every inner substep, md_step.c:117).  The chain update needs every
@@ -592,6 +762,13 @@ __global__ void k_resetpos(int n, const SysP *__restrict__ sp, const int *__rest
   }
 }
 
+// accumulator of quantity k of k_group_init / k_group_small:
+// ecorr pot, prs, t0 t1 t2 t4 t5 t8 | bond v, w, t[9] | bend v, w, t[9]
+__device__ __forceinline__ int group_slot(int k) {
+  return k < 2 ? ACC_POT_ECORR + k : k < 8 ? ACC_PRS_ECORRT + sym6(k - 2) : k < 19 ? ACC_VBOND + k - 8
+       : k == 19 ? (int)ACC_VBEND : ACC_WBEND + k - 20;
+}
+
 // start of force(1) (md_fcntr.c:64-73): zero fxl (and fxs), add the
 // excluded-pair correction of every group (ecorr, md_ewald.c:385-453), and
 // collect the group's bonded energies and virials (getvbond / getvbend; the
@@ -693,14 +870,136 @@ __global__ void k_group_init(StepP P, const int *__restrict__ gwork, int ngw, co
       v[29] += dudcos * (zi * c1z + zj * c2z + zk * c3z);
     }
   }
-  const int slots[30] = {ACC_POT_ECORR, ACC_PRS_ECORR, ACC_PRS_ECORRT + 0, ACC_PRS_ECORRT + 1,
-                         ACC_PRS_ECORRT + 2, ACC_PRS_ECORRT + 4, ACC_PRS_ECORRT + 5, ACC_PRS_ECORRT + 8,
-                         ACC_VBOND, ACC_WBOND, ACC_WBONDT + 0, ACC_WBONDT + 1, ACC_WBONDT + 2,
-                         ACC_WBONDT + 3, ACC_WBONDT + 4, ACC_WBONDT + 5, ACC_WBONDT + 6, ACC_WBONDT + 7,
-                         ACC_WBONDT + 8, ACC_VBEND, ACC_WBEND, ACC_WBENDT + 0, ACC_WBENDT + 1,
-                         ACC_WBENDT + 2, ACC_WBENDT + 3, ACC_WBENDT + 4, ACC_WBENDT + 5, ACC_WBENDT + 6,
-                         ACC_WBENDT + 7, ACC_WBENDT + 8};
-  sys_acc<30>(v, sy, acc, slots);
+  sys_acc<30>(v, sy, acc, group_slot);
+}
+
+// k_group_init for molecules of at most three atoms, three excluded pairs, two
+// bonds and one bend: positions, charges and forces in registers, the terms
+// unrolled (their erf, exp and acos overlap).  The ecorr forces are added to
+// fxl, or -- where the kernel runs beside the k-space -- written to `part`,
+// one triple per charged atom, which k_kforce_sum adds.
+__global__ void __launch_bounds__(128) k_group_small(
+    StepP P, const int *__restrict__ gwork, int ngw, const int *__restrict__ gaoff, const int *__restrict__ gatoms,
+    const double *__restrict__ pos, const double *__restrict__ q, double *__restrict__ fxl, double *__restrict__ part,
+    const int *__restrict__ qidx, const int *__restrict__ gcoff, const int2 *__restrict__ cij,
+    const int *__restrict__ gboff, const int4 *__restrict__ bij, const double2 *__restrict__ bp,
+    const int *__restrict__ geoff, const int4 *__restrict__ eijk, const double2 *__restrict__ ep,
+    double *__restrict__ acc, const SysP *__restrict__ sp, const int *__restrict__ sys_of,
+    const int *__restrict__ gs) {
+  if (gated_off(gs, 0)) return;
+  const int gi = blockIdx.x * blockDim.x + threadIdx.x;
+  const int n = P.n;
+  double v[30];
+#pragma unroll
+  for (int k = 0; k < 30; k++) v[k] = 0.;
+  int sy = -1;
+  if (gi < ngw) {
+    const int g = gwork[gi], a0 = gaoff[g], na = gaoff[g + 1] - a0;
+    int id[3];
+    double x[3][3], qa[3], f[3][3];
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      id[a] = gatoms[a0 + (a < na ? a : 0)];
+      qa[a] = q[id[a]];
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        x[a][d] = pos[d * n + id[a]];
+        f[a][d] = 0.;
+      }
+    }
+    auto local = [&](int i) { return i == id[0] ? 0 : (i == id[1] ? 1 : 2); };
+    sy = sys_of[id[0]];
+    const double kappa = sp[sy].kappa, kappa2 = sp[sy].kappa2;
+    const double sqrt_pi = 1. / sqrt(M_PI);
+    const int c0 = gcoff[g], nc = gcoff[g + 1] - c0, b0 = gboff[g], nb = gboff[g + 1] - b0, e0 = geoff[g],
+              ne = geoff[g + 1] - e0;
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      if (c >= nc) break;
+      const int2 ij = cij[c0 + c];
+      const int i = local(ij.x), j = local(ij.y);
+      double r[3];
+#pragma unroll
+      for (int d = 0; d < 3; d++) r[d] = pick(x, i, d) - pick(x, j, d);
+      const double dis2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2], dis = sqrt(dis2);
+      const double qi = i == 0 ? qa[0] : (i == 1 ? qa[1] : qa[2]), qj = j == 0 ? qa[0] : (j == 1 ? qa[1] : qa[2]);
+      const double qijr = qi * qj / dis, erfr = erf(dis * kappa);
+      v[0] += -qijr * erfr;
+      double dv = -qijr * (-2. * kappa * exp(-kappa2 * dis2) * sqrt_pi + erfr / dis);
+      v[1] += dis * dv;
+      dv /= dis;
+      v[2] += dv * r[0] * r[0]; v[3] += dv * r[0] * r[1]; v[4] += dv * r[0] * r[2];
+      v[5] += dv * r[1] * r[1]; v[6] += dv * r[1] * r[2]; v[7] += dv * r[2] * r[2];
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        add_to(f, i, d, r[d] * dv);
+        add_to(f, j, d, -(r[d] * dv));
+      }
+    }
+    // getvbond (md_fbond.c:160-207), harmonic
+#pragma unroll
+    for (int b = 0; b < 2; b++) {
+      if (b >= nb) break;
+      const int4 ij = bij[b0 + b];
+      const double2 p = bp[b0 + b];
+      const int i = local(ij.x), j = local(ij.y);
+      double r[3];
+#pragma unroll
+      for (int d = 0; d < 3; d++) r[d] = pick(x, i, d) - pick(x, j, d);
+      const double dis = sqrt(r[0] * r[0] + r[1] * r[1] + r[2] * r[2]), dr = dis - p.x;
+      v[8] += .5 * p.y * dr * dr;
+      const double fk = p.y * dr / dis;
+      v[9] -= fk * dis * dis;
+#pragma unroll
+      for (int k = 0; k < 9; k++) v[10 + k] -= fk * r[k % 3] * r[k / 3];
+    }
+    // getvbend (md_fbend.c:295-398), harmonic, with its virial
+    if (ne > 0) {
+      const int4 ijk = eijk[e0];
+      const double2 p = ep[e0];
+      const int i = local(ijk.x), j = local(ijk.y), k = local(ijk.z);
+      double a[3], b[3];
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        a[d] = pick(x, i, d) - pick(x, j, d);
+        b[d] = pick(x, k, d) - pick(x, j, d);
+      }
+      const double al = a[0] * a[0] + a[1] * a[1] + a[2] * a[2], bl = b[0] * b[0] + b[1] * b[1] + b[2] * b[2];
+      const double r11 = 1. / sqrt(al * bl);
+      double costh = (a[0] * b[0] + a[1] * b[1] + a[2] * b[2]) * r11;
+      costh = costh < 1. ? costh : 1.;
+      costh = costh > -1. ? costh : -1.;
+      const double th = fabs(costh) >= 1. ? 1. : acos(costh), dth = th - p.x;
+      v[19] += .5 * p.y * dth * dth;
+      const double dudth = fabs(costh) >= 1. ? 0. : p.y * dth;
+      const double dthdcos = fabs(costh) >= 1. ? -1. : -1. / sqrt(1. - costh * costh);
+      const double dudcos = dudth * dthdcos;
+      double c1[3], c2[3], c3[3];
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        c1[d] = costh * a[d] / al - b[d] * r11;
+        c2[d] = -costh * (a[d] / al + b[d] / bl) + (a[d] + b[d]) * r11;
+        c3[d] = costh * b[d] / bl - a[d] * r11;
+      }
+      v[20] += dudcos * (a[0] * c1[0] + a[1] * c1[1] + a[2] * c1[2] - b[0] * c3[0] - b[1] * c3[1] - b[2] * c3[2]);
+#pragma unroll
+      for (int m = 0; m < 9; m++) {
+        const int r = m % 3, c = m / 3;                    // tensor element: position component r, cosine gradient c
+        v[21 + m] += dudcos * (pick(x, i, r) * c1[c] + pick(x, j, r) * c2[c] + pick(x, k, r) * c3[c]);
+      }
+    }
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      if (a >= na || nc == 0) break;
+      const int jq = part ? qidx[id[a]] : -1;
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        if (!part) fxl[d * n + id[a]] += f[a][d];
+        else if (jq >= 0) part[(size_t)3 * jq + d] = f[a][d];
+      }
+    }
+  }
+  sys_acc<30>(v, sy, acc, group_slot);
 }
 
 // energies and virials of the cross bonds, torsions and 1-4 pairs, per group
@@ -779,21 +1078,18 @@ __global__ void k_intra_energy(StepP P, const int *__restrict__ gaoff, const int
       }
     }
   }
-  int slots[42];
-  slots[0] = ACC_VBOND;
-  slots[1] = ACC_WBOND;
-  slots[11] = ACC_VTORS;
-  slots[21] = ACC_VONFO;
-  slots[22] = ACC_WONFO;
-  slots[32] = ACC_VONFO_E;
+  double lo[21], hi[21];
 #pragma unroll
-  for (int k = 0; k < 9; k++) {
-    slots[2 + k] = ACC_WBONDXT + k;
-    slots[12 + k] = ACC_WTORST + k;
-    slots[23 + k] = ACC_WONFOT + k;
-    slots[33 + k] = ACC_WONFOET + k;
+  for (int k = 0; k < 21; k++) {
+    lo[k] = v[k];
+    hi[k] = v[21 + k];
   }
-  sys_acc<42>(v, sy, acc, slots);
+  sys_acc<21>(lo, sy, acc, [](int k) {
+    return k < 2 ? ACC_VBOND + k : k < 11 ? ACC_WBONDXT + k - 2 : k == 11 ? (int)ACC_VTORS : ACC_WTORST + k - 12;
+  });
+  sys_acc<21>(hi, sy, acc, [](int k) {
+    return k == 0 ? (int)ACC_VONFO : k < 11 ? ACC_WONFO + k - 1 : k == 11 ? (int)ACC_VONFO_E : ACC_WONFOET + k - 12;
+  });
 }
 
 // end of force(1) / force(0): rmass (utils/md_util.new.c:219) and, inside
@@ -838,9 +1134,9 @@ __global__ void k_finish(int n, int level, int kick, int rm_l, int rm_s, double 
   }
   if (i == 0 && advance_step) istate[IS_ISTEP] += 1;
   if (level == 1) {
-    const int slots[6] = {ACC_P2MT + 0, ACC_P2MT + 1, ACC_P2MT + 2, ACC_P2MT + 4, ACC_P2MT + 5, ACC_P2MT + 8};
-    if (batch) sys_acc<6>(v, sy, acc, slots);
-    else block_acc<6>(v, acc, slots);
+    const auto slot = [](int k) { return ACC_P2MT + sym6(k); };
+    if (batch) sys_acc<6>(v, sy, acc, slot);
+    else block_acc<6>(v, acc, slot);
   }
 }
 
@@ -1273,6 +1569,28 @@ int step_setup(Ctx *c, const cm3d_nb_system *systems, int nsys) {
     if (!work.empty()) CK(cudaMemcpy(c->grp_work, work.data(), sizeof(int) * work.size(), cudaMemcpyHostToDevice));
   }
   if ((rc = upload_intra(c, ih, gid, ng))) return rc;
+  // molecules small enough for the register form of the inner level
+  c->small_mol = 0;
+  if (!c->has_intra_x && !c->intra.frz) {
+    int ma = 0, mb2 = 0, me2 = 0, mc2 = 0;
+    for (int g = 0; g < ng; g++) {
+      ma = std::max(ma, aoff[g + 1] - aoff[g]);
+      mb2 = std::max(mb2, boff[g + 1] - boff[g]);
+      me2 = std::max(me2, eoff[g + 1] - eoff[g]);
+    }
+    for (int g = 0; g < ng; g++) mc2 = std::max(mc2, coff[g + 1] - coff[g]);
+    c->small_mol = ma == 1 && mb2 + me2 + mc2 == 0 ? 1 : (ma <= 3 && mb2 <= 2 && me2 <= 1 && mc2 <= 3 ? 3 : 0);
+    if (c->small_mol == 3 && nc > 0) {
+      // force(1)'s molecule terms beside the k-space: their forces go by charge
+      std::vector<int> qi((size_t)n, -1), ich((size_t)c->ncharge);
+      if (c->ncharge > 0) CK(cudaMemcpy(ich.data(), c->icharge, sizeof(int) * ich.size(), cudaMemcpyDeviceToHost));
+      for (int k = 0; k < c->ncharge; k++) qi[(size_t)ich[(size_t)k]] = k;
+      c->ecorr_side = true;
+      for (int b = 0; b < nc; b++) c->ecorr_side = c->ecorr_side && qi[(size_t)mc[b].x] >= 0 && qi[(size_t)mc[b].y] >= 0;
+      CK(cudaMalloc(&c->qidx, sizeof(int) * (size_t)n));
+      CK(cudaMemcpy(c->qidx, qi.data(), sizeof(int) * (size_t)n, cudaMemcpyHostToDevice));
+    }
+  }
   return nvt_setup(c, systems, nsys);
 }
 
@@ -1304,7 +1622,32 @@ int run_tors_level(Ctx *c) {
   return CM3D_NB_OK;
 }
 
-int group_init(Ctx *c, bool zero_fxs) {
+// the molecules' ecorr forces and their ecorr, bond and bend energies on
+// stream st: forces added to fxl, or (small molecules) written to `part`
+int group_terms(Ctx *c, cudaStream_t st, double *part) {
+  if (c->ngwork == 0) return CM3D_NB_OK;
+  StepP P = step_params(c);
+  if (c->small_mol == 3) {
+    const int B = c->ngwork < 128 * c->num_sms ? 32 : 128;
+    k_group_small<<<grid_for(c->ngwork, B), B, 0, st>>>(P, c->grp_work, c->ngwork, c->grp_atom_off, c->grp_atoms,
+                                                        c->pos, c->q, c->fxl, part, c->qidx, c->grp_ecorr_off,
+                                                        c->ecorr_ij, c->grp_bond_off, c->bond_ij, c->bond_p,
+                                                        c->grp_bend_off, c->bend_ijk, c->bend_p, c->acc, c->sp,
+                                                        c->sys_of, c->gate);
+  } else {
+    k_group_init<<<grid_for(c->ngwork, 128), 128, 0, st>>>(P, c->grp_work, c->ngwork, c->grp_atom_off, c->grp_atoms,
+                                                           c->pos, c->q, c->fxl, c->fxs, c->grp_ecorr_off,
+                                                           c->ecorr_ij, c->grp_bond_off, c->bond_ij, c->bond_p,
+                                                           c->grp_bend_off, c->bend_ijk, c->bend_p, c->acc, c->sp,
+                                                           c->sys_of, c->gate);
+  }
+  c->launches++;
+  CKL(c);
+  return CM3D_NB_OK;
+}
+
+// side: the molecule terms run beside the k-space already (kspace_fork)
+int group_init(Ctx *c, bool zero_fxs, bool side) {
   StepP P = step_params(c);
   const int B = 128;
   cudaEvent_t e0;
@@ -1313,13 +1656,9 @@ int group_init(Ctx *c, bool zero_fxs) {
   // the host-driven path that finishes it computes them again from here)
   CK(cudaMemsetAsync(c->fxl, 0, sizeof(double) * 3 * (size_t)c->n, c->st));
   if (zero_fxs) CK(cudaMemsetAsync(c->fxs, 0, sizeof(double) * 3 * (size_t)c->n, c->st));
-  if (c->ngwork > 0) {
-    k_group_init<<<grid_for(c->ngwork, B), B, 0, c->st>>>(P, c->grp_work, c->ngwork, c->grp_atom_off, c->grp_atoms,
-                                                          c->pos, c->q, c->fxl, c->fxs, c->grp_ecorr_off,
-                                                          c->ecorr_ij, c->grp_bond_off, c->bond_ij, c->bond_p,
-                                                          c->grp_bend_off, c->bend_ijk, c->bend_p, c->acc, c->sp,
-                                                          c->sys_of, c->gate);
-    c->launches++;
+  if (!side) {
+    int rc = group_terms(c, c->st, nullptr);
+    if (rc) return rc;
   }
   if (c->has_intra_x) {
     k_intra_energy<<<grid_for(c->ngroups, B), B, 0, c->st>>>(P, c->grp_atom_off, c->grp_atoms, c->pos, c->q,
@@ -1392,7 +1731,7 @@ int run_force(Ctx *c, int iflg) {
   }
   if (iflg == 1) {
     if ((rc = zero_acc(c))) return rc;
-    if ((rc = group_init(c, true))) return rc;
+    if ((rc = group_init(c, true, false))) return rc;
     if ((rc = pair_forces(c, 1, 3))) return rc;
     if ((rc = kspace_forces(c))) return rc;
     return finish_level1(c, 0, 0, false);
@@ -1415,7 +1754,7 @@ static int close_level(Ctx *c, int intr, bool ks_forked = false) {
   StepP P = step_params(c);
   if (intr == c->nres_lrf - 1) {
     if (!ks_forked && (rc = zero_acc(c))) return rc;
-    if ((rc = group_init(c, P.use_fxs))) return rc;
+    if ((rc = group_init(c, P.use_fxs, ks_forked && c->ecorr_side))) return rc;
     if ((rc = pair_forces(c, 1, 3))) return rc;
     if ((rc = ks_forked ? kspace_join(c) : kspace_forces(c))) return rc;
     return finish_level1(c, P.dter, P.dter1, true);
@@ -1458,12 +1797,22 @@ static int one_level(Ctx *c, int intr, bool gated) {
         c->launches += 4;
       }
   } else {
+    if (c->small_mol) {
+      // few molecules: one warp per block, so that they spread over the SMs
+      const int BS = c->ngroups < 128 * c->num_sms ? 32 : 128;
+      auto inner = c->small_mol == 1 ? k_inner_small<1> : k_inner_small<3>;
+      inner<<<grid_for(c->ngroups, BS), BS, 0, c->st>>>(P, intr, c->grp_atom_off, c->grp_atoms, c->pos, c->vel, c->mass,
+                                                        c->fxl, c->fxs, c->fxa, c->dxn, c->grp_bond_off, c->bond_ij,
+                                                        c->bond_p, c->grp_bend_off, c->bend_ijk, c->bend_p, c->sp,
+                                                        c->sys_of, c->sreb, c->istate, c->gate);
+    } else {
     auto inner = c->has_intra_x || c->intra.frz ? k_inner<true> : k_inner<false>;
     inner<<<grid_for(c->ngroups, B), B, 0, c->st>>>(P, intr, c->grp_atom_off, c->grp_atoms, c->pos, c->vel,
                                                       c->mass, c->fxl, c->fxs, c->fxa, c->dxn, c->grp_bond_off,
                                                       c->bond_ij, c->bond_p, c->grp_bend_off, c->bend_ijk,
                                                       c->bend_p, c->sp, c->sys_of, c->sreb, c->istate, c->gate,
                                                       c->intra, c->q, c->fxr, c->stat);
+    }
     c->launches++;
   }
   tend(c, 3, e0);
