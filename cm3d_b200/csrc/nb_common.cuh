@@ -363,6 +363,16 @@ struct Ctx {
   int ks_tiles = 0, ks_tile_atoms = 0, kf_split = 1;
   bool ks_small = false;                // batch of systems with <= 32 charges: one-warp k-space tiles
   size_t kf_smem = 0;
+  // large k sums of one system (k_sfac_gemm, k_kforce_reg)
+  bool kr_on = false;
+  int kr_kcm = 0, kr_atoms = 0, kr_tiles = 0;   // largest |kc|; atoms per structure-factor block and their number
+  int *kr_perm = nullptr;               // rows in order of falling length
+  int *kr_split = nullptr;              // first row of each force split
+  int kr_nent = 0, kr_cap = 0;          // force coefficients: entries, most of one split (+2)
+  int4 *kr_hdr = nullptr;               // per row {ka, kb, largest |kc|, first entry}, one more at the end
+  int2 *kr_kidx = nullptr;              // per entry {k of +kc, k of -kc}
+  float4 *kr_coef = nullptr;
+  float2 *kr_btab = nullptr;            // cos, sin of kc theta, [kc][charge]
   double *kf_part = nullptr;            // per row split partial reciprocal forces (mixed, split > 1)
   int2 *ecorr_pairs = nullptr;          // CM3D's iecorr/jecorr order
   // ---- bonded groups (connected components of bonds/bends/ecorr)

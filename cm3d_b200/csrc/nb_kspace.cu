@@ -24,7 +24,9 @@
 // the recurrence along one row.  The plain mode does everything in FP64 with
 // CM3D's expressions (rk = x aka + y akb + z akc, md_ewald.c:264).
 #include <math.h>
+#include <stdlib.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "nb_common.cuh"
@@ -328,8 +330,8 @@ __global__ void __launch_bounds__(KS_THREADS) k_kforce_mixed(int nq, const uint4
       for (int m = 0; m < A; m++) {
         const int jq = abase + m * blockDim.x + threadIdx.x;
         if (jq < aend) {
-          const size_t o = ((size_t)blockIdx.y * nq + jq) * 3;
-          part[o] = part[o + 1] = part[o + 2] = 0.0;
+          const size_t o = (size_t)3 * blockIdx.y * nq + jq;
+          part[o] = part[o + nq] = part[o + 2 * (size_t)nq] = 0.0;
         }
       }
     return;
@@ -447,10 +449,10 @@ __global__ void __launch_bounds__(KS_THREADS) k_kforce_mixed(int nq, const uint4
     double fz = __dmul_rn(t, fma(hmati[8], U2[m], fma(hmati[5], U1[m], __dmul_rn(hmati[2], U0[m]))));
     if (part) {
       // one partial per row split, summed in a fixed order by k_kforce_sum
-      const size_t o = ((size_t)blockIdx.y * nq + jq[m]) * 3;
+      const size_t o = (size_t)3 * blockIdx.y * nq + jq[m];
       part[o] = fx;
-      part[o + 1] = fy;
-      part[o + 2] = fz;
+      part[o + nq] = fy;
+      part[o + 2 * (size_t)nq] = fz;
     } else if (atomic) {
       atomicAdd(fxl + i, fx);
       atomicAdd(fxl + n + i, fy);
@@ -460,6 +462,429 @@ __global__ void __launch_bounds__(KS_THREADS) k_kforce_mixed(int nq, const uint4
       fxl[n + i] += fy;
       fxl[2 * n + i] += fz;
     }
+  }
+}
+
+// ---------------------------------------------- mixed mode, large k sums
+// One system with many atoms and k-vectors.  With phi = 2 pi (ka s_a + kb s_b)
+// and theta = 2 pi s_c, exp(i (phi +- kc theta)) needs only cos and sin of phi
+// (per row and atom) and of kc theta (per kc and atom, the same for every
+// row), so that a row's k and -k along c share their products:
+//   structure factors: sums over atoms of (tq cos phi, tq sin phi) x
+//     (cos kc theta, sin kc theta), four products for two k -- a matrix
+//     product, tiled in shared memory with its sums in registers;
+//   forces: per row and atom the sums over kc of A(k)'s combinations p, q, s,
+//     t (k_kforce_reg) times cos, sin kc theta, which stay in registers.
+// No phase recursion: cos and sin come from the exact fixed-point phases.  (FP32 products and sums as in k_sfac_mixed; a structure
+// factor's FP32 sums run over at most SG_ATOMS / slices atoms before FP64.)
+// 331,776 charges x 19,400 k: structure factors 2.38 -> 1.32 ms, forces 2.12 ->
+// 1.46 ms, the forces' error a fifth; bound by FP32 issue and the latency of
+// the shared-memory operands (FMA pipe 41% and 55% busy).
+constexpr int SG_ROWS = 64;        // rows per block
+constexpr int SG_TR = 8;           // rows per thread
+constexpr int SG_TK = 4;           // kc per thread
+constexpr int SG_THREADS = 192;
+constexpr int SG_CHUNK = 64;       // atoms staged at a time
+constexpr int SG_ATOMS = 512;      // atoms per block (most)
+constexpr int KR_MAX = 24;         // largest |kc|: kc groups of the sums, registers of the forces
+constexpr int KR_A = 2;            // atoms per thread, forces (four: 1.66 ms instead of 1.46 at 331,776 charges)
+constexpr int KR_THREADS = 128;
+
+// cos and sin of a fixed-point phase (2^32 = one turn): the nearest quarter
+// turn is taken off exactly and the rest, within pi/4, goes through the Taylor
+// polynomials (sin to x^9, cos to x^8: truncation 2e-9 and 3e-8), so both are
+// good to an FP32 rounding or two, where the fast intrinsics are off by up to
+// 5e-7 -- which the small, screened S(k) of a neutral liquid would feel.
+__device__ __forceinline__ void phase_cs(unsigned phi, float &c, float &s) {
+  const unsigned quarter = (phi + 0x20000000u) >> 30;
+  const float x = (float)(int)(phi - (quarter << 30)) * 1.4629180792671596e-09f;   // 2 pi / 2^32
+  const float y = x * x;
+  float sp = fmaf(y, 2.7557319e-06f, -1.9841270e-04f);       // 1/9!, 1/7!
+  sp = fmaf(y, sp, 8.3333333e-03f);                          // 1/5!
+  sp = fmaf(y, sp, -1.6666667e-01f);                         // 1/3!
+  sp = fmaf(x * y, sp, x);
+  float cp = fmaf(y, 2.4801587e-05f, -1.3888889e-03f);       // 1/8!, 1/6!
+  cp = fmaf(y, cp, 4.1666667e-02f);                          // 1/4!
+  cp = fmaf(y, cp, -0.5f);
+  cp = fmaf(y, cp, 1.0f);
+  const float a = (quarter & 1) ? sp : cp, b = (quarter & 1) ? cp : sp;
+  c = __uint_as_float(__float_as_uint(a) ^ (((quarter + 1) & 2) << 30));
+  s = __uint_as_float(__float_as_uint(b) ^ ((quarter & 2) << 30));
+}
+
+// asynchronous 8-byte copy to shared memory
+__device__ __forceinline__ void cp_async8(void *dst, const void *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+
+// fixed-point phases (k_kprep) and cos, sin of kc theta, kc = 0 .. kcmax
+__global__ void k_kprep_reg(int nq, int kcmax, const int *__restrict__ icharge, int n, const double *__restrict__ pos,
+                            const double *__restrict__ q, const double *__restrict__ hmati,
+                            uint4 *__restrict__ kfrac, float2 *__restrict__ btab, const int *__restrict__ gs) {
+  if (gated_off(gs, 0)) return;
+  const int jq = blockIdx.x * blockDim.x + threadIdx.x;
+  if (jq >= nq) return;
+  const int i = icharge[jq];
+  const double x = pos[i], y = pos[n + i], z = pos[2 * n + i];
+  unsigned u[3];
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    const double s = x * hmati[3 * d] + y * hmati[3 * d + 1] + z * hmati[3 * d + 2];
+    const double f = s - floor(s);
+    u[d] = (unsigned)((unsigned long long)(f * 4294967296.0) & 0xffffffffull);
+  }
+  kfrac[jq] = make_uint4(u[0], u[1], u[2], __float_as_uint((float)(q[i] * sqrt(4.0 * M_PI))));   // md_ewald.c:202
+  for (int k = blockIdx.y; k <= kcmax; k += gridDim.y) {
+    float sn, cs;
+    phase_cs((unsigned)k * u[2], cs, sn);
+    btab[(size_t)k * nq + jq] = make_float2(cs, sn);
+  }
+}
+
+// Partial S(k) of SG_ROWS rows (in order of falling length, rowperm) over one
+// range of atoms.  Thread: SG_TR rows x SG_TK kc, every nslice-th staged atom.
+// Both operands are staged twice over: while a chunk is multiplied the next
+// one's (tq cos phi, tq sin phi) are formed and the one after that's cos, sin
+// kc theta are on their way (cp.async), one barrier per chunk.
+struct SgSmem {
+  // As[buffer][atom][P 0-3, P 4-7, Q 0-3, Q 4-7][row group][4]: a warp's
+  // 16-byte reads are contiguous (Bs likewise: [atom][kc pair][kc group]{c, s, c, s})
+  float4 As[2][SG_CHUNK][4][SG_ROWS / SG_TR];
+  uint4 us[3][SG_CHUNK];
+  int4 row[SG_ROWS];                                 // {first kc, length, first k, -}; length 0: no row
+};
+
+__global__ void __launch_bounds__(SG_THREADS, 2) k_sfac_gemm(
+    int nq, int atoms_per_block, const uint4 *__restrict__ kfrac, const float2 *__restrict__ btab, int nrows,
+    const int4 *__restrict__ rows, const int *__restrict__ row_k0, const int *__restrict__ rowperm, int ktot,
+    double2 *__restrict__ spart, const int *__restrict__ gs) {
+  if (gated_off(gs, 0)) return;
+  extern __shared__ __align__(16) unsigned char sg_smem[];
+  SgSmem &M = *reinterpret_cast<SgSmem *>(sg_smem);
+  const int rbase = blockIdx.y * SG_ROWS;
+  // the longest row is the first: its largest |kc| sets the kc groups
+  const int4 top = rows[rowperm[rbase]];
+  const int kcm = max(abs(top.z), abs(top.z + top.w - 1));
+  const int ng = kcm / SG_TK + 1, ntile = (SG_ROWS / SG_TR) * ng;
+  // (an atom's 2 ng float4 and one of padding: the copies of 32 atoms' values
+  // then spread over the banks)
+  const int bst = 2 * ng + 1;
+  float4 *Bs[3];
+#pragma unroll
+  for (int b = 0; b < 3; b++) Bs[b] = reinterpret_cast<float4 *>(sg_smem + sizeof(SgSmem)) + (size_t)b * SG_CHUNK * bst;
+  const int nslice = SG_THREADS / ntile;
+  const int tile = threadIdx.x % ntile, slice = threadIdx.x / ntile;
+  const int rg = tile / ng, kg = tile - rg * ng;
+  const bool work = slice < nslice;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int a_beg = blockIdx.x * atoms_per_block, a_end = min(nq, a_beg + atoms_per_block);
+  const int nch = (a_end - a_beg + SG_CHUNK - 1) / SG_CHUNK;
+  // this lane's two rows, for the phases: rows lane % 4 and lane % 4 + 4 of
+  // group lane / 4, so that a warp's stores are contiguous
+  const int ra = rbase + (lane >> 2) * SG_TR + (lane & 3);
+  int2 r0 = make_int2(0, 0), r1 = r0;
+  if (threadIdx.x < SG_ROWS) {
+    int4 r = make_int4(0, 0, 0, 0);
+    if (rbase + (int)threadIdx.x < nrows) {
+      const int rid = rowperm[rbase + threadIdx.x];
+      const int4 w = rows[rid];
+      r = make_int4(w.z, w.w, row_k0[rid], 0);
+    }
+    M.row[threadIdx.x] = r;
+  }
+  if (ra < nrows) {
+    const int4 r = rows[rowperm[ra]];
+    r0 = make_int2(r.x, r.y);
+  }
+  if (ra + 4 < nrows) {
+    const int4 r = rows[rowperm[ra + 4]];
+    r1 = make_int2(r.x, r.y);
+  }
+  // chunk ch's kc phases and fixed-point phases on their way (one group)
+  auto fetch = [&](int ch) {
+    if (ch < nch) {
+      const int a0 = a_beg + ch * SG_CHUNK, na = min(SG_CHUNK, a_end - a0);
+      float4 *B = Bs[ch % 3];
+      for (int e = threadIdx.x; e < SG_CHUNK * (kcm + 1); e += SG_THREADS) {
+        const int k = e / SG_CHUNK, a = e - k * SG_CHUNK;
+        float2 *dst = reinterpret_cast<float2 *>(B + a * bst + ((k >> 1) & 1) * ng + (k >> 2)) + (k & 1);
+        if (a < na) cp_async8(dst, btab + (size_t)k * nq + a0 + a);
+        else *dst = make_float2(0.f, 0.f);
+      }
+      if (threadIdx.x < SG_CHUNK) {
+        uint2 *dst = reinterpret_cast<uint2 *>(&M.us[ch % 3][threadIdx.x]);
+        if ((int)threadIdx.x < na) {
+          const uint2 *src = reinterpret_cast<const uint2 *>(kfrac + a0 + threadIdx.x);
+          cp_async8(dst, src);
+          cp_async8(dst + 1, src + 1);
+        } else {
+          dst[0] = dst[1] = make_uint2(0u, 0u);
+        }
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // (tq cos phi, tq sin phi) of the block's rows for chunk ch
+  auto form = [&](int ch) {
+    for (int a = warp; a < SG_CHUNK; a += SG_THREADS / 32) {
+      const uint4 u = M.us[ch % 3][a];
+      const float tq = __uint_as_float(u.w);
+      float *A = reinterpret_cast<float *>(M.As[ch & 1][a]);
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int2 row = h ? r1 : r0;
+        float sn, cs;
+        phase_cs((unsigned)row.x * u.x + (unsigned)row.y * u.y, cs, sn);
+        A[h * 32 + lane] = tq * cs;
+        A[64 + h * 32 + lane] = tq * sn;
+      }
+    }
+  };
+  float2 acc[SG_TR / 2][SG_TK][4];                   // row pairs: Pc, Ps, Qc, Qs
+#pragma unroll
+  for (int r = 0; r < SG_TR / 2; r++)
+#pragma unroll
+    for (int k = 0; k < SG_TK; k++)
+#pragma unroll
+      for (int m = 0; m < 4; m++) acc[r][k][m] = make_float2(0.f, 0.f);
+  // (kc above kcm in the last group are never written: zero them once)
+  for (int b = 0; b < 3; b++)
+    for (int e = threadIdx.x; e < SG_CHUNK * (ng * SG_TK - kcm - 1); e += SG_THREADS) {
+      const int k = kcm + 1 + e / SG_CHUNK, a = e % SG_CHUNK;
+      reinterpret_cast<float2 *>(Bs[b] + a * bst + ((k >> 1) & 1) * ng + (k >> 2))[k & 1] = make_float2(0.f, 0.f);
+    }
+  fetch(0);
+  fetch(1);
+  asm volatile("cp.async.wait_group 1;" ::: "memory");
+  __syncthreads();
+  form(0);
+  for (int ch = 0; ch < nch; ch++) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                                 // chunk ch is formed, ch + 1 fetched, ch - 1 no longer read
+    fetch(ch + 2);
+    if (ch + 1 < nch) form(ch + 1);
+    if (work) {
+      const float4(*A)[4][SG_ROWS / SG_TR] = M.As[ch & 1];
+      const float4 *B = Bs[ch % 3];
+#pragma unroll 2
+      for (int a = slice; a < SG_CHUNK; a += nslice) {
+        const float4 p0 = A[a][0][rg], p1 = A[a][1][rg], q0 = A[a][2][rg], q1 = A[a][3][rg];
+        const float4 b0 = B[a * bst + kg], b1 = B[a * bst + ng + kg];
+        const float2 P[4] = {make_float2(p0.x, p0.y), make_float2(p0.z, p0.w), make_float2(p1.x, p1.y),
+                             make_float2(p1.z, p1.w)};
+        const float2 Q[4] = {make_float2(q0.x, q0.y), make_float2(q0.z, q0.w), make_float2(q1.x, q1.y),
+                             make_float2(q1.z, q1.w)};
+        const float C[4] = {b0.x, b0.z, b1.x, b1.z}, S[4] = {b0.y, b0.w, b1.y, b1.w};
+#pragma unroll
+        for (int k = 0; k < SG_TK; k++) {
+          const float2 c2 = make_float2(C[k], C[k]), s2 = make_float2(S[k], S[k]);
+#pragma unroll
+          for (int r = 0; r < SG_TR / 2; r++) {
+            acc[r][k][0] = __ffma2_rn(P[r], c2, acc[r][k][0]);
+            acc[r][k][1] = __ffma2_rn(P[r], s2, acc[r][k][1]);
+            acc[r][k][2] = __ffma2_rn(Q[r], c2, acc[r][k][2]);
+            acc[r][k][3] = __ffma2_rn(Q[r], s2, acc[r][k][3]);
+          }
+        }
+      }
+    }
+  }
+  // the slices in FP64, in order, one kc of the thread's at a time; then
+  // S(+-kc) = (Pc -+ Qs) + i (Qc +- Ps)
+  float *red = reinterpret_cast<float *>(M.As);      // [slice][tile][row of the group][4]
+  for (int k = 0; k < SG_TK; k++) {
+    __syncthreads();
+    if (work) {
+#pragma unroll
+      for (int kk = 0; kk < SG_TK; kk++)
+        if (kk == k) {
+#pragma unroll
+          for (int r = 0; r < SG_TR; r++)
+#pragma unroll
+            for (int m = 0; m < 4; m++)
+              red[((slice * ntile + tile) * SG_TR + r) * 4 + m] = (r & 1) ? acc[r / 2][kk][m].y : acc[r / 2][kk][m].x;
+        }
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < ntile * SG_TR; e += SG_THREADS) {
+      const int tl = e / SG_TR, r = e - tl * SG_TR;
+      const int g = tl / ng, kc = (tl - g * ng) * SG_TK + k;
+      const int4 row = M.row[g * SG_TR + r];
+      const int kp = kc - row.x, km = -kc - row.x;   // places of +kc and -kc in the row
+      const bool inp = kp >= 0 && kp < row.y, inm = kc > 0 && km >= 0 && km < row.y;
+      if (!inp && !inm) continue;
+      double v[4] = {0., 0., 0., 0.};
+      for (int sl = 0; sl < nslice; sl++) {
+        const float4 x = reinterpret_cast<const float4 *>(red)[(sl * ntile + tl) * SG_TR + r];
+        v[0] += x.x;
+        v[1] += x.y;
+        v[2] += x.z;
+        v[3] += x.w;
+      }
+      double2 *out = spart + (size_t)blockIdx.x * ktot + row.z;
+      if (inp) out[kp] = make_double2(v[0] - v[3], v[2] + v[1]);
+      if (inm) out[km] = make_double2(v[0] + v[3], v[2] - v[1]);
+    }
+  }
+}
+
+// k_sred over many tiles: 32 k per block, eight threads each over the tiles
+__global__ void __launch_bounds__(256) k_sred_tiles(int ktot, int ntiles, const double2 *__restrict__ spart,
+                                                    double2 *__restrict__ sk, const int *__restrict__ gs) {
+  if (gated_off(gs, 0)) return;
+  __shared__ double2 part[8][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int k = blockIdx.x * 32 + lane;
+  double sr = 0, si = 0;
+  if (k < ktot) {
+#pragma unroll 4
+    for (int t = w; t < ntiles; t += 8) {
+      const double2 p = spart[(size_t)t * ktot + k];
+      sr += p.x;
+      si += p.y;
+    }
+  }
+  part[w][lane] = make_double2(sr, si);
+  __syncthreads();
+  if (w == 0 && k < ktot) {
+    for (int v = 1; v < 8; v++) {
+      sr += part[v][lane].x;
+      si += part[v][lane].y;
+    }
+    sk[k] = make_double2(sr, si);
+  }
+}
+
+// The force kernel's coefficients, once per step: entry e is (row, kc >= 0)
+// with kidx[e] = {k of +kc, k of -kc} (-1: not in the set).  With A(+kc) = (a,
+// b), A(-kc) = (a', b'): p = a + a', q = b - b', s = a - a', t = b + b'.
+__global__ void k_kcoef(int nent, const int2 *__restrict__ kidx, const float2 *__restrict__ akf,
+                        float4 *__restrict__ coef, const int *__restrict__ gs) {
+  if (gated_off(gs, 0)) return;
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= nent) return;
+  const int2 k = kidx[e];
+  const float2 z = make_float2(0.f, 0.f);
+  const float2 ap = k.x >= 0 ? akf[k.x] : z, am = k.y >= 0 ? akf[k.y] : z;
+  coef[e] = make_float4(ap.x + am.x, ap.y - am.y, ap.x - am.x, ap.y + am.y);
+}
+
+// Forces of KR_A atoms per thread over the rows of one split.  A row
+// contributes
+//   W0 = sin phi sum (p c + q s_) + cos phi sum (s s_ - t c)
+//   W1 = sin phi sum kc (s c + t s_) + cos phi sum kc (p s_ - q c)
+// (c, s_: cos, sin kc theta), summed in FP32 within the row and in FP64 over
+// rows, as k_kforce_mixed does.  hdr: per row {ka, kb, largest |kc|, first
+// entry}; a split's headers and coefficients are copied to shared memory.
+template <int KM>
+__global__ void __launch_bounds__(KR_THREADS) k_kforce_reg(
+    int nq, const uint4 *__restrict__ kfrac, const float2 *__restrict__ btab, const int *__restrict__ split_row,
+    const int4 *__restrict__ ghdr, const float4 *__restrict__ gcoef, int cap, const double *__restrict__ hmati,
+    double *__restrict__ part, const int *__restrict__ gs) {
+  if (gated_off(gs, 0)) return;
+  extern __shared__ float4 coef[];                   // cap coefficients, then the headers
+  int4 *hdr = reinterpret_cast<int4 *>(coef + cap);
+  const int r0 = split_row[blockIdx.y], nr = split_row[blockIdx.y + 1] - r0;
+  for (int r = threadIdx.x; r < nr; r += KR_THREADS) hdr[r] = ghdr[r0 + r];
+  {
+    const int e0 = ghdr[r0].w, e1 = ghdr[r0 + nr].w;   // (one header past the last row)
+    for (int e = threadIdx.x; e < e1 - e0; e += KR_THREADS) coef[e] = gcoef[e0 + e];
+  }
+  const int e_first = ghdr[r0].w;
+  const int a0 = blockIdx.x * (KR_THREADS * KR_A) + threadIdx.x;
+  unsigned u0[KR_A], u1[KR_A];
+  float tq[KR_A];
+  float2 c[KM][KR_A / 2], sv[KM][KR_A / 2];          // kc = 1 .. KM, atoms in pairs
+  double U0[KR_A], U1[KR_A], U2[KR_A];
+#pragma unroll
+  for (int m = 0; m < KR_A; m++) {
+    const int j = a0 + m * KR_THREADS;
+    const uint4 u = j < nq ? kfrac[j] : make_uint4(0, 0, 0, 0);
+    u0[m] = u.x;
+    u1[m] = u.y;
+    tq[m] = __uint_as_float(u.w);
+    U0[m] = U1[m] = U2[m] = 0.0;
+#pragma unroll
+    for (int k = 0; k < KM; k++) {
+      const float2 b = j < nq ? btab[(size_t)(k + 1) * nq + j] : make_float2(0.f, 0.f);
+      if (m & 1) {
+        c[k][m / 2].y = b.x;
+        sv[k][m / 2].y = b.y;
+      } else {
+        c[k][m / 2].x = b.x;
+        sv[k][m / 2].x = b.y;
+      }
+    }
+  }
+  __syncthreads();
+  {
+    for (int r = 0; r < nr; r++) {
+      const int4 h = hdr[r];
+      const float4 *cf = coef + (h.w - e_first);
+      float2 X0[KR_A / 2], Y0[KR_A / 2], X1[KR_A / 2], Y1[KR_A / 2];
+      // kc in pairs (a row's entries are padded to one and an even number with
+      // zeros), the next pair's coefficients loaded a pair ahead; the last
+      // row's may be read past its end, not used
+      float4 g0 = cf[1], g1 = cf[2];
+      {
+        const float4 f = cf[0];
+#pragma unroll
+        for (int m = 0; m < KR_A / 2; m++) {
+          X0[m] = make_float2(f.x, f.x);
+          Y0[m] = make_float2(-f.w, -f.w);
+          X1[m] = Y1[m] = make_float2(0.f, 0.f);
+        }
+      }
+#pragma unroll
+      for (int k2 = 0; k2 < KM; k2 += 2) {
+        if (k2 >= h.z) break;
+        const float4 f2[2] = {g0, g1};
+        g0 = cf[k2 + 3];
+        g1 = cf[k2 + 4];
+#pragma unroll
+        for (int w = 0; w < 2; w++) {
+          const int k = k2 + w;
+          const float4 f = f2[w];
+          const float2 p = make_float2(f.x, f.x), q = make_float2(f.y, f.y), s = make_float2(f.z, f.z),
+                       t = make_float2(f.w, f.w), nq2 = make_float2(-f.y, -f.y), nt = make_float2(-f.w, -f.w);
+          const float2 kc2 = make_float2((float)(k + 1), (float)(k + 1));
+#pragma unroll
+          for (int m = 0; m < KR_A / 2; m++) {
+            X0[m] = __ffma2_rn(p, c[k][m], X0[m]);
+            Y0[m] = __ffma2_rn(s, sv[k][m], Y0[m]);
+            const float2 x1 = __fmul2_rn(s, c[k][m]), y1 = __fmul2_rn(p, sv[k][m]);
+            X0[m] = __ffma2_rn(q, sv[k][m], X0[m]);
+            Y0[m] = __ffma2_rn(nt, c[k][m], Y0[m]);
+            X1[m] = __ffma2_rn(kc2, __ffma2_rn(t, sv[k][m], x1), X1[m]);
+            Y1[m] = __ffma2_rn(kc2, __ffma2_rn(nq2, c[k][m], y1), Y1[m]);
+          }
+        }
+      }
+#pragma unroll
+      for (int m = 0; m < KR_A; m++) {
+        float sn, cs;
+        phase_cs((unsigned)h.x * u0[m] + (unsigned)h.y * u1[m], cs, sn);
+        const float x0 = (m & 1) ? X0[m / 2].y : X0[m / 2].x, y0 = (m & 1) ? Y0[m / 2].y : Y0[m / 2].x;
+        const float x1 = (m & 1) ? X1[m / 2].y : X1[m / 2].x, y1 = (m & 1) ? Y1[m / 2].y : Y1[m / 2].x;
+        const double W0 = (double)fmaf(sn, x0, cs * y0), W1 = (double)fmaf(sn, x1, cs * y1);
+        U0[m] = fma((double)h.x, W0, U0[m]);
+        U1[m] = fma((double)h.y, W0, U1[m]);
+        U2[m] += W1;
+      }
+    }
+  }
+  const double TPI = 2.0 * M_PI;
+#pragma unroll
+  for (int m = 0; m < KR_A; m++) {
+    const int j = a0 + m * KR_THREADS;
+    if (j >= nq) continue;
+    // F = tq 2 pi H^-T U  (k = 2 pi H^-T n, md_ewald.c:248-251)
+    const double t = TPI * (double)tq[m];
+    const size_t o = (size_t)3 * blockIdx.y * nq + j;
+    part[o] = t * (hmati[0] * U0[m] + hmati[3] * U1[m] + hmati[6] * U2[m]);
+    part[o + nq] = t * (hmati[1] * U0[m] + hmati[4] * U1[m] + hmati[7] * U2[m]);
+    part[o + 2 * (size_t)nq] = t * (hmati[2] * U0[m] + hmati[5] * U1[m] + hmati[8] * U2[m]);
   }
 }
 
@@ -477,10 +902,10 @@ __global__ void k_kforce_sum(int nq, int nsplit, const double *__restrict__ part
   double fx = 0, fy = 0, fz = 0;
 #pragma unroll 8
   for (int y = 0; y < nsplit; y++) {
-    const size_t o = ((size_t)y * nq + jq) * 3;
+    const size_t o = (size_t)3 * y * nq + jq;
     fx += part[o];
-    fy += part[o + 1];
-    fz += part[o + 2];
+    fy += part[o + nq];
+    fz += part[o + 2 * (size_t)nq];
   }
   fxl[i] = f0 + fx;
   fxl[n + i] = f1 + fy;
@@ -593,6 +1018,137 @@ __global__ void k_kforce_plain(int nq, const double4 *__restrict__ kp, const int
 }
 
 // ------------------------------------------------------------------ host
+// The large-sum kernels' layout, where they apply: at least KR_MIN_SUM atoms x
+// k-vectors (below that the sums take microseconds and the older kernels, with
+// their smaller tiles, are as fast: 24,000 charges x 1526 k 28 + 24 us) and rows of
+// |kc| up to KR_MAX.
+constexpr double KR_MIN_SUM = 5e7;
+static int kr_km(int kcm) { return kcm <= 8 ? 8 : kcm <= 12 ? 12 : kcm <= 16 ? 16 : KR_MAX; }
+static int kspace_reg_setup(Ctx *c, const std::vector<int4> &rows) {
+  int kcm = 0;
+  auto top = [](const int4 &r) { return std::max(std::abs(r.z), std::abs(r.z + r.w - 1)); };
+  for (const int4 &r : rows) kcm = std::max(kcm, top(r));
+  if ((double)c->ncharge * c->ktot < KR_MIN_SUM || kcm > KR_MAX || kcm < 1) return CM3D_NB_OK;
+  const int nr = (int)rows.size();
+  std::vector<int> perm((size_t)nr);
+  for (int r = 0; r < nr; r++) perm[(size_t)r] = r;
+  std::stable_sort(perm.begin(), perm.end(), [&](int a, int b) { return top(rows[(size_t)a]) > top(rows[(size_t)b]); });
+  // structure factors: atom ranges of at most SG_ATOMS, small enough for
+  // three blocks per SM
+  const int ry = (nr + SG_ROWS - 1) / SG_ROWS;
+  int per = SG_ATOMS;
+  while (per > 2 * SG_CHUNK && (long long)((c->ncharge + per - 1) / per) * ry < 3LL * c->num_sms) per /= 2;
+  c->kr_atoms = per;
+  c->kr_tiles = (c->ncharge + per - 1) / per;
+  // forces: the rows in splits of similar numbers of coefficients, each within
+  // 48 KB of shared memory, enough of them for four blocks per SM
+  const int ft = (c->ncharge + KR_THREADS * KR_A - 1) / (KR_THREADS * KR_A);
+  long long total = 0;
+  auto entries = [&](const int4 &r) { return 1 + (top(r) + 1) / 2 * 2; };
+  for (const int4 &r : rows) total += entries(r);
+  const long long cap = 36 * 1024 / (long long)sizeof(float4);   // (+ headers: 48 KB)
+  long long want = std::max<long long>((total + cap - 1) / cap, (4LL * c->num_sms + ft - 1) / ft);
+  want = std::min<long long>(want, nr);
+  std::vector<int> sr(1, 0);
+  long long run = 0, most = 0;
+  for (int r = 0; r < nr; r++) {
+    const long long e = entries(rows[(size_t)r]);
+    if (run > 0 && (run + e > cap || run * want >= total || r - sr.back() >= 512)) {
+      sr.push_back(r);
+      most = std::max(most, run);
+      run = 0;
+    }
+    run += e;
+  }
+  most = std::max(most, run);
+  sr.push_back(nr);
+  c->kf_split = (int)sr.size() - 1;
+  // each row's header and coefficient entries, and the entries' k
+  std::vector<int4> hdr;
+  std::vector<int2> kidx;
+  int rows_most = 0, k0 = 0;
+  for (int r = 0; r < nr; r++) {
+    const int4 w = rows[(size_t)r];
+    hdr.push_back(make_int4(w.x, w.y, top(w), (int)kidx.size()));
+    for (int kc = 0; kc < entries(w); kc++) {
+      const int kp = kc - w.z, km = -kc - w.z;
+      kidx.push_back(make_int2(kp >= 0 && kp < w.w ? k0 + kp : -1, kc > 0 && km >= 0 && km < w.w ? k0 + km : -1));
+    }
+    k0 += w.w;
+  }
+  hdr.push_back(make_int4(0, 0, 0, (int)kidx.size()));
+  for (int s = 0; s < c->kf_split; s++) rows_most = std::max(rows_most, sr[(size_t)s + 1] - sr[(size_t)s]);
+  c->kr_cap = (int)most + 4;
+  c->kf_smem = (size_t)c->kr_cap * sizeof(float4) + (size_t)rows_most * sizeof(int4);
+  c->kr_nent = (int)kidx.size();
+  CK(cudaMalloc(&c->kr_hdr, sizeof(int4) * hdr.size()));
+  CK(cudaMemcpy(c->kr_hdr, hdr.data(), sizeof(int4) * hdr.size(), cudaMemcpyHostToDevice));
+  CK(cudaMalloc(&c->kr_kidx, sizeof(int2) * kidx.size()));
+  CK(cudaMemcpy(c->kr_kidx, kidx.data(), sizeof(int2) * kidx.size(), cudaMemcpyHostToDevice));
+  CK(cudaMalloc(&c->kr_coef, sizeof(float4) * kidx.size()));
+  c->kr_kcm = kcm;
+  CK(cudaMalloc(&c->kr_perm, sizeof(int) * perm.size()));
+  CK(cudaMemcpy(c->kr_perm, perm.data(), sizeof(int) * perm.size(), cudaMemcpyHostToDevice));
+  CK(cudaMalloc(&c->kr_split, sizeof(int) * sr.size()));
+  CK(cudaMemcpy(c->kr_split, sr.data(), sizeof(int) * sr.size(), cudaMemcpyHostToDevice));
+  // (rows above kcm, up to the force kernel's register count, stay zero)
+  const size_t bt = sizeof(float2) * (size_t)(kr_km(kcm) + 1) * (size_t)c->ncharge;
+  CK(cudaMalloc(&c->kr_btab, bt));
+  CK(cudaMemset(c->kr_btab, 0, bt));
+  cudaFree(c->spart);
+  c->spart = nullptr;
+  CK(cudaMalloc(&c->spart, sizeof(double2) * (size_t)c->kr_tiles * (size_t)c->ktot));
+  CK(cudaMalloc(&c->kf_part, sizeof(double) * 3 * ((size_t)c->kf_split + 1) * c->ncharge));
+  CK(cudaMemset(c->kf_part, 0, sizeof(double) * 3 * ((size_t)c->kf_split + 1) * c->ncharge));
+  c->kr_on = true;
+  return CM3D_NB_OK;
+}
+
+template <int KM>
+static void launch_kforce_reg(Ctx *c, cudaStream_t st) {
+  const dim3 g((c->ncharge + KR_THREADS * KR_A - 1) / (KR_THREADS * KR_A), c->kf_split);
+  k_kforce_reg<KM><<<g, KR_THREADS, c->kf_smem, st>>>(c->ncharge, c->kfrac, c->kr_btab, c->kr_split, c->kr_hdr,
+                                                      c->kr_coef, c->kr_cap, c->acc + ACC_COUNT, c->kf_part, c->gate);
+}
+
+// force(1)'s k-space with the large-sum kernels; the forces stay in the
+// partials unless they are to be added here (!defer)
+static int kspace_run_reg(Ctx *c, cudaStream_t st, bool defer, double vol) {
+  const double *dhmati = c->acc + ACC_COUNT;
+  const int nq = c->ncharge;
+  cudaEvent_t e0;
+  tbegin(c, 1, &e0);
+  k_kprep_reg<<<dim3(grid_for(nq, 128), 4), 128, 0, st>>>(nq, c->kr_kcm, c->icharge, c->n, c->pos, c->q, dhmati, c->kfrac,
+                                                          c->kr_btab, c->gate);
+  const size_t bsm = sizeof(SgSmem) + 3 * sizeof(float4) * SG_CHUNK * (size_t)(2 * (c->kr_kcm / SG_TK + 1) + 1);
+  static unsigned long long attr_devs = 0;
+  if (c->dev < 64 && !(attr_devs & (1ull << c->dev))) {
+    CK(cudaFuncSetAttribute(k_sfac_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, 120 * 1024));
+    attr_devs |= 1ull << c->dev;
+  }
+  k_sfac_gemm<<<dim3(c->kr_tiles, (c->nrows + SG_ROWS - 1) / SG_ROWS), SG_THREADS, bsm, st>>>(
+      nq, c->kr_atoms, c->kfrac, c->kr_btab, c->nrows, c->rows, c->row_k0, c->kr_perm, c->ktot, c->spart, c->gate);
+  k_sred_tiles<<<(c->ktot + 31) / 32, 256, 0, st>>>(c->ktot, c->kr_tiles, c->spart, c->sk, c->gate);
+  k_sred<false><<<std::min(grid_for(c->ktot, 64), c->num_sms * 4), 64, 0, st>>>(
+      c->ktot, 1, c->sk, c->ka_d, c->kb_d, c->kc_d, dhmati, 1.0 / vol, c->falp2, c->sk, c->akf, nullptr, c->acc, nullptr,
+      nullptr, c->gate);
+  k_kcoef<<<grid_for(c->kr_nent, 128), 128, 0, st>>>(c->kr_nent, c->kr_kidx, c->akf, c->kr_coef, c->gate);
+  switch (kr_km(c->kr_kcm)) {
+    case 8: launch_kforce_reg<8>(c, st); break;
+    case 12: launch_kforce_reg<12>(c, st); break;
+    case 16: launch_kforce_reg<16>(c, st); break;
+    default: launch_kforce_reg<KR_MAX>(c, st);
+  }
+  c->launches += 6;
+  if (!defer) {
+    k_kforce_sum<<<grid_for(nq, 256), 256, 0, st>>>(nq, c->kf_split, c->kf_part, c->icharge, c->n, c->fxl, c->gate);
+    c->launches++;
+  }
+  tend(c, 1, e0);
+  CKL(c);
+  return CM3D_NB_OK;
+}
+
 // k rows, tiles and partial-S(k) layout of every system (SysP fields q0 ..
 // spart0), all systems' rows / k-vectors concatenated
 int kspace_setup(Ctx *c) {
@@ -671,6 +1227,11 @@ int kspace_setup(Ctx *c) {
     CK(cudaMalloc(&c->akd, sizeof(double2) * (size_t)c->ktot));
   }
   CK(cudaMalloc(&c->kposd, sizeof(double4) * (size_t)c->ncharge));
+  if (mixed && c->nsys == 1) {
+    int rc2 = kspace_reg_setup(c, rows);
+    if (rc2) return rc2;
+    if (c->kr_on) return CM3D_NB_OK;
+  }
   // split the rows over enough blocks to fill the machine in the force pass
   int split = 1;
   while ((long long)c->ftiles_tot * split < (long long)c->num_sms * 4 && split < nrows_max) split *= 2;
@@ -770,6 +1331,7 @@ static int kspace_run(Ctx *c, cudaStream_t st, bool defer) {
   double vol = c->hmat[0] * (c->hmat[4] * c->hmat[8] - c->hmat[5] * c->hmat[7]) +
                c->hmat[1] * (c->hmat[5] * c->hmat[6] - c->hmat[3] * c->hmat[8]) +
                c->hmat[2] * (c->hmat[3] * c->hmat[7] - c->hmat[4] * c->hmat[6]);
+  if (c->kr_on) return kspace_run_reg(c, st, defer, vol);
   cudaEvent_t e0;
   tbegin(c, 1, &e0);
   const bool mixed = c->mode == CM3D_NB_MIXED;

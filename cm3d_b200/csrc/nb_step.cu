@@ -412,8 +412,8 @@ __device__ __forceinline__ void mol_bond(Mol3 &M, int i, int j, double2 par) {
   double x[3];
 #pragma unroll
   for (int d = 0; d < 3; d++) x[d] = pick(M.p, i, d) - pick(M.p, j, d);
-  const double r = sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]);
-  const double fr = par.y * (r - par.x) / r;
+  const double r2 = x[0] * x[0] + x[1] * x[1] + x[2] * x[2], ri = rsqrt(r2);
+  const double fr = par.y * (r2 * ri - par.x) * ri;
 #pragma unroll
   for (int d = 0; d < 3; d++) {
     add_to(M.f, i, d, -(x[d] * fr));
@@ -431,16 +431,18 @@ __device__ __forceinline__ void mol_bend(Mol3 &M, int i, int j, int k, double2 p
   }
   const double al = a[0] * a[0] + a[1] * a[1] + a[2] * a[2];
   const double bl = b[0] * b[0] + b[1] * b[1] + b[2] * b[2];
-  const double r11 = 1. / sqrt(al * bl), costh = (a[0] * b[0] + a[1] * b[1] + a[2] * b[2]) * r11;
+  const double r11 = rsqrt(al * bl), costh = (a[0] * b[0] + a[1] * b[1] + a[2] * b[2]) * r11;
   double dudth = 0., dthdcos = -1.;
   if (fabs(costh) < 1.) {
     dudth = par.y * (acos(costh) - par.x);
-    dthdcos = -1. / sqrt(1. - costh * costh);
+    dthdcos = -rsqrt(1. - costh * costh);
   }
   const double dudcos = dudth * dthdcos;
+  // cos / |a|^2 = (a.b) r11 / |a|^2 and cos / |b|^2: r11^2 = 1 / (|a|^2 |b|^2)
+  const double ca = costh * r11 * r11 * bl, cb = costh * r11 * r11 * al;
 #pragma unroll
   for (int d = 0; d < 3; d++) {
-    const double d1 = costh * a[d] / al - b[d] * r11, d3 = costh * b[d] / bl - a[d] * r11;
+    const double d1 = ca * a[d] - b[d] * r11, d3 = cb * b[d] - a[d] * r11;
     add_to(M.f, i, d, dudcos * d1);
     add_to(M.f, j, d, dudcos * (-d1 - d3));
     add_to(M.f, k, d, dudcos * d3);
@@ -881,7 +883,7 @@ __global__ void k_group_init(StepP P, const int *__restrict__ gwork, int ngw, co
 __global__ void __launch_bounds__(128) k_group_small(
     StepP P, const int *__restrict__ gwork, int ngw, const int *__restrict__ gaoff, const int *__restrict__ gatoms,
     const double *__restrict__ pos, const double *__restrict__ q, double *__restrict__ fxl, double *__restrict__ part,
-    const int *__restrict__ qidx, const int *__restrict__ gcoff, const int2 *__restrict__ cij,
+    int nq, const int *__restrict__ qidx, const int *__restrict__ gcoff, const int2 *__restrict__ cij,
     const int *__restrict__ gboff, const int4 *__restrict__ bij, const double2 *__restrict__ bp,
     const int *__restrict__ geoff, const int4 *__restrict__ eijk, const double2 *__restrict__ ep,
     double *__restrict__ acc, const SysP *__restrict__ sp, const int *__restrict__ sys_of,
@@ -995,7 +997,7 @@ __global__ void __launch_bounds__(128) k_group_small(
 #pragma unroll
       for (int d = 0; d < 3; d++) {
         if (!part) fxl[d * n + id[a]] += f[a][d];
-        else if (jq >= 0) part[(size_t)3 * jq + d] = f[a][d];
+        else if (jq >= 0) part[(size_t)d * nq + jq] = f[a][d];
       }
     }
   }
@@ -1630,7 +1632,7 @@ int group_terms(Ctx *c, cudaStream_t st, double *part) {
   if (c->small_mol == 3) {
     const int B = c->ngwork < 128 * c->num_sms ? 32 : 128;
     k_group_small<<<grid_for(c->ngwork, B), B, 0, st>>>(P, c->grp_work, c->ngwork, c->grp_atom_off, c->grp_atoms,
-                                                        c->pos, c->q, c->fxl, part, c->qidx, c->grp_ecorr_off,
+                                                        c->pos, c->q, c->fxl, part, c->ncharge, c->qidx, c->grp_ecorr_off,
                                                         c->ecorr_ij, c->grp_bond_off, c->bond_ij, c->bond_p,
                                                         c->grp_bend_off, c->bend_ijk, c->bend_p, c->acc, c->sp,
                                                         c->sys_of, c->gate);
