@@ -95,7 +95,7 @@ static void destroy(Ctx *c) {
                   c->fxr, c->intra_buf, c->ithm, c->nhc, c->cwl, c->cwn, c->cw_tf, c->cw_tg, c->cw_tl,
                   c->cw_part, c->nvt_kin, c->nvt_chsum, c->th_atoms, c->th_choff, c->th_chunk,
                   c->cw_sys, c->cw_sitems, c->cw_items, c->cw_gidx, c->cw_scan, c->grp_work, c->smeta, c->xspan, c->qidx,
-                  c->kr_perm, c->kr_split, c->kr_btab, c->kr_hdr, c->kr_kidx, c->kr_coef};
+                  c->rad_cm, c->rad, c->dxi, c->kr_perm, c->kr_split, c->kr_btab, c->kr_hdr, c->kr_kidx, c->kr_coef};
   cw_destroy(c);
   for (void *p : ptrs)
     if (p) cudaFree(p);
@@ -163,8 +163,48 @@ static void box_widths(SysP &P, const SysH &H) {
   for (int d = 0; d < 3; d++) {
     const double w = box_width(H, d);
     if (w < 2.0 * H.rlist) P.smallbox = 1;
-    P.near_s[d] = 0.5 - 1.01 * H.skin / w - 1e-6;
+    P.near_s[d] = 0.5 - 1.01 * (H.skin + H.extra) / w - 1e-6;
   }
+}
+
+// How far the engine's own lists reach beyond CM3D's.  nrefsh's schedule --
+// RESETPOS, the snapshot, its counters -- is CM3D's, by CM3D's skin; a list
+// only has to hold every pair within the cut-offs until it is built again, and
+// with a thin skin (0.5 A in the water decks: a rebuild every two steps) the
+// build costs several times the pairs of a thicker shell.  The lists therefore
+// take a skin of LIST_SKIN of the largest cut-off, if that is more than CM3D's,
+// and are built when an atom has moved half of it (dxi) -- checked every step
+// beside nrefsh's own test.  Not where the wider radius would take the grid
+// below 3 cells per axis or the box below two list radii, nor where the list
+// radii given are not the cut-offs plus the skin.  (us per step, list skins of
+// 0.5 -- CM3D's own --, 1, 1.5, 2 and 2.5 A: 12,288 water atoms 235, 181, 162,
+// 161, 207; 37 boxes of 27,000 atoms 221, -, 210, 188, 217.  331,776 water
+// atoms with CM3D's 1.5 A, 4.80 ms; 2 A, 4.53; 2.5 A, 5.13.)
+constexpr double LIST_SKIN = 0.2;
+static double list_skin(const SysH &H, double rc_max, bool consistent, double cell_scale) {
+  double extra = LIST_SKIN * rc_max - H.skin;
+  if (!consistent || !(H.skin > 0.0) || !(extra > 0.0)) return 0.0;
+  for (int d = 0; d < 3; d++) {
+    const double w = box_width(H, d);
+    if (floor(w / (H.rlist_cm * cell_scale)) >= 3) extra = std::min(extra, (1.0 - 1e-9) * w / (3.0 * cell_scale) - H.rlist_cm);
+    if (w >= 2.0 * H.rlist_cm) extra = std::min(extra, (1.0 - 1e-9) * 0.5 * w - H.rlist_cm);
+  }
+  return extra > 0.01 * rc_max ? extra : 0.0;
+}
+
+// the squared list radius `extra` beyond one of CM3D's
+static double widened(double r2, double extra) {
+  if (!(extra > 0.0) || r2 < 0.0) return r2;
+  const double r = sqrt(r2) + extra;
+  return r * r;
+}
+
+// the list radii and skin of a system's own lists from its `extra`
+static void list_radii(SysP &P, SysH &H) {
+  H.rlist = H.rlist_cm + H.extra;
+  P.rmaxl_list2_e = widened(P.rmaxl_skin2_e, H.extra);
+  P.rmaxs_list2_e = widened(P.rmaxs_skin2_e, H.extra);
+  P.listq = H.extra > 0.0 ? .25 * (H.skin + H.extra) * (H.skin + H.extra) : -1.0;
 }
 
 static int create(const cm3d_nb_system *systems, int nsys, const cm3d_nb_options *opt, Ctx **out) {
@@ -271,7 +311,8 @@ static int create(const cm3d_nb_system *systems, int nsys, const cm3d_nb_options
   const size_t n3 = 3 * (size_t)n;
   std::vector<double> pos(n3), vel(n3), mass(n), q(n);
   std::vector<int> itype(n), sys_of(n), map, ich, eoff(n + 1, 0), eidx, coff(n + 1, 0), cidx;
-  std::vector<double> vtab, dvtab, swt, icut, coultab, dcoultab, switchse;
+  std::vector<double> vtab, dvtab, swt, icut, coultab, dcoultab, switchse, rad_cm, rad;
+  bool any_extra = false;
   int a0 = 0, inter0 = 0, ncoul = 0;
   for (int sy = 0; sy < nsys; sy++) {
     const cm3d_nb_system *s = systems + sy;
@@ -338,7 +379,10 @@ static int create(const cm3d_nb_system *systems, int nsys, const cm3d_nb_options
     P.inter0 = inter0;
     P.ninter = s->ninter;
     for (int k = 0; k < s->ntypes * s->ntypes; k++) map.push_back(s->map[k] >= 0 ? inter0 + s->map[k] : -1);
-    double r2 = 0;
+    double r2 = 0, rc2 = 0;
+    // the lists' radii are the cut-offs plus the skin
+    bool consistent = true;
+    auto covers = [&](double skin2, double cut2) { return sqrt(skin2) >= sqrt(cut2) + s->skin_ter - 1e-9; };
     for (int in = 0; in < s->ninter; in++) {
       icut.push_back(s->rmaxs_cut2[in]);
       icut.push_back(s->rmins_cut2[in]);
@@ -349,6 +393,8 @@ static int create(const cm3d_nb_system *systems, int nsys, const cm3d_nb_options
       icut.push_back(s->dx2tab[in]);
       icut.push_back(s->vtab[(size_t)in * nt + nt - 4]);
       r2 = std::max(r2, s->rmaxl_skin2[in]);
+      rc2 = std::max(rc2, s->rmaxl_cut2[in]);
+      consistent = consistent && covers(s->rmaxl_skin2[in], s->rmaxl_cut2[in]) && covers(s->rmaxs_skin2[in], s->rmaxs_cut2[in]);
       for (int k = 0; k < nt; k++) {
         vtab.push_back(s->vtab[(size_t)in * nt + k]);
         dvtab.push_back(s->dvtab[(size_t)in * nt + k]);
@@ -374,6 +420,8 @@ static int create(const cm3d_nb_system *systems, int nsys, const cm3d_nb_options
       P.offc = (float)(s->rmins_coul2 * s->dx2coul);
       P.tablast_e = (float)s->coultab[nt - 4];
       r2 = std::max(r2, s->rmaxl_skin2_e);
+      rc2 = std::max(rc2, s->rmaxl_coul2);
+      consistent = consistent && covers(s->rmaxl_skin2_e, s->rmaxl_coul2) && covers(s->rmaxs_skin2_e, s->rmaxs_coul2);
       H.ktot = s->ktot;
       H.ka.assign(s->ka, s->ka + s->ktot);
       H.kb.assign(s->kb, s->kb + s->ktot);
@@ -382,8 +430,17 @@ static int create(const cm3d_nb_system *systems, int nsys, const cm3d_nb_options
       P.coul = -1;
       P.rmaxl_skin2_e = P.rmaxs_skin2_e = -1.0;
     }
-    H.rlist = sqrt(r2);
+    H.rlist_cm = sqrt(r2);
     H.skin = s->skin_ter;
+    H.extra = c->mode == CM3D_NB_MIXED ? list_skin(H, sqrt(rc2), consistent, c->cell_scale) : 0.0;
+    list_radii(P, H);
+    any_extra = any_extra || H.extra > 0.0;
+    for (int in = 0; in < s->ninter; in++) {
+      rad_cm.push_back(s->rmaxs_skin2[in]);
+      rad_cm.push_back(s->rmaxl_skin2[in]);
+      rad.push_back(widened(s->rmaxs_skin2[in], H.extra));
+      rad.push_back(widened(s->rmaxl_skin2[in], H.extra));
+    }
     box_widths(P, H);
     a0 += ns;
   }
@@ -440,6 +497,9 @@ static int create(const cm3d_nb_system *systems, int nsys, const cm3d_nb_options
   if ((rc = upload(&c->dvtab, dvtab.data(), dvtab.size()))) return rc;
   if ((rc = upload(&c->switchs, swt.data(), swt.size()))) return rc;
   if ((rc = upload(&c->icut, icut.data(), icut.size()))) return rc;
+  if ((rc = upload(&c->rad_cm, rad_cm.data(), rad_cm.size()))) return rc;
+  if ((rc = upload(&c->rad, rad.data(), rad.size()))) return rc;
+  if (any_extra && (rc = upload(&c->dxi, pos.data(), n3))) return rc;
   if ((rc = upload(&c->coultab, coultab.data(), coultab.size()))) return rc;
   if ((rc = upload(&c->dcoultab, dcoultab.data(), dcoultab.size()))) return rc;
   if ((rc = upload(&c->switchse, switchse.data(), switchse.size()))) return rc;
@@ -479,7 +539,8 @@ static int create(const cm3d_nb_system *systems, int nsys, const cm3d_nb_options
   if ((rc = upload(&c->acc, acc0.data(), acc0.size()))) return rc;
   if ((rc = upload<long long>(&c->stat, nullptr, ST_COUNT))) return rc;
   if ((rc = upload<int>(&c->istate, nullptr, IS_COUNT))) return rc;
-  if ((rc = upload<int>(&c->sreb, nullptr, (size_t)nsys))) return rc;
+  if ((rc = upload<int>(&c->sreb, nullptr, 2 * (size_t)nsys))) return rc;
+  c->lreb = c->sreb + nsys;
   if ((rc = upload<int>(&c->slast, nullptr, (size_t)nsys))) return rc;
   if ((rc = upload<long long>(&c->sstat, nullptr, (size_t)nsys * SS_COUNT))) return rc;
   CK(cudaMallocHost(&c->h_acc, sizeof(double) * (size_t)nsys * ACC_STRIDE));
@@ -695,12 +756,36 @@ int cm3d_nb_set_box(cm3d_nb_ctx *ctx, const double hmat[9]) {
   }
   if (H.iperd == 3)
     for (int d = 0; d < 3; d++)
-      if (box_width(H, d) / P.nc[d] < H.rlist) {
+      if (box_width(H, d) / H.nc_cm[d] < H.rlist_cm) {
         set_error("set_box: the box shrank below the cell grid (%d cells of width %g < list radius %g along "
                   "direction %d); create a new context for this box",
-                  P.nc[d], box_width(H, d) / P.nc[d], H.rlist, d);
+                  H.nc_cm[d], box_width(H, d) / H.nc_cm[d], H.rlist_cm, d);
         return CM3D_NB_ERR_STATE;
       }
+  // A box that moves: the engine's lists go back to CM3D's radii and schedule
+  // (a list kept longer would meet box changes its skin does not measure),
+  // built from the positions of CM3D's last rebuild in the box as it was.
+  if (c->hs[0].extra > 0.0) {
+    int rc;
+    c->hs[0].extra = 0.0;
+    list_radii(c->h_sp[0], c->hs[0]);
+    box_widths(c->h_sp[0], c->hs[0]);
+    cell_shifts(c->h_sp[0], c->hs[0]);
+    c->rlist_max = c->hs[0].rlist;
+    CK(cudaStreamSynchronize(c->st));
+    CK(cudaMemcpy(c->sp, c->h_sp.data(), sizeof(SysP), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(c->rad, c->rad_cm, sizeof(double) * 2 * (size_t)c->ninter, cudaMemcpyDeviceToDevice));
+    if (c->lists_built) {
+      std::swap(c->pos, c->dxn);
+      c->no_snapshot = true;
+      rc = build_lists(c, false, true);
+      std::swap(c->pos, c->dxn);
+      c->no_snapshot = false;
+      if (rc) return rc;
+    }
+    H.extra = 0.0;
+    list_radii(P, H);
+  }
   box_widths(P, H);
   cell_shifts(P, H);
   c->hs[0] = H;
@@ -773,10 +858,10 @@ int cm3d_nb_nrefsh(cm3d_nb_ctx *ctx, int istep, int *rebuilt) {
   if ((rc = reset_positions(c))) return rc;
   CK(cudaMemcpyAsync(c->h_istate, c->istate, sizeof(int) * IS_COUNT, cudaMemcpyDeviceToHost, c->st));
   CK(cudaStreamSynchronize(c->st));
-  if (c->h_istate[IS_REBUILD]) {
-    if ((rc = build_lists(c, false, false))) return rc;
-    if (rebuilt) *rebuilt = 1;
-  }
+  if (c->h_istate[IS_LREBUILD]) rc = build_lists(c, false, false);
+  else if (c->h_istate[IS_REBUILD]) rc = take_snapshot(c, false, false, false);
+  if (rc) return rc;
+  if (rebuilt && c->h_istate[IS_REBUILD]) *rebuilt = 1;
   return CM3D_NB_OK;
 }
 

@@ -83,6 +83,8 @@ struct SysP {
   float hF[9], hiF[9];
   double h[9], hi[9];
   double rmaxl_skin2_e, rmaxs_skin2_e;   // -1 without charges
+  double rmaxl_list2_e, rmaxs_list2_e;   // the same radii of the engine's own lists
+  double listq;              // (list skin / 2)^2 of the engine's own lists; -1: they follow nrefsh's rebuilds
   double skin2q;             // (skin / 2)^2
   double near_s[3];          // small boxes: |fractional displacement| above which a listed pair
                              // may change its nearest image before the next rebuild
@@ -107,19 +109,20 @@ enum {
 enum {
   IS_ISTEP = 0,           // SIMPARMS.istep of the step being taken
   IS_ISTEPLAST = 1,       // md_finter.c:48 static isteplast
-  IS_REBUILD = 2,         // rebuild requested by the displacement check
-  IS_HALT = 3,            // a device-side rebuild outgrew a list: the rest
+  IS_REBUILD = 2,         // nrefsh: an atom moved more than skin / 2 (md_finter.c:63)
+  IS_LREBUILD = 3,        // the engine's own lists are to be built again (see list_skin)
+  IS_HALT = 4,            // a device-side rebuild outgrew a list: the rest
                           // of the captured step does nothing, the host
                           // grows the buffers and finishes the step
-  IS_INTR = 4,            // RESPA level (intr) the step is in
+  IS_INTR = 5,            // RESPA level (intr) the step is in
   IS_COUNT = 8
 };
 
 // Gate of kernels that run inside a captured step: with gs == nullptr (host
 // driven) never skip; otherwise skip once the step is halted, and list-build
-// kernels (need_rebuild) also when no rebuild was requested.
+// kernels (need_rebuild) also when no list is to be built.
 __device__ __forceinline__ bool gated_off(const int *gs, int need_rebuild) {
-  return gs && (gs[IS_HALT] != 0 || (need_rebuild && gs[IS_REBUILD] == 0));
+  return gs && (gs[IS_HALT] != 0 || (need_rebuild && gs[IS_LREBUILD] == 0));
 }
 // per-system counters (sstat[s * SS_COUNT + ...])
 enum { SS_REBUILDS = 0, SS_RESETS = 1, SS_COUNT = 2 };
@@ -207,8 +210,11 @@ struct SysH {
   double hmat[9], hmati[9];
   double vlrc = 0, wlrc = 0, ewald_self = 0, ewald_bkg = 0;
   double scale14 = 1, scale14e = 1;   // ONFO.scale_onefour / scale_onefour_e
-  double rlist = 0;          // largest list radius (LJ or charges, with skin)
+  double rlist = 0;          // largest radius of the engine's own lists
+  double rlist_cm = 0;       // largest list radius of CM3D (LJ or charges, with skin)
+  int nc_cm[3] = {1, 1, 1};  //   and the cells per axis it leaves room for (set_box's limit)
   double skin = 0;           // INTER.skin_ter
+  double extra = 0;          // the engine's own lists reach this far beyond CM3D's (list_skin)
   double rmaxl_coul2 = 0, dx2coul = 0, rmins_coul2 = 0;   // charges: cut-off^2, table spacing, table start^2
   std::vector<int4> krows;   // k rows {ka, kb, kc0, len} of the system's k set
   std::vector<int> krow_k0;  // first k of each row (system-local)
@@ -249,6 +255,7 @@ struct Ctx {
   int *sys_of = nullptr;               // per atom: its system
   int *cell_sys = nullptr;             // per cell: its system
   int *sreb = nullptr;                 // per system: rebuild requested (nrefsh)
+  int *lreb = nullptr;                 // per system: the engine's own lists are to be built (in sreb's allocation)
   int *slast = nullptr;                // per system: md_finter.c's isteplast
   long long *sstat = nullptr;          // per system: SS_* counters
   long long *h_sstat = nullptr;
@@ -334,6 +341,7 @@ struct Ctx {
   double *pos = nullptr, *vel = nullptr, *fxl = nullptr, *fxs = nullptr, *fxa = nullptr;
   double *fxr = nullptr;                // torsion level (torsions + 1-4 pairs)
   double *mass = nullptr, *q = nullptr, *dxn = nullptr, *snap = nullptr;
+  double *dxi = nullptr;                // positions the engine's own lists were built from (a list skin beyond CM3D's)
   int *itype = nullptr;
   // ---- parameters on device
   int *map = nullptr;                   // ntypes^2
@@ -341,6 +349,7 @@ struct Ctx {
   double *icut = nullptr;               // 8*ninter: rmaxs_cut2 rmins_cut2 rmaxl_cut2
                                         // rminl_cut2 rmaxs_skin2 rmaxl_skin2 dx2tab vt[ntm4]
   double *coultab = nullptr, *dcoultab = nullptr, *switchse = nullptr;
+  double *rad_cm = nullptr, *rad = nullptr;   // per interaction {rmaxs, rmaxl}^2 list radii: CM3D's, the engine's own
   int *excl_off = nullptr, *excl_idx = nullptr, *cexcl_off = nullptr, *cexcl_idx = nullptr;
   // FP32 coefficient tables (mixed): per index k two float4
   //   LJ:   {dv0, dvA, dvB, v0} {vA, vB, sw0, swA}  + swB in a third
@@ -548,6 +557,7 @@ std::recursive_mutex &device_mutex();           // nb_capi.cu
 using DevLock = std::lock_guard<std::recursive_mutex>;
 int list_setup(Ctx *c);                         // nb_list.cu
 void cell_shifts(SysP &P, const SysH &H);       // nb_list.cu
+int take_snapshot(Ctx *c, bool device_flag, bool all, bool lists);   // nb_list.cu
 int refresh_corners(Ctx *c);                    // nb_list.cu: cell corners under a new box
 int pair_forces(Ctx *c, int iflg, int which);   // nb_pair.cu: which 0 LJ, 1 elec, 2 fused
 int pair_setup(Ctx *c);                         // nb_pair.cu

@@ -1622,7 +1622,7 @@ int cw_convert(Ctx *c, bool device_flag, bool all) {
   int *halt = device_flag ? c->istate + IS_HALT : nullptr;
   if (c->cw_batch) {
     // only the atoms of the compact systems being rebuilt (all: every one)
-    k_cw_scan<<<1, 1024, 0, c->st>>>(c->nsys, c->sp, c->cw_sys, c->sreb, all ? 1 : 0, c->cw_scan, gate);
+    k_cw_scan<<<1, 1024, 0, c->st>>>(c->nsys, c->sp, c->cw_sys, c->lreb, all ? 1 : 0, c->cw_scan, gate);
     k_cw_convert_sys<<<8 * c->num_sms, 256, 0, c->st>>>(c->nsys, c->cw_scan, c->sp, c->cw_cap, c->n, c->cw_words,
                                                          c->cw_row, c->cell_start, c->cell_of, c->cell_atoms, c->nlen,
                                                          c->nbr_stride, c->nbr, c->cwl, c->cwn, c->stat, halt, gate);

@@ -223,7 +223,8 @@ struct ListK {
   const float4 *xq;
   const double *pos;
   const int *itype, *map;
-  const double *icut, *q;
+  const double *rad, *q;               // list radii^2 of the lists being built, {s, l} per interaction
+  int own;                             // the engine's own lists (otherwise CM3D's half lists)
   const int *excl_off, *excl_idx, *cexcl_off, *cexcl_idx;
   const int4 *cimg;
   const int2 *smeta, *xspan;
@@ -244,7 +245,7 @@ __device__ __noinline__ uint32_t exact_entry(const SysP &P, const ListK &K, int 
   const int4 ci = K.cimg[i];
   const bool qi = K.q[i] != 0.0;
   const double xi = pos[i], yi = pos[n + i], zi = pos[2 * n + i];
-  const double *__restrict__ icut = K.icut;
+  const double rl_e = K.own ? P.rmaxl_list2_e : P.rmaxl_skin2_e, rs_e = K.own ? P.rmaxs_list2_e : P.rmaxs_skin2_e;
   const int intr = K.map[P.map0 + ti * P.ntypes + K.itype[j]];
   const bool lj_ok = intr >= 0;
   const bool el_ok = qi && K.q[j] != 0.0;
@@ -262,13 +263,13 @@ __device__ __noinline__ uint32_t exact_entry(const SysP &P, const ListK &K, int 
   const double ez = __dadd_rn(__dadd_rn(__dmul_rn(sx, P.h[6]), __dmul_rn(sy, P.h[7])), __dmul_rn(sz, P.h[8]));
   const double r2 = r2_ref(ex, ey, ez);
   uint32_t en = 0;
-  if (lj_ok && r2 < icut[8 * intr + 5] && !(P.excl && excluded(i, j, K.excl_off, K.excl_idx))) {
+  if (lj_ok && r2 < K.rad[2 * intr + 1] && !(P.excl && excluded(i, j, K.excl_off, K.excl_idx))) {
     en |= ENT_LJ;
-    if (r2 < icut[8 * intr + 4]) en |= ENT_LJS;
+    if (r2 < K.rad[2 * intr]) en |= ENT_LJS;
   }
-  if (el_ok && r2 < P.rmaxl_skin2_e && !(P.cexcl && excluded(i, j, K.cexcl_off, K.cexcl_idx))) {
+  if (el_ok && r2 < rl_e && !(P.cexcl && excluded(i, j, K.cexcl_off, K.cexcl_idx))) {
     en |= ENT_EL;
-    if (r2 < P.rmaxs_skin2_e) en |= ENT_ELS;
+    if (r2 < rs_e) en |= ENT_ELS;
   }
   if (!en) return 0;
   // small boxes: the atoms may move skin/2 each before the next rebuild, so a
@@ -477,13 +478,13 @@ __device__ __forceinline__ ListAtom list_atom(const SysP &P, const ListK &K, int
   if (A.rows && lane < P.ntypes) {
     const int intr = K.map[P.map0 + A.ti * P.ntypes + lane];
     if (intr >= 0) {
-      A.rl = (float)K.icut[8 * intr + 5];
-      A.rs = (float)K.icut[8 * intr + 4];
+      A.rl = (float)K.rad[2 * intr + 1];
+      A.rs = (float)K.rad[2 * intr];
     }
   }
   if (meta.y & 1) {
-    A.el = (float)P.rmaxl_skin2_e;
-    A.es = (float)P.rmaxs_skin2_e;
+    A.el = (float)(K.own ? P.rmaxl_list2_e : P.rmaxl_skin2_e);
+    A.es = (float)(K.own ? P.rmaxs_list2_e : P.rmaxs_skin2_e);
   }
   A.near = fmaf(4e-5f, P.lim2_image, 2e-3f);
   const int2 x = K.xspan[meta.x];
@@ -527,8 +528,8 @@ __device__ __forceinline__ uint32_t list_flags(const SysP &P, const ListK &K, co
     rl = rs = -1.f;
     const int intr = on ? K.map[P.map0 + A.ti * P.ntypes + tj] : -1;
     if (intr >= 0) {
-      rl = (float)K.icut[8 * intr + 5];
-      rs = (float)K.icut[8 * intr + 4];
+      rl = (float)K.rad[2 * intr + 1];
+      rs = (float)K.rad[2 * intr];
     }
   }
   const bool qj = (mj.y & 1) != 0;
@@ -917,7 +918,7 @@ __global__ void __launch_bounds__(LT_WARPS * 32, 5) k_list_tile(
   if (rows)
     for (int k = threadIdx.x; k < ntypes * ntypes; k += LT_WARPS * 32) {
       const int intr = K.map[P.map0 + k];
-      M.radii[k] = intr >= 0 ? make_float2((float)K.icut[8 * intr + 5], (float)K.icut[8 * intr + 4])
+      M.radii[k] = intr >= 0 ? make_float2((float)K.rad[2 * intr + 1], (float)K.rad[2 * intr])
                              : make_float2(-1.f, -1.f);
     }
   __syncthreads();
@@ -928,7 +929,7 @@ __global__ void __launch_bounds__(LT_WARPS * 32, 5) k_list_tile(
     if (halt) *halt = 1;
   }
   const float near_r = fmaf(4e-5f, P.lim2_image, 2e-3f);
-  const float el_r = (float)P.rmaxl_skin2_e, es_r = (float)P.rmaxs_skin2_e;
+  const float el_r = (float)P.rmaxl_list2_e, es_r = (float)P.rmaxs_list2_e;
   // the threshold's room for the rounding of the larger terms (coordinates of
   // up to two cells); the survivors' distances are formed anew
   float lim;
@@ -1031,8 +1032,8 @@ __global__ void __launch_bounds__(LT_WARPS * 32, 5) k_list_tile(
           } else if (on) {
             const int intr = K.map[P.map0 + (at.y >> 1) * ntypes + (mj.y >> 1)];
             if (intr >= 0) {
-              rl = (float)K.icut[8 * intr + 5];
-              rs = (float)K.icut[8 * intr + 4];
+              rl = (float)K.rad[2 * intr + 1];
+              rs = (float)K.rad[2 * intr];
             }
           }
           const bool qq = qi && (mj.y & 1);
@@ -1152,11 +1153,12 @@ __global__ void k_rebuild_cells(int nsys, const SysP *__restrict__ sp, const int
 // instead (same decisions).
 constexpr int LW_THREADS = 256;
 constexpr size_t LW_BYTES_PER_ATOM = sizeof(float4) + 2 * sizeof(int);   // s_x (w: type, charge), s_u, s_j
-constexpr long long LW_MAX_CAP = 2048;     // largest staged neighbourhood (48 KB)
+constexpr int LW_MIN_ATOMS = 1024;          // atoms per SM from which neighbourhoods are staged
+constexpr long long LW_MAX_CAP = 2944;     // largest staged neighbourhood (69 KB: 3 blocks per SM)
 
 __global__ void __launch_bounds__(LW_THREADS, 3) k_list_win(
     const __grid_constant__ ListK K, int nsys, const int *__restrict__ rb_scan, const SysP *__restrict__ sp,
-    int stride, int cap, int parts, uint32_t *__restrict__ nbr, int *__restrict__ nlen,
+    int stride, int cap, uint32_t *__restrict__ nbr, int *__restrict__ nlen,
     long long *__restrict__ stat, int *__restrict__ halt, const int *__restrict__ gate) {
   if (gated_off(gate, 1)) return;
   extern __shared__ float4 s_x[];                        // cap
@@ -1167,10 +1169,8 @@ __global__ void __launch_bounds__(LW_THREADS, 3) k_list_win(
   __shared__ int s_cs[27], s_off[27], s_code[27], s_tot, s_nw;
   __shared__ float4 s_sh[27];
   const int warp = threadIdx.x >> 5;
-  const int total = rb_scan[nsys] * parts;
-  for (int item = blockIdx.x; item < total; item += gridDim.x) {
-    // rebuilt cell v, every parts-th round of its atoms from `part` on
-    const int v = item / parts, part = item - v * parts;
+  const int total = rb_scan[nsys];
+  for (int v = blockIdx.x; v < total; v += gridDim.x) {
     // the system of rebuilt cell v: the last s with rb_scan[s] <= v (systems
     // without rebuilt cells share their successor's value and are passed)
     int sa = 0, sb = nsys;
@@ -1245,7 +1245,7 @@ __global__ void __launch_bounds__(LW_THREADS, 3) k_list_win(
     const int kind = grid_kind(P);
     const bool prune = kind == G_STENCIL && ortho(P);
     const float3 cw = cell_width(P);
-    for (int t = lo + part * (LW_THREADS / 32) + warp; t < hi; t += parts * (LW_THREADS / 32)) {
+    for (int t = lo + warp; t < hi; t += LW_THREADS / 32) {
       if (staged)
         full_list_atom<true>(P, K, t, stride, nbr, nlen, stat, halt, qs[warp], qrs[warp], kind, prune && nw == 27, cw,
                              s_x, s_u, s_j, tot, s_off, s_code, nw);
@@ -1301,26 +1301,48 @@ int refresh_corners(Ctx *c) {
   return CM3D_NB_OK;
 }
 
-// dxn = pos of the rebuilt systems (ngbr_list.c:577-580) and, per rebuilt
-// system, isteplast = istep (md_finter.c:98)
+// The positions rebuilds refer to.  nrefsh's rebuilds (sreb): dxn = pos
+// (ngbr_list.c:577-580), isteplast = istep (md_finter.c:98); event = 0 leaves
+// them alone.  The engine's own lists (lreb; dxi null: they follow nrefsh's
+// rebuilds): dxi = pos.
 __global__ void k_snapshot(int n, const SysP *__restrict__ sp, const int *__restrict__ sys_of,
-                           const int *__restrict__ sreb, int all, const double *__restrict__ pos,
-                           double *__restrict__ dxn, int *__restrict__ slast, long long *__restrict__ sstat,
+                           const int *__restrict__ sreb, const int *__restrict__ lreb, int all, int event, int lists,
+                           const double *__restrict__ pos, double *__restrict__ dxn, double *__restrict__ dxi,
+                           int *__restrict__ slast, long long *__restrict__ sstat,
                            const int *__restrict__ gate, const int *__restrict__ istate,
                            long long *__restrict__ stat) {
-  if (gated_off(gate, 1)) return;
+  if (gate && (gate[IS_HALT] != 0 || (gate[IS_REBUILD] == 0 && gate[IS_LREBUILD] == 0))) return;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i == 0) atomicAdd((unsigned long long *)(stat + ST_REBUILDS), 1ull);
+  if (i == 0 && event && (!gate || gate[IS_REBUILD] != 0)) atomicAdd((unsigned long long *)(stat + ST_REBUILDS), 1ull);
   if (i >= n) return;
   const int s = sys_of[i];
-  if (sys_skip(s, sreb, all)) return;
-  dxn[i] = pos[i];
-  dxn[n + i] = pos[n + i];
-  dxn[2 * n + i] = pos[2 * n + i];
+  const double x = pos[i], y = pos[n + i], z = pos[2 * n + i];
+  if (dxi && lists && (all || lreb[s] != 0)) {
+    dxi[i] = x;
+    dxi[n + i] = y;
+    dxi[2 * n + i] = z;
+  }
+  if (!event || sys_skip(s, sreb, all)) return;
+  dxn[i] = x;
+  dxn[n + i] = y;
+  dxn[2 * n + i] = z;
   if (i == sp[s].a0) {
     slast[s] = istate[IS_ISTEP];
     sstat[(size_t)s * SS_COUNT + SS_REBUILDS] += 1;
   }
+}
+
+// nrefsh's snapshot (unless no_snapshot; in a host-driven pass if the flag it
+// read back asks for it) and, with `lists`, that of the lists just built
+int take_snapshot(Ctx *c, bool device_flag, bool all, bool lists) {
+  const bool event = !c->no_snapshot && (all || device_flag || c->h_istate[IS_REBUILD] != 0);
+  k_snapshot<<<grid_for(c->n, 256), 256, 0, c->st>>>(c->n, c->sp, c->sys_of, c->sreb, c->lreb, all ? 1 : 0,
+                                                      event ? 1 : 0, lists ? 1 : 0, c->pos, c->dxn, c->dxi,
+                                                      c->slast, c->sstat, device_flag ? c->istate : nullptr, c->istate,
+                                                      c->stat);
+  c->launches++;
+  CKL(c);
+  return CM3D_NB_OK;
 }
 
 // --------------------------------------------------------------- host side
@@ -1368,15 +1390,18 @@ int list_setup(Ctx *c) {
   double est_max = 32.0;
   for (int s = 0; s < c->nsys; s++) {
     SysP &P = c->h_sp[s];
-    const SysH &H = c->hs[s];
+    SysH &H = c->hs[s];
     int tot = 1;
     for (int d = 0; d < 3; d++) {
       double w = 1.0 / sqrt(H.hmati[3 * d] * H.hmati[3 * d] + H.hmati[3 * d + 1] * H.hmati[3 * d + 1] +
                             H.hmati[3 * d + 2] * H.hmati[3 * d + 2]);
-      int m = H.rlist > 0 ? (int)floor(w / (H.rlist * c->cell_scale)) : 1;
-      m = m < 1 ? 1 : (m > 1000 ? 1000 : m);
-      P.nc[d] = m;
-      tot *= m;
+      auto cells = [&](double rl) {
+        const int m = rl > 0 ? (int)floor(w / (rl * c->cell_scale)) : 1;
+        return m < 1 ? 1 : (m > 1000 ? 1000 : m);
+      };
+      P.nc[d] = cells(H.rlist);
+      H.nc_cm[d] = cells(H.rlist_cm);
+      tot *= P.nc[d];
     }
     P.c0 = c0;
     P.ncells = tot;
@@ -1448,9 +1473,14 @@ int list_setup(Ctx *c) {
     // a neighbourhood of thousands of atoms leaves one block per SM: the
     // warp-per-atom walk through global memory keeps more warps in flight
     if (c->lw_cap < 64 || cap > LW_MAX_CAP) c->lw_cap = 0;
+    // with a few cells per block the staging of the largest neighbourhood is
+    // what the kernel waits for, and a warp per atom fills the GPU sooner (per
+    // step, 37 boxes of 27,000 atoms in all: 45 us staged, 21 us walked; 648
+    // water atoms: 5.3 and 5.6; 1024 boxes of 953,000 atoms: 406 and 510)
+    if (c->n < LW_MIN_ATOMS * c->num_sms) c->lw_cap = 0;
     const char *lk = getenv("CM3D_NB_LIST_KERNEL");
     if (lk && strcmp(lk, "walk") == 0) c->lw_cap = 0;
-    c->list_tile = 1;
+    c->list_tile = cap > LW_MAX_CAP ? 1 : 0;
     for (int sy = 0; sy < c->nsys; sy++)
       for (int d = 0; d < 3; d++)
         if (c->h_sp[sy].nc[d] < 3) c->list_tile = 0;
@@ -1532,7 +1562,7 @@ static ListCaps caps(Ctx *c) {
 
 // Build the lists from the current positions.  `all`: every system (set-up,
 // get_ngbr, export); otherwise only the systems whose displacement test
-// asked for it (sreb).  With device_flag the kernels are also gated on the
+// asked for it (lreb).  With device_flag the kernels are also gated on the
 // device rebuild flag (graph replay) and the capacities are not re-checked on
 // the host.  The plain engine always builds CM3D's half lists (its pair
 // kernels walk them); the mixed engine builds its full list and the half
@@ -1546,24 +1576,24 @@ int build_lists(Ctx *c, bool device_flag, bool all) {
   cudaEvent_t e0;
   tbegin(c, 2, &e0);
   int4 *cimg = c->cimg;
-  k_cell_zero<<<grid_for(c->ncells, B), B, 0, c->st>>>(c->ncells, c->cell_sys, c->sreb, al, c->cell_cursor, gate);
-  k_cell_assign<<<grid_for(n, B), B, 0, c->st>>>(n, c->pos, c->sp, c->sys_of, c->sreb, al, c->cell_of,
+  k_cell_zero<<<grid_for(c->ncells, B), B, 0, c->st>>>(c->ncells, c->cell_sys, c->lreb, al, c->cell_cursor, gate);
+  k_cell_assign<<<grid_for(n, B), B, 0, c->st>>>(n, c->pos, c->sp, c->sys_of, c->lreb, al, c->cell_of,
                                                   c->cell_cursor, cimg, gate);
-  k_cell_scan<<<c->nsys, 256, 0, c->st>>>(c->sp, c->sreb, al, c->cell_cursor, c->cell_start, gate);
-  k_cell_fill<<<grid_for(n, B), B, 0, c->st>>>(n, c->sys_of, c->sreb, al, c->cell_of, c->cell_start,
+  k_cell_scan<<<c->nsys, 256, 0, c->st>>>(c->sp, c->lreb, al, c->cell_cursor, c->cell_start, gate);
+  k_cell_fill<<<grid_for(n, B), B, 0, c->st>>>(n, c->sys_of, c->lreb, al, c->cell_of, c->cell_start,
                                                 c->cell_cursor, c->cell_atoms, gate);
   {
     // enough blocks for four per SM where the grid allows it
     const int per_block = std::max(1, std::min(SORT_CELLS, c->ncells / std::max(1, 4 * c->num_sms)));
     k_cell_sort<<<(c->ncells + per_block - 1) / per_block, SORT_THREADS, 0, c->st>>>(
-        c->ncells, per_block, c->cell_sys, c->sreb, al, c->cell_start, c->itype, c->cell_atoms, gate);
+        c->ncells, per_block, c->cell_sys, c->lreb, al, c->cell_start, c->itype, c->cell_atoms, gate);
   }
-  k_sorted_init<<<grid_for(n, B), B, 0, c->st>>>(n, c->sp, c->sys_of, c->sreb, al, c->cell_atoms, cimg, c->itype,
+  k_sorted_init<<<grid_for(n, B), B, 0, c->st>>>(n, c->sp, c->sys_of, c->lreb, al, c->cell_atoms, cimg, c->itype,
                                                   c->pos, c->q, c->rank, c->styp, c->smeta, c->corner, c->xq, gate);
   c->launches += 6;
   const long long warps_threads = 32LL * n;
   int *halt = device_flag ? c->istate + IS_HALT : nullptr;
-  const ListK K = {n, c->cell_atoms, c->cell_start, c->cell_of, c->xq, c->pos, c->itype, c->map, c->icut, c->q,
+  ListK K = {n, c->cell_atoms, c->cell_start, c->cell_of, c->xq, c->pos, c->itype, c->map, c->rad, c->q, 1,
                    c->excl_off, c->excl_idx, c->cexcl_off, c->cexcl_idx, cimg, c->smeta, c->xspan};
   bool direct = false;                       // the list kernel wrote the compact lists as well
   if (c->mode == CM3D_NB_MIXED) {
@@ -1581,15 +1611,10 @@ int build_lists(Ctx *c, bool device_flag, bool all) {
         int per_sm = 1;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_list_win, LW_THREADS, smem);
         long long grid = (long long)c->num_sms * (per_sm > 0 ? per_sm : 1);
-        // a grid of few cells is split into parts of the cells' atoms until
-        // the resident blocks all have work (8 cells of 81 water atoms run on
-        // 8 of the 148 SMs: 135 us, split and with FP32 minimum images 9 us)
-        int parts = 1;
-        while ((long long)c->ncells * parts < grid && parts * (LW_THREADS / 32) < c->lw_atoms) parts++;
-        if (grid > (long long)c->ncells * parts) grid = (long long)c->ncells * parts;
-        k_rebuild_cells<<<1, 1024, 0, c->st>>>(c->nsys, c->sp, c->sreb, al, c->rb_scan, gate);
+        if (grid > c->ncells) grid = c->ncells;
+        k_rebuild_cells<<<1, 1024, 0, c->st>>>(c->nsys, c->sp, c->lreb, al, c->rb_scan, gate);
         k_list_win<<<(int)grid, LW_THREADS, smem, c->st>>>(K, c->nsys, c->rb_scan, c->sp, c->nbr_stride, c->lw_cap,
-                                                           parts, c->nbr, c->nlen, c->stat, halt, gate);
+                                                           c->nbr, c->nlen, c->stat, halt, gate);
         c->launches++;
       } else if (c->list_tile) {
         int rc = CM3D_NB_OK;
@@ -1603,11 +1628,11 @@ int build_lists(Ctx *c, bool device_flag, bool all) {
         while (group > 8 && (long long)n / group < 2LL * c->num_sms) group /= 2;
         const int parts = (c->lw_atoms + group - 1) / group;
         const auto kern = compact ? k_list_tile<true> : k_list_tile<false>;
-        kern<<<c->ncells * parts, LT_WARPS * 32, 0, c->st>>>(K, group, parts, c->sp, c->cell_sys, c->sreb, al,
+        kern<<<c->ncells * parts, LT_WARPS * 32, 0, c->st>>>(K, group, parts, c->sp, c->cell_sys, c->lreb, al,
                                                              c->nbr_stride, c->nbr, c->nlen, W, c->stat, halt, gate);
         direct = compact;
       } else {
-        k_list_full<<<grid_for(warps_threads, 256), 256, 0, c->st>>>(K, c->sp, c->sys_of, c->sreb, al, c->nbr_stride,
+        k_list_full<<<grid_for(warps_threads, 256), 256, 0, c->st>>>(K, c->sp, c->sys_of, c->lreb, al, c->nbr_stride,
                                                                      c->nbr, c->nlen, c->stat, halt, gate);
       }
       c->launches++;
@@ -1626,6 +1651,9 @@ int build_lists(Ctx *c, bool device_flag, bool all) {
     if (rc) return rc;
   }
   if (want_half) {
+    // CM3D's lists, by CM3D's radii
+    K.rad = c->rad_cm;
+    K.own = 0;
     k_list_half<false><<<grid_for(warps_threads, 256), 256, 0, c->st>>>(
         K, c->sp, c->sys_of, caps(c), c->cnt, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, c->stat, nullptr,
         gate);
@@ -1646,10 +1674,9 @@ int build_lists(Ctx *c, bool device_flag, bool all) {
         halt, gate);
     c->launches++;
   }
-  if (!c->no_snapshot) {
-    k_snapshot<<<grid_for(n, B), B, 0, c->st>>>(n, c->sp, c->sys_of, c->sreb, al, c->pos, c->dxn, c->slast,
-                                                 c->sstat, gate, c->istate, c->stat);
-    c->launches++;
+  if (!c->no_snapshot || c->dxi) {
+    const int rc = take_snapshot(c, device_flag, all, true);
+    if (rc) return rc;
   }
   CKL(c);
   tend(c, 2, e0);

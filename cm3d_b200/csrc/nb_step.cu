@@ -285,6 +285,29 @@ __global__ void k_bonded(StepP P, const int *__restrict__ gaoff, const int *__re
   }
 }
 
+// What a displacement test raises: nrefsh's rebuild (far) and the building of
+// the engine's own lists (lfar; their lists follow nrefsh's rebuilds where
+// listq < 0).  A list test on positions that RESETPOS then pulls back holds for
+// the pulled ones too: they lie between them and nrefsh's snapshot, which
+// passed the test.
+__device__ __forceinline__ void raise_rebuild(int sy, double listq, bool far, bool lfar, int *__restrict__ sreb,
+                                              int *__restrict__ lreb, int *__restrict__ istate) {
+  if (far) {
+    sreb[sy] = 1;
+    istate[IS_REBUILD] = 1;
+  }
+  if (listq < 0. ? far : lfar) {
+    lreb[sy] = 1;
+    istate[IS_LREBUILD] = 1;
+  }
+}
+
+// squared displacement of atom i from the snapshot d
+__device__ __forceinline__ double moved2(int i, int n, const double *__restrict__ pos, const double *__restrict__ d) {
+  const double xc = d[i] - pos[i], yc = d[n + i] - pos[n + i], zc = d[2 * n + i] - pos[2 * n + i];
+  return xc * xc + yc * yc + zc * zc;
+}
+
 // One pass of md_step.c:95-136 for level `intr`: the kick with the
 // nonbonded accelerations, the ninrra x ninnra inner loop with force(2) on
 // this group, then nrefsh's displacement test.
@@ -292,11 +315,13 @@ template <bool INTRA>
 __global__ void k_inner(StepP P, int intr, const int *__restrict__ gaoff, const int *__restrict__ gatoms,
                         double *__restrict__ pos, double *__restrict__ vel, const double *__restrict__ mass,
                         const double *__restrict__ fxl, const double *__restrict__ fxs, double *__restrict__ fxa,
-                        const double *__restrict__ dxn, const int *__restrict__ gboff,
+                        const double *__restrict__ dxn, const double *__restrict__ dxi,
+                        const int *__restrict__ gboff,
                         const int4 *__restrict__ bij, const double2 *__restrict__ bp,
                         const int *__restrict__ geoff, const int4 *__restrict__ eijk,
                         const double2 *__restrict__ ep, const SysP *__restrict__ sp,
-                        const int *__restrict__ sys_of, int *__restrict__ sreb, int *__restrict__ istate,
+                        const int *__restrict__ sys_of, int *__restrict__ sreb, int *__restrict__ lreb,
+                        int *__restrict__ istate,
                         const int *__restrict__ gs, IntraDev X, const double *__restrict__ q,
                         double *__restrict__ fxr, long long *__restrict__ stat) {
   if (gated_off(gs, 0)) return;
@@ -373,17 +398,14 @@ __global__ void k_inner(StepP P, int intr, const int *__restrict__ gaoff, const 
   }
   // nrefsh: any |r - r_last|^2 > skin^2/4 (md_finter.c:63-71), per system
   const int sy = sys_of[gatoms[a0]];
-  const double skin2q = sp[sy].skin2q;
-  bool far = false;
+  const double skin2q = sp[sy].skin2q, listq = sp[sy].listq;
+  bool far = false, lfar = false;
   for (int a = a0; a < a1; a++) {
-    int i = gatoms[a];
-    double xc = dxn[i] - pos[i], yc = dxn[n + i] - pos[n + i], zc = dxn[2 * n + i] - pos[2 * n + i];
-    if (xc * xc + yc * yc + zc * zc > skin2q) far = true;
+    const int i = gatoms[a];
+    far |= moved2(i, n, pos, dxn) > skin2q;
+    if (listq >= 0.) lfar |= moved2(i, n, pos, dxi) > listq;
   }
-  if (far) {
-    sreb[sy] = 1;
-    istate[IS_REBUILD] = 1;
-  }
+  raise_rebuild(sy, listq, far, lfar, sreb, lreb, istate);
 }
 
 // k_inner for a context whose molecules all have at most NA atoms (NA 1: no
@@ -454,10 +476,10 @@ __global__ void __launch_bounds__(128) k_inner_small(
     StepP P, int intr, const int *__restrict__ gaoff, const int *__restrict__ gatoms, double *__restrict__ pos,
     double *__restrict__ vel, const double *__restrict__ mass, const double *__restrict__ fxl,
     const double *__restrict__ fxs, double *__restrict__ fxa, const double *__restrict__ dxn,
-    const int *__restrict__ gboff, const int4 *__restrict__ bij, const double2 *__restrict__ bp,
+    const double *__restrict__ dxi, const int *__restrict__ gboff, const int4 *__restrict__ bij, const double2 *__restrict__ bp,
     const int *__restrict__ geoff, const int4 *__restrict__ eijk, const double2 *__restrict__ ep,
-    const SysP *__restrict__ sp, const int *__restrict__ sys_of, int *__restrict__ sreb, int *__restrict__ istate,
-    const int *__restrict__ gs) {
+    const SysP *__restrict__ sp, const int *__restrict__ sys_of, int *__restrict__ sreb, int *__restrict__ lreb,
+    int *__restrict__ istate, const int *__restrict__ gs) {
   if (gated_off(gs, 0)) return;
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g == 0) istate[IS_INTR] = intr;
@@ -471,7 +493,7 @@ __global__ void __launch_bounds__(128) k_inner_small(
   Mol3 M;
   double rm[NA];
   const int sy = sys_of[id[0]];
-  const double skin2q = sp[sy].skin2q;
+  const double skin2q = sp[sy].skin2q, listq = sp[sy].listq;
 #pragma unroll
   for (int a = 0; a < NA; a++) {
     rm[a] = 1. / mass[id[a]];
@@ -536,11 +558,11 @@ __global__ void __launch_bounds__(128) k_inner_small(
       for (int d = 0; d < 3; d++) M.v[a][d] += P.dta2 * M.f[a][d];
   }
   // results, and nrefsh: any |r - r_last|^2 > skin^2/4 (md_finter.c:63-71)
-  bool far = false;
+  bool far = false, lfar = false;
 #pragma unroll
   for (int a = 0; a < NA; a++) {
     if (a >= na) break;
-    double c2 = 0.;
+    double c2 = 0., l2 = 0.;
 #pragma unroll
     for (int d = 0; d < 3; d++) {
       const int x = d * n + id[a];
@@ -549,13 +571,15 @@ __global__ void __launch_bounds__(128) k_inner_small(
       if (NA > 1) fxa[x] = M.f[a][d];
       const double c = dxn[x] - M.p[a][d];
       c2 = d == 0 ? c * c : c2 + c * c;
+      if (listq >= 0.) {
+        const double l = dxi[x] - M.p[a][d];
+        l2 = d == 0 ? l * l : l2 + l * l;
+      }
     }
-    if (c2 > skin2q) far = true;
+    far |= c2 > skin2q;
+    lfar |= l2 > listq;
   }
-  if (far) {
-    sreb[sy] = 1;
-    istate[IS_REBUILD] = 1;
-  }
+  raise_rebuild(sy, listq, far, lfar, sreb, lreb, istate);
 }
 
 // ---- NVT: the inner level with Nose-Hoover chains (intnhc_new,
@@ -651,13 +675,15 @@ __global__ void k_nvt_chain(int ntherm, int nchain, double dta2, double *__restr
 __global__ void k_nvt_c(StepP P, int tors_end, int level_end, const int *__restrict__ gaoff,
                         const int *__restrict__ gatoms, double *__restrict__ pos, double *__restrict__ vel,
                         const double *__restrict__ mass, const double *__restrict__ q, double *__restrict__ fxa,
-                        double *__restrict__ fxr, const double *__restrict__ dxn, const int *__restrict__ gboff,
+                        double *__restrict__ fxr, const double *__restrict__ dxn, const double *__restrict__ dxi,
+                        const int *__restrict__ gboff,
                         const int4 *__restrict__ bij, const double2 *__restrict__ bp,
                         const int *__restrict__ geoff, const int4 *__restrict__ eijk,
                         const double2 *__restrict__ ep, const int *__restrict__ ithm,
                         const double *__restrict__ veta, const SysP *__restrict__ sp,
-                        const int *__restrict__ sys_of, int *__restrict__ sreb, int *__restrict__ istate,
-                        IntraDev X, long long *__restrict__ stat, const int *__restrict__ gs) {
+                        const int *__restrict__ sys_of, int *__restrict__ sreb, int *__restrict__ lreb,
+                        int *__restrict__ istate, IntraDev X, long long *__restrict__ stat,
+                        const int *__restrict__ gs) {
   if (gated_off(gs, 0)) return;
   int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= P.ngroups) return;
@@ -709,32 +735,28 @@ __global__ void k_nvt_c(StepP P, int tors_end, int level_end, const int *__restr
   }
   if (level_end) {
     const int sy = sys_of[gatoms[a0]];
-    const double skin2q = sp[sy].skin2q;
-    bool far = false;
+    const double skin2q = sp[sy].skin2q, listq = sp[sy].listq;
+    bool far = false, lfar = false;
     for (int a = a0; a < a1; a++) {
       const int i = gatoms[a];
-      const double xc = dxn[i] - pos[i], yc = dxn[n + i] - pos[n + i], zc = dxn[2 * n + i] - pos[2 * n + i];
-      if (xc * xc + yc * yc + zc * zc > skin2q) far = true;
+      far |= moved2(i, n, pos, dxn) > skin2q;
+      if (listq >= 0.) lfar |= moved2(i, n, pos, dxi) > listq;
     }
-    if (far) {
-      sreb[sy] = 1;
-      istate[IS_REBUILD] = 1;
-    }
+    raise_rebuild(sy, listq, far, lfar, sreb, lreb, istate);
   }
 }
 
 // standalone displacement test (cm3d_nb_nrefsh)
 __global__ void k_disp(int n, const SysP *__restrict__ sp, const int *__restrict__ sys_of,
-                       const double *__restrict__ pos, const double *__restrict__ dxn, int *__restrict__ sreb,
+                       const double *__restrict__ pos, const double *__restrict__ dxn,
+                       const double *__restrict__ dxi, int *__restrict__ sreb, int *__restrict__ lreb,
                        int *__restrict__ istate) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int sy = sys_of[i];
-  double xc = dxn[i] - pos[i], yc = dxn[n + i] - pos[n + i], zc = dxn[2 * n + i] - pos[2 * n + i];
-  if (xc * xc + yc * yc + zc * zc > sp[sy].skin2q) {
-    sreb[sy] = 1;
-    istate[IS_REBUILD] = 1;
-  }
+  const double listq = sp[sy].listq;
+  raise_rebuild(sy, listq, moved2(i, n, pos, dxn) > sp[sy].skin2q, listq >= 0. && moved2(i, n, pos, dxi) > listq, sreb,
+                lreb, istate);
 }
 
 // RESETPOS (md_finter.c:79-95): if a rebuild is due fewer than 3 steps after
@@ -1694,15 +1716,17 @@ static int finish_level0(Ctx *c, double dts2, bool kick) {
 
 // clear the rebuild requests (the any-system flag and every system's own)
 static int clear_rebuild(Ctx *c) {
-  CK(cudaMemsetAsync(c->istate + IS_REBUILD, 0, sizeof(int), c->st));
-  CK(cudaMemsetAsync(c->sreb, 0, sizeof(int) * (size_t)c->nsys, c->st));
+  static_assert(IS_LREBUILD == IS_REBUILD + 1, "the two flags are cleared together");
+  CK(cudaMemsetAsync(c->istate + IS_REBUILD, 0, 2 * sizeof(int), c->st));
+  CK(cudaMemsetAsync(c->sreb, 0, sizeof(int) * 2 * (size_t)c->nsys, c->st));
   return CM3D_NB_OK;
 }
 
 int check_displacement(Ctx *c) {
   int rc;
   if ((rc = clear_rebuild(c))) return rc;
-  k_disp<<<grid_for(c->n, 256), 256, 0, c->st>>>(c->n, c->sp, c->sys_of, c->pos, c->dxn, c->sreb, c->istate);
+  k_disp<<<grid_for(c->n, 256), 256, 0, c->st>>>(c->n, c->sp, c->sys_of, c->pos, c->dxn, c->dxi, c->sreb, c->lreb,
+                                                  c->istate);
   c->launches++;
   CKL(c);
   return CM3D_NB_OK;
@@ -1793,9 +1817,9 @@ static int one_level(Ctx *c, int intr, bool gated) {
                                                                c->gate);
         k_nvt_c<<<grid_for(c->ngroups, B), B, 0, c->st>>>(
             P, intra == c->nres_intra - 1, inrra == c->nres_tors - 1 && intra == c->nres_intra - 1,
-            c->grp_atom_off, c->grp_atoms, c->pos, c->vel, c->mass, c->q, c->fxa, c->fxr, c->dxn,
+            c->grp_atom_off, c->grp_atoms, c->pos, c->vel, c->mass, c->q, c->fxa, c->fxr, c->dxn, c->dxi,
             c->grp_bond_off, c->bond_ij, c->bond_p, c->grp_bend_off, c->bend_ijk, c->bend_p, c->ithm, veta,
-            c->sp, c->sys_of, c->sreb, c->istate, c->intra, c->stat, c->gate);
+            c->sp, c->sys_of, c->sreb, c->lreb, c->istate, c->intra, c->stat, c->gate);
         c->launches += 4;
       }
   } else {
@@ -1804,15 +1828,15 @@ static int one_level(Ctx *c, int intr, bool gated) {
       const int BS = c->ngroups < 128 * c->num_sms ? 32 : 128;
       auto inner = c->small_mol == 1 ? k_inner_small<1> : k_inner_small<3>;
       inner<<<grid_for(c->ngroups, BS), BS, 0, c->st>>>(P, intr, c->grp_atom_off, c->grp_atoms, c->pos, c->vel, c->mass,
-                                                        c->fxl, c->fxs, c->fxa, c->dxn, c->grp_bond_off, c->bond_ij,
+                                                        c->fxl, c->fxs, c->fxa, c->dxn, c->dxi, c->grp_bond_off, c->bond_ij,
                                                         c->bond_p, c->grp_bend_off, c->bend_ijk, c->bend_p, c->sp,
-                                                        c->sys_of, c->sreb, c->istate, c->gate);
+                                                        c->sys_of, c->sreb, c->lreb, c->istate, c->gate);
     } else {
     auto inner = c->has_intra_x || c->intra.frz ? k_inner<true> : k_inner<false>;
     inner<<<grid_for(c->ngroups, B), B, 0, c->st>>>(P, intr, c->grp_atom_off, c->grp_atoms, c->pos, c->vel,
-                                                      c->mass, c->fxl, c->fxs, c->fxa, c->dxn, c->grp_bond_off,
+                                                      c->mass, c->fxl, c->fxs, c->fxa, c->dxn, c->dxi, c->grp_bond_off,
                                                       c->bond_ij, c->bond_p, c->grp_bend_off, c->bend_ijk,
-                                                      c->bend_p, c->sp, c->sys_of, c->sreb, c->istate, c->gate,
+                                                      c->bend_p, c->sp, c->sys_of, c->sreb, c->lreb, c->istate, c->gate,
                                                       c->intra, c->q, c->fxr, c->stat);
     }
     c->launches++;
@@ -1842,8 +1866,10 @@ static int one_level(Ctx *c, int intr, bool gated) {
   } else {
     CK(cudaMemcpyAsync(c->h_istate, c->istate, sizeof(int) * IS_COUNT, cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
-    if (c->h_istate[IS_REBUILD]) {
+    if (c->h_istate[IS_LREBUILD]) {
       if ((rc = build_lists(c, false, false))) return rc;
+    } else if (c->h_istate[IS_REBUILD]) {
+      if ((rc = take_snapshot(c, false, false, false))) return rc;
     }
   }
   return close_level(c, intr, fork);

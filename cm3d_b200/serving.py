@@ -71,7 +71,9 @@ def device_bytes(system) -> int:
     r2 = float(np.max(system["rmaxl_skin2"])) if system["ninter"] > 0 else 0.0
     if int(system.get("ktot", 0)) > 0:
         r2 = max(r2, float(system.get("rmaxl_skin2_e", 0.0)))
+    # the engine's own lists take a skin of at least 20% of the cut-off
     rl = math.sqrt(r2)
+    rl = max(rl, 1.2 * (rl - float(system.get("skin", rl))))
     stride = min(1.3 * n / vol * 4.0 / 3.0 * math.pi * rl ** 3 + 64.0, n + 31.0)
     ktot = int(system.get("ktot", 0))
     kbytes = ktot * (math.ceil(n / 2048) * 16 + 64)
