@@ -606,7 +606,7 @@ int finish_steps(Ctx *c);                       // nb_step.cu
 int query_steps(Ctx *c, int *done);             // nb_step.cu
 int run_force(Ctx *c, int iflg);                // nb_step.cu
 int run_bonded(Ctx *c);                         // nb_step.cu
-int group_init(Ctx *c, bool zero_fxs, bool side);   // nb_step.cu
+int group_init(Ctx *c, bool zero_fxs, bool side, bool zeroed);   // nb_step.cu
 int finish_level1(Ctx *c, double dter, double dter1, bool kick);   // nb_step.cu
 int check_displacement(Ctx *c);                 // nb_step.cu
 int reset_positions(Ctx *c);                    // nb_step.cu

@@ -759,16 +759,32 @@ __global__ void k_disp(int n, const SysP *__restrict__ sp, const int *__restrict
                 lreb, istate);
 }
 
+// What the kernel before the forces clears for them in a replayed step: as
+// graph nodes of their own, these and the rebuild requests that k_finish clears
+// were five memsets of some 2 us each, launch and drain, on the step's path
+// (argon, 2048 atoms with thermostats: 82 us per step, 72 without them).
+struct ZeroSpan {
+  double *fxl = nullptr, *fxs = nullptr;
+  double *acc = nullptr;
+  int nacc = 0;              // ACC_COUNT per system
+};
+
 // RESETPOS (md_finter.c:79-95): if a rebuild is due fewer than 3 steps after
 // the system's previous one, pull every atom that moved more than skin/2
 // back toward its position at the last rebuild (by CM3D's factor skin2/d^2)
 __global__ void k_resetpos(int n, const SysP *__restrict__ sp, const int *__restrict__ sys_of,
                            const int *__restrict__ sreb, const int *__restrict__ slast, double *__restrict__ pos,
                            const double *__restrict__ dxn, const int *__restrict__ istate,
-                           long long *__restrict__ stat, long long *__restrict__ sstat) {
-  if (istate[IS_REBUILD] == 0 || istate[IS_HALT] != 0) return;
+                           long long *__restrict__ stat, long long *__restrict__ sstat, ZeroSpan Z) {
+  if (istate[IS_HALT] != 0) return;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
+  for (int k = i; k < Z.nacc; k += gridDim.x * blockDim.x) Z.acc[(size_t)(k / ACC_COUNT) * ACC_STRIDE + k % ACC_COUNT] = 0.;
   if (i >= n) return;
+  for (int d = 0; d < 3; d++) {
+    if (Z.fxl) Z.fxl[d * n + i] = 0.;
+    if (Z.fxs) Z.fxs[d * n + i] = 0.;
+  }
+  if (istate[IS_REBUILD] == 0) return;
   const int sy = sys_of[i];
   if (sreb[sy] == 0 || istate[IS_ISTEP] - slast[sy] >= 3) return;
   if (i == sp[sy].a0) {
@@ -1123,9 +1139,17 @@ __global__ void k_finish(int n, int level, int kick, int rm_l, int rm_s, double 
                          const double *__restrict__ mass, double *__restrict__ fxl, double *__restrict__ fxs,
                          double *__restrict__ vel, double *__restrict__ acc, int *__restrict__ istate,
                          int advance_step, const int *__restrict__ sys_of, int batch,
-                         const int *__restrict__ gs, const unsigned char *__restrict__ frz) {
+                         const int *__restrict__ gs, const unsigned char *__restrict__ frz, int *__restrict__ reb,
+                         int nreb) {
   if (gated_off(gs, 0)) return;
   int i = blockIdx.x * blockDim.x + threadIdx.x;
+  // a replayed level leaves the rebuild requests cleared for the next one (a
+  // halted one keeps them for the host-driven path that finishes it)
+  for (int k = i; k < nreb; k += gridDim.x * blockDim.x) reb[k] = 0;
+  if (i == 0 && nreb > 0) {
+    istate[IS_REBUILD] = 0;
+    istate[IS_LREBUILD] = 0;
+  }
   double v[6] = {0, 0, 0, 0, 0, 0};
   int sy = -1;
   if (i < n) {
@@ -1671,15 +1695,14 @@ int group_terms(Ctx *c, cudaStream_t st, double *part) {
 }
 
 // side: the molecule terms run beside the k-space already (kspace_fork)
-int group_init(Ctx *c, bool zero_fxs, bool side) {
+// (zeroed: and the force arrays start from zero already)
+int group_init(Ctx *c, bool zero_fxs, bool side, bool zeroed) {
   StepP P = step_params(c);
   const int B = 128;
   cudaEvent_t e0;
   tbegin(c, 3, &e0);
-  // the force arrays start from zero (a halted graph step zeroes them too:
-  // the host-driven path that finishes it computes them again from here)
-  CK(cudaMemsetAsync(c->fxl, 0, sizeof(double) * 3 * (size_t)c->n, c->st));
-  if (zero_fxs) CK(cudaMemsetAsync(c->fxs, 0, sizeof(double) * 3 * (size_t)c->n, c->st));
+  if (!zeroed) CK(cudaMemsetAsync(c->fxl, 0, sizeof(double) * 3 * (size_t)c->n, c->st));
+  if (zero_fxs && !zeroed) CK(cudaMemsetAsync(c->fxs, 0, sizeof(double) * 3 * (size_t)c->n, c->st));
   if (!side) {
     int rc = group_terms(c, c->st, nullptr);
     if (rc) return rc;
@@ -1699,7 +1722,7 @@ int finish_level1(Ctx *c, double dter, double dter1, bool kick) {
   bool rs = c->need_short || c->nres_lrf > 1;
   k_finish<<<grid_for(c->n, B), B, 0, c->st>>>(c->n, 1, kick ? 1 : 0, 1, rs ? 1 : 0, dter, dter1, c->mass, c->fxl,
                                                c->fxs, c->vel, c->acc, c->istate, kick ? 1 : 0, c->sys_of,
-                                               c->nsys > 1, c->gate, c->intra.frz);
+                                               c->nsys > 1, c->gate, c->intra.frz, c->sreb, c->gate ? 2 * c->nsys : 0);
   c->launches++;
   CKL(c);
   return CM3D_NB_OK;
@@ -1708,7 +1731,7 @@ int finish_level1(Ctx *c, double dter, double dter1, bool kick) {
 static int finish_level0(Ctx *c, double dts2, bool kick) {
   k_finish<<<grid_for(c->n, 256), 256, 0, c->st>>>(c->n, 0, kick ? 1 : 0, 0, 1, 0, dts2, c->mass, c->fxl, c->fxs,
                                                    c->vel, c->acc, c->istate, 0, c->sys_of, c->nsys > 1, c->gate,
-                                                   c->intra.frz);
+                                                   c->intra.frz, c->sreb, c->gate ? 2 * c->nsys : 0);
   c->launches++;
   CKL(c);
   return CM3D_NB_OK;
@@ -1732,13 +1755,15 @@ int check_displacement(Ctx *c) {
   return CM3D_NB_OK;
 }
 
-int reset_positions(Ctx *c) {
+static int reset_positions(Ctx *c, const ZeroSpan &Z) {
   k_resetpos<<<grid_for(c->n, 256), 256, 0, c->st>>>(c->n, c->sp, c->sys_of, c->sreb, c->slast, c->pos, c->dxn,
-                                                      c->istate, c->stat, c->sstat);
+                                                      c->istate, c->stat, c->sstat, Z);
   c->launches++;
   CKL(c);
   return CM3D_NB_OK;
 }
+
+int reset_positions(Ctx *c) { return reset_positions(c, ZeroSpan()); }
 
 // zero every accumulator force(1) and getvireal fill, in every system
 static int zero_acc(Ctx *c) {
@@ -1757,7 +1782,7 @@ int run_force(Ctx *c, int iflg) {
   }
   if (iflg == 1) {
     if ((rc = zero_acc(c))) return rc;
-    if ((rc = group_init(c, true, false))) return rc;
+    if ((rc = group_init(c, true, false, false))) return rc;
     if ((rc = pair_forces(c, 1, 3))) return rc;
     if ((rc = kspace_forces(c))) return rc;
     return finish_level1(c, 0, 0, false);
@@ -1775,12 +1800,12 @@ int run_force(Ctx *c, int iflg) {
 // force(1) + kick on the last level, force(0) + kick otherwise.  ks_forked:
 // the accumulators were zeroed and the k-space runs on the side stream
 // already (kspace_fork), joined here after the pair forces.
-static int close_level(Ctx *c, int intr, bool ks_forked = false) {
+static int close_level(Ctx *c, int intr, bool ks_forked = false, bool zeroed = false) {
   int rc;
   StepP P = step_params(c);
   if (intr == c->nres_lrf - 1) {
-    if (!ks_forked && (rc = zero_acc(c))) return rc;
-    if ((rc = group_init(c, P.use_fxs, ks_forked && c->ecorr_side))) return rc;
+    if (!ks_forked && !zeroed && (rc = zero_acc(c))) return rc;
+    if ((rc = group_init(c, P.use_fxs, ks_forked && c->ecorr_side, zeroed))) return rc;
     if ((rc = pair_forces(c, 1, 3))) return rc;
     if ((rc = ks_forked ? kspace_join(c) : kspace_forces(c))) return rc;
     return finish_level1(c, P.dter, P.dter1, true);
@@ -1797,7 +1822,7 @@ static int one_level(Ctx *c, int intr, bool gated) {
   int rc;
   StepP P = step_params(c);
   const int B = 128;
-  if ((rc = clear_rebuild(c))) return rc;
+  if (!gated && (rc = clear_rebuild(c))) return rc;
   cudaEvent_t e0;
   tbegin(c, 3, &e0);
   if (c->ntherm > 0) {
@@ -1843,7 +1868,15 @@ static int one_level(Ctx *c, int intr, bool gated) {
   }
   tend(c, 3, e0);
   CKL(c);
-  if ((rc = reset_positions(c))) return rc;
+  ZeroSpan Z;
+  const bool zeroed = gated && intr == c->nres_lrf - 1;
+  if (zeroed) {
+    Z.fxl = c->fxl;
+    Z.fxs = P.use_fxs ? c->fxs : nullptr;
+    Z.acc = c->acc;
+    Z.nacc = ACC_COUNT * c->nsys;
+  }
+  if ((rc = reset_positions(c, Z))) return rc;
   if (intr == c->nres_lrf - 1 && c->ho_pos) {
     // the step's positions are final: their copy to the registered host
     // buffer runs on a third stream beside the rest of the step (joined at
@@ -1858,7 +1891,7 @@ static int one_level(Ctx *c, int intr, bool gated) {
   // the side stream while the lists are rebuilt and the pair forces run
   const bool fork = intr == c->nres_lrf - 1 && kspace_async_ok(c);
   if (fork) {
-    if ((rc = zero_acc(c))) return rc;
+    if (!zeroed && (rc = zero_acc(c))) return rc;
     if ((rc = kspace_fork(c))) return rc;
   }
   if (gated) {
@@ -1872,7 +1905,7 @@ static int one_level(Ctx *c, int intr, bool gated) {
       if ((rc = take_snapshot(c, false, false, false))) return rc;
     }
   }
-  return close_level(c, intr, fork);
+  return close_level(c, intr, fork, zeroed);
 }
 
 static int one_step(Ctx *c, bool gated) {
@@ -1926,7 +1959,9 @@ int launch_steps(Ctx *c, int istep0, int nsteps) {
     return CM3D_NB_OK;
   }
   // graph replay: one captured step, every kernel gated on the device state
-  // (rebuild flag; halt after a list overflow)
+  // (rebuild flag; halt after a list overflow), the rebuild requests cleared
+  // once here and by each level's last kernel
+  if ((rc = clear_rebuild(c))) return rc;
   if (!c->graph) {
     DevLock lock(device_mutex());
     cudaGraph_t g;
