@@ -95,7 +95,7 @@ static void destroy(Ctx *c) {
                   c->fxr, c->intra_buf, c->ithm, c->nhc, c->cwl, c->cwn, c->cw_tf, c->cw_tg, c->cw_tl,
                   c->cw_part, c->nvt_kin, c->nvt_chsum, c->th_atoms, c->th_choff, c->th_chunk,
                   c->cw_sys, c->cw_sitems, c->cw_items, c->cw_gidx, c->cw_scan, c->grp_work, c->smeta, c->xspan, c->qidx,
-                  c->rad_cm, c->rad, c->dxi, c->kr_perm, c->kr_split, c->kr_btab, c->kr_hdr, c->kr_kidx, c->kr_coef};
+                  c->rad_cm, c->rad, c->dxi, c->bin_keys, c->kr_perm, c->kr_split, c->kr_btab, c->kr_hdr, c->kr_kidx, c->kr_coef};
   cw_destroy(c);
   for (void *p : ptrs)
     if (p) cudaFree(p);

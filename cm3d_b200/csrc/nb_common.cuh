@@ -416,6 +416,8 @@ struct Ctx {
   // ---- cell grid and lists
   int nc[3] = {1, 1, 1}, ncells = 1;
   int *cell_of = nullptr, *cell_start = nullptr, *cell_cursor = nullptr, *cell_atoms = nullptr;
+  long long *bin_keys = nullptr;        // k_bin's scratch: the atoms of each cell before they are ordered
+  int bin_cluster = 0;                  //   and its blocks per system (0: the grid-wide kernels)
   int *rank = nullptr;                  // original -> sorted
   int *cnt = nullptr;                   // 5 per atom counts (t s te se full)
   long long *off = nullptr;             // 5*(n+1) exclusive offsets

@@ -54,16 +54,9 @@ __global__ void k_cell_zero(int ncells, const int *__restrict__ cell_sys, const 
   cell_count[c] = 0;
 }
 
-__global__ void k_cell_assign(int n, const double *__restrict__ pos, const SysP *__restrict__ sp,
-                              const int *__restrict__ sys_of, const int *__restrict__ sreb, int all,
-                              int *__restrict__ cell_of, int *__restrict__ cell_count, int4 *__restrict__ cimg,
-                              const int *__restrict__ gate) {
-  if (gated_off(gate, 1)) return;
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const int s = sys_of[i];
-  if (sys_skip(s, sreb, all)) return;
-  const SysP &P = sp[s];
+// the cell of atom i (and its image, in cimg)
+__device__ __forceinline__ int place_in_cell(const SysP &P, int n, int i, const double *__restrict__ pos,
+                                             int4 *__restrict__ cimg) {
   double x = pos[i], y = pos[n + i], z = pos[2 * n + i];
   double sv[3];
   for (int d = 0; d < 3; d++)
@@ -79,9 +72,21 @@ __global__ void k_cell_assign(int n, const double *__restrict__ pos, const SysP 
     img[d] = (int)fl;
     cc[d] = c;
   }
-  int cell = P.c0 + (cc[0] * P.nc[1] + cc[1]) * P.nc[2] + cc[2];
-  cell_of[i] = cell;
   cimg[i] = make_int4(cc[0] | (cc[1] << 10) | (cc[2] << 20), img[0], img[1], img[2]);
+  return P.c0 + (cc[0] * P.nc[1] + cc[1]) * P.nc[2] + cc[2];
+}
+
+__global__ void k_cell_assign(int n, const double *__restrict__ pos, const SysP *__restrict__ sp,
+                              const int *__restrict__ sys_of, const int *__restrict__ sreb, int all,
+                              int *__restrict__ cell_of, int *__restrict__ cell_count, int4 *__restrict__ cimg,
+                              const int *__restrict__ gate) {
+  if (gated_off(gate, 1)) return;
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int s = sys_of[i];
+  if (sys_skip(s, sreb, all)) return;
+  const int cell = place_in_cell(sp[s], n, i, pos, cimg);
+  cell_of[i] = cell;
   atomicAdd(cell_count + cell, 1);
 }
 
@@ -213,6 +218,144 @@ __global__ void __launch_bounds__(SORT_THREADS) k_cell_sort(int ncells, int per_
       }
       __syncthreads();
     }
+  }
+}
+
+// What the sorted order holds of each atom: rank, type, the FP64 corner of the
+// atom's cell (held fixed until the next rebuild) and FP32 cell-relative
+// coordinates + charge.
+struct Sorted {
+  const int *itype;
+  const double *pos, *q;
+  int *rank, *styp;
+  int2 *smeta;
+  double *corner;
+  float4 *xq;
+};
+
+// atom i, whose cell and image are ci, at sorted place t
+__device__ __forceinline__ void sorted_place(const SysP &P, const Sorted &S, int n, int t, int i, int4 ci) {
+  const double *h = P.h;
+  double o0 = (double)ci.y + (double)(ci.x & 1023) / P.nc[0];
+  double o1 = (double)ci.z + (double)((ci.x >> 10) & 1023) / P.nc[1];
+  double o2 = (double)ci.w + (double)((ci.x >> 20) & 1023) / P.nc[2];
+  double c0 = h[0] * o0 + h[1] * o1 + h[2] * o2;
+  double c1 = h[3] * o0 + h[4] * o1 + h[5] * o2;
+  double c2 = h[6] * o0 + h[7] * o1 + h[8] * o2;
+  S.corner[t] = c0;
+  S.corner[n + t] = c1;
+  S.corner[2 * n + t] = c2;
+  const double q = S.q[i];
+  S.xq[t] = make_float4((float)(S.pos[i] - c0), (float)(S.pos[n + i] - c1), (float)(S.pos[2 * n + i] - c2), (float)q);
+  S.rank[i] = t;
+  S.styp[t] = S.itype[i];
+  S.smeta[t] = make_int2(i, S.itype[i] * 2 + (q != 0.0 ? 1 : 0));
+}
+
+__global__ void k_sorted_init(int n, const SysP *__restrict__ sp, const int *__restrict__ sys_of,
+                              const int *__restrict__ sreb, int all, const int *__restrict__ cell_atoms,
+                              const int4 *__restrict__ cimg, const __grid_constant__ Sorted S,
+                              const int *__restrict__ gate) {
+  if (gated_off(gate, 1)) return;
+  int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  const int s = sys_of[t];
+  if (sys_skip(s, sreb, all)) return;
+  const int i = cell_atoms[t];
+  sorted_place(sp[s], S, n, t, i, cimg[i]);
+}
+
+// The six binning kernels (k_cell_zero .. k_sorted_init) in one, a cluster of
+// `nb` blocks per system with its barriers between the stages: same cells, same
+// order.  For systems of up to BIN_ATOMS atoms, where the six are launches and
+// little else -- on the steps that build nothing, too: they are replayed every
+// step and each costs some 2 us to find that out (us per step, six kernels and
+// one: 648 water atoms 70, 65; 2048 argon 72, 66; 2048 charged 86, 82; 37 boxes
+// 183, 176; 12,288 water atoms 148, 147).
+//
+// A stage reads what other blocks wrote before the barrier; nothing read
+// earlier in the kernel is read again after another block's write, except the
+// counters, which go through L2.
+constexpr int BIN_THREADS = 1024, BIN_CLUSTER = 8, BIN_ATOMS = 4 * BIN_CLUSTER * BIN_THREADS;
+__device__ __forceinline__ void bin_sync(int nb) {
+  if (nb == 1) {
+    __syncthreads();
+    return;
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__global__ void __launch_bounds__(BIN_THREADS, 1) k_bin(
+    int n, int nb, const SysP *__restrict__ sp, const int *__restrict__ sreb, int all, const __grid_constant__ Sorted S,
+    int4 *cimg, int *cell_of, int *count, int *cell_start, long long *keys, int *cell_atoms,
+    const int *__restrict__ gate) {
+  if (gated_off(gate, 1)) return;
+  const int s = blockIdx.x / nb, rank = blockIdx.x - s * nb;
+  if (sys_skip(s, sreb, all)) return;                     // whole clusters
+  const SysP &P = sp[s];
+  const int m = P.ncells, c0 = P.c0, a0 = P.a0, a1 = P.a0 + P.n;
+  const int t0 = rank * BIN_THREADS + threadIdx.x, nt = nb * BIN_THREADS;
+  for (int k = t0; k < m; k += nt) count[c0 + k] = 0;
+  bin_sync(nb);
+  for (int i = a0 + t0; i < a1; i += nt) {
+    const int cell = place_in_cell(P, n, i, S.pos, cimg);
+    cell_of[i] = cell;
+    atomicAdd(count + cell, 1);
+  }
+  bin_sync(nb);
+  if (rank == 0) {
+    // cell_start: exclusive scan of the counts, `chunk` cells per thread
+    __shared__ int part[32];
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const int chunk = (m + BIN_THREADS - 1) / BIN_THREADS;
+    const int lo = min(m, t * chunk), hi = min(m, lo + chunk);
+    int sum = 0;
+    for (int k = lo; k < hi; k++) sum += __ldcg(count + c0 + k);
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    if (lane == 31) part[w] = incl;
+    __syncthreads();
+    if (w == 0) {
+      int v = part[lane];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += u;
+      }
+      part[lane] = v;
+    }
+    __syncthreads();
+    int run = a0 + incl - sum + (w > 0 ? part[w - 1] : 0);
+    for (int k = lo; k < hi; k++) {
+      const int cnt = __ldcg(count + c0 + k);
+      cell_start[c0 + k] = run;
+      count[c0 + k] = 0;
+      run += cnt;
+    }
+    if (t == BIN_THREADS - 1) cell_start[c0 + m] = a1;
+  }
+  bin_sync(nb);
+  for (int i = a0 + t0; i < a1; i += nt) {
+    const int cell = cell_of[i];                          // this thread's own
+    keys[cell_start[cell] + atomicAdd(count + cell, 1)] = sort_key(S.itype, i);
+  }
+  bin_sync(nb);
+  // k_cell_sort's order: each atom's place is the number of smaller keys in
+  // its cell (neighbouring threads share the cell and read the same key)
+  for (int u = a0 + t0; u < a1; u += nt) {
+    const long long key = keys[u];
+    const int i = (int)(key & 0xffffffffLL);
+    const int cell = __ldcg(cell_of + i);
+    const int lo = cell_start[cell], hi = cell_start[cell + 1];
+    int r = 0;
+#pragma unroll 4
+    for (int v = lo; v < hi; v++) r += keys[v] < key;
+    cell_atoms[lo + r] = i;
+    sorted_place(P, S, n, lo + r, i, __ldcg(cimg + i));
   }
 }
 
@@ -1255,37 +1398,8 @@ __global__ void __launch_bounds__(LW_THREADS, 3) k_list_win(
   }
 }
 
-// sorted-order arrays: rank, type, the FP64 corner of the atom's cell (held
-// fixed until the next rebuild) and FP32 cell-relative coordinates + charge
-__global__ void k_sorted_init(int n, const SysP *__restrict__ sp, const int *__restrict__ sys_of,
-                              const int *__restrict__ sreb, int all, const int *__restrict__ cell_atoms,
-                              const int4 *__restrict__ cimg, const int *__restrict__ itype,
-                              const double *__restrict__ pos, const double *__restrict__ q, int *__restrict__ rank,
-                              int *__restrict__ styp, int2 *__restrict__ smeta, double *__restrict__ corner,
-                              float4 *__restrict__ xq,
-                              const int *__restrict__ gate) {
-  if (gated_off(gate, 1)) return;
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  const int s = sys_of[t];
-  if (sys_skip(s, sreb, all)) return;
-  const SysP &P = sp[s];
-  int i = cell_atoms[t];
-  int4 ci = cimg[i];
-  const double *h = P.h;
-  double o0 = (double)ci.y + (double)(ci.x & 1023) / P.nc[0];
-  double o1 = (double)ci.z + (double)((ci.x >> 10) & 1023) / P.nc[1];
-  double o2 = (double)ci.w + (double)((ci.x >> 20) & 1023) / P.nc[2];
-  double c0 = h[0] * o0 + h[1] * o1 + h[2] * o2;
-  double c1 = h[3] * o0 + h[4] * o1 + h[5] * o2;
-  double c2 = h[6] * o0 + h[7] * o1 + h[8] * o2;
-  corner[t] = c0;
-  corner[n + t] = c1;
-  corner[2 * n + t] = c2;
-  xq[t] = make_float4((float)(pos[i] - c0), (float)(pos[n + i] - c1), (float)(pos[2 * n + i] - c2), (float)q[i]);
-  rank[i] = t;
-  styp[t] = itype[i];
-  smeta[t] = make_int2(i, itype[i] * 2 + (q[i] != 0.0 ? 1 : 0));
+static Sorted sorted_arrays(const Ctx *c) {
+  return {c->itype, c->pos, c->q, c->rank, c->styp, c->smeta, c->corner, c->xq};
 }
 
 // The cell corners (and FP32 cell-relative positions) under a new box: every
@@ -1293,9 +1407,8 @@ __global__ void k_sorted_init(int n, const SysP *__restrict__ sp, const int *__r
 // pair kernels' shifts, also H-derived, are updated beside this).
 int refresh_corners(Ctx *c) {
   if (c->mode != CM3D_NB_MIXED || !c->lists_built) return CM3D_NB_OK;
-  k_sorted_init<<<grid_for(c->n, 256), 256, 0, c->st>>>(c->n, c->sp, c->sys_of, c->sreb, 1, c->cell_atoms,
-                                                        c->cimg, c->itype, c->pos, c->q, c->rank, c->styp,
-                                                        c->smeta, c->corner, c->xq, nullptr);
+  k_sorted_init<<<grid_for(c->n, 256), 256, 0, c->st>>>(c->n, c->sp, c->sys_of, c->sreb, 1, c->cell_atoms, c->cimg,
+                                                        sorted_arrays(c), nullptr);
   c->launches++;
   CKL(c);
   return CM3D_NB_OK;
@@ -1443,6 +1556,16 @@ int list_setup(Ctx *c) {
   CK(cudaMemset(c->cell_cursor, 0, sizeof(int) * ((size_t)c0 + 1)));
   CK(cudaMalloc(&c->cell_atoms, sizeof(int) * (size_t)c->n));
   CK(cudaMalloc(&c->rank, sizeof(int) * (size_t)c->n));
+  int n_max = 0;
+  for (int s = 0; s < c->nsys; s++) n_max = std::max(n_max, c->h_sp[s].n);
+  if (n_max <= BIN_ATOMS) {
+    // an atom per thread, while the clusters of a batch fit the GPU side by side
+    c->bin_cluster = 1;
+    while (c->bin_cluster < BIN_CLUSTER && c->bin_cluster * BIN_THREADS < n_max &&
+           2 * c->bin_cluster * c->nsys <= c->num_sms)
+      c->bin_cluster *= 2;
+    CK(cudaMalloc(&c->bin_keys, sizeof(long long) * (size_t)c->n));
+  }
   CK(cudaMalloc(&c->cnt, sizeof(int) * 4 * (size_t)c->n));
   CK(cudaMalloc(&c->off, sizeof(long long) * 4 * ((size_t)c->n + 1)));
   CK(cudaMalloc(&c->ltot, sizeof(long long) * LT_COUNT));
@@ -1576,21 +1699,36 @@ int build_lists(Ctx *c, bool device_flag, bool all) {
   cudaEvent_t e0;
   tbegin(c, 2, &e0);
   int4 *cimg = c->cimg;
-  k_cell_zero<<<grid_for(c->ncells, B), B, 0, c->st>>>(c->ncells, c->cell_sys, c->lreb, al, c->cell_cursor, gate);
-  k_cell_assign<<<grid_for(n, B), B, 0, c->st>>>(n, c->pos, c->sp, c->sys_of, c->lreb, al, c->cell_of,
-                                                  c->cell_cursor, cimg, gate);
-  k_cell_scan<<<c->nsys, 256, 0, c->st>>>(c->sp, c->lreb, al, c->cell_cursor, c->cell_start, gate);
-  k_cell_fill<<<grid_for(n, B), B, 0, c->st>>>(n, c->sys_of, c->lreb, al, c->cell_of, c->cell_start,
-                                                c->cell_cursor, c->cell_atoms, gate);
-  {
+  if (c->bin_cluster > 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(c->nsys * c->bin_cluster));
+    cfg.blockDim = dim3(BIN_THREADS);
+    cfg.stream = c->st;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)c->bin_cluster;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    CK(cudaLaunchKernelEx(&cfg, k_bin, n, c->bin_cluster, (const SysP *)c->sp, (const int *)c->lreb, al,
+                          sorted_arrays(c), cimg, c->cell_of, c->cell_cursor, c->cell_start, c->bin_keys,
+                          c->cell_atoms, gate));
+    c->launches++;
+  } else {
+    k_cell_zero<<<grid_for(c->ncells, B), B, 0, c->st>>>(c->ncells, c->cell_sys, c->lreb, al, c->cell_cursor, gate);
+    k_cell_assign<<<grid_for(n, B), B, 0, c->st>>>(n, c->pos, c->sp, c->sys_of, c->lreb, al, c->cell_of,
+                                                    c->cell_cursor, cimg, gate);
+    k_cell_scan<<<c->nsys, 256, 0, c->st>>>(c->sp, c->lreb, al, c->cell_cursor, c->cell_start, gate);
+    k_cell_fill<<<grid_for(n, B), B, 0, c->st>>>(n, c->sys_of, c->lreb, al, c->cell_of, c->cell_start,
+                                                  c->cell_cursor, c->cell_atoms, gate);
     // enough blocks for four per SM where the grid allows it
     const int per_block = std::max(1, std::min(SORT_CELLS, c->ncells / std::max(1, 4 * c->num_sms)));
     k_cell_sort<<<(c->ncells + per_block - 1) / per_block, SORT_THREADS, 0, c->st>>>(
         c->ncells, per_block, c->cell_sys, c->lreb, al, c->cell_start, c->itype, c->cell_atoms, gate);
+    k_sorted_init<<<grid_for(n, B), B, 0, c->st>>>(n, c->sp, c->sys_of, c->lreb, al, c->cell_atoms, cimg,
+                                                    sorted_arrays(c), gate);
+    c->launches += 6;
   }
-  k_sorted_init<<<grid_for(n, B), B, 0, c->st>>>(n, c->sp, c->sys_of, c->lreb, al, c->cell_atoms, cimg, c->itype,
-                                                  c->pos, c->q, c->rank, c->styp, c->smeta, c->corner, c->xq, gate);
-  c->launches += 6;
   const long long warps_threads = 32LL * n;
   int *halt = device_flag ? c->istate + IS_HALT : nullptr;
   ListK K = {n, c->cell_atoms, c->cell_start, c->cell_of, c->xq, c->pos, c->itype, c->map, c->rad, c->q, 1,
