@@ -244,6 +244,103 @@ struct IntraDev {
   const unsigned char *frz = nullptr;   // per atom: frozen (nullptr: none)
 };
 
+// The sums of the compact pair kernels' items: 16 quantities per item.
+enum { CQ_EEL = 0, CQ_QQ_UNUSED, CQ_VE0, CQ_VE1, CQ_VE2, CQ_VE4, CQ_VE5, CQ_VE8,
+       CQ_ELJ, CQ_VSH, CQ_VL0, CQ_VL1, CQ_VL2, CQ_VL4, CQ_VL5, CQ_VL8, CQ_COUNT };
+
+struct EnergyItems {
+  const double *part = nullptr;     // CQ_COUNT doubles per item; null: nothing to sum
+  const int2 *sitems = nullptr;     // a batch: {first, count} of every system's items (0: not on the compact path)
+  const SysP *sp = nullptr;
+  int nitems = 0;                   // one system
+  int mask = 0;                     // 1: LJ, 2: electrostatics
+  int count = 0;                    // systems
+};
+
+// Sum of the items' partials into CM3D's accumulators: one block, warp q
+// sums quantity q over the items (fixed order), then one thread applies the
+// sums in a fixed order (several quantities feed one accumulator); each pair
+// was counted from both ends, hence 1/2.
+__device__ __forceinline__ void cw_apply(int mask, const double *v, double *acc) {
+  if (mask & 2) {
+    // (CM3D's shifted sum spothe, finter_e.c:197, is read by nothing --
+    // getsvirter_e reports spote -- and this path does not form it)
+    acc[ACC_SPOTE] += v[CQ_EEL];
+    acc[ACC_SPRSE] -= v[CQ_VE0] + v[CQ_VE4] + v[CQ_VE8];
+    acc[ACC_SPRSET + 0] -= v[CQ_VE0];
+    acc[ACC_SPRSET + 1] -= v[CQ_VE1];
+    acc[ACC_SPRSET + 2] -= v[CQ_VE2];
+    acc[ACC_SPRSET + 4] -= v[CQ_VE4];
+    acc[ACC_SPRSET + 5] -= v[CQ_VE5];
+    acc[ACC_SPRSET + 8] -= v[CQ_VE8];
+  }
+  if (mask & 1) {
+    acc[ACC_SPOTL] += v[CQ_ELJ];
+    acc[ACC_SPOTHL] += v[CQ_ELJ] - v[CQ_VSH];
+    acc[ACC_SPRSL] -= v[CQ_VL0] + v[CQ_VL4] + v[CQ_VL8];
+    acc[ACC_SPRSLT + 0] -= v[CQ_VL0];
+    acc[ACC_SPRSLT + 1] -= v[CQ_VL1];
+    acc[ACC_SPRSLT + 2] -= v[CQ_VL2];
+    acc[ACC_SPRSLT + 4] -= v[CQ_VL4];
+    acc[ACC_SPRSLT + 5] -= v[CQ_VL5];
+    acc[ACC_SPRSLT + 8] -= v[CQ_VL8];
+  }
+}
+
+// One block of ER_THREADS sums system sy's items into its accumulators: 16
+// threads to an item (a 128-byte row), ER_THREADS / 16 items at a time.
+constexpr int ER_THREADS = 256;
+__device__ __forceinline__ void energy_sums(const EnergyItems &E, int sy, double *acc) {
+  const int2 r = E.sitems ? E.sitems[sy] : make_int2(0, E.nitems);
+  if (r.y == 0) return;
+  __shared__ double s_q[ER_THREADS];
+  const int q = threadIdx.x % CQ_COUNT, it0 = threadIdx.x / CQ_COUNT;
+  double s = 0.0;
+#pragma unroll 8
+  for (int it = it0; it < r.y; it += ER_THREADS / CQ_COUNT) s += E.part[(size_t)(r.x + it) * CQ_COUNT + q];
+  s_q[threadIdx.x] = s;
+  __syncthreads();
+  if (threadIdx.x < CQ_COUNT) {
+    s = 0.0;
+    for (int k = 0; k < ER_THREADS / CQ_COUNT; k++) s += s_q[k * CQ_COUNT + q];
+    s_q[q] = 0.5 * s;
+    __syncwarp(0xffff);
+    if (q == 0) {
+      int m = E.mask;
+      if (E.sitems) m &= (E.sp[sy].ninter > 0 ? 1 : 0) | (E.sp[sy].coul >= 0 ? 2 : 0);
+      cw_apply(m, s_q, acc + (size_t)sy * ACC_STRIDE);
+    }
+  }
+}
+
+// Sum of charge jq's partial k-space forces (one triple per split; jq < 0:
+// none).  SL > 1: a block of SL warps, warp `slice` taking every SL-th split of
+// 32 charges; the first warp returns the sums.
+template <int SL>
+__device__ __forceinline__ void split_sum(const double *__restrict__ part, int nsplit, int nq, int jq, int slice,
+                                          double (&ks)[3]) {
+  ks[0] = ks[1] = ks[2] = 0.0;
+  if (jq >= 0) {
+#pragma unroll 4
+    for (int y = slice; y < nsplit; y += SL) {
+      const double *p = part + (size_t)3 * y * nq + jq;
+      ks[0] += p[0];
+      ks[1] += p[nq];
+      ks[2] += p[2 * (size_t)nq];
+    }
+  }
+  if (SL > 1) {
+    __shared__ double s_k[SL][3][32];
+    const int lane = threadIdx.x & 31;
+    for (int d = 0; d < 3; d++) s_k[slice][d][lane] = ks[d];
+    __syncthreads();
+    if (slice == 0)
+      for (int w = 1; w < SL; w++)
+        for (int d = 0; d < 3; d++) ks[d] += s_k[w][d][lane];
+  }
+}
+constexpr int SPLIT_WARPS = 8;
+
 struct Ctx {
   // ---- configuration
   int dev = 0;
@@ -386,7 +483,9 @@ struct Ctx {
   int2 *ecorr_pairs = nullptr;          // CM3D's iecorr/jecorr order
   // ---- bonded groups (connected components of bonds/bends/ecorr)
   int ngroups = 0;
-  int *qidx = nullptr;                  // per atom: its place in icharge, -1 uncharged (small_mol 3)
+  int *qidx = nullptr;                  // per atom: its place in icharge, -1 uncharged
+  bool defer_energy = false;            // the compact energy sums wait for the level's last kernel
+  EnergyItems energy_items;             //   here
   bool ecorr_side = false;              // force(1)'s molecule terms run beside the k-space (all ecorr atoms charged)
   int small_mol = 0;                    // every molecule has at most this many atoms (1, 3; 0: more) and simple terms
   int *grp_atom_off = nullptr, *grp_atoms = nullptr;
@@ -609,7 +708,7 @@ int query_steps(Ctx *c, int *done);             // nb_step.cu
 int run_force(Ctx *c, int iflg);                // nb_step.cu
 int run_bonded(Ctx *c);                         // nb_step.cu
 int group_init(Ctx *c, bool zero_fxs, bool side, bool zeroed);   // nb_step.cu
-int finish_level1(Ctx *c, double dter, double dter1, bool kick);   // nb_step.cu
+int finish_level1(Ctx *c, double dter, double dter1, bool kick, bool kparts);   // nb_step.cu
 int check_displacement(Ctx *c);                 // nb_step.cu
 int reset_positions(Ctx *c);                    // nb_step.cu
 

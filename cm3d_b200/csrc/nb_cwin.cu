@@ -63,8 +63,6 @@ constexpr int CW_RF = 8;                    // copies of the erfc force table (l
 constexpr int CW_RG = 8;                    // copies of the erfc energy table
 
 // per-item FP64 sums (each pair is seen from both ends: k_cw_ereduce halves)
-enum { CQ_EEL = 0, CQ_QQ_UNUSED, CQ_VE0, CQ_VE1, CQ_VE2, CQ_VE4, CQ_VE5, CQ_VE8,
-       CQ_ELJ, CQ_VSH, CQ_VL0, CQ_VL1, CQ_VL2, CQ_VL4, CQ_VL5, CQ_VL8, CQ_COUNT };
 
 struct CwP {
   int n, ncx, ncy, ncz, nitems, nsplit, cap, words;   // words: 8-byte words per atom slot
@@ -1075,74 +1073,12 @@ __global__ void __launch_bounds__(NG *GW * 32, 1) k_pair_cs(
   if (lane == 0 && under) atomicAdd((unsigned long long *)(stat + ST_UNDERFLOW), under);
 }
 
-// Sum of the items' partials into CM3D's accumulators: one block, warp q
-// sums quantity q over the items (fixed order), then one thread applies the
-// sums in a fixed order (several quantities feed one accumulator); each pair
-// was counted from both ends, hence 1/2.
-__device__ void cw_apply(int mask, const double *v, double *acc) {
-  if (mask & 2) {
-    // (CM3D's shifted sum spothe, finter_e.c:197, is read by nothing --
-    // getsvirter_e reports spote -- and this path does not form it)
-    acc[ACC_SPOTE] += v[CQ_EEL];
-    acc[ACC_SPRSE] -= v[CQ_VE0] + v[CQ_VE4] + v[CQ_VE8];
-    acc[ACC_SPRSET + 0] -= v[CQ_VE0];
-    acc[ACC_SPRSET + 1] -= v[CQ_VE1];
-    acc[ACC_SPRSET + 2] -= v[CQ_VE2];
-    acc[ACC_SPRSET + 4] -= v[CQ_VE4];
-    acc[ACC_SPRSET + 5] -= v[CQ_VE5];
-    acc[ACC_SPRSET + 8] -= v[CQ_VE8];
-  }
-  if (mask & 1) {
-    acc[ACC_SPOTL] += v[CQ_ELJ];
-    acc[ACC_SPOTHL] += v[CQ_ELJ] - v[CQ_VSH];
-    acc[ACC_SPRSL] -= v[CQ_VL0] + v[CQ_VL4] + v[CQ_VL8];
-    acc[ACC_SPRSLT + 0] -= v[CQ_VL0];
-    acc[ACC_SPRSLT + 1] -= v[CQ_VL1];
-    acc[ACC_SPRSLT + 2] -= v[CQ_VL2];
-    acc[ACC_SPRSLT + 4] -= v[CQ_VL4];
-    acc[ACC_SPRSLT + 5] -= v[CQ_VL5];
-    acc[ACC_SPRSLT + 8] -= v[CQ_VL8];
-  }
-}
-
-__global__ void __launch_bounds__(CQ_COUNT * 32) k_cw_ereduce(int nitems, int mask, double tablast_e,
-                                                               const double *__restrict__ ipart,
-                                                               double *__restrict__ acc, const int *__restrict__ gs) {
+// The compact systems' energy sums as a kernel of their own (force calls; a
+// step sums them in its last kernel, beside the kick).
+__global__ void __launch_bounds__(ER_THREADS) k_cw_ereduce(const __grid_constant__ EnergyItems E,
+                                                           double *__restrict__ acc, const int *__restrict__ gs) {
   if (gated_off(gs, 0)) return;
-  __shared__ double s_q[CQ_COUNT];
-  const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double s = 0.0;
-  for (int it = lane; it < nitems; it += 32) s += ipart[(size_t)it * CQ_COUNT + q];
-  s = warp_sum(s);
-  if (lane == 0) s_q[q] = 0.5 * s;
-  __syncthreads();
-  if (threadIdx.x == 0) cw_apply(mask, s_q, acc);
-}
-
-// The same for a batch's compact systems: block per system, its items
-// {first, count} (none: a gather-kernel system, nothing to do), its own
-// accumulators; LJ sums where it has LJ interactions, electrostatic ones
-// where it has charges.
-__global__ void __launch_bounds__(CQ_COUNT * 32) k_cw_ereduce_sys(int mask, const int2 *__restrict__ sitems,
-                                                                   const SysP *__restrict__ sp,
-                                                                   const double *__restrict__ ipart,
-                                                                   double *__restrict__ acc,
-                                                                   const int *__restrict__ gs) {
-  if (gated_off(gs, 0)) return;
-  const int sy = blockIdx.x;
-  const int2 r = sitems[sy];
-  if (r.y == 0) return;
-  __shared__ double s_q[CQ_COUNT];
-  const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  double s = 0.0;
-  for (int it = lane; it < r.y; it += 32) s += ipart[(size_t)(r.x + it) * CQ_COUNT + q];
-  s = warp_sum(s);
-  if (lane == 0) s_q[q] = 0.5 * s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const int m = mask & ((sp[sy].ninter > 0 ? 1 : 0) | (sp[sy].coul >= 0 ? 2 : 0));
-    cw_apply(m, s_q, acc + (size_t)sy * ACC_STRIDE);
-  }
+  energy_sums(E, blockIdx.x, acc);
 }
 
 // ------------------------------------------------------------------ host
@@ -1760,10 +1696,13 @@ int cw_pairs(Ctx *c, int mask, double *fout) {
 }
 
 int cw_ereduce(Ctx *c, int mask) {
-  if (c->cw_batch)
-    k_cw_ereduce_sys<<<c->nsys, CQ_COUNT * 32, 0, c->st>>>(mask, c->cw_sitems, c->sp, c->cw_part, c->acc, c->gate);
-  else
-    k_cw_ereduce<<<1, CQ_COUNT * 32, 0, c->st>>>(c->cw_nitems, mask, c->tablast_e, c->cw_part, c->acc, c->gate);
+  const EnergyItems E = {c->cw_part, c->cw_batch ? c->cw_sitems : nullptr, c->sp, c->cw_nitems, mask,
+                         c->cw_batch ? c->nsys : 1};
+  if (c->defer_energy) {
+    c->energy_items = E;
+    return CM3D_NB_OK;
+  }
+  k_cw_ereduce<<<E.count, ER_THREADS, 0, c->st>>>(E, c->acc, c->gate);
   c->launches++;
   CKL(c);
   return CM3D_NB_OK;

@@ -448,7 +448,7 @@ __global__ void __launch_bounds__(KS_THREADS) k_kforce_mixed(int nq, const uint4
     double fy = __dmul_rn(t, fma(hmati[7], U2[m], fma(hmati[4], U1[m], __dmul_rn(hmati[1], U0[m]))));
     double fz = __dmul_rn(t, fma(hmati[8], U2[m], fma(hmati[5], U1[m], __dmul_rn(hmati[2], U0[m]))));
     if (part) {
-      // one partial per row split, summed in a fixed order by k_kforce_sum
+      // one partial per row split, summed in a fixed order by split_sum
       const size_t o = (size_t)3 * blockIdx.y * nq + jq[m];
       part[o] = fx;
       part[o + nq] = fy;
@@ -888,28 +888,29 @@ __global__ void __launch_bounds__(KR_THREADS) k_kforce_reg(
   }
 }
 
-// the row splits' partial reciprocal forces of every charged atom (and the
-// molecule terms' partial, where they run beside the k-space), summed in
-// split order (deterministic: the same result whatever else the device runs);
-// eight partials' loads in flight at a time
-__global__ void k_kforce_sum(int nq, int nsplit, const double *__restrict__ part, const int *__restrict__ icharge,
-                             int n, double *__restrict__ fxl, const int *__restrict__ gs) {
+// fxl += the partial forces of every charge, in split order (a force call's; a
+// step adds them in its last kernel)
+template <int SL>
+__global__ void __launch_bounds__(256) k_kforce_sum(int nq, int nsplit, const double *__restrict__ part,
+                                                    const int *__restrict__ icharge, int n, double *__restrict__ fxl,
+                                                    const int *__restrict__ gs) {
   if (gated_off(gs, 0)) return;
-  const int jq = blockIdx.x * blockDim.x + threadIdx.x;
-  if (jq >= nq) return;
+  const int slice = SL > 1 ? threadIdx.x >> 5 : 0;
+  const int jq = SL > 1 ? blockIdx.x * 32 + (threadIdx.x & 31) : blockIdx.x * blockDim.x + threadIdx.x;
+  double ks[3];
+  split_sum<SL>(part, nsplit, nq, jq < nq ? jq : -1, slice, ks);
+  if (slice > 0 || jq >= nq) return;
   const int i = icharge[jq];
-  const double f0 = fxl[i], f1 = fxl[n + i], f2 = fxl[2 * n + i];
-  double fx = 0, fy = 0, fz = 0;
-#pragma unroll 8
-  for (int y = 0; y < nsplit; y++) {
-    const size_t o = (size_t)3 * y * nq + jq;
-    fx += part[o];
-    fy += part[o + nq];
-    fz += part[o + 2 * (size_t)nq];
-  }
-  fxl[i] = f0 + fx;
-  fxl[n + i] = f1 + fy;
-  fxl[2 * n + i] = f2 + fz;
+  for (int d = 0; d < 3; d++) fxl[d * n + i] += ks[d];
+}
+
+static void kforce_sum(Ctx *c, int nsplit, cudaStream_t st) {
+  const int nq = c->ncharge;
+  if (nq < 256 * c->num_sms)
+    k_kforce_sum<SPLIT_WARPS><<<(nq + 31) / 32, 256, 0, st>>>(nq, nsplit, c->kf_part, c->icharge, c->n, c->fxl, c->gate);
+  else
+    k_kforce_sum<1><<<grid_for(nq, 256), 256, 0, st>>>(nq, nsplit, c->kf_part, c->icharge, c->n, c->fxl, c->gate);
+  c->launches++;
 }
 
 // ------------------------------------------------------------ plain FP64
@@ -1141,8 +1142,7 @@ static int kspace_run_reg(Ctx *c, cudaStream_t st, bool defer, double vol) {
   }
   c->launches += 6;
   if (!defer) {
-    k_kforce_sum<<<grid_for(nq, 256), 256, 0, st>>>(nq, c->kf_split, c->kf_part, c->icharge, c->n, c->fxl, c->gate);
-    c->launches++;
+    kforce_sum(c, c->kf_split, st);
   }
   tend(c, 1, e0);
   CKL(c);
@@ -1313,9 +1313,7 @@ static int kspace_forces_batch(Ctx *c, cudaStream_t st, bool defer) {
                                                                  c->fxl, part, c->sp, c->ftile_sys, c->gate);
   c->launches += 4;
   if (part && !defer) {
-    k_kforce_sum<<<grid_for(c->ncharge, 256), 256, 0, st>>>(c->ncharge, c->kf_split, part, c->icharge, c->n,
-                                                                c->fxl, c->gate);
-    c->launches++;
+    kforce_sum(c, c->kf_split, st);
   }
   tend(c, 1, e0);
   CKL(c);
@@ -1367,9 +1365,7 @@ static int kspace_run(Ctx *c, cudaStream_t st, bool defer) {
                                                             0, c->fxl, split > 1 || defer ? c->kf_part : nullptr,
                                                             nullptr, nullptr, c->gate);
     if (split > 1 && !defer) {
-      k_kforce_sum<<<grid_for(c->ncharge, 256), 256, 0, st>>>(c->ncharge, split, c->kf_part, c->icharge,
-                                                                  c->n, c->fxl, c->gate);
-      c->launches++;
+      kforce_sum(c, split, st);
     }
   } else {
     dim3 gf((c->ncharge + 255) / 256, split);
@@ -1408,15 +1404,10 @@ int kspace_fork(Ctx *c) {
   return CM3D_NB_OK;
 }
 
-// Join: the main stream waits for the forked k-space and adds its partial
-// forces to fxl in split order (after the pair forces, as without the fork)
+// Join: the main stream waits for the forked k-space; the level's last kernel
+// adds its partial forces to fxl in split order, after the pair forces
 int kspace_join(Ctx *c) {
   CK(cudaStreamWaitEvent(c->st, c->ev_join, 0));
-  const int B = c->ncharge < 256 * c->num_sms ? 64 : 256;
-  k_kforce_sum<<<grid_for(c->ncharge, B), B, 0, c->st>>>(c->ncharge, c->kf_split + (c->ecorr_side ? 1 : 0), c->kf_part,
-                                                         c->icharge, c->n, c->fxl, c->gate);
-  c->launches++;
-  CKL(c);
   return CM3D_NB_OK;
 }
 

@@ -917,7 +917,7 @@ __global__ void k_group_init(StepP P, const int *__restrict__ gwork, int ngw, co
 // bonds and one bend: positions, charges and forces in registers, the terms
 // unrolled (their erf, exp and acos overlap).  The ecorr forces are added to
 // fxl, or -- where the kernel runs beside the k-space -- written to `part`,
-// one triple per charged atom, which k_kforce_sum adds.
+// one triple per charged atom, which split_sum adds.
 __global__ void __launch_bounds__(128) k_group_small(
     StepP P, const int *__restrict__ gwork, int ngw, const int *__restrict__ gaoff, const int *__restrict__ gatoms,
     const double *__restrict__ pos, const double *__restrict__ q, double *__restrict__ fxl, double *__restrict__ part,
@@ -1132,20 +1132,45 @@ __global__ void k_intra_energy(StepP P, const int *__restrict__ gaoff, const int
   });
 }
 
-// end of force(1) / force(0): rmass (utils/md_util.new.c:219) and, inside
-// step(), the closing kick of md_step.c:139-145; then the kinetic tensor of
-// get_p2mt (md_fcntr.c:332-354) for geteng
-__global__ void k_finish(int n, int level, int kick, int rm_l, int rm_s, double dk_l, double dk_s,
+// The k-space's partial forces, one triple per split and charged atom
+struct KParts {
+  const double *part = nullptr;     // null: none to add
+  const int *qidx = nullptr;
+  int nsplit = 0, nq = 0;
+};
+
+// end of force(1) / force(0): the partial k-space forces into fxl, rmass
+// (utils/md_util.new.c:219) and, inside step(), the closing kick of
+// md_step.c:139-145; then the kinetic tensor of get_p2mt (md_fcntr.c:332-354)
+// for geteng.  The last E.count blocks sum the compact pair kernels' energies.
+//
+// Bound by latency in small systems: SL warps of a block share the splits of 32
+// atoms, so that their loads are in flight at once, and the sums that were
+// kernels before and beside this one are part of it (us per step, before and
+// after: 2048 argon atoms 66, 62; 2048 charged ones, 32 splits, 81, 64; 12,288
+// water atoms 147, 136; 37 boxes 174, 160).
+template <int SL>
+__global__ void __launch_bounds__(256) k_finish(
+                         int n, int level, int kick, int rm_l, int rm_s, double dk_l, double dk_s,
                          const double *__restrict__ mass, double *__restrict__ fxl, double *__restrict__ fxs,
                          double *__restrict__ vel, double *__restrict__ acc, int *__restrict__ istate,
                          int advance_step, const int *__restrict__ sys_of, int batch,
                          const int *__restrict__ gs, const unsigned char *__restrict__ frz, int *__restrict__ reb,
-                         int nreb) {
+                         int nreb, const __grid_constant__ KParts K, const __grid_constant__ EnergyItems E) {
   if (gated_off(gs, 0)) return;
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int nb = gridDim.x - E.count;                     // blocks of atoms
+  if ((int)blockIdx.x >= nb) {
+    energy_sums(E, blockIdx.x - nb, acc);
+    return;
+  }
+  const int slice = SL > 1 ? threadIdx.x >> 5 : 0;
+  int i = SL > 1 ? blockIdx.x * 32 + (threadIdx.x & 31) : blockIdx.x * blockDim.x + threadIdx.x;
+  double ks[3];
+  if (K.part) split_sum<SL>(K.part, K.nsplit, K.nq, i < n ? K.qidx[i] : -1, slice, ks);
+  if (slice > 0) i = n;                                   // the first warp goes on
   // a replayed level leaves the rebuild requests cleared for the next one (a
   // halted one keeps them for the host-driven path that finishes it)
-  for (int k = i; k < nreb; k += gridDim.x * blockDim.x) reb[k] = 0;
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nreb; k += nb * blockDim.x) reb[k] = 0;
   if (i == 0 && nreb > 0) {
     istate[IS_REBUILD] = 0;
     istate[IS_LREBUILD] = 0;
@@ -1160,7 +1185,8 @@ __global__ void k_finish(int n, int level, int kick, int rm_l, int rm_s, double 
     const bool frozen = frz && frz[i];
     for (int d = 0; d < 3; d++) {
       int x = d * n + i;
-      if (rm_l) fxl[x] *= r;
+      if (K.part) fxl[x] = (fxl[x] + ks[d]) * (rm_l ? r : 1.);
+      else if (rm_l) fxl[x] *= r;
       if (rm_s) fxs[x] *= r;
       if (frozen) {
         if (level == 1) fxl[x] = 0.;
@@ -1617,6 +1643,13 @@ int step_setup(Ctx *c, const cm3d_nb_system *systems, int nsys) {
     if (!work.empty()) CK(cudaMemcpy(c->grp_work, work.data(), sizeof(int) * work.size(), cudaMemcpyHostToDevice));
   }
   if ((rc = upload_intra(c, ih, gid, ng))) return rc;
+  std::vector<int> qi((size_t)n, -1), ich((size_t)c->ncharge);
+  if (c->ncharge > 0) {
+    CK(cudaMemcpy(ich.data(), c->icharge, sizeof(int) * ich.size(), cudaMemcpyDeviceToHost));
+    for (int k = 0; k < c->ncharge; k++) qi[(size_t)ich[(size_t)k]] = k;
+    CK(cudaMalloc(&c->qidx, sizeof(int) * (size_t)n));
+    CK(cudaMemcpy(c->qidx, qi.data(), sizeof(int) * (size_t)n, cudaMemcpyHostToDevice));
+  }
   // molecules small enough for the register form of the inner level
   c->small_mol = 0;
   if (!c->has_intra_x && !c->intra.frz) {
@@ -1630,13 +1663,8 @@ int step_setup(Ctx *c, const cm3d_nb_system *systems, int nsys) {
     c->small_mol = ma == 1 && mb2 + me2 + mc2 == 0 ? 1 : (ma <= 3 && mb2 <= 2 && me2 <= 1 && mc2 <= 3 ? 3 : 0);
     if (c->small_mol == 3 && nc > 0) {
       // force(1)'s molecule terms beside the k-space: their forces go by charge
-      std::vector<int> qi((size_t)n, -1), ich((size_t)c->ncharge);
-      if (c->ncharge > 0) CK(cudaMemcpy(ich.data(), c->icharge, sizeof(int) * ich.size(), cudaMemcpyDeviceToHost));
-      for (int k = 0; k < c->ncharge; k++) qi[(size_t)ich[(size_t)k]] = k;
       c->ecorr_side = true;
       for (int b = 0; b < nc; b++) c->ecorr_side = c->ecorr_side && qi[(size_t)mc[b].x] >= 0 && qi[(size_t)mc[b].y] >= 0;
-      CK(cudaMalloc(&c->qidx, sizeof(int) * (size_t)n));
-      CK(cudaMemcpy(c->qidx, qi.data(), sizeof(int) * (size_t)n, cudaMemcpyHostToDevice));
     }
   }
   return nvt_setup(c, systems, nsys);
@@ -1717,21 +1745,30 @@ int group_init(Ctx *c, bool zero_fxs, bool side, bool zeroed) {
   return CM3D_NB_OK;
 }
 
-int finish_level1(Ctx *c, double dter, double dter1, bool kick) {
-  const int B = 256;
+int finish_level1(Ctx *c, double dter, double dter1, bool kick, bool kparts) {
+  const int B = ER_THREADS;
   bool rs = c->need_short || c->nres_lrf > 1;
-  k_finish<<<grid_for(c->n, B), B, 0, c->st>>>(c->n, 1, kick ? 1 : 0, 1, rs ? 1 : 0, dter, dter1, c->mass, c->fxl,
-                                               c->fxs, c->vel, c->acc, c->istate, kick ? 1 : 0, c->sys_of,
-                                               c->nsys > 1, c->gate, c->intra.frz, c->sreb, c->gate ? 2 * c->nsys : 0);
+  KParts K;
+  if (kparts) K = {c->kf_part, c->qidx, c->kf_split + (c->ecorr_side ? 1 : 0), c->ncharge};
+  const EnergyItems E = c->energy_items;
+  c->energy_items = EnergyItems();
+  // warps share an atom's splits while a thread per atom does not fill the GPU
+  const bool sl = K.part && c->n < B * c->num_sms;
+  const auto kern = sl ? k_finish<SPLIT_WARPS> : k_finish<1>;
+  const int blocks = (sl ? (c->n + 31) / 32 : (c->n + B - 1) / B) + E.count;
+  kern<<<blocks, B, 0, c->st>>>(c->n, 1, kick ? 1 : 0, 1, rs ? 1 : 0, dter, dter1, c->mass, c->fxl, c->fxs, c->vel,
+                                c->acc, c->istate, kick ? 1 : 0, c->sys_of, c->nsys > 1, c->gate, c->intra.frz,
+                                c->sreb, c->gate ? 2 * c->nsys : 0, K, E);
   c->launches++;
   CKL(c);
   return CM3D_NB_OK;
 }
 
 static int finish_level0(Ctx *c, double dts2, bool kick) {
-  k_finish<<<grid_for(c->n, 256), 256, 0, c->st>>>(c->n, 0, kick ? 1 : 0, 0, 1, 0, dts2, c->mass, c->fxl, c->fxs,
+  k_finish<1><<<grid_for(c->n, 256), 256, 0, c->st>>>(c->n, 0, kick ? 1 : 0, 0, 1, 0, dts2, c->mass, c->fxl, c->fxs,
                                                    c->vel, c->acc, c->istate, 0, c->sys_of, c->nsys > 1, c->gate,
-                                                   c->intra.frz, c->sreb, c->gate ? 2 * c->nsys : 0);
+                                                   c->intra.frz, c->sreb, c->gate ? 2 * c->nsys : 0, KParts(),
+                                                   EnergyItems());
   c->launches++;
   CKL(c);
   return CM3D_NB_OK;
@@ -1785,7 +1822,7 @@ int run_force(Ctx *c, int iflg) {
     if ((rc = group_init(c, true, false, false))) return rc;
     if ((rc = pair_forces(c, 1, 3))) return rc;
     if ((rc = kspace_forces(c))) return rc;
-    return finish_level1(c, 0, 0, false);
+    return finish_level1(c, 0, 0, false, false);
   }
   if (iflg == 0) {
     CK(cudaMemsetAsync(c->fxs, 0, sizeof(double) * 3 * (size_t)c->n, c->st));
@@ -1806,9 +1843,12 @@ static int close_level(Ctx *c, int intr, bool ks_forked = false, bool zeroed = f
   if (intr == c->nres_lrf - 1) {
     if (!ks_forked && !zeroed && (rc = zero_acc(c))) return rc;
     if ((rc = group_init(c, P.use_fxs, ks_forked && c->ecorr_side, zeroed))) return rc;
-    if ((rc = pair_forces(c, 1, 3))) return rc;
+    c->defer_energy = true;
+    rc = pair_forces(c, 1, 3);
+    c->defer_energy = false;
+    if (rc) return rc;
     if ((rc = ks_forked ? kspace_join(c) : kspace_forces(c))) return rc;
-    return finish_level1(c, P.dter, P.dter1, true);
+    return finish_level1(c, P.dter, P.dter1, true, ks_forked);
   }
   CK(cudaMemsetAsync(c->fxs, 0, sizeof(double) * 3 * (size_t)c->n, c->st));
   if ((rc = pair_forces(c, 0, 3))) return rc;
