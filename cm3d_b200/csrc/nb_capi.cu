@@ -620,6 +620,7 @@ static double *block_of(Ctx *c, int which) {
 }
 
 static int pull_acc(Ctx *c) {
+  if (c->acc_here) return CM3D_NB_OK;
   CK(cudaMemcpyAsync(c->h_acc, c->acc, sizeof(double) * (size_t)c->nsys * ACC_STRIDE, cudaMemcpyDeviceToHost,
                      c->st));
   CK(cudaStreamSynchronize(c->st));
@@ -697,7 +698,7 @@ void cm3d_nb_destroy(cm3d_nb_ctx *ctx) {
 }
 
 // every entry point first finishes asynchronously launched steps
-#define CTX                                         \
+#define CTX_READ                                    \
   Ctx *c = reinterpret_cast<Ctx *>(ctx);            \
   if (!c) {                                         \
     set_error("null context");                      \
@@ -711,9 +712,19 @@ void cm3d_nb_destroy(cm3d_nb_ctx *ctx) {
       if (_rc) return _rc;                          \
     }                                               \
   } while (0)
+// any call that may change the accumulators: a copy made with the steps is stale
+#define CTX  \
+  CTX_READ;  \
+  c->acc_here = false
 
+// (blocks that lie back to back, as in a (3, n) array, go in one copy)
 static int put3(Ctx *c, double *dst, const double *x, const double *y, const double *z) {
   const size_t n = c->n;
+  if (y == x + n && z == y + n) {
+    CK(cudaMemcpyAsync(dst, x, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, c->st));
+    CK(cudaStreamSynchronize(c->st));
+    return CM3D_NB_OK;
+  }
   CK(cudaMemcpyAsync(dst, x, sizeof(double) * n, cudaMemcpyHostToDevice, c->st));
   CK(cudaMemcpyAsync(dst + n, y, sizeof(double) * n, cudaMemcpyHostToDevice, c->st));
   CK(cudaMemcpyAsync(dst + 2 * n, z, sizeof(double) * n, cudaMemcpyHostToDevice, c->st));
@@ -723,6 +734,11 @@ static int put3(Ctx *c, double *dst, const double *x, const double *y, const dou
 
 static int get3(Ctx *c, const double *src, double *x, double *y, double *z) {
   const size_t n = c->n;
+  if (y == x + n && z == y + n) {
+    CK(cudaMemcpyAsync(x, src, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, c->st));
+    CK(cudaStreamSynchronize(c->st));
+    return CM3D_NB_OK;
+  }
   CK(cudaMemcpyAsync(x, src, sizeof(double) * n, cudaMemcpyDeviceToHost, c->st));
   CK(cudaMemcpyAsync(y, src + n, sizeof(double) * n, cudaMemcpyDeviceToHost, c->st));
   CK(cudaMemcpyAsync(z, src + 2 * n, sizeof(double) * n, cudaMemcpyDeviceToHost, c->st));
@@ -809,7 +825,7 @@ int cm3d_nb_set_box(cm3d_nb_ctx *ctx, const double hmat[9]) {
 }
 
 int cm3d_nb_get_positions(cm3d_nb_ctx *ctx, double *px, double *py, double *pz) {
-  CTX;
+  CTX_READ;
   return get3(c, c->pos, px, py, pz);
 }
 int cm3d_nb_set_velocities(cm3d_nb_ctx *ctx, const double *vx, const double *vy, const double *vz) {
@@ -817,7 +833,7 @@ int cm3d_nb_set_velocities(cm3d_nb_ctx *ctx, const double *vx, const double *vy,
   return put3(c, c->vel, vx, vy, vz);
 }
 int cm3d_nb_get_velocities(cm3d_nb_ctx *ctx, double *vx, double *vy, double *vz) {
-  CTX;
+  CTX_READ;
   return get3(c, c->vel, vx, vy, vz);
 }
 int cm3d_nb_get_forces(cm3d_nb_ctx *ctx, int which, double *fx, double *fy, double *fz) {
@@ -852,8 +868,7 @@ int cm3d_nb_nrefsh(cm3d_nb_ctx *ctx, int istep, int *rebuilt) {
     set_error("nrefsh() before get_ngbr()");
     return CM3D_NB_ERR_STATE;
   }
-  c->h_istate[IS_ISTEP] = istep;
-  CK(cudaMemcpyAsync(c->istate + IS_ISTEP, c->h_istate + IS_ISTEP, sizeof(int), cudaMemcpyHostToDevice, c->st));
+  if ((rc = begin_steps(c, istep))) return rc;
   if ((rc = check_displacement(c))) return rc;
   if ((rc = reset_positions(c))) return rc;
   CK(cudaMemcpyAsync(c->h_istate, c->istate, sizeof(int) * IS_COUNT, cudaMemcpyDeviceToHost, c->st));
@@ -1083,7 +1098,7 @@ int cm3d_nb_step_query(cm3d_nb_ctx *ctx, int *done) {
 }
 
 int cm3d_nb_step_wait(cm3d_nb_ctx *ctx) {
-  CTX;   // finishes the pending steps
+  CTX_READ;   // finishes the pending steps
   return CM3D_NB_OK;
 }
 
@@ -1143,7 +1158,7 @@ int cm3d_nb_get_energies(cm3d_nb_ctx *ctx, cm3d_nb_energies *e) {
 }
 
 int cm3d_nb_get_system_energies(cm3d_nb_ctx *ctx, int sys, cm3d_nb_energies *e) {
-  CTX;
+  CTX_READ;
   int rc;
   if (sys < 0 || sys >= c->nsys) {
     set_error("get_system_energies: system %d of %d", sys, c->nsys);
@@ -1155,7 +1170,7 @@ int cm3d_nb_get_system_energies(cm3d_nb_ctx *ctx, int sys, cm3d_nb_energies *e) 
 }
 
 int cm3d_nb_get_all_energies(cm3d_nb_ctx *ctx, cm3d_nb_energies *e) {
-  CTX;
+  CTX_READ;
   int rc;
   if ((rc = pull_acc(c))) return rc;
   for (int s = 0; s < c->nsys; s++) energies_of(c, s, e + s);

@@ -484,6 +484,7 @@ struct Ctx {
   // ---- bonded groups (connected components of bonds/bends/ecorr)
   int ngroups = 0;
   int *qidx = nullptr;                  // per atom: its place in icharge, -1 uncharged
+  bool acc_coming = false, acc_here = false;   // h_acc: on its way with the steps' state, valid until the next change
   bool defer_energy = false;            // the compact energy sums wait for the level's last kernel
   EnergyItems energy_items;             //   here
   bool ecorr_side = false;              // force(1)'s molecule terms run beside the k-space (all ecorr atoms charged)
@@ -659,6 +660,8 @@ using DevLock = std::lock_guard<std::recursive_mutex>;
 int list_setup(Ctx *c);                         // nb_list.cu
 void cell_shifts(SysP &P, const SysH &H);       // nb_list.cu
 int take_snapshot(Ctx *c, bool device_flag, bool all, bool lists);   // nb_list.cu
+constexpr int ACC_WITH_STATE = 64;              // most systems whose accumulators are copied after every step call
+int begin_steps(Ctx *c, int istep);              // nb_step.cu
 int refresh_corners(Ctx *c);                    // nb_list.cu: cell corners under a new box
 int pair_forces(Ctx *c, int iflg, int which);   // nb_pair.cu: which 0 LJ, 1 elec, 2 fused
 int pair_setup(Ctx *c);                         // nb_pair.cu

@@ -1782,9 +1782,28 @@ static int clear_rebuild(Ctx *c) {
   return CM3D_NB_OK;
 }
 
+// The step number of the next step (or test) and cleared rebuild requests, in
+// one launch where a copy from the host and two memsets took three.
+__global__ void k_begin(int istep, int *__restrict__ istate, int *__restrict__ reb, int nreb) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < nreb) reb[i] = 0;
+  if (i == 0) {
+    istate[IS_ISTEP] = istep;
+    istate[IS_REBUILD] = 0;
+    istate[IS_LREBUILD] = 0;
+  }
+}
+
+int begin_steps(Ctx *c, int istep) {
+  c->h_istate[IS_ISTEP] = istep;
+  k_begin<<<grid_for(2 * c->nsys, 256), 256, 0, c->st>>>(istep, c->istate, c->sreb, 2 * c->nsys);
+  c->launches++;
+  CKL(c);
+  return CM3D_NB_OK;
+}
+
+// (after begin_steps)
 int check_displacement(Ctx *c) {
-  int rc;
-  if ((rc = clear_rebuild(c))) return rc;
   k_disp<<<grid_for(c->n, 256), 256, 0, c->st>>>(c->n, c->sp, c->sys_of, c->pos, c->dxn, c->dxi, c->sreb, c->lreb,
                                                   c->istate);
   c->launches++;
@@ -1963,12 +1982,6 @@ static int one_step(Ctx *c, bool gated) {
   return host_outputs_tail(c);
 }
 
-static int set_istep(Ctx *c, int istep) {
-  c->h_istate[IS_ISTEP] = istep;
-  CK(cudaMemcpyAsync(c->istate + IS_ISTEP, c->h_istate + IS_ISTEP, sizeof(int), cudaMemcpyHostToDevice, c->st));
-  return CM3D_NB_OK;
-}
-
 // the end of a step with registered host outputs: join the positions' copy
 // and copy the velocities
 int host_outputs_tail(Ctx *c) {
@@ -1996,7 +2009,7 @@ int launch_steps(Ctx *c, int istep0, int nsteps) {
     return CM3D_NB_ERR_STATE;
   }
   if (nsteps <= 0) return CM3D_NB_OK;
-  if ((rc = set_istep(c, istep0))) return rc;
+  if ((rc = begin_steps(c, istep0))) return rc;
   cudaEvent_t e4;
   if (!c->use_graph || c->timing.on) {
     tbegin(c, 4, &e4);
@@ -2007,8 +2020,7 @@ int launch_steps(Ctx *c, int istep0, int nsteps) {
   }
   // graph replay: one captured step, every kernel gated on the device state
   // (rebuild flag; halt after a list overflow), the rebuild requests cleared
-  // once here and by each level's last kernel
-  if ((rc = clear_rebuild(c))) return rc;
+  // by begin_steps and by each level's last kernel
   if (!c->graph) {
     DevLock lock(device_mutex());
     cudaGraph_t g;
@@ -2032,6 +2044,11 @@ int launch_steps(Ctx *c, int istep0, int nsteps) {
   }
   tend(c, 4, e4);
   CK(cudaMemcpyAsync(c->h_istate, c->istate, sizeof(int) * IS_COUNT, cudaMemcpyDeviceToHost, c->st));
+  // a few systems' accumulators come with the state: the energies read after
+  // the steps then need no round trip of their own
+  c->acc_coming = c->nsys <= ACC_WITH_STATE;
+  if (c->acc_coming)
+    CK(cudaMemcpyAsync(c->h_acc, c->acc, sizeof(double) * (size_t)c->nsys * ACC_STRIDE, cudaMemcpyDeviceToHost, c->st));
   if (!c->step_ev) CK(cudaEventCreateWithFlags(&c->step_ev, cudaEventDisableTiming));
   CK(cudaEventRecord(c->step_ev, c->st));
   c->pending = true;
@@ -2054,7 +2071,10 @@ int finish_steps(Ctx *c) {
   }
   CK(cudaEventSynchronize(c->step_ev));
   c->pending = false;
-  if (!c->h_istate[IS_HALT]) return CM3D_NB_OK;
+  if (!c->h_istate[IS_HALT]) {
+    c->acc_here = c->acc_coming;
+    return CM3D_NB_OK;
+  }
   const int istep0 = c->pend_istep0, nsteps = c->pend_nsteps;
   c->overflows_host++;
   const int failed = c->h_istate[IS_ISTEP], intr = c->h_istate[IS_INTR];
