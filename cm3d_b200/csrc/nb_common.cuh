@@ -341,6 +341,32 @@ __device__ __forceinline__ void split_sum(const double *__restrict__ part, int n
 }
 constexpr int SPLIT_WARPS = 8;
 
+// A barrier over a cluster of nb blocks; what its threads wrote before is
+// visible after.
+__device__ __forceinline__ void cluster_sync(int nb) {
+  if (nb == 1) {
+    __syncthreads();
+    return;
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+template <typename... K, typename... A>
+static inline cudaError_t cluster_launch(void (*kern)(K...), int blocks, int cluster, int threads, cudaStream_t st,
+                                         A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)blocks);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.stream = st;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = (unsigned)cluster;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
 struct Ctx {
   // ---- configuration
   int dev = 0;

@@ -277,14 +277,6 @@ __global__ void k_sorted_init(int n, const SysP *__restrict__ sp, const int *__r
 // earlier in the kernel is read again after another block's write, except the
 // counters, which go through L2.
 constexpr int BIN_THREADS = 1024, BIN_CLUSTER = 8, BIN_ATOMS = 4 * BIN_CLUSTER * BIN_THREADS;
-__device__ __forceinline__ void bin_sync(int nb) {
-  if (nb == 1) {
-    __syncthreads();
-    return;
-  }
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __global__ void __launch_bounds__(BIN_THREADS, 1) k_bin(
     int n, int nb, const SysP *__restrict__ sp, const int *__restrict__ sreb, int all, const __grid_constant__ Sorted S,
     int4 *cimg, int *cell_of, int *count, int *cell_start, long long *keys, int *cell_atoms,
@@ -296,13 +288,13 @@ __global__ void __launch_bounds__(BIN_THREADS, 1) k_bin(
   const int m = P.ncells, c0 = P.c0, a0 = P.a0, a1 = P.a0 + P.n;
   const int t0 = rank * BIN_THREADS + threadIdx.x, nt = nb * BIN_THREADS;
   for (int k = t0; k < m; k += nt) count[c0 + k] = 0;
-  bin_sync(nb);
+  cluster_sync(nb);
   for (int i = a0 + t0; i < a1; i += nt) {
     const int cell = place_in_cell(P, n, i, S.pos, cimg);
     cell_of[i] = cell;
     atomicAdd(count + cell, 1);
   }
-  bin_sync(nb);
+  cluster_sync(nb);
   if (rank == 0) {
     // cell_start: exclusive scan of the counts, `chunk` cells per thread
     __shared__ int part[32];
@@ -338,12 +330,12 @@ __global__ void __launch_bounds__(BIN_THREADS, 1) k_bin(
     }
     if (t == BIN_THREADS - 1) cell_start[c0 + m] = a1;
   }
-  bin_sync(nb);
+  cluster_sync(nb);
   for (int i = a0 + t0; i < a1; i += nt) {
     const int cell = cell_of[i];                          // this thread's own
     keys[cell_start[cell] + atomicAdd(count + cell, 1)] = sort_key(S.itype, i);
   }
-  bin_sync(nb);
+  cluster_sync(nb);
   // k_cell_sort's order: each atom's place is the number of smaller keys in
   // its cell (neighbouring threads share the cell and read the same key)
   for (int u = a0 + t0; u < a1; u += nt) {
@@ -1700,19 +1692,9 @@ int build_lists(Ctx *c, bool device_flag, bool all) {
   tbegin(c, 2, &e0);
   int4 *cimg = c->cimg;
   if (c->bin_cluster > 0) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(c->nsys * c->bin_cluster));
-    cfg.blockDim = dim3(BIN_THREADS);
-    cfg.stream = c->st;
-    cudaLaunchAttribute at = {};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = (unsigned)c->bin_cluster;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    CK(cudaLaunchKernelEx(&cfg, k_bin, n, c->bin_cluster, (const SysP *)c->sp, (const int *)c->lreb, al,
-                          sorted_arrays(c), cimg, c->cell_of, c->cell_cursor, c->cell_start, c->bin_keys,
-                          c->cell_atoms, gate));
+    CK(cluster_launch(k_bin, c->nsys * c->bin_cluster, c->bin_cluster, BIN_THREADS, c->st, n, c->bin_cluster,
+                      (const SysP *)c->sp, (const int *)c->lreb, al, sorted_arrays(c), cimg, c->cell_of,
+                      c->cell_cursor, c->cell_start, c->bin_keys, c->cell_atoms, gate));
     c->launches++;
   } else {
     k_cell_zero<<<grid_for(c->ncells, B), B, 0, c->st>>>(c->ncells, c->cell_sys, c->lreb, al, c->cell_cursor, gate);

@@ -586,83 +586,110 @@ __global__ void __launch_bounds__(128) k_inner_small(
 // integrate/md_therm.new.c:278-333, called between the two half drifts of
 // every inner substep, md_step.c:117).  The chain update needs every
 // thermostat's kinetic sum, a reduction over all groups, so each inner
-// substep runs as four launches: k_nvt_a (kicks, first half drift, the
-// first velocity scaling, each atom's kinetic term), k_nvt_ksum (the
-// thermostats' kinetic sums in a fixed order), k_nvt_chain (one thread per
-// thermostat) and k_nvt_c (second scaling, second half drift, bonded
-// forces, kicks and, at the level's end, the displacement test).
+// substep has four stages: nvt_first (kicks, first half drift, the first
+// velocity scaling, each atom's kinetic term), nvt_chunk (the thermostats'
+// kinetic sums in a fixed order), nvt_chain (one thread per thermostat) and
+// nvt_second (second scaling, second half drift, bonded forces, kicks and, at
+// the level's end, the displacement test) -- in one cluster of blocks
+// (k_nvt_cluster) or a launch each (k_nvt_a, k_nvt_ksum, k_nvt_chain, k_nvt_c).
 
-__device__ __forceinline__ double nhc_factor(int thm, int nchain, double dta2, const double *__restrict__ veta) {
-  return exp(-dta2 * (thm >= 0 ? veta[(size_t)thm * nchain] : 0.));
+// (through L2: in k_nvt_cluster another block's thread updates the chains)
+__device__ __forceinline__ double nhc_factor(int thm, int nchain, double dta2, const double *veta) {
+  return exp(-dta2 * (thm >= 0 ? __ldcg(veta + (size_t)thm * nchain) : 0.));
 }
 
-__global__ void k_nvt_a(StepP P, int intr, int level_start, int tors_start, const int *__restrict__ gaoff,
-                        const int *__restrict__ gatoms, double *__restrict__ pos, double *__restrict__ vel,
-                        const double *__restrict__ mass, const double *__restrict__ fxl,
-                        const double *__restrict__ fxs, const double *__restrict__ fxa,
-                        const double *__restrict__ fxr, const int *__restrict__ ithm,
-                        const double *__restrict__ veta, double *__restrict__ kin, IntraDev X,
-                        int *__restrict__ istate, const int *__restrict__ gs) {
-  if (gated_off(gs, 0)) return;
-  int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g == 0 && level_start) istate[IS_INTR] = intr;
-  if (g >= P.ngroups) return;
+struct NvtK {
+  const int *gaoff, *gatoms, *ithm;
+  double *pos, *vel;
+  const double *mass, *q, *fxl, *fxs, *veta;
+  double *fxa, *fxr, *kin;
+  const double *dxn, *dxi;
+  const int *gboff;
+  const int4 *bij;
+  const double2 *bp;
+  const int *geoff;
+  const int4 *eijk;
+  const double2 *ep;
+  const SysP *sp;
+  const int *sys_of;
+  int *sreb, *lreb, *istate;
+  IntraDev X;
+  long long *stat;
+};
+
+// group g: kicks, first half drift, first velocity scaling, kinetic terms
+__device__ __forceinline__ void nvt_first(const StepP &P, const NvtK &K, int g, int intr, bool level_start,
+                                          bool tors_start) {
   const int n = P.n;
+  double *pos = K.pos, *vel = K.vel;
+  const IntraDev &X = K.X;
   const bool tors = X.tor_off && (X.tor_off[g + 1] > X.tor_off[g] || X.o14_off[g + 1] > X.o14_off[g]);
-  for (int a = gaoff[g]; a < gaoff[g + 1]; a++) {
-    const int i = gatoms[a];
+  for (int a = K.gaoff[g]; a < K.gaoff[g + 1]; a++) {
+    const int i = K.gatoms[a];
     for (int d = 0; d < 3; d++) {
       const int x = d * n + i;
       if (level_start) {
-        if (intr == 0) vel[x] += P.dter * fxl[x] + (P.use_fxs ? P.dter1 * fxs[x] : 0.0);
-        else vel[x] += P.dts2 * fxs[x];
+        if (intr == 0) vel[x] += P.dter * K.fxl[x] + (P.use_fxs ? P.dter1 * K.fxs[x] : 0.0);
+        else vel[x] += P.dts2 * K.fxs[x];
       }
-      if (tors_start && tors) vel[x] += P.dtr2 * fxr[x];
-      vel[x] += P.dta2 * fxa[x];
+      if (tors_start && tors) vel[x] += P.dtr2 * K.fxr[x];
+      vel[x] += P.dta2 * K.fxa[x];
       pos[x] += P.dta2 * vel[x];
     }
-    const int thm = ithm[i];
-    const double e = nhc_factor(thm, P.nchain, P.dta2, veta);
+    const int thm = K.ithm[i];
+    const double e = nhc_factor(thm, P.nchain, P.dta2, K.veta);
     vel[i] *= e;
     vel[n + i] *= e;
     vel[2 * n + i] *= e;
-    // this atom's kinetic term; k_nvt_ksum adds them per thermostat in a
+    // this atom's kinetic term; nvt_chunk adds them per thermostat in a
     // fixed order (atoms without a thermostat are in no chunk)
-    kin[i] = mass[i] * (vel[i] * vel[i] + vel[n + i] * vel[n + i] + vel[2 * n + i] * vel[2 * n + i]);
+    K.kin[i] = K.mass[i] * (vel[i] * vel[i] + vel[n + i] * vel[n + i] + vel[2 * n + i] * vel[2 * n + i]);
   }
+}
+
+__global__ void k_nvt_a(StepP P, int intr, int level_start, int tors_start, const __grid_constant__ NvtK K,
+                        const int *__restrict__ gs) {
+  if (gated_off(gs, 0)) return;
+  int g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g == 0 && level_start) K.istate[IS_INTR] = intr;
+  if (g < P.ngroups) nvt_first(P, K, g, intr, level_start, tors_start);
 }
 
 // the kinetic sums of the thermostats' chunks: one warp per chunk, a lane-
 // strided sum and the warp's fixed shuffle tree (the same order every step,
 // alone or in a batch)
+// one warp: chunk ch's kinetic sum
+__device__ __forceinline__ void nvt_chunk(int ch, const int2 *__restrict__ chunk, const int *__restrict__ atoms,
+                                          const double *kin, double *chsum) {
+  const int lane = threadIdx.x & 31;
+  const int2 r = chunk[ch];
+  double s = 0.0;
+#pragma unroll 4
+  for (int k = r.x + lane; k < r.y; k += 32) s += __ldcg(kin + atoms[k]);
+  s = warp_sum(s);
+  if (lane == 0) chsum[ch] = s;
+}
+
 __global__ void k_nvt_ksum(int nchunks, const int2 *__restrict__ chunk, const int *__restrict__ atoms,
                            const double *__restrict__ kin, double *__restrict__ chsum, const int *__restrict__ gs) {
   if (gated_off(gs, 0)) return;
-  const int ch = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (ch >= nchunks) return;
-  const int2 r = chunk[ch];
-  double s = 0.0;
-  for (int k = r.x + lane; k < r.y; k += 32) s += kin[atoms[k]];
-  s = warp_sum(s);
-  if (lane == 0) chsum[ch] = s;
+  const int ch = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (ch < nchunks) nvt_chunk(ch, chunk, atoms, kin, chsum);
 }
 
 // the chain half step of one thermostat, in intnhc_new's order: links from
 // the top, forces (forcen_new, md_therm.new.c:175-198), velocities and
 // positions, the recurrence, links from the bottom
-__global__ void k_nvt_chain(int ntherm, int nchain, double dta2, double *__restrict__ nhc,
-                            const double *__restrict__ chsum, const int *__restrict__ choff,
-                            const int *__restrict__ gs) {
-  if (gated_off(gs, 0)) return;
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= ntherm) return;
+// thermostat j's chain
+__device__ __forceinline__ void nvt_chain(int j, int ntherm, int nchain, double dta2, double *__restrict__ nhc,
+                                          const double *chsum, const int *__restrict__ choff) {
   const size_t tc = (size_t)ntherm * nchain, o = (size_t)j * nchain;
   const double *m = nhc + o, *gk = nhc + tc + o;
   double *eta = nhc + 2 * tc + o, *v = nhc + 3 * tc + o, *f = nhc + 4 * tc + o;
   const double dta = 2. * dta2;
   for (int i = 0; i < nchain - 1; i++) v[i] *= exp(-dta2 * v[i + 1]);
   double p2m = 0.0;
-  for (int k = choff[j]; k < choff[j + 1]; k++) p2m += chsum[k];
+  for (int k = choff[j]; k < choff[j + 1]; k++) p2m += __ldcg(chsum + k);
   f[0] = (p2m - gk[0]) / m[0];
   for (int i = 1; i < nchain; i++) f[i] = (m[i - 1] * v[i - 1] * v[i - 1] - gk[i]) / m[i];
   for (int i = 0; i < nchain; i++) v[i] += dta2 * f[i];
@@ -672,29 +699,27 @@ __global__ void k_nvt_chain(int ntherm, int nchain, double dta2, double *__restr
   for (int i = nchain - 2; i >= 0; i--) v[i] *= exp(-dta2 * v[i + 1]);
 }
 
-__global__ void k_nvt_c(StepP P, int tors_end, int level_end, const int *__restrict__ gaoff,
-                        const int *__restrict__ gatoms, double *__restrict__ pos, double *__restrict__ vel,
-                        const double *__restrict__ mass, const double *__restrict__ q, double *__restrict__ fxa,
-                        double *__restrict__ fxr, const double *__restrict__ dxn, const double *__restrict__ dxi,
-                        const int *__restrict__ gboff,
-                        const int4 *__restrict__ bij, const double2 *__restrict__ bp,
-                        const int *__restrict__ geoff, const int4 *__restrict__ eijk,
-                        const double2 *__restrict__ ep, const int *__restrict__ ithm,
-                        const double *__restrict__ veta, const SysP *__restrict__ sp,
-                        const int *__restrict__ sys_of, int *__restrict__ sreb, int *__restrict__ lreb,
-                        int *__restrict__ istate, IntraDev X, long long *__restrict__ stat,
-                        const int *__restrict__ gs) {
+__global__ void k_nvt_chain(int ntherm, int nchain, double dta2, double *__restrict__ nhc,
+                            const double *__restrict__ chsum, const int *__restrict__ choff,
+                            const int *__restrict__ gs) {
   if (gated_off(gs, 0)) return;
-  int g = blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= P.ngroups) return;
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j < ntherm) nvt_chain(j, ntherm, nchain, dta2, nhc, chsum, choff);
+}
+
+// group g: second scaling and half drift, the bonded (and torsion) forces at
+// the new positions and their kicks; at the level's end the displacement tests
+__device__ __forceinline__ void nvt_second(const StepP &P, const NvtK &K, int g, bool tors_end, bool level_end) {
   const int n = P.n;
-  const int a0 = gaoff[g], a1 = gaoff[g + 1];
+  double *pos = K.pos, *vel = K.vel, *fxa = K.fxa, *fxr = K.fxr;
+  const IntraDev &X = K.X;
+  const int a0 = K.gaoff[g], a1 = K.gaoff[g + 1];
   const bool has_bx = X.bx_off && X.bx_off[g + 1] > X.bx_off[g];
-  const bool bonded = gboff[g + 1] > gboff[g] || geoff[g + 1] > geoff[g] || has_bx;
+  const bool bonded = K.gboff[g + 1] > K.gboff[g] || K.geoff[g + 1] > K.geoff[g] || has_bx;
   const bool tors = X.tor_off && (X.tor_off[g + 1] > X.tor_off[g] || X.o14_off[g + 1] > X.o14_off[g]);
   for (int a = a0; a < a1; a++) {
-    const int i = gatoms[a];
-    const double e = nhc_factor(ithm[i], P.nchain, P.dta2, veta);
+    const int i = K.gatoms[a];
+    const double e = nhc_factor(K.ithm[i], P.nchain, P.dta2, K.veta);
     for (int d = 0; d < 3; d++) {
       const int x = d * n + i;
       vel[x] *= e;
@@ -703,47 +728,89 @@ __global__ void k_nvt_c(StepP P, int tors_end, int level_end, const int *__restr
   }
   if (bonded) {
     for (int a = a0; a < a1; a++) {
-      const int i = gatoms[a];
+      const int i = K.gatoms[a];
       fxa[i] = fxa[n + i] = fxa[2 * n + i] = 0.;
     }
-    group_bonded(g, n, pos, fxa, gboff, bij, bp, geoff, eijk, ep);
+    group_bonded(g, n, pos, fxa, K.gboff, K.bij, K.bp, K.geoff, K.eijk, K.ep);
     if (has_bx) group_bondx(g, n, pos, fxa, X);
     for (int a = a0; a < a1; a++) {
-      const int i = gatoms[a];
-      const double r = 1. / mass[i];
+      const int i = K.gatoms[a];
+      const double r = 1. / K.mass[i];
       fxa[i] *= r; fxa[n + i] *= r; fxa[2 * n + i] *= r;
       if (X.frz && X.frz[i]) freeze_one(i, n, vel, fxa);
     }
   }
   for (int a = a0; a < a1; a++) {
-    const int i = gatoms[a];
+    const int i = K.gatoms[a];
     for (int d = 0; d < 3; d++) vel[d * n + i] += P.dta2 * fxa[d * n + i];
   }
   if (tors_end && tors) {
     for (int a = a0; a < a1; a++) {
-      const int i = gatoms[a];
+      const int i = K.gatoms[a];
       fxr[i] = fxr[n + i] = fxr[2 * n + i] = 0.;
     }
-    group_tors_level(g, n, pos, q, fxr, X, stat);
+    group_tors_level(g, n, pos, K.q, fxr, X, K.stat);
     for (int a = a0; a < a1; a++) {
-      const int i = gatoms[a];
-      const double r = 1. / mass[i];
+      const int i = K.gatoms[a];
+      const double r = 1. / K.mass[i];
       fxr[i] *= r; fxr[n + i] *= r; fxr[2 * n + i] *= r;
       if (X.frz && X.frz[i]) freeze_one(i, n, vel, fxr);
       for (int d = 0; d < 3; d++) vel[d * n + i] += P.dtr2 * fxr[d * n + i];
     }
   }
   if (level_end) {
-    const int sy = sys_of[gatoms[a0]];
-    const double skin2q = sp[sy].skin2q, listq = sp[sy].listq;
+    const int sy = K.sys_of[K.gatoms[a0]];
+    const double skin2q = K.sp[sy].skin2q, listq = K.sp[sy].listq;
     bool far = false, lfar = false;
     for (int a = a0; a < a1; a++) {
-      const int i = gatoms[a];
-      far |= moved2(i, n, pos, dxn) > skin2q;
-      if (listq >= 0.) lfar |= moved2(i, n, pos, dxi) > listq;
+      const int i = K.gatoms[a];
+      far |= moved2(i, n, pos, K.dxn) > skin2q;
+      if (listq >= 0.) lfar |= moved2(i, n, pos, K.dxi) > listq;
     }
-    raise_rebuild(sy, listq, far, lfar, sreb, lreb, istate);
+    raise_rebuild(sy, listq, far, lfar, K.sreb, K.lreb, K.istate);
   }
+}
+
+__global__ void k_nvt_c(StepP P, int tors_end, int level_end, const __grid_constant__ NvtK K,
+                        const int *__restrict__ gs) {
+  if (gated_off(gs, 0)) return;
+  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g < P.ngroups) nvt_second(P, K, g, tors_end, level_end);
+}
+
+// All substeps of a level in one cluster of blocks, with its barriers where the
+// grid-wide form starts a new kernel: for systems whose four launches per
+// substep wait for one another longer than they work (us per step, grid-wide and one cluster: argon of 864
+// atoms 52, 50; 2048, 62, 60; 4000, 69, 66; 6912 and two groups a thread, 74,
+// 78; water under 8 substeps, 648 atoms 161, 138; 3000, 199, 170; 8232, 280, 268).  What another
+// block wrote (kinetic terms, chunk sums, chain velocities) is read through L2.
+constexpr int NVT_THREADS = 512;
+struct ChainK {
+  int nchunks, ntherm;
+  const int2 *chunk;
+  const int *atoms, *choff;
+  double *chsum, *nhc;
+};
+__global__ void __launch_bounds__(NVT_THREADS, 1) k_nvt_cluster(StepP P, int intr, int ntors, int nintra, int nb,
+                                                                const __grid_constant__ NvtK K,
+                                                                const __grid_constant__ ChainK C,
+                                                                const int *__restrict__ gs) {
+  if (gated_off(gs, 0)) return;                           // the whole cluster
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, nt = nb * blockDim.x;
+  if (t == 0) K.istate[IS_INTR] = intr;
+  for (int it = 0; it < ntors; it++)
+    for (int ia = 0; ia < nintra; ia++) {
+      for (int g = t; g < P.ngroups; g += nt) nvt_first(P, K, g, intr, it == 0 && ia == 0, ia == 0);
+      cluster_sync(nb);
+      // few chunks: the first block sums them and turns the chains by itself
+      const bool lone = C.nchunks <= (int)blockDim.x / 32;
+      for (int ch = t >> 5; ch < C.nchunks; ch += nt >> 5) nvt_chunk(ch, C.chunk, C.atoms, K.kin, C.chsum);
+      cluster_sync(lone ? 1 : nb);
+      for (int j = t; j < C.ntherm; j += nt) nvt_chain(j, C.ntherm, P.nchain, P.dta2, C.nhc, C.chsum, C.choff);
+      cluster_sync(nb);
+      for (int g = t; g < P.ngroups; g += nt)
+        nvt_second(P, K, g, ia == nintra - 1, it == ntors - 1 && ia == nintra - 1);
+    }
 }
 
 // standalone displacement test (cm3d_nb_nrefsh)
@@ -1884,6 +1951,7 @@ static int close_level(Ctx *c, int intr, bool ks_forked = false, bool zeroed = f
 // RESPA level `intr` of one outer step (md_step.c:95-146); with `gated` the
 // rebuild kernels are gated on the device flag (graph capture), otherwise
 // the host reads the flag and rebuilds
+constexpr int NVT_CLUSTER_GROUPS = 8 * NVT_THREADS;    // one cluster's threads
 static int one_level(Ctx *c, int intr, bool gated) {
   int rc;
   StepP P = step_params(c);
@@ -1892,27 +1960,34 @@ static int one_level(Ctx *c, int intr, bool gated) {
   cudaEvent_t e0;
   tbegin(c, 3, &e0);
   if (c->ntherm > 0) {
-    // NVT: four launches per inner substep (k_nvt_a, k_nvt_ksum, k_nvt_chain, k_nvt_c)
     const size_t tc = (size_t)c->ntherm * c->nchain;
-    double *veta = c->nhc + 3 * tc;
-    for (int inrra = 0; inrra < c->nres_tors; inrra++)
-      for (int intra = 0; intra < c->nres_intra; intra++) {
-        k_nvt_a<<<grid_for(c->ngroups, B), B, 0, c->st>>>(P, intr, inrra == 0 && intra == 0, intra == 0,
-                                                          c->grp_atom_off, c->grp_atoms, c->pos, c->vel, c->mass,
-                                                          c->fxl, c->fxs, c->fxa, c->fxr, c->ithm, veta, c->nvt_kin,
-                                                          c->intra, c->istate, c->gate);
-        k_nvt_ksum<<<grid_for(32LL * c->nth_chunks, 256), 256, 0, c->st>>>(c->nth_chunks, c->th_chunk, c->th_atoms,
-                                                                          c->nvt_kin, c->nvt_chsum, c->gate);
-        k_nvt_chain<<<grid_for(c->ntherm, 64), 64, 0, c->st>>>(c->ntherm, c->nchain, P.dta2, c->nhc, c->nvt_chsum,
-                                                               c->th_choff,
-                                                               c->gate);
-        k_nvt_c<<<grid_for(c->ngroups, B), B, 0, c->st>>>(
-            P, intra == c->nres_intra - 1, inrra == c->nres_tors - 1 && intra == c->nres_intra - 1,
-            c->grp_atom_off, c->grp_atoms, c->pos, c->vel, c->mass, c->q, c->fxa, c->fxr, c->dxn, c->dxi,
-            c->grp_bond_off, c->bond_ij, c->bond_p, c->grp_bend_off, c->bend_ijk, c->bend_p, c->ithm, veta,
-            c->sp, c->sys_of, c->sreb, c->lreb, c->istate, c->intra, c->stat, c->gate);
-        c->launches += 4;
-      }
+    const NvtK K = {c->grp_atom_off, c->grp_atoms, c->ithm, c->pos, c->vel, c->mass, c->q, c->fxl, c->fxs,
+                    c->nhc + 3 * tc, c->fxa, c->fxr, c->nvt_kin, c->dxn, c->dxi, c->grp_bond_off, c->bond_ij,
+                    c->bond_p, c->grp_bend_off, c->bend_ijk, c->bend_p, c->sp, c->sys_of, c->sreb, c->lreb,
+                    c->istate, c->intra, c->stat};
+    if (c->ngroups <= NVT_CLUSTER_GROUPS) {
+      const ChainK C = {c->nth_chunks, c->ntherm, c->th_chunk, c->th_atoms, c->th_choff, c->nvt_chsum, c->nhc};
+      // the groups over as many SMs as the cluster has, two warps a block at least
+      int nb = 1;
+      while (nb < 8 && nb * 64 < c->ngroups) nb *= 2;
+      const int nthreads = std::max(64, (c->ngroups + nb * 32 - 1) / (nb * 32) * 32);
+      CK(cluster_launch(k_nvt_cluster, nb, nb, nthreads, c->st, P, intr, c->nres_tors, c->nres_intra, nb, K, C,
+                        (const int *)c->gate));
+      c->launches++;
+    } else {
+      // four launches per inner substep
+      for (int inrra = 0; inrra < c->nres_tors; inrra++)
+        for (int intra = 0; intra < c->nres_intra; intra++) {
+          k_nvt_a<<<grid_for(c->ngroups, B), B, 0, c->st>>>(P, intr, inrra == 0 && intra == 0, intra == 0, K, c->gate);
+          k_nvt_ksum<<<grid_for(32LL * c->nth_chunks, 256), 256, 0, c->st>>>(c->nth_chunks, c->th_chunk, c->th_atoms,
+                                                                            c->nvt_kin, c->nvt_chsum, c->gate);
+          k_nvt_chain<<<grid_for(c->ntherm, 64), 64, 0, c->st>>>(c->ntherm, c->nchain, P.dta2, c->nhc, c->nvt_chsum,
+                                                                 c->th_choff, c->gate);
+          k_nvt_c<<<grid_for(c->ngroups, B), B, 0, c->st>>>(
+              P, intra == c->nres_intra - 1, inrra == c->nres_tors - 1 && intra == c->nres_intra - 1, K, c->gate);
+          c->launches += 4;
+        }
+    }
   } else {
     if (c->small_mol) {
       // few molecules: one warp per block, so that they spread over the SMs
