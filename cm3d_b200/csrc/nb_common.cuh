@@ -391,7 +391,7 @@ struct Ctx {
   double *ered = nullptr;              // k_ereduce: per-block partial sums of one large system
   unsigned *ered_done = nullptr;       // k_ereduce: blocks finished per quantity
   int lw_cap = 0;                      // staged list build: neighbourhood atoms per block (0: off)
-  int list_tile = 0;                   // tiled list build: every system has 3 or more cells per axis
+  int list_tile = 0;                   // tiled list build: crowded grids of 3 or more cells per axis
   int lw_atoms = 1;                    //   and atoms of its fullest cell (mean count + 25%)
   int *grp_work = nullptr;             // groups with ecorr pairs, bonds or bends (device)
   int ngwork = 0;

@@ -34,7 +34,7 @@
 // pairs of one atom in FP32 (about 20 pairs for 32 lanes per atom) and then
 // adds that chunk in FP64: forces across the atom's lanes (fixed shuffle
 // tree), energies and virials into per-lane FP64 sums that the block adds up
-// per work item and k_cw_ereduce adds over items, all in a fixed order.  The
+// per work item and energy_sums adds over items, all in a fixed order.  The
 // results do not depend on timing: a run repeats bit for bit.
 #include <math.h>
 #include <stdlib.h>
@@ -62,7 +62,7 @@ constexpr int CW_STATIC_SMEM = 6144;        // >= the kernel's static shared arr
 constexpr int CW_RF = 8;                    // copies of the erfc force table (lane l reads copy l % 8)
 constexpr int CW_RG = 8;                    // copies of the erfc energy table
 
-// per-item FP64 sums (each pair is seen from both ends: k_cw_ereduce halves)
+// per-item FP64 sums (each pair is seen from both ends: energy_sums halves)
 
 struct CwP {
   int n, ncx, ncy, ncz, nitems, nsplit, cap, words;   // words: 8-byte words per atom slot
