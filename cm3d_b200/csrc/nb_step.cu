@@ -802,8 +802,10 @@ __global__ void __launch_bounds__(NVT_THREADS, 1) k_nvt_cluster(StepP P, int int
     for (int ia = 0; ia < nintra; ia++) {
       for (int g = t; g < P.ngroups; g += nt) nvt_first(P, K, g, intr, it == 0 && ia == 0, ia == 0);
       cluster_sync(nb);
-      // few chunks: the first block sums them and turns the chains by itself
-      const bool lone = C.nchunks <= (int)blockDim.x / 32;
+      // few chunks and chains: the first block sums them and turns the chains by
+      // itself (a thermostat without atoms has a chain and no chunk: with more
+      // thermostats than the block has threads another block turns some)
+      const bool lone = C.nchunks <= (int)blockDim.x / 32 && C.ntherm <= (int)blockDim.x;
       for (int ch = t >> 5; ch < C.nchunks; ch += nt >> 5) nvt_chunk(ch, C.chunk, C.atoms, K.kin, C.chsum);
       cluster_sync(lone ? 1 : nb);
       for (int j = t; j < C.ntherm; j += nt) nvt_chain(j, C.ntherm, P.nchain, P.dta2, C.nhc, C.chsum, C.choff);
