@@ -124,6 +124,14 @@ enum {
 __device__ __forceinline__ bool gated_off(const int *gs, int need_rebuild) {
   return gs && (gs[IS_HALT] != 0 || (need_rebuild && gs[IS_LREBUILD] == 0));
 }
+// The gate of kernels that may run while the halt is being raised -- the list
+// kernels, whose own blocks raise it, and the k-space and molecule terms, which
+// run beside them -- and whose threads work together.  Threads that read the
+// flag one by one could disagree, and those that stayed would index with what
+// those that left had not written; here one yes takes the whole block.
+__device__ __forceinline__ bool block_gated_off(const int *gs, int need_rebuild) {
+  return gs && __syncthreads_or(gated_off(gs, need_rebuild));
+}
 // per-system counters (sstat[s * SS_COUNT + ...])
 enum { SS_REBUILDS = 0, SS_RESETS = 1, SS_COUNT = 2 };
 

@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(256) k_cw_convert(int ncx, int ncy, int ncz, i
                                                     const uint32_t *__restrict__ nbr, uint2 *__restrict__ cwl,
                                                     int2 *__restrict__ cwn, long long *__restrict__ stat,
                                                     int *__restrict__ halt, const int *__restrict__ gs) {
-  if (gated_off(gs, 1)) return;
+  if (block_gated_off(gs, 1)) return;
   const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (t >= n) return;                                  // whole warps
   cw_convert_atom(t, threadIdx.x & 31, ncx, ncy, ncz, 0, cap, n, words, row, cell_start, cell_of, sorig, nlen,
@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(256) k_cw_convert_sys(int nsys, const int *__r
                                                         const uint32_t *__restrict__ nbr, uint2 *__restrict__ cwl,
                                                         int2 *__restrict__ cwn, long long *__restrict__ stat,
                                                         int *__restrict__ halt, const int *__restrict__ gs) {
-  if (gated_off(gs, 1)) return;
+  if (block_gated_off(gs, 1)) return;
   const int total = scan[nsys];
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   for (int v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; v < total; v += nwarps) {

@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(KS_THREADS, 2) k_sfac_mixed(int nq, const uint
                                                            const SysP *__restrict__ sp,
                                                            const int *__restrict__ tile_sys,
                                                            const int *__restrict__ gs) {
-  if (gated_off(gs, 0)) return;
+  if (block_gated_off(gs, 0)) return;
   __shared__ float2 red[KS_THREADS / 32][MAX_ROWLEN];
   // this block's atoms [abase, aend), rows [rbeg, rend) and partial-S(k) base
   int abase = blockIdx.x * (blockDim.x * A), aend = nq, rbeg = 0, rend = nrows;
@@ -243,7 +243,7 @@ __global__ void k_sred(int ktot, int ntiles, const double2 *__restrict__ spart, 
                        double rvol_one, double falp2_one, double2 *__restrict__ sk, float2 *__restrict__ akf,
                        double2 *__restrict__ akd, double *__restrict__ acc, const SysP *__restrict__ sp,
                        const int *__restrict__ k_sys, const int *__restrict__ gs) {
-  if (gated_off(gs, 0)) return;
+  if (block_gated_off(gs, 0)) return;
   double v[11] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
   const double TPI = 2.0 * M_PI;
   int sys = -1;
@@ -302,7 +302,7 @@ __global__ void __launch_bounds__(KS_THREADS) k_kforce_mixed(int nq, const uint4
                                                              const SysP *__restrict__ sp,
                                                              const int *__restrict__ tile_sys,
                                                              const int *__restrict__ gs) {
-  if (gated_off(gs, 0)) return;
+  if (block_gated_off(gs, 0)) return;
   extern __shared__ float2 ak_s[];
   // this block's charged atoms [abase, aend), rows [r0, r1) and k range
   int r0, r1, kend, abase, aend;
@@ -559,7 +559,7 @@ __global__ void __launch_bounds__(SG_THREADS, 2) k_sfac_gemm(
     int nq, int atoms_per_block, const uint4 *__restrict__ kfrac, const float2 *__restrict__ btab, int nrows,
     const int4 *__restrict__ rows, const int *__restrict__ row_k0, const int *__restrict__ rowperm, int ktot,
     double2 *__restrict__ spart, const int *__restrict__ gs) {
-  if (gated_off(gs, 0)) return;
+  if (block_gated_off(gs, 0)) return;
   extern __shared__ __align__(16) unsigned char sg_smem[];
   SgSmem &M = *reinterpret_cast<SgSmem *>(sg_smem);
   const int rbase = blockIdx.y * SG_ROWS;
@@ -732,7 +732,7 @@ __global__ void __launch_bounds__(SG_THREADS, 2) k_sfac_gemm(
 // k_sred over many tiles: 32 k per block, eight threads each over the tiles
 __global__ void __launch_bounds__(256) k_sred_tiles(int ktot, int ntiles, const double2 *__restrict__ spart,
                                                     double2 *__restrict__ sk, const int *__restrict__ gs) {
-  if (gated_off(gs, 0)) return;
+  if (block_gated_off(gs, 0)) return;
   __shared__ double2 part[8][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int k = blockIdx.x * 32 + lane;
@@ -782,7 +782,7 @@ __global__ void __launch_bounds__(KR_THREADS) k_kforce_reg(
     int nq, const uint4 *__restrict__ kfrac, const float2 *__restrict__ btab, const int *__restrict__ split_row,
     const int4 *__restrict__ ghdr, const float4 *__restrict__ gcoef, int cap, const double *__restrict__ hmati,
     double *__restrict__ part, const int *__restrict__ gs) {
-  if (gated_off(gs, 0)) return;
+  if (block_gated_off(gs, 0)) return;
   extern __shared__ float4 coef[];                   // cap coefficients, then the headers
   int4 *hdr = reinterpret_cast<int4 *>(coef + cap);
   const int r0 = split_row[blockIdx.y], nr = split_row[blockIdx.y + 1] - r0;
@@ -894,7 +894,7 @@ template <int SL>
 __global__ void __launch_bounds__(256) k_kforce_sum(int nq, int nsplit, const double *__restrict__ part,
                                                     const int *__restrict__ icharge, int n, double *__restrict__ fxl,
                                                     const int *__restrict__ gs) {
-  if (gated_off(gs, 0)) return;
+  if (block_gated_off(gs, 0)) return;
   const int slice = SL > 1 ? threadIdx.x >> 5 : 0;
   const int jq = SL > 1 ? blockIdx.x * 32 + (threadIdx.x & 31) : blockIdx.x * blockDim.x + threadIdx.x;
   double ks[3];
@@ -920,7 +920,7 @@ __global__ void __launch_bounds__(KS_THREADS) k_sfac_plain(int nq, const double4
                                                            int ktot, const double *__restrict__ hmati,
                                                            double2 *__restrict__ spart,
                                                            const int *__restrict__ gs) {
-  if (gated_off(gs, 0)) return;
+  if (block_gated_off(gs, 0)) return;
   __shared__ double2 red[KS_THREADS / 32][MAX_ROWLEN];
   const int tile = blockIdx.x;
   const int r0 = blockIdx.y * rows_per_block;
@@ -966,7 +966,7 @@ __global__ void k_kforce_plain(int nq, const double4 *__restrict__ kp, const int
                                int rows_per_split, const double2 *__restrict__ akd, int ktot,
                                const double *__restrict__ hmati, int atomic, double *__restrict__ fxl,
                                const int *__restrict__ gs) {
-  if (gated_off(gs, 0)) return;
+  if (block_gated_off(gs, 0)) return;
   const int jq = blockIdx.x * blockDim.x + threadIdx.x;
   const int r0 = blockIdx.y * rows_per_split;
   const int r1 = min(nrows, r0 + rows_per_split);

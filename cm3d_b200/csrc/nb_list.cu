@@ -713,7 +713,7 @@ __global__ void __launch_bounds__(256) k_list_half(
     int *__restrict__ cnt, const long long *__restrict__ off,
     const long long *__restrict__ tot, int2 *__restrict__ l0, int2 *__restrict__ l1, int2 *__restrict__ l2,
     int2 *__restrict__ l3, long long *__restrict__ stat, int *__restrict__ halt, const int *__restrict__ gate) {
-  if (gated_off(gate, 1)) return;
+  if (block_gated_off(gate, 1)) return;
   __shared__ int qs[256 / 32][LQ];
   __shared__ float qrs[256 / 32][LQ];
   const int n = K.n;
@@ -938,7 +938,7 @@ __global__ void __launch_bounds__(256, 3) k_list_full(
     const __grid_constant__ ListK K, const SysP *__restrict__ sp, const int *__restrict__ sys_of,
     const int *__restrict__ sreb, int all, int stride, uint32_t *__restrict__ nbr, int *__restrict__ nlen,
     long long *__restrict__ stat, int *__restrict__ halt, const int *__restrict__ gate) {
-  if (gated_off(gate, 1)) return;
+  if (block_gated_off(gate, 1)) return;
   __shared__ int qs[256 / 32][LQ];
   __shared__ float qrs[256 / 32][LQ];
   const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -1001,7 +1001,7 @@ __global__ void __launch_bounds__(LT_WARPS * 32, 5) k_list_tile(
     const int *__restrict__ cell_sys, const int *__restrict__ sreb, int all, int stride, uint32_t *__restrict__ nbr,
     int *__restrict__ nlen, const __grid_constant__ CompactOut W, long long *__restrict__ stat,
     int *__restrict__ halt, const int *__restrict__ gate) {
-  if (gated_off(gate, 1)) return;
+  if (block_gated_off(gate, 1)) return;
   __shared__ TileSmem M;
   const int cell = blockIdx.x / parts, part = blockIdx.x - cell * parts;
   const int sy = cell_sys[cell];
@@ -1295,7 +1295,7 @@ __global__ void __launch_bounds__(LW_THREADS, 3) k_list_win(
     const __grid_constant__ ListK K, int nsys, const int *__restrict__ rb_scan, const SysP *__restrict__ sp,
     int stride, int cap, uint32_t *__restrict__ nbr, int *__restrict__ nlen,
     long long *__restrict__ stat, int *__restrict__ halt, const int *__restrict__ gate) {
-  if (gated_off(gate, 1)) return;
+  if (block_gated_off(gate, 1)) return;
   extern __shared__ float4 s_x[];                        // cap
   int *s_u = reinterpret_cast<int *>(s_x + cap);         // cap: sorted index | shift code << ENT_CODE_SHIFT
   int *s_j = s_u + cap;                                  // cap: atom index

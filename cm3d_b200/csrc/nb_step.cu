@@ -897,7 +897,7 @@ __global__ void k_group_init(StepP P, const int *__restrict__ gwork, int ngw, co
                              const double2 *__restrict__ ep, double *__restrict__ acc,
                              const SysP *__restrict__ sp, const int *__restrict__ sys_of,
                              const int *__restrict__ gs) {
-  if (gated_off(gs, 0)) return;
+  if (block_gated_off(gs, 0)) return;
   const int gi = blockIdx.x * blockDim.x + threadIdx.x;
   const int n = P.n;
   // ecorr: pot, prs, t0 t1 t2 t4 t5 t8 | bond: v, w, t0..t8 | bend: v, w, t0..t8
@@ -995,7 +995,7 @@ __global__ void __launch_bounds__(128) k_group_small(
     const int *__restrict__ geoff, const int4 *__restrict__ eijk, const double2 *__restrict__ ep,
     double *__restrict__ acc, const SysP *__restrict__ sp, const int *__restrict__ sys_of,
     const int *__restrict__ gs) {
-  if (gated_off(gs, 0)) return;
+  if (block_gated_off(gs, 0)) return;
   const int gi = blockIdx.x * blockDim.x + threadIdx.x;
   const int n = P.n;
   double v[30];
