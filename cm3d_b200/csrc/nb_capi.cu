@@ -150,12 +150,6 @@ static void box_params(SysP &P, SysH &H) {
   }
 }
 
-// width of the box along each direction (1 / |row d of H^-1|)
-static double box_width(const SysH &H, int d) {
-  return 1.0 / sqrt(H.hmati[3 * d] * H.hmati[3 * d] + H.hmati[3 * d + 1] * H.hmati[3 * d + 1] +
-                    H.hmati[3 * d + 2] * H.hmati[3 * d + 2]);
-}
-
 // boxes narrower than two list radii need the on-the-fly minimum image (for
 // the pairs near the image boundary, see near_s)
 static void box_widths(SysP &P, const SysH &H) {
@@ -180,14 +174,45 @@ static void box_widths(SysP &P, const SysH &H) {
 // 0.5 -- CM3D's own --, 1, 1.5, 2 and 2.5 A: 12,288 water atoms 235, 181, 162,
 // 161, 207; 37 boxes of 27,000 atoms 221, -, 210, 188, 217.  331,776 water
 // atoms with CM3D's 1.5 A, 4.80 ms; 2 A, 4.53; 2.5 A, 5.13.)
-constexpr double LIST_SKIN = 0.2;
-static double list_skin(const SysH &H, double rc_max, bool consistent, double cell_scale) {
+//
+// Wider lists make fewer, wider cells, and cells too wide for a window beside
+// the tables (`slots`) lose the compact pair kernel, which takes half the
+// gather kernel's time or less.  Where CM3D's own radius has room for it the
+// skin stops at the last grid that has, unless that leaves less than
+// LIST_SKIN_LEAST of the cut-off: then the builds saved are worth more.  (us
+// per step, CM3D's lists, the full skin in the gather kernel, the skin that
+// keeps the compact one, windows of 7142 slots: 10,125 water atoms 185, 139,
+// 111 with 1.6 A in all; 17,496: 212, 184, 159 with 1.2 A; 46,875: 511, 430,
+// 389 with 1.1 A; but 27,783: 350, 300, 329 with 0.86 A, and 8232: 148, 119,
+// 122 with 0.86 A.  The windows beside four copies of the erfc tables now leave
+// room for the full skin in all of these but the 10,125 and 8232.)  In a batch
+// all systems or none run in the compact kernel: there the skin always stops.
+constexpr double LIST_SKIN = 0.2, LIST_SKIN_LEAST = 0.1;
+static double list_skin(const SysH &H, double rc_max, bool consistent, double cell_scale, long long slots, bool batch) {
   double extra = LIST_SKIN * rc_max - H.skin;
   if (!consistent || !(H.skin > 0.0) || !(extra > 0.0)) return 0.0;
+  // the most a radius can grow with m cells of it left along direction d
+  auto room = [&](int d, int m) { return (1.0 - 1e-9) * box_width(H, d) / (m * cell_scale) - H.rlist_cm; };
   for (int d = 0; d < 3; d++) {
+    if (cells_along(H, d, H.rlist_cm, cell_scale) >= 3) extra = std::min(extra, room(d, 3));
     const double w = box_width(H, d);
-    if (floor(w / (H.rlist_cm * cell_scale)) >= 3) extra = std::min(extra, (1.0 - 1e-9) * w / (3.0 * cell_scale) - H.rlist_cm);
     if (w >= 2.0 * H.rlist_cm) extra = std::min(extra, (1.0 - 1e-9) * 0.5 * w - H.rlist_cm);
+  }
+  auto fits = [&](double x) {
+    double cells = 1.0;
+    for (int d = 0; d < 3; d++) {
+      const int m = cells_along(H, d, H.rlist_cm + x, cell_scale);
+      if (m < 3) return false;
+      cells *= m;
+    }
+    return cw_window(H.n, cells) <= (double)slots;
+  };
+  if (extra > 0.0 && fits(0.0) && !fits(extra)) {
+    double kept = 0.0;
+    for (int d = 0; d < 3; d++)
+      for (int m = cells_along(H, d, H.rlist_cm, cell_scale); m >= 3; m--)
+        if (room(d, m) > kept && room(d, m) < extra && fits(room(d, m))) kept = room(d, m);
+    if (batch || H.skin + kept >= LIST_SKIN_LEAST * rc_max) extra = kept;
   }
   return extra > 0.01 * rc_max ? extra : 0.0;
 }
@@ -312,6 +337,8 @@ static int create(const cm3d_nb_system *systems, int nsys, const cm3d_nb_options
   std::vector<double> pos(n3), vel(n3), mass(n), q(n);
   std::vector<int> itype(n), sys_of(n), map, ich, eoff(n + 1, 0), eidx, coff(n + 1, 0), cidx;
   std::vector<double> vtab, dvtab, swt, icut, coultab, dcoultab, switchse, rad_cm, rad;
+  std::vector<double> rc_max((size_t)nsys, 0.0);
+  std::vector<char> cut_and_skin((size_t)nsys, 0);
   bool any_extra = false;
   int a0 = 0, inter0 = 0, ncoul = 0;
   for (int sy = 0; sy < nsys; sy++) {
@@ -432,7 +459,20 @@ static int create(const cm3d_nb_system *systems, int nsys, const cm3d_nb_options
     }
     H.rlist_cm = sqrt(r2);
     H.skin = s->skin_ter;
-    H.extra = c->mode == CM3D_NB_MIXED ? list_skin(H, sqrt(rc2), consistent, c->cell_scale) : 0.0;
+    rc_max[sy] = sqrt(rc2);
+    cut_and_skin[sy] = consistent;
+    a0 += ns;
+  }
+  c->ncoul = ncoul;
+  c->ncharge = (int)ich.size();
+  c->ninter = inter0;
+  // the engine's own list radii
+  const long long slots = cw_slots(c);
+  for (int sy = 0; sy < nsys; sy++) {
+    const cm3d_nb_system *s = systems + sy;
+    SysP &P = c->h_sp[sy];
+    SysH &H = c->hs[sy];
+    H.extra = c->mode == CM3D_NB_MIXED ? list_skin(H, rc_max[sy], cut_and_skin[sy], c->cell_scale, slots, nsys > 1) : 0.0;
     list_radii(P, H);
     any_extra = any_extra || H.extra > 0.0;
     for (int in = 0; in < s->ninter; in++) {
@@ -442,11 +482,7 @@ static int create(const cm3d_nb_system *systems, int nsys, const cm3d_nb_options
       rad.push_back(widened(s->rmaxl_skin2[in], H.extra));
     }
     box_widths(P, H);
-    a0 += ns;
   }
-  c->ncoul = ncoul;
-  c->ncharge = (int)ich.size();
-  c->ninter = inter0;
   // the scalar fields describe system 0 (the plain engine and the single-system
   // paths read them)
   {

@@ -426,6 +426,7 @@ struct Ctx {
   float4 *cw_tl = nullptr;             // LJ, 2 float4 per knot
   float cw_lj1[4] = {0, 0, 0, 0};      // the one LJ interaction: rc^2, dx2tab, offset, vt
   int cw_nsplit = 1, cw_nitems = 0;    // work items: cells x parts
+  int cw_rt = 8;                       // copies of the erfc tables in the compact kernel's shared memory
   int cw_nt = 512;                     // threads per pair-kernel block (512 or 640; autotuner)
   double *cw_part = nullptr;           // per-item FP64 energy/virial sums
   // a batch: the systems with >= 3 cells per axis in the compact kernel (in
@@ -693,6 +694,11 @@ std::recursive_mutex &device_mutex();           // nb_capi.cu
 using DevLock = std::lock_guard<std::recursive_mutex>;
 int list_setup(Ctx *c);                         // nb_list.cu
 void cell_shifts(SysP &P, const SysH &H);       // nb_list.cu
+double box_width(const SysH &H, int d);          // nb_list.cu
+int cells_along(const SysH &H, int d, double rlist, double cell_scale);   // nb_list.cu
+long long cw_slots(const Ctx *c);               // nb_cwin.cu: window slots of the compact kernel
+// the compact kernels' window: the mean 27 cells hold, a quarter more and 64
+inline double cw_window(double n, double ncells) { return 1.25 * 27.0 * n / ncells + 64.0; }
 int take_snapshot(Ctx *c, bool device_flag, bool all, bool lists);   // nb_list.cu
 constexpr int ACC_WITH_STATE = 64;              // most systems whose accumulators are copied after every step call
 int begin_steps(Ctx *c, int istep);              // nb_step.cu

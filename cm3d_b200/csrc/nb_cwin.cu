@@ -36,6 +36,7 @@
 // tree), energies and virials into per-lane FP64 sums that the block adds up
 // per work item and energy_sums adds over items, all in a fixed order.  The
 // results do not depend on timing: a run repeats bit for bit.
+#include <limits.h>
 #include <math.h>
 #include <stdlib.h>
 #include <string.h>
@@ -59,8 +60,12 @@ constexpr int CW_MAX_CAP = 16382;           // window slots (the dummy slot `cap
 constexpr float CW_MAGIC = 12582912.0f;     // 1.5 * 2^23: p + MAGIC rounded toward zero holds floor(p)
 constexpr unsigned CW_MAGIC_BITS = 0x4B400000u;
 constexpr int CW_STATIC_SMEM = 6144;        // >= the kernel's static shared arrays (5.2 KB)
-constexpr int CW_RF = 8;                    // copies of the erfc force table (lane l reads copy l % 8)
-constexpr int CW_RG = 8;                    // copies of the erfc energy table
+// Copies of the erfc force and energy tables (lane l reads copy l % 8): eight
+// keep the lanes' reads off one another's banks; four, for windows that do not
+// fit beside eight, leave room for 3072 more atoms and make the pairs 7% slower
+// (41,472 water atoms 111 and 119 us) where the gather kernel takes twice as
+// long (27,783 atoms in 13 A cells: 105 us, gather 147).
+constexpr int CW_RT = 8, CW_RT_FEW = 4;
 
 // per-item FP64 sums (each pair is seen from both ends: energy_sums halves)
 
@@ -336,7 +341,7 @@ constexpr int CW_WAIT_LIMIT = 1 << 22;
 // addresses less MAGIC_BITS knots, so that the float bits of the split
 // coordinate address the knot directly (k * stride = bits * stride - MAGIC_BITS
 // * stride, mod 2^32).
-template <int RF = CW_RF, int RG = CW_RG>
+template <int RF, int RG>
 __device__ __forceinline__ void cw_elec(const CwP &P, float qj, float dx, float dy, float dz, float r2,
                                         unsigned tfb, unsigned tgb, CwAcc &A) {
   A.r2min = fminf(A.r2min, r2);
@@ -395,7 +400,7 @@ __device__ __forceinline__ void cw_lj(const CwP &P, float dx, float dy, float dz
 // serve them all -- given as {system, cell of the system, part, parts};
 // each item's cell grid and shifts come from its system's SysP, and its
 // partial sums go to item0 + item.
-template <bool HAS_EL, int LJM, bool BATCH = false, int NT = CW_THREADS>
+template <bool HAS_EL, int LJM, bool BATCH, int NT, int RT>
 __global__ void __launch_bounds__(NT, 1) k_pair_cw(
     CwP P, const float4 *__restrict__ xq, const int *__restrict__ styp, const int *__restrict__ sorig,
     const int *__restrict__ cell_start, const int2 *__restrict__ cwn, const uint2 *__restrict__ cwl,
@@ -407,9 +412,9 @@ __global__ void __launch_bounds__(NT, 1) k_pair_cw(
   if (gated_off(gs, 0)) return;
   extern __shared__ float4 sm[];
   // tables first (16-byte aligned), then the window
-  float4 *tf = sm;                                                    // ntable * CW_RF
-  float2 *tg = reinterpret_cast<float2 *>(tf + (HAS_EL ? P.ntable * CW_RF : 0));   // ntable * CW_RG
-  float4 *tl = reinterpret_cast<float4 *>(tg + (HAS_EL ? P.ntable * CW_RG : 0));   // 2 ninter ntable
+  float4 *tf = sm;                                                    // ntable * RT
+  float2 *tg = reinterpret_cast<float2 *>(tf + (HAS_EL ? P.ntable * RT : 0));   // ntable * RT
+  float4 *tl = reinterpret_cast<float4 *>(tg + (HAS_EL ? P.ntable * RT : 0));   // 2 ninter ntable
   const int nl = LJM ? 2 * P.ninter * P.ntable : 0;
   float4 *wx = tl + nl;                                               // cap + 1 staged atoms
   unsigned char *wt = reinterpret_cast<unsigned char *>(wx + P.cap + 1);   // LJM 2: their types
@@ -424,8 +429,10 @@ __global__ void __launch_bounds__(NT, 1) k_pair_cw(
   if (!BATCH)
     for (int k = threadIdx.x; k < 54; k += blockDim.x) s_shift[k] = gshift[k];
   if (HAS_EL) {
-    for (int k = threadIdx.x; k < P.ntable * CW_RF; k += blockDim.x) tf[k] = gtf[k / CW_RF];
-    for (int k = threadIdx.x; k < P.ntable * CW_RG; k += blockDim.x) tg[k] = gtg[k / CW_RG];
+    for (int k = threadIdx.x; k < P.ntable * RT; k += blockDim.x) {
+      tf[k] = gtf[k / RT];
+      tg[k] = gtg[k / RT];
+    }
   }
   for (int k = threadIdx.x; k < nl; k += blockDim.x) tl[k] = gtl[k];
   if (LJM == 2) {
@@ -450,10 +457,10 @@ __global__ void __launch_bounds__(NT, 1) k_pair_cw(
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   constexpr int NWARP = NT / 32;
   // this lane's table copies and the window as 32-bit shared addresses
-  const unsigned tfb = (unsigned)__cvta_generic_to_shared(tf + (lane & (CW_RF - 1))) -
-                       CW_MAGIC_BITS * (unsigned)(CW_RF * sizeof(float4));
-  const unsigned tgb = (unsigned)__cvta_generic_to_shared(tg + (lane & (CW_RG - 1))) -
-                       CW_MAGIC_BITS * (unsigned)(CW_RG * sizeof(float2));
+  const unsigned tfb = (unsigned)__cvta_generic_to_shared(tf + (lane & (RT - 1))) -
+                       CW_MAGIC_BITS * (unsigned)(RT * sizeof(float4));
+  const unsigned tgb = (unsigned)__cvta_generic_to_shared(tg + (lane & (RT - 1))) -
+                       CW_MAGIC_BITS * (unsigned)(RT * sizeof(float2));
   const unsigned wxb = (unsigned)__cvta_generic_to_shared(wx);
   unsigned long long under = 0;
 
@@ -609,7 +616,7 @@ __global__ void __launch_bounds__(NT, 1) k_pair_cw(
         float4 xj;
         float dx, dy, dz;
         const float r2 = geom(e, xj, dx, dy, dz);
-        if (HAS_EL) cw_elec(P, (e & CW_EL) ? xj.w : 0.f, dx, dy, dz, (e & CW_EL) ? r2 : 3.0e38f, tfb, tgb, Acc);
+        if (HAS_EL) cw_elec<RT, RT>(P, (e & CW_EL) ? xj.w : 0.f, dx, dy, dz, (e & CW_EL) ? r2 : 3.0e38f, tfb, tgb, Acc);
         lj_pair(e, dx, dy, dz, r2, Acc);
       };
       auto back_pair = [&](uint32_t e, CwAcc &Acc) {
@@ -617,7 +624,7 @@ __global__ void __launch_bounds__(NT, 1) k_pair_cw(
           float4 xj;
           float dx, dy, dz;
           const float r2 = geom(e, xj, dx, dy, dz);
-          cw_elec(P, xj.w, dx, dy, dz, r2, tfb, tgb, Acc);
+          cw_elec<RT, RT>(P, xj.w, dx, dy, dz, r2, tfb, tgb, Acc);
         }
       };
       // block b's word of this lane; the next two are in flight
@@ -1084,7 +1091,7 @@ __global__ void __launch_bounds__(ER_THREADS) k_cw_ereduce(const __grid_constant
 // ------------------------------------------------------------------ host
 static int cw_ljm_of(int ninter) { return ninter == 0 ? 0 : (ninter == 1 ? 1 : 2); }
 
-static size_t cw_table_bytes(bool el, int ljm, int ninter, int ntable, int rf = CW_RF, int rg = CW_RG) {
+static size_t cw_table_bytes(bool el, int ljm, int ninter, int ntable, int rf, int rg) {
   size_t b = 0;
   if (el) b += (size_t)ntable * (rf * sizeof(float4) + rg * sizeof(float2));
   if (ljm) b += (size_t)2 * ninter * ntable * sizeof(float4);
@@ -1188,6 +1195,42 @@ static int cw_words_for(long long stride) {
   return std::max(cw_words_row(stride, CW_ROW), cw_words_row(stride, CS_LPA));
 }
 
+// window slots beside tables of `tables` bytes for `windows` windows a block
+static long long cw_room(const Ctx *c, size_t fixed, size_t tables, int ljm, int windows) {
+  const size_t budget = c->smem_optin > fixed ? c->smem_optin - fixed : 0;
+  const size_t per_slot = sizeof(float4) + (ljm == 2 ? 1 : 0), pad = (size_t)16 * windows;
+  const long long room = budget > tables + pad ? (long long)((budget - tables - pad) / (per_slot * windows)) - 1 : 0;
+  return std::min<long long>(room, CW_MAX_CAP);
+}
+
+// The window slots that the tables of the context's systems leave the compact
+// kernel (32 lanes per atom); no limit where CM3D's own list radii leave it out
+// already.  The 8-lane kernel of a batch has less room, and is no reason to
+// stop: where only its windows no longer fit, the longer lists in the gather
+// kernel are as fast (us per step, the narrow grid and the wide one: 64 boxes
+// of 1400 charged atoms 298, 298; 200 of them 755, 756; 64 of 1500 328, 322).
+long long cw_slots(const Ctx *c) {
+  long long cap = CW_MAX_CAP;
+  double window = 0.0;
+  for (int s = 0; s < c->nsys; s++) {
+    const SysP &S = c->h_sp[s];
+    const SysH &H = c->hs[s];
+    const bool el = S.coul >= 0;
+    const int ljm = cw_ljm_of(S.ninter);
+    double cells = 1.0;
+    bool grid = el || ljm;
+    for (int d = 0; d < 3; d++) {
+      const int m = cells_along(H, d, H.rlist_cm, c->cell_scale);
+      cells *= m;
+      grid = grid && m >= 3;
+    }
+    if (!grid || S.ntypes > 16 || S.ninter > 64) continue;       // never in the compact kernels
+    cap = std::min(cap, cw_room(c, CW_STATIC_SMEM, cw_table_bytes(el, ljm, S.ninter, c->ntable, CW_RT_FEW, CW_RT_FEW), ljm, 1));
+    window = std::max(window, cw_window(S.n, cells));
+  }
+  return window > (double)cap ? LLONG_MAX : cap;
+}
+
 static int cw_setup_batch(Ctx *c);
 
 // Whether the compact path can run this context, and its tables and window
@@ -1204,14 +1247,16 @@ int cw_setup(Ctx *c) {
   if (c->ntypes > 16 || c->ninter > 64) return CM3D_NB_OK;       // static map / cut-off arrays
   const int ljm = cw_ljm_of(c->ninter);
   const bool el = c->ncharge > 0;
-  const double mean_window = 27.0 * (double)c->n / (double)c->ncells;
-  const size_t want_cap = (size_t)(1.25 * mean_window) + 64;
-  const size_t budget = c->smem_optin > CW_STATIC_SMEM ? c->smem_optin - CW_STATIC_SMEM : 0;
-  const size_t per_slot = sizeof(float4) + (ljm == 2 ? 1 : 0);
-  const size_t tb = cw_table_bytes(el, ljm, c->ninter, c->ntable);
-  if (tb + (want_cap + 1) * per_slot + 16 > budget) return CM3D_NB_OK;
-  long long cap = (long long)((budget - tb - 16) / per_slot) - 1;
-  cap = cw_env_cap(std::min<long long>(cap, CW_MAX_CAP));
+  size_t tb = 0;
+  long long cap = 0;
+  for (int rt : {CW_RT, CW_RT_FEW}) {
+    c->cw_rt = rt;
+    tb = cw_table_bytes(el, ljm, c->ninter, c->ntable, rt, rt);
+    cap = cw_room(c, CW_STATIC_SMEM, tb, ljm, 1);
+    if (cw_window(c->n, c->ncells) <= (double)cap) break;
+  }
+  if (cw_window(c->n, c->ncells) > (double)cap) return CM3D_NB_OK;
+  cap = cw_env_cap(cap);
   c->cw_cap = c->cw_cap32 = (int)cap;
   c->cw_row = CW_ROW;
   c->cw_smem = tb + ((size_t)cap + 1) * sizeof(float4) + (ljm == 2 ? (size_t)cap + 1 : 0);
@@ -1359,21 +1404,21 @@ static int cw_setup_batch(Ctx *c) {
     }
     gid[s] = g;
     cwsys[s] = 1;
-    want_window = std::max(want_window, 27.0 * (double)S.n / (double)S.ncells);
+    want_window = std::max(want_window, cw_window(S.n, S.ncells));
   }
   if (groups->empty()) return CM3D_NB_OK;
   // one window capacity for all groups: what shared memory leaves next to
   // the largest tables, and at least the largest mean window x 1.25 + 64
-  const size_t budget = c->smem_optin > CW_STATIC_SMEM ? c->smem_optin - CW_STATIC_SMEM : 0;
-  long long cap = CW_MAX_CAP;
-  for (const CwGroup &G : *groups) {
-    const size_t tb = cw_table_bytes(G.el, G.ljm, G.P.ninter, nt);
-    const size_t per_slot = sizeof(float4) + (G.ljm == 2 ? 1 : 0);
-    const long long room = budget > tb + 16 ? (long long)((budget - tb - 16) / per_slot) - 1 : 0;
-    cap = std::min(cap, room);
+  long long cap = 0;
+  for (int rt : {CW_RT, CW_RT_FEW}) {
+    c->cw_rt = rt;
+    cap = CW_MAX_CAP;
+    for (const CwGroup &G : *groups)
+      cap = std::min(cap, cw_room(c, CW_STATIC_SMEM, cw_table_bytes(G.el, G.ljm, G.P.ninter, nt, rt, rt), G.ljm, 1));
+    if (want_window <= (double)cap) break;
   }
   cap = cw_env_cap(cap);
-  if ((double)cap < 1.25 * want_window + 64.0) {
+  if ((double)cap < want_window) {
     groups->clear();
     return CM3D_NB_OK;
   }
@@ -1381,14 +1426,10 @@ static int cw_setup_batch(Ctx *c) {
   // k_pair_cs: CS_NG windows per block next to the tables
   const size_t budget8 = c->smem_optin > CS_STATIC_SMEM ? c->smem_optin - CS_STATIC_SMEM : 0;
   long long cap8 = CW_MAX_CAP;
-  for (const CwGroup &G : *groups) {
-    const size_t tb = cw_table_bytes(G.el, G.ljm, G.P.ninter, nt, CS_RF, CS_RG);
-    const size_t per_slot = sizeof(float4) + (G.ljm == 2 ? 1 : 0);
-    const long long room = budget8 > tb + 16 * CS_NG ? (long long)((budget8 - tb - 16 * CS_NG) / (per_slot * CS_NG)) - 1 : 0;
-    cap8 = std::min(cap8, room);
-  }
+  for (const CwGroup &G : *groups)
+    cap8 = std::min(cap8, cw_room(c, CS_STATIC_SMEM, cw_table_bytes(G.el, G.ljm, G.P.ninter, nt, CS_RF, CS_RG), G.ljm, CS_NG));
   cap8 = cw_env_cap(cap8);
-  c->cw_cap8 = (double)cap8 >= 1.25 * want_window + 64.0 ? (int)cap8 : 0;
+  c->cw_cap8 = (double)cap8 >= want_window ? (int)cap8 : 0;
   // the layout: 32 lanes per atom (a system runs as it does alone) until
   // the autotuner finds the 8-lane kernel faster (cells of a few tens of
   // atoms); CM3D_NB_CW_ROW=8 starts there
@@ -1417,7 +1458,7 @@ static int cw_setup_batch(Ctx *c) {
     atf.insert(atf.end(), gtf[g].begin(), gtf[g].end());
     atg.insert(atg.end(), gtg[g].begin(), gtg[g].end());
     atl.insert(atl.end(), gtl[g].begin(), gtl[g].end());
-    const size_t tb = cw_table_bytes(G.el, G.ljm, G.P.ninter, nt);
+    const size_t tb = cw_table_bytes(G.el, G.ljm, G.P.ninter, nt, c->cw_rt, c->cw_rt);
     G.smem = (tb + ((size_t)c->cw_cap32 + 1) * sizeof(float4) + (G.ljm == 2 ? (size_t)c->cw_cap32 + 1 : 0) + 15) /
              16 * 16;
     if (c->cw_cap8 > 0) {
@@ -1573,10 +1614,10 @@ int cw_convert(Ctx *c, bool device_flag, bool all) {
   return cw_check(c, device_flag);
 }
 
-template <bool EL, int LJM, bool BATCH, int NT>
-static void cw_launch_nt(Ctx *c, const CwP &P, size_t smem, double *fout, const float4 *tf, const float2 *tg,
+template <bool EL, int LJM, bool BATCH, int NT, int RT>
+static void cw_launch_rt(Ctx *c, const CwP &P, size_t smem, double *fout, const float4 *tf, const float2 *tg,
                          const float4 *tl, const int4 *items, int item0) {
-  auto kern = k_pair_cw<EL, LJM, BATCH, NT>;
+  auto kern = k_pair_cw<EL, LJM, BATCH, NT, RT>;
   static unsigned long long attr_devs = 0;
   if (c->dev < 64 && !(attr_devs & (1ull << c->dev))) {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(c->smem_optin - CW_STATIC_SMEM));
@@ -1586,6 +1627,14 @@ static void cw_launch_nt(Ctx *c, const CwP &P, size_t smem, double *fout, const 
   kern<<<grid, NT, smem, c->st>>>(P, c->xq, c->styp, c->cell_atoms, c->cell_start, c->cwn, c->cwl, c->shift,
                                           c->map, c->fcut, tf, tg, tl, fout, c->cw_part, c->stat, c->gate, items,
                                           c->sp, item0);
+}
+
+// (without charges there is no table to copy)
+template <bool EL, int LJM, bool BATCH, int NT>
+static void cw_launch_nt(Ctx *c, const CwP &P, size_t smem, double *fout, const float4 *tf, const float2 *tg,
+                         const float4 *tl, const int4 *items, int item0) {
+  if (EL && c->cw_rt == CW_RT_FEW) cw_launch_rt<EL, LJM, BATCH, NT, EL ? CW_RT_FEW : CW_RT>(c, P, smem, fout, tf, tg, tl, items, item0);
+  else cw_launch_rt<EL, LJM, BATCH, NT, CW_RT>(c, P, smem, fout, tf, tg, tl, items, item0);
 }
 
 template <bool EL, int LJM, bool BATCH>

@@ -1461,6 +1461,18 @@ static void stencil(int nc, int *s, int *ns) {
   }
 }
 
+// width of the box along each direction (1 / |row d of H^-1|)
+double box_width(const SysH &H, int d) {
+  return 1.0 / sqrt(H.hmati[3 * d] * H.hmati[3 * d] + H.hmati[3 * d + 1] * H.hmati[3 * d + 1] +
+                    H.hmati[3 * d + 2] * H.hmati[3 * d + 2]);
+}
+
+// cells along direction d for lists of radius rlist
+int cells_along(const SysH &H, int d, double rlist, double cell_scale) {
+  const int m = rlist > 0 ? (int)floor(box_width(H, d) / (rlist * cell_scale)) : 1;
+  return m < 1 ? 1 : (m > 1000 ? 1000 : m);
+}
+
 // Cell grids of every system (cells at least one list radius wide in every
 // fractional direction: plane spacing 1 / |row d of hmati|), their stencils,
 // the 27 cell-corner shifts and the FP32 prefilter radius; fills the cell
@@ -1483,11 +1495,8 @@ void cell_shifts(SysP &P, const SysH &H) {
   // FP32 minimum images in the list tests of a coarse grid: candidates lie
   // within two cells, so cells of at most 4 list radii bound the displacement
   P.image_ok = 1;
-  for (int d = 0; d < 3; d++) {
-    const double w = 1.0 / sqrt(H.hmati[3 * d] * H.hmati[3 * d] + H.hmati[3 * d + 1] * H.hmati[3 * d + 1] +
-                                H.hmati[3 * d + 2] * H.hmati[3 * d + 2]);
-    if (!(w / P.nc[d] <= 4.0 * H.rlist)) P.image_ok = 0;
-  }
+  for (int d = 0; d < 3; d++)
+    if (!(box_width(H, d) / P.nc[d] <= 4.0 * H.rlist)) P.image_ok = 0;
 }
 
 int list_setup(Ctx *c) {
@@ -1498,14 +1507,8 @@ int list_setup(Ctx *c) {
     SysH &H = c->hs[s];
     int tot = 1;
     for (int d = 0; d < 3; d++) {
-      double w = 1.0 / sqrt(H.hmati[3 * d] * H.hmati[3 * d] + H.hmati[3 * d + 1] * H.hmati[3 * d + 1] +
-                            H.hmati[3 * d + 2] * H.hmati[3 * d + 2]);
-      auto cells = [&](double rl) {
-        const int m = rl > 0 ? (int)floor(w / (rl * c->cell_scale)) : 1;
-        return m < 1 ? 1 : (m > 1000 ? 1000 : m);
-      };
-      P.nc[d] = cells(H.rlist);
-      H.nc_cm[d] = cells(H.rlist_cm);
+      P.nc[d] = cells_along(H, d, H.rlist, c->cell_scale);
+      H.nc_cm[d] = cells_along(H, d, H.rlist_cm, c->cell_scale);
       tot *= P.nc[d];
     }
     P.c0 = c0;
