@@ -790,7 +790,7 @@ int cm3d_nb_set_positions(cm3d_nb_ctx *ctx, const double *px, const double *py, 
 // derived from H -- H^-1, the volume, the small-box test, the cell grid's
 // neighbour shifts and the device copies the kernels read -- follows it; the
 // grid keeps its cell counts, which stays valid while every cell is at least
-// a list radius wide.
+// a list radius wide.  (The first call takes the grid that CM3D's radii give.)
 int cm3d_nb_set_box(cm3d_nb_ctx *ctx, const double hmat[9]) {
   CTX;
   DevLock lock(device_mutex());
@@ -814,29 +814,38 @@ int cm3d_nb_set_box(cm3d_nb_ctx *ctx, const double hmat[9]) {
                   H.nc_cm[d], box_width(H, d) / H.nc_cm[d], H.rlist_cm, d);
         return CM3D_NB_ERR_STATE;
       }
-  // A box that moves: the engine's lists go back to CM3D's radii and schedule
-  // (a list kept longer would meet box changes its skin does not measure),
-  // built from the positions of CM3D's last rebuild in the box as it was.
+  // A box that moves: the engine's lists go back to CM3D's radii, grid and
+  // schedule (a list kept longer would meet box changes its skin does not
+  // measure), built from the positions of CM3D's last rebuild in the box as it
+  // was.
   if (c->hs[0].extra > 0.0) {
     int rc;
+    CK(cudaStreamSynchronize(c->st));
+    if (c->graph) cudaGraphExecDestroy(c->graph);   // it holds the old grid
+    c->graph = nullptr;
     c->hs[0].extra = 0.0;
     list_radii(c->h_sp[0], c->hs[0]);
     box_widths(c->h_sp[0], c->hs[0]);
-    cell_shifts(c->h_sp[0], c->hs[0]);
     c->rlist_max = c->hs[0].rlist;
-    CK(cudaStreamSynchronize(c->st));
+    if ((rc = grid_setup(c))) return rc;
     CK(cudaMemcpy(c->sp, c->h_sp.data(), sizeof(SysP), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(c->rad, c->rad_cm, sizeof(double) * 2 * (size_t)c->ninter, cudaMemcpyDeviceToDevice));
+    cw_regrid(c);
     if (c->lists_built) {
       std::swap(c->pos, c->dxn);
       c->no_snapshot = true;
       rc = build_lists(c, false, true);
       std::swap(c->pos, c->dxn);
       c->no_snapshot = false;
-      if (rc) return rc;
+      if (rc) {
+        c->lists_built = false;                     // no lists on this grid
+        return rc;
+      }
     }
-    H.extra = 0.0;
-    list_radii(P, H);
+    H = c->hs[0];
+    P = c->h_sp[0];
+    memcpy(H.hmat, hmat, sizeof H.hmat);
+    box_params(P, H);
   }
   box_widths(P, H);
   cell_shifts(P, H);

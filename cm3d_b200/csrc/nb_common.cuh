@@ -693,6 +693,9 @@ int build_lists(Ctx *c, bool device_flag, bool all);   // nb_list.cu
 std::recursive_mutex &device_mutex();           // nb_capi.cu
 using DevLock = std::lock_guard<std::recursive_mutex>;
 int list_setup(Ctx *c);                         // nb_list.cu
+int grid_setup(Ctx *c);                         // nb_list.cu: the cell grids (again, for other radii)
+void cw_regrid(Ctx *c);                         // nb_cwin.cu: the compact path on another grid
+inline int cells_cm(const SysH &H) { return H.nc_cm[0] * H.nc_cm[1] * H.nc_cm[2]; }
 void cell_shifts(SysP &P, const SysH &H);       // nb_list.cu
 double box_width(const SysH &H, int d);          // nb_list.cu
 int cells_along(const SysH &H, int d, double rlist, double cell_scale);   // nb_list.cu

@@ -1233,18 +1233,11 @@ long long cw_slots(const Ctx *c) {
 
 static int cw_setup_batch(Ctx *c);
 
-// Whether the compact path can run this context, and its tables and window
-// size: one system with at least 3 cells per axis (a batch: cw_setup_batch),
-// the full force level without the RESPA switch copy, a window of the mean
-// size (x 1.25, + 64) next to the tables in the shared memory a block may use.
-int cw_setup(Ctx *c) {
-  c->cw_ok = 0;
-  if (c->mode != CM3D_NB_MIXED) return CM3D_NB_OK;
-  if (c->need_short || c->nres_lrf > 1) return CM3D_NB_OK;
-  if (cw_env_off()) return CM3D_NB_OK;
-  if (c->nsys > 1) return cw_setup_batch(c);
-  if (c->nc[0] < 3 || c->nc[1] < 3 || c->nc[2] < 3) return CM3D_NB_OK;
-  if (c->ntypes > 16 || c->ninter > 64) return CM3D_NB_OK;       // static map / cut-off arrays
+// Whether the compact path fits one system's grid: at least 3 cells per axis
+// and a window of the mean size (x 1.25, + 64) next to the tables in the shared
+// memory a block may use; its table copies and window size.
+static bool cw_fit(Ctx *c) {
+  if (c->nc[0] < 3 || c->nc[1] < 3 || c->nc[2] < 3) return false;
   const int ljm = cw_ljm_of(c->ninter);
   const bool el = c->ncharge > 0;
   size_t tb = 0;
@@ -1255,12 +1248,28 @@ int cw_setup(Ctx *c) {
     cap = cw_room(c, CW_STATIC_SMEM, tb, ljm, 1);
     if (cw_window(c->n, c->ncells) <= (double)cap) break;
   }
-  if (cw_window(c->n, c->ncells) > (double)cap) return CM3D_NB_OK;
+  if (cw_window(c->n, c->ncells) > (double)cap) return false;
   cap = cw_env_cap(cap);
   c->cw_cap = c->cw_cap32 = (int)cap;
-  c->cw_row = CW_ROW;
   c->cw_smem = tb + ((size_t)cap + 1) * sizeof(float4) + (ljm == 2 ? (size_t)cap + 1 : 0);
   c->cw_smem = (c->cw_smem + 15) / 16 * 16;
+  return true;
+}
+
+// Whether the compact path can run this context, and its tables: one system
+// whose grid it fits (a batch: cw_setup_batch), the full force level without
+// the RESPA switch copy.
+int cw_setup(Ctx *c) {
+  c->cw_ok = 0;
+  if (c->mode != CM3D_NB_MIXED) return CM3D_NB_OK;
+  if (c->need_short || c->nres_lrf > 1) return CM3D_NB_OK;
+  if (cw_env_off()) return CM3D_NB_OK;
+  if (c->nsys > 1) return cw_setup_batch(c);
+  if (c->ntypes > 16 || c->ninter > 64) return CM3D_NB_OK;       // static map / cut-off arrays
+  if (!cw_fit(c)) return CM3D_NB_OK;
+  const int ljm = cw_ljm_of(c->ninter);
+  const bool el = c->ncharge > 0;
+  c->cw_row = CW_ROW;
   c->cw_words = cw_words_for(c->nbr_stride);
   CK(cudaMalloc(&c->cwl, sizeof(uint2) * (size_t)c->n * (size_t)c->cw_words));
   CK(cudaMalloc(&c->cwn, sizeof(int2) * (size_t)c->n));
@@ -1307,7 +1316,7 @@ int cw_setup(Ctx *c) {
   // per SM (each part stages its cell's window again); the autotuner may
   // choose another split (room for the largest)
   const int want = (4 * c->num_sms + c->ncells - 1) / c->ncells;
-  CK(cudaMalloc(&c->cw_part, sizeof(double) * CQ_COUNT * (size_t)c->ncells * CW_MAX_SPLIT));
+  CK(cudaMalloc(&c->cw_part, sizeof(double) * CQ_COUNT * (size_t)std::max(c->ncells, cells_cm(c->hs[0])) * CW_MAX_SPLIT));
   cw_set_split(c, std::max(1, std::min(want, CW_MAX_SPLIT)));
   c->cw_ok = 1;
   c->cw_use = 1;
@@ -1511,6 +1520,23 @@ void cw_set_split(Ctx *c, int nsplit) {
   if (c->cw_batch) return;
   c->cw_nsplit = std::max(1, std::min(nsplit, CW_MAX_SPLIT));
   c->cw_nitems = c->ncells * c->cw_nsplit;
+}
+
+// The compact path of one system on another cell grid, with the autotuner's
+// choices where it was open before.  Where it cannot be opened (no memory for
+// it) the system runs in the other kernels.
+void cw_regrid(Ctx *c) {
+  const int ok = c->cw_ok, use = c->cw_use, split = c->cw_nsplit;
+  if (!c->cwl) {
+    if (cw_setup(c)) {
+      c->cw_ok = c->cw_use = 0;
+      cudaGetLastError();
+    }
+    return;
+  }
+  c->cw_ok = cw_fit(c);
+  c->cw_use = c->cw_ok && (!ok || use);
+  cw_set_split(c, split);
 }
 
 // A batch's compact-list layout and the kernel that reads it: row 32

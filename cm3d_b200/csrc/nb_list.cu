@@ -1473,10 +1473,6 @@ int cells_along(const SysH &H, int d, double rlist, double cell_scale) {
   return m < 1 ? 1 : (m > 1000 ? 1000 : m);
 }
 
-// Cell grids of every system (cells at least one list radius wide in every
-// fractional direction: plane spacing 1 / |row d of hmati|), their stencils,
-// the 27 cell-corner shifts and the FP32 prefilter radius; fills the cell
-// fields of c->h_sp and allocates the binning and list arrays.
 // the 27 neighbour-cell displacements of a system's grid (one cell step
 // along each box vector), as FP32 hi + lo parts
 void cell_shifts(SysP &P, const SysH &H) {
@@ -1499,9 +1495,13 @@ void cell_shifts(SysP &P, const SysH &H) {
     if (!(box_width(H, d) / P.nc[d] <= 4.0 * H.rlist)) P.image_ok = 0;
 }
 
-int list_setup(Ctx *c) {
+// Cell grids of every system (cells at least one list radius wide in every
+// fractional direction: plane spacing 1 / |row d of hmati|), their stencils,
+// the 27 cell-corner shifts and the FP32 prefilter radius, in the cell fields
+// of c->h_sp, and the list kernel for such cells.  At set-up, and again where a
+// moving box takes the list radius back.
+int grid_setup(Ctx *c) {
   int c0 = 0;
-  double est_max = 32.0;
   for (int s = 0; s < c->nsys; s++) {
     SysP &P = c->h_sp[s];
     SysH &H = c->hs[s];
@@ -1526,58 +1526,19 @@ int list_setup(Ctx *c) {
     P.lim2 = pre ? (float)(rl * rl) : INFINITY;
     P.lim2_image = (float)(rl * rl);
     cell_shifts(P, H);
-    // first guess of the full-list slot: 1.3 x the mean number of atoms in
-    // a list sphere, plus 64
-    double vol = fabs(H.hmat[0] * (H.hmat[4] * H.hmat[8] - H.hmat[5] * H.hmat[7]) +
-                      H.hmat[1] * (H.hmat[5] * H.hmat[6] - H.hmat[3] * H.hmat[8]) +
-                      H.hmat[2] * (H.hmat[3] * H.hmat[7] - H.hmat[4] * H.hmat[6]));
-    double r = H.rlist;
-    double est = 1.3 * (double)H.n / vol * (4.0 / 3.0) * M_PI * r * r * r + 64.0;
-    if (est > (double)H.n + 31.0) est = (double)H.n + 31.0;
-    if (est > est_max) est_max = est;
   }
   c->ncells = c0;
   c->nc[0] = c->h_sp[0].nc[0];
   c->nc[1] = c->h_sp[0].nc[1];
   c->nc[2] = c->h_sp[0].nc[2];
-  std::vector<int> cell_sys(c0);
-  for (int s = 0; s < c->nsys; s++)
-    for (int k = 0; k < c->h_sp[s].ncells; k++) cell_sys[c->h_sp[s].c0 + k] = s;
-  CK(cudaMalloc(&c->cell_sys, sizeof(int) * (size_t)c0));
-  CK(cudaMemcpy(c->cell_sys, cell_sys.data(), sizeof(int) * (size_t)c0, cudaMemcpyHostToDevice));
-  CK(cudaMalloc(&c->cell_of, sizeof(int) * (size_t)c->n));
-  CK(cudaMalloc(&c->cell_start, sizeof(int) * ((size_t)c0 + 1)));
-  CK(cudaMalloc(&c->cell_cursor, sizeof(int) * ((size_t)c0 + 1)));
-  CK(cudaMemset(c->cell_cursor, 0, sizeof(int) * ((size_t)c0 + 1)));
-  CK(cudaMalloc(&c->cell_atoms, sizeof(int) * (size_t)c->n));
-  CK(cudaMalloc(&c->rank, sizeof(int) * (size_t)c->n));
-  int n_max = 0;
-  for (int s = 0; s < c->nsys; s++) n_max = std::max(n_max, c->h_sp[s].n);
-  if (n_max <= BIN_ATOMS) {
-    // an atom per thread, while the clusters of a batch fit the GPU side by side
-    c->bin_cluster = 1;
-    while (c->bin_cluster < BIN_CLUSTER && c->bin_cluster * BIN_THREADS < n_max &&
-           2 * c->bin_cluster * c->nsys <= c->num_sms)
-      c->bin_cluster *= 2;
-    CK(cudaMalloc(&c->bin_keys, sizeof(long long) * (size_t)c->n));
-  }
-  CK(cudaMalloc(&c->cnt, sizeof(int) * 4 * (size_t)c->n));
-  CK(cudaMalloc(&c->off, sizeof(long long) * 4 * ((size_t)c->n + 1)));
-  CK(cudaMalloc(&c->ltot, sizeof(long long) * LT_COUNT));
-  CK(cudaMallocHost(&c->h_ltot, sizeof(long long) * LT_COUNT));
-  CK(cudaMalloc(&c->styp, sizeof(int) * (size_t)c->n));
-  CK(cudaMalloc(&c->smeta, sizeof(int2) * (size_t)c->n));
-  CK(cudaMalloc(&c->corner, sizeof(double) * 3 * (size_t)c->n));
-  CK(cudaMalloc(&c->xq, sizeof(float4) * (size_t)c->n));
-  CK(cudaMalloc(&c->cimg, sizeof(int4) * (size_t)c->n));
   // system 0's shifts (the single-system pair kernel keeps them in shared memory)
-  CK(cudaMalloc(&c->shift, sizeof(float4) * 54));
   CK(cudaMemcpy(c->shift, c->h_sp[0].shift, sizeof(float4) * 27, cudaMemcpyHostToDevice));
   CK(cudaMemcpy(c->shift + 27, c->h_sp[0].shift_lo, sizeof(float4) * 27, cudaMemcpyHostToDevice));
   if (c->mode == CM3D_NB_MIXED) {
     // staged list build: room for 1.6x the largest mean stencil neighbourhood
     // (+64), within the shared memory a block may opt into
     double nb_max = 0;
+    c->lw_atoms = 1;
     for (int sy = 0; sy < c->nsys; sy++) {
       const SysP &S = c->h_sp[sy];
       const double per_cell = (double)S.n / (double)(S.ncells > 0 ? S.ncells : 1);
@@ -1603,6 +1564,60 @@ int list_setup(Ctx *c) {
       for (int d = 0; d < 3; d++)
         if (c->h_sp[sy].nc[d] < 3) c->list_tile = 0;
     if (lk && strcmp(lk, "walk") == 0) c->list_tile = 0;
+  }
+  return CM3D_NB_OK;
+}
+
+// The grids, and the binning and list arrays.
+int list_setup(Ctx *c) {
+  CK(cudaMalloc(&c->shift, sizeof(float4) * 54));
+  int rc = grid_setup(c);
+  if (rc) return rc;
+  // (one system: room for the grid of CM3D's radii as well, which set_box takes up)
+  const int ncells = std::max(c->ncells, c->nsys == 1 ? cells_cm(c->hs[0]) : 0);
+  std::vector<int> cell_sys((size_t)ncells, 0);
+  for (int s = 0; s < c->nsys; s++)
+    for (int k = 0; k < c->h_sp[s].ncells; k++) cell_sys[(size_t)c->h_sp[s].c0 + k] = s;
+  CK(cudaMalloc(&c->cell_sys, sizeof(int) * (size_t)ncells));
+  CK(cudaMemcpy(c->cell_sys, cell_sys.data(), sizeof(int) * (size_t)ncells, cudaMemcpyHostToDevice));
+  CK(cudaMalloc(&c->cell_start, sizeof(int) * ((size_t)ncells + 1)));
+  CK(cudaMalloc(&c->cell_cursor, sizeof(int) * ((size_t)ncells + 1)));
+  CK(cudaMemset(c->cell_cursor, 0, sizeof(int) * ((size_t)ncells + 1)));
+  double est_max = 32.0;
+  for (const SysH &H : c->hs) {
+    // first guess of the full-list slot: 1.3 x the mean number of atoms in
+    // a list sphere, plus 64
+    double vol = fabs(H.hmat[0] * (H.hmat[4] * H.hmat[8] - H.hmat[5] * H.hmat[7]) +
+                      H.hmat[1] * (H.hmat[5] * H.hmat[6] - H.hmat[3] * H.hmat[8]) +
+                      H.hmat[2] * (H.hmat[3] * H.hmat[7] - H.hmat[4] * H.hmat[6]));
+    double r = H.rlist;
+    double est = 1.3 * (double)H.n / vol * (4.0 / 3.0) * M_PI * r * r * r + 64.0;
+    if (est > (double)H.n + 31.0) est = (double)H.n + 31.0;
+    if (est > est_max) est_max = est;
+  }
+  CK(cudaMalloc(&c->cell_of, sizeof(int) * (size_t)c->n));
+  CK(cudaMalloc(&c->cell_atoms, sizeof(int) * (size_t)c->n));
+  CK(cudaMalloc(&c->rank, sizeof(int) * (size_t)c->n));
+  int n_max = 0;
+  for (int s = 0; s < c->nsys; s++) n_max = std::max(n_max, c->h_sp[s].n);
+  if (n_max <= BIN_ATOMS) {
+    // an atom per thread, while the clusters of a batch fit the GPU side by side
+    c->bin_cluster = 1;
+    while (c->bin_cluster < BIN_CLUSTER && c->bin_cluster * BIN_THREADS < n_max &&
+           2 * c->bin_cluster * c->nsys <= c->num_sms)
+      c->bin_cluster *= 2;
+    CK(cudaMalloc(&c->bin_keys, sizeof(long long) * (size_t)c->n));
+  }
+  CK(cudaMalloc(&c->cnt, sizeof(int) * 4 * (size_t)c->n));
+  CK(cudaMalloc(&c->off, sizeof(long long) * 4 * ((size_t)c->n + 1)));
+  CK(cudaMalloc(&c->ltot, sizeof(long long) * LT_COUNT));
+  CK(cudaMallocHost(&c->h_ltot, sizeof(long long) * LT_COUNT));
+  CK(cudaMalloc(&c->styp, sizeof(int) * (size_t)c->n));
+  CK(cudaMalloc(&c->smeta, sizeof(int2) * (size_t)c->n));
+  CK(cudaMalloc(&c->corner, sizeof(double) * 3 * (size_t)c->n));
+  CK(cudaMalloc(&c->xq, sizeof(float4) * (size_t)c->n));
+  CK(cudaMalloc(&c->cimg, sizeof(int4) * (size_t)c->n));
+  if (c->mode == CM3D_NB_MIXED) {
     CK(cudaMalloc(&c->rb_scan, sizeof(int) * ((size_t)c->nsys + 1)));
     CK(cudaMalloc(&c->nlen, sizeof(int) * 2 * (size_t)c->n));
     CK(cudaMemset(c->nlen, 0, sizeof(int) * 2 * (size_t)c->n));
