@@ -780,9 +780,10 @@ __global__ void k_nvt_c(StepP P, int tors_end, int level_end, const __grid_const
 
 // All substeps of a level in one cluster of blocks, with its barriers where the
 // grid-wide form starts a new kernel: for systems whose four launches per
-// substep wait for one another longer than they work (us per step, grid-wide and one cluster: argon of 864
-// atoms 52, 50; 2048, 62, 60; 4000, 69, 66; 6912 and two groups a thread, 74,
-// 78; water under 8 substeps, 648 atoms 161, 138; 3000, 199, 170; 8232, 280, 268).  What another
+// substep wait for one another longer than they work (us per step, grid-wide
+// and one cluster: argon of 864 atoms 52, 50; 2048, 62, 60; 4000, 69, 66; 6912
+// and two groups a thread, 74, 78; water under 8 substeps, 648 atoms 161, 138;
+// 3000, 199, 170; 8232, 280, 268; nvt_in_cluster draws the line).  What another
 // block wrote (kinetic terms, chunk sums, chain velocities) is read through L2.
 constexpr int NVT_THREADS = 512;
 struct ChainK {
@@ -1950,10 +1951,26 @@ static int close_level(Ctx *c, int intr, bool ks_forked = false, bool zeroed = f
   return finish_level0(c, P.dts2, true);
 }
 
+// Whether the thermostatted inner level runs in one cluster (k_nvt_cluster): a
+// group per thread, and no more atoms than its eight SMs move through memory in
+// the time that the launches of the grid-wide form take -- more of them where
+// the level has several substeps, and four launches each, and with few groups,
+// whose threads wait for their own atoms' terms either way.  (us per step,
+// cluster and grid-wide; chains of 1 to 32 atoms, one substep: 3072 groups of 2
+// atoms 68, 68; 4096 of 2, 73, 70; 2048 of 4, 87, 80; 4096 of 4, 117, 92; but
+// 1024 of 8, 117, 119; 1024 of 32, 506, 510; 512 of 32, 353, 462.  Water, one
+// and four substeps: 2197 molecules 148, 148 and 221, 239; 2744, 177, 174 and
+// 271, 275; 3375, 175, 171 and 275, 275; 4096, 155, 143 and 255, 230.)
+constexpr int NVT_CLUSTER_GROUPS = 8 * NVT_THREADS, NVT_FEW_GROUPS = 1024;
+static bool nvt_in_cluster(const Ctx *c) {
+  if (c->ngroups > NVT_CLUSTER_GROUPS) return false;
+  const bool few = c->ngroups <= NVT_FEW_GROUPS;
+  return c->n <= (few ? 32768 : c->nres_tors * c->nres_intra > 1 ? 10240 : 6144);
+}
+
 // RESPA level `intr` of one outer step (md_step.c:95-146); with `gated` the
 // rebuild kernels are gated on the device flag (graph capture), otherwise
 // the host reads the flag and rebuilds
-constexpr int NVT_CLUSTER_GROUPS = 8 * NVT_THREADS;    // one cluster's threads
 static int one_level(Ctx *c, int intr, bool gated) {
   int rc;
   StepP P = step_params(c);
@@ -1967,7 +1984,7 @@ static int one_level(Ctx *c, int intr, bool gated) {
                     c->nhc + 3 * tc, c->fxa, c->fxr, c->nvt_kin, c->dxn, c->dxi, c->grp_bond_off, c->bond_ij,
                     c->bond_p, c->grp_bend_off, c->bend_ijk, c->bend_p, c->sp, c->sys_of, c->sreb, c->lreb,
                     c->istate, c->intra, c->stat};
-    if (c->ngroups <= NVT_CLUSTER_GROUPS) {
+    if (nvt_in_cluster(c)) {
       const ChainK C = {c->nth_chunks, c->ntherm, c->th_chunk, c->th_atoms, c->th_choff, c->nvt_chsum, c->nhc};
       // the groups over as many SMs as the cluster has, two warps a block at least
       int nb = 1;
