@@ -1288,7 +1288,9 @@ __global__ void k_rebuild_cells(int nsys, const SysP *__restrict__ sp, const int
 // instead (same decisions).
 constexpr int LW_THREADS = 256;
 constexpr size_t LW_BYTES_PER_ATOM = sizeof(float4) + 2 * sizeof(int);   // s_x (w: type, charge), s_u, s_j
-constexpr int LW_MIN_ATOMS = 1024;          // atoms per SM from which neighbourhoods are staged
+constexpr int LW_MIN_ATOMS = 1024;          // atoms per SM from which neighbourhoods are staged,
+constexpr int LW_MIN_EVEN = 400;            //   and where the largest is at most LW_EVEN times the mean
+constexpr double LW_EVEN = 1.5;
 constexpr long long LW_MAX_CAP = 2944;     // largest staged neighbourhood (69 KB: 3 blocks per SM)
 
 __global__ void __launch_bounds__(LW_THREADS, 3) k_list_win(
@@ -1537,12 +1539,14 @@ int grid_setup(Ctx *c) {
   if (c->mode == CM3D_NB_MIXED) {
     // staged list build: room for 1.6x the largest mean stencil neighbourhood
     // (+64), within the shared memory a block may opt into
-    double nb_max = 0;
+    double nb_max = 0, nb_sum = 0;
     c->lw_atoms = 1;
     for (int sy = 0; sy < c->nsys; sy++) {
       const SysP &S = c->h_sp[sy];
       const double per_cell = (double)S.n / (double)(S.ncells > 0 ? S.ncells : 1);
-      nb_max = std::max(nb_max, per_cell * S.nsx * S.nsy * S.nsz);
+      const double nb = per_cell * S.nsx * S.nsy * S.nsz;
+      nb_max = std::max(nb_max, nb);
+      nb_sum += nb * S.n;
       c->lw_atoms = std::max(c->lw_atoms, (int)(1.25 * per_cell) + 1);
     }
     c->lw_smem_max = c->smem_optin > 8192 ? c->smem_optin - 8192 : 0;
@@ -1553,10 +1557,16 @@ int grid_setup(Ctx *c) {
     // warp-per-atom walk through global memory keeps more warps in flight
     if (c->lw_cap < 64 || cap > LW_MAX_CAP) c->lw_cap = 0;
     // with a few cells per block the staging of the largest neighbourhood is
-    // what the kernel waits for, and a warp per atom fills the GPU sooner (per
-    // step, 37 boxes of 27,000 atoms in all: 45 us staged, 21 us walked; 648
-    // water atoms: 5.3 and 5.6; 1024 boxes of 953,000 atoms: 406 and 510)
-    if (c->n < LW_MIN_ATOMS * c->num_sms) c->lw_cap = 0;
+    // what the kernel waits for, and a warp per atom fills the GPU sooner: in
+    // ragged batches up to 1024 atoms per SM, in even ones, whose blocks finish
+    // together, up to 400.  (us per step, walked and staged.  Ragged, the
+    // largest neighbourhood 2.3 times the mean: 27,000 atoms 99, 131; 71,000,
+    // 181, 210; 131,000, 284, 300; 216,000, 429, 428.  Even: 24,600 atoms 57,
+    // 57; 49,000 charged 151, 155; 64,000, 86, 78; 64,000 charged 204, 189;
+    // 108,000 in one box 140, 131; 150,000, 163, 149.  1.47 times: 85,000,
+    // 119, 112.)
+    const bool even = nb_max * c->n <= LW_EVEN * nb_sum;
+    if (c->n < (even ? LW_MIN_EVEN : LW_MIN_ATOMS) * c->num_sms) c->lw_cap = 0;
     const char *lk = getenv("CM3D_NB_LIST_KERNEL");
     if (lk && strcmp(lk, "walk") == 0) c->lw_cap = 0;
     c->list_tile = cap > LW_MAX_CAP ? 1 : 0;
