@@ -271,12 +271,17 @@ __global__ void k_sorted_init(int n, const SysP *__restrict__ sp, const int *__r
 // little else -- on the steps that build nothing, too: they are replayed every
 // step and each costs some 2 us to find that out (us per step, six kernels and
 // one: 648 water atoms 70, 65; 2048 argon 72, 66; 2048 charged 86, 82; 37 boxes
-// 183, 176; 12,288 water atoms 148, 147).
+// 183, 176; 12,288 water atoms 132, 128; 32,000 argon 89, 85; 8 boxes of 32,000
+// 558, 550; 100 of 3000 water atoms 2991, 2931; 31,944 water atoms 411, 411.
+// The FP64 engine, whose builds are as frequent as CM3D's: 32,000 argon atoms
+// 96, 90; 1536 water atoms 151, 149; 5184, 370, 369; but 12,288, 722, 728;
+// 24,000, 1523, 1542).
 //
 // A stage reads what other blocks wrote before the barrier; nothing read
 // earlier in the kernel is read again after another block's write, except the
 // counters, which go through L2.
 constexpr int BIN_THREADS = 1024, BIN_CLUSTER = 8, BIN_ATOMS = 4 * BIN_CLUSTER * BIN_THREADS;
+constexpr double BIN_PLAIN_PAIRS = 1e6;     // FP64 engine: most atoms x atoms per cell
 __global__ void __launch_bounds__(BIN_THREADS, 1) k_bin(
     int n, int nb, const SysP *__restrict__ sp, const int *__restrict__ sreb, int all, const __grid_constant__ Sorted S,
     int4 *cimg, int *cell_of, int *count, int *cell_start, long long *keys, int *cell_atoms,
@@ -1610,7 +1615,10 @@ int list_setup(Ctx *c) {
   CK(cudaMalloc(&c->rank, sizeof(int) * (size_t)c->n));
   int n_max = 0;
   for (int s = 0; s < c->nsys; s++) n_max = std::max(n_max, c->h_sp[s].n);
-  if (n_max <= BIN_ATOMS) {
+  // (the FP64 engine, which builds its lists at CM3D's frequency: not where
+  // each atom is ordered among hundreds in its cell, by eight SMs)
+  const bool crowded = c->mode == CM3D_NB_PLAIN_FP64 && (double)n_max * n_max > BIN_PLAIN_PAIRS * c->ncells;
+  if (n_max <= BIN_ATOMS && !crowded) {
     // an atom per thread, while the clusters of a batch fit the GPU side by side
     c->bin_cluster = 1;
     while (c->bin_cluster < BIN_CLUSTER && c->bin_cluster * BIN_THREADS < n_max &&
