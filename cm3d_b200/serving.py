@@ -61,23 +61,52 @@ class Job:
         return None if self.finished is None else self.finished - self.arrival
 
 
+def _kspace_bytes(nq: int, ktot: int) -> float:
+    """The reciprocal space's work arrays for nq charges and a spherical half set
+    of ktot k-vectors: per-tile structure factors, partial forces of every split,
+    phases and their tables.  Follows kspace_setup and kspace_reg_setup in
+    csrc/nb_kspace.cu on 148 SMs."""
+    if nq == 0 or ktot == 0:
+        return 0.0
+    sms = 148
+    kmax = (1.5 * ktot / math.pi) ** (1.0 / 3.0)
+    rows = math.ceil(0.5 * math.pi * kmax * kmax) + 1
+    fixed = 96.0 * ktot + 48.0 * nq
+    if nq * ktot >= 5e7 and kmax < 25.0:
+        # the large-sum kernels: tiles of 512 atoms, fewer where they are few
+        per = 512
+        while per > 128 and math.ceil(nq / per) * math.ceil(rows / 64) < 3 * sms:
+            per //= 2
+        split = max(math.ceil((0.5 * ktot + 2 * rows) / 2304), math.ceil(4 * sms / math.ceil(nq / 256))) + 1
+        return fixed + 16.0 * ktot * math.ceil(nq / per) + 24.0 * nq * (split + 1) + 8.0 * nq * 25
+    split = 1
+    while math.ceil(nq / 512) * split < 4 * sms and split < rows:
+        split *= 2
+    return fixed + 16.0 * ktot * math.ceil(nq / 2048) + 24.0 * nq * (min(split, rows) + 1)
+
+
 def device_bytes(system) -> int:
-    """Estimate of a job's device memory: per-atom state, the full neighbour
-    list (1.3 x the mean number of atoms in a list sphere + 64 entries per
-    atom, 4 bytes each), the k-space work arrays, plus a fixed part."""
+    """Estimate of a job's device memory, the admission control's: per-atom state,
+    the master list (slots of 1.3 x the mean number of atoms in a list sphere + 64
+    entries, 4 bytes each) and its compact form (2 bytes each, in blocks of 128
+    per segment), the k-space work arrays, plus a fixed part for the driver's
+    2 MB pages."""
     n = int(system.natoms)
     h = np.asarray(system["hmat"], float).reshape(3, 3)
     vol = abs(float(np.linalg.det(h)))
     r2 = float(np.max(system["rmaxl_skin2"])) if system["ninter"] > 0 else 0.0
-    if int(system.get("ktot", 0)) > 0:
+    ktot = int(system.get("ktot", 0))
+    if ktot > 0:
         r2 = max(r2, float(system.get("rmaxl_skin2_e", 0.0)))
-    # the engine's own lists take a skin of at least 20% of the cut-off
+    # the engine's own lists take up to 20% of the cut-off as skin
     rl = math.sqrt(r2)
     rl = max(rl, 1.2 * (rl - float(system.get("skin", rl))))
     stride = min(1.3 * n / vol * 4.0 / 3.0 * math.pi * rl ** 3 + 64.0, n + 31.0)
-    ktot = int(system.get("ktot", 0))
-    kbytes = ktot * (math.ceil(n / 2048) * 16 + 64)
-    return int(n * (4.0 * stride + 420.0) + kbytes + (8 << 20))
+    stride = 32.0 * math.ceil(stride / 32.0)
+    lists = 4.0 * stride + 256.0 * (math.ceil(stride / 128.0) + 1.0)
+    charge = system.get("qch", None)
+    nq = n if charge is None else int(np.count_nonzero(charge))
+    return int(n * (lists + 640.0) + _kspace_bytes(nq, ktot) + (8 << 20))
 
 
 class Server:
