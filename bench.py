@@ -232,16 +232,19 @@ def roofline(eng, steps: int, istep0: int, fp32_tflops: float, hbm_gbs: float) -
     t_bw = nbytes / (hbm_gbs * 1e9)
     t_fl = flops / (fp32_tflops * 1e12)
     # DRAM bytes per launch from an ncu capture (profiles/pair_kernel_traffic.json),
-    # used only while the kernel's source is the one that was captured
+    # used only while the kernel's source, and that of the lists it reads, are
+    # the ones that were captured
     kind, tpa = eng.pair_kernel()
     traffic, traffic_src = None, "no capture of this kernel"
     try:
         import hashlib
         with open(os.path.join(ROOT, "profiles", "pair_kernel_traffic.json")) as fh:
             tr = json.load(fh).get(eng.workload_name, {})
-        src = os.path.join(ROOT, "cm3d_b200", "csrc", "nb_cwin.cu" if kind == "compact" else "nb_pair.cu")
-        with open(src, "rb") as fh:
-            sha = hashlib.sha256(fh.read()).hexdigest()[:16]
+        h = hashlib.sha256()
+        for src in ("nb_cwin.cu" if kind == "compact" else "nb_pair.cu", "nb_list.cu", "nb_capi.cu"):
+            with open(os.path.join(ROOT, "cm3d_b200", "csrc", src), "rb") as fh:
+                h.update(fh.read())
+        sha = h.hexdigest()[:16]
         if tr.get("pair_kernel") == kind and tr.get("source_sha16") == sha:
             traffic = tr.get("dram_bytes_per_launch")
             traffic_src = f"{tr.get('source')} (captured {tr.get('date')}, kernel source sha {sha})"

@@ -265,10 +265,8 @@ struct EnergyItems {
   int count = 0;                    // systems
 };
 
-// Sum of the items' partials into CM3D's accumulators: one block, warp q
-// sums quantity q over the items (fixed order), then one thread applies the
-// sums in a fixed order (several quantities feed one accumulator); each pair
-// was counted from both ends, hence 1/2.
+// A system's sums over its items (energy_sums) into CM3D's accumulators: one
+// thread, in a fixed order (several quantities feed one accumulator).
 __device__ __forceinline__ void cw_apply(int mask, const double *v, double *acc) {
   if (mask & 2) {
     // (CM3D's shifted sum spothe, finter_e.c:197, is read by nothing --
@@ -296,7 +294,9 @@ __device__ __forceinline__ void cw_apply(int mask, const double *v, double *acc)
 }
 
 // One block of ER_THREADS sums system sy's items into its accumulators: 16
-// threads to an item (a 128-byte row), ER_THREADS / 16 items at a time.
+// threads to an item (a 128-byte row), ER_THREADS / 16 items at a time, then
+// thread q quantity q over those, in a fixed order; each pair was counted from
+// both ends, hence 1/2.
 constexpr int ER_THREADS = 256;
 __device__ __forceinline__ void energy_sums(const EnergyItems &E, int sy, double *acc) {
   const int2 r = E.sitems ? E.sitems[sy] : make_int2(0, E.nitems);

@@ -9,7 +9,8 @@
 //
 // The master full list (nb_list.cu: per cell-sorted atom, 32-bit entries of
 // sorted index + cell-shift code + list flags) is rewritten after every
-// rebuild into a compact list (k_cw_convert):
+// rebuild into a compact list (by k_cw_convert, where the list kernel has not
+// written it beside the master list itself, k_list_tile):
 //
 //   * a 16-bit entry holds the index of j in the 27-cell window of i's cell
 //     (the window a pair-kernel block stages in shared memory, each cell
@@ -24,10 +25,11 @@
 //     which spreads a warp's window loads over the shared-memory banks.
 //
 // The pair kernel (k_pair_cw) keeps the tables in shared memory replicated
-// RF (RG) times, lane l reading copy l % RF: with RF = 8 the 16-byte force
+// RT times, lane l reading copy l % RT: with RT = 8 the 16-byte force
 // coefficients a lane reads always lie in bank group l % 8, so a warp's 32
 // random table reads take 4 shared-memory wavefronts -- the minimum for 512
-// bytes -- instead of the ~7 that random 16-byte reads cost.
+// bytes -- instead of the ~7 that random 16-byte reads cost (RT = 4 where
+// wide cells need the room, CW_RT_FEW).
 //
 // Precision and order: distances, interpolation and the per-pair products
 // are FP32 (cell-relative coordinates, as in nb_pair.cu); each lane sums its
@@ -66,8 +68,6 @@ constexpr int CW_STATIC_SMEM = 6144;        // >= the kernel's static shared arr
 // (41,472 water atoms 111 and 119 us) where the gather kernel takes twice as
 // long (27,783 atoms in 13 A cells: 105 us, gather 147).
 constexpr int CW_RT = 8, CW_RT_FEW = 4;
-
-// per-item FP64 sums (each pair is seen from both ends: energy_sums halves)
 
 struct CwP {
   int n, ncx, ncy, ncz, nitems, nsplit, cap, words;   // words: 8-byte words per atom slot

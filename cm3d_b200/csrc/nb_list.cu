@@ -5,14 +5,17 @@
 // ngbr_liste (ngbr_list.c:103-143) and the link-cell helpers get_lnklist /
 // get_lnklist_e (energy/control/set_link.c:203-300).
 //
-// Pair membership is decided exactly as CM3D decides it: the displacement is
-// taken in FP64, folded with CM3D's period() arithmetic (md_period.new.c:39-52,
-// CM3D's anint and operation order, no FMA contraction -- this file is
-// compiled with -fmad=false as well) and compared with the per-interaction
-// radius rmaxl_skin2[map[ti][tj]] / rmaxs_skin2 (LJ, after the map == -1 and
-// exclusion tests) or rmaxl_skin2_e / rmaxs_skin2_e (charged atoms, after the
-// charge-exclusion test).  The resulting pair sets are bit-identical to
-// CM3D's.  The cell grid itself is our own: cells at least one list radius
+// Pair membership comes out as CM3D decides it.  exact_entry takes the
+// displacement in FP64, folds it with CM3D's period() arithmetic
+// (md_period.new.c:39-52, CM3D's anint and operation order, no FMA contraction
+// -- this file is compiled with -fmad=false as well) and compares with the
+// per-interaction radius rmaxl_skin2[map[ti][tj]] / rmaxs_skin2 (LJ, after the
+// map == -1 and exclusion tests) or rmaxl_skin2_e / rmaxs_skin2_e (charged
+// atoms, after the charge-exclusion test).  A pair whose FP32 distance is
+// further from every radius than a margin of some ten times its error, and
+// whose image FP32 can tell, is decided by that distance (list_flags, fold);
+// all others go through exact_entry.  The resulting pair sets are bit-identical
+// to CM3D's.  The cell grid itself is our own: cells at least one list radius
 // wide, atoms counting-sorted by cell (inside a cell by atom type, then atom
 // index), and a stencil of unique neighbour cells, so every pair within range
 // is seen exactly once per direction whatever CM3D's ncell_div is.
@@ -20,7 +23,7 @@
 // A context may hold several independent systems (SysP, nb_common.cuh): each
 // has its own box, cell grid and parameters, its cells and atoms occupy
 // contiguous ranges, and a system is rebuilt only when its own displacement
-// test asked for it (sreb[s]) unless the build covers every system (`all`).
+// test asked for it (lreb[s]) unless the build covers every system (`all`).
 //
 // Outputs
 //   lst[0..3]  CM3D's four half lists t, s, te, se as (i, j) with i < j
@@ -937,8 +940,9 @@ __device__ __forceinline__ void full_list_atom(
   }
 }
 
-// Mixed mode, warp per atom over every atom (the candidates walked in global
-// memory): the fallback of k_list_win.
+// Mixed mode, warp per atom over every atom, the candidates walked in global
+// memory: small and ragged contexts and coarse grids, whose neighbourhoods are
+// neither staged (k_list_win) nor tiled (k_list_tile).
 __global__ void __launch_bounds__(256, 3) k_list_full(
     const __grid_constant__ ListK K, const SysP *__restrict__ sp, const int *__restrict__ sys_of,
     const int *__restrict__ sreb, int all, int stride, uint32_t *__restrict__ nbr, int *__restrict__ nlen,
@@ -1285,9 +1289,10 @@ __global__ void k_rebuild_cells(int nsys, const SysP *__restrict__ sp, const int
 // moved by their cell's shift, sorted index + the cell's shift code, atom
 // index, type and charge flag) in shared memory once, then its warps build
 // the cell's atoms' lists from it: the prefilter reads shared memory, and in
-// a grid of 3 or more cells per axis the list flags come from the FP32
-// distance (fast_flags) except within a margin of a list radius, where the
-// FP64 test decides -- the same lists as the FP64 test of every candidate.
+// the list flags come from the FP32 distance (list_flags; in a grid of fewer
+// than 3 cells per axis that of the minimum image) except within a margin of a
+// list radius, where the FP64 test decides -- the same lists as the FP64 test
+// of every candidate.
 // Blocks walk the cells of the systems being rebuilt; a cell whose
 // neighbourhood holds more than `cap` atoms is walked in global memory
 // instead (same decisions).

@@ -414,8 +414,11 @@ __global__ void k_inner(StepP P, int intr, const int *__restrict__ gaoff, const 
 // positions, velocities and bonded accelerations stay in registers through
 // the ninrra x ninnra substeps.  The general kernel passes every one of them
 // through global memory, whose latency, not the arithmetic, is its time (4096
-// water molecules, 4 substeps: 26 us; here 9 us).  An atom's local index
-// selects among registers; the sums are k_inner's, in its order.
+// water molecules, 4 substeps, cold caches: 32 us; here 15 us).  An atom's
+// local index selects among registers.  The terms are added in k_inner's order;
+// a bond's and a bend's factors are formed with reciprocal roots (mol_bond,
+// mol_bend) where CM3D divides by the root, which differs in the last bits
+// (5e-14 of the forces against 64-bit references, as before).
 struct Mol3 {
   double p[3][3], v[3][3], f[3][3];      // [atom][component]
 };
