@@ -79,6 +79,7 @@ struct SysP {
   float lim2;                // FP32 list prefilter radius^2 (inf = off)
   float lim2_image;          //   and that of a minimum-image distance (grids of fewer than 3 cells)
   int image_ok;              // the grid allows FP32 minimum images in the list tests
+  int sheared;               // the box vectors are not along the axes
   float rc2_el, dx2c, offc, tablast_e;
   float hF[9], hiF[9];
   double h[9], hi[9];

@@ -468,7 +468,10 @@ __device__ __forceinline__ int grid_kind(const SysP &P) {
 // squared distance and leaves the image's shift code (CODE_EXACT where FP32
 // cannot tell, see above) and near-image bit in `code`.  The displacement is
 // a difference of coordinates no larger than a box of at most 8 list radii
-// per axis, so s carries an error of about 1e-7; 1e-5 is the margin.
+// per axis, so s carries an error of about 1e-7; 1e-5 is the margin.  In a
+// sheared box the two images of a pair half a box apart are not equally long,
+// and the other one may be within a list radius where this one is not: such a
+// pair returns 0 and so gets to its FP64 test.
 __device__ __forceinline__ float fold(const SysP &P, float dx, float dy, float dz, int &code) {
   const float sx = P.hiF[0] * dx + P.hiF[1] * dy + P.hiF[2] * dz;
   const float sy = P.hiF[3] * dx + P.hiF[4] * dy + P.hiF[5] * dz;
@@ -479,7 +482,8 @@ __device__ __forceinline__ float fold(const SysP &P, float dx, float dy, float d
   dz -= P.hF[6] * mx + P.hF[7] * my + P.hF[8] * mz;
   const float ax = fabsf(sx - mx), ay = fabsf(sy - my), az = fabsf(sz - mz);
   constexpr float EPS = 1e-5f;
-  bool exact = ax > 0.5f - EPS || ay > 0.5f - EPS || az > 0.5f - EPS;
+  const bool half = ax > 0.5f - EPS || ay > 0.5f - EPS || az > 0.5f - EPS;
+  bool exact = half;
   int near = 0;
   if (P.smallbox) {
     const float nx = (float)P.near_s[0], ny = (float)P.near_s[1], nz = (float)P.near_s[2];
@@ -490,7 +494,7 @@ __device__ __forceinline__ float fold(const SysP &P, float dx, float dy, float d
             kz = code % 3 - 1 - (int)mz * P.nc[2];
   exact |= kx < -1 || kx > 1 || ky < -1 || ky > 1 || kz < -1 || kz > 1;
   code = exact ? CODE_EXACT << ENT_CODE_SHIFT : ((kx + 1) * 9 + (ky + 1) * 3 + (kz + 1)) << ENT_CODE_SHIFT | near;
-  return fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+  return half && P.sheared ? 0.f : fmaf(dz, dz, fmaf(dy, dy, dx * dx));
 }
 
 template <class Decide>
@@ -699,7 +703,7 @@ __device__ __forceinline__ void append(uint32_t *__restrict__ out, int stride, u
   nb += __popc(bb);
 }
 
-__device__ __forceinline__ bool ortho(const SysP &P) {
+__host__ __device__ __forceinline__ bool ortho(const SysP &P) {
   return P.h[1] == 0. && P.h[2] == 0. && P.h[3] == 0. && P.h[5] == 0. && P.h[6] == 0. && P.h[7] == 0.;
 }
 // edges of an orthorhombic box's cells
@@ -1503,6 +1507,7 @@ void cell_shifts(SysP &P, const SysH &H) {
   // FP32 minimum images in the list tests of a coarse grid: candidates lie
   // within two cells, so cells of at most 4 list radii bound the displacement
   P.image_ok = 1;
+  P.sheared = ortho(P) ? 0 : 1;
   for (int d = 0; d < 3; d++)
     if (!(box_width(H, d) / P.nc[d] <= 4.0 * H.rlist)) P.image_ok = 0;
 }
