@@ -753,33 +753,51 @@ void cm3d_nb_destroy(cm3d_nb_ctx *ctx) {
   CTX_READ;  \
   c->acc_here = false
 
-// (blocks that lie back to back, as in a (3, n) array, go in one copy)
-static int put3(Ctx *c, double *dst, const double *x, const double *y, const double *z) {
-  const size_t n = c->n;
-  if (y == x + n && z == y + n) {
-    CK(cudaMemcpyAsync(dst, x, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, c->st));
-    CK(cudaStreamSynchronize(c->st));
-    return CM3D_NB_OK;
+// Three blocks of host memory to or from the device.  Blocks that lie back to
+// back, as in a (3, n) array, go in one copy, if all or none of them are
+// page-locked: a copy over memory that is partly page-locked is not allowed.
+// (Nor may the driver take one over blocks that were page-locked one by one.)
+static int copy3(Ctx *c, double *const dst[3], const double *const src[3], const double *const host[3],
+                 cudaMemcpyKind kind) {
+  const size_t n = c->n, b = sizeof(double) * n;
+  bool whole = host[1] == host[0] + n && host[2] == host[1] + n;
+  cudaMemoryType type = cudaMemoryTypeUnregistered;
+  for (int k = 0; whole && k < 3; k++) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, host[k]) != cudaSuccess) {
+      cudaGetLastError();
+      whole = false;
+      break;
+    }
+    whole = k == 0 || a.type == type;
+    type = a.type;
   }
-  CK(cudaMemcpyAsync(dst, x, sizeof(double) * n, cudaMemcpyHostToDevice, c->st));
-  CK(cudaMemcpyAsync(dst + n, y, sizeof(double) * n, cudaMemcpyHostToDevice, c->st));
-  CK(cudaMemcpyAsync(dst + 2 * n, z, sizeof(double) * n, cudaMemcpyHostToDevice, c->st));
+  if (whole) {
+    const cudaError_t e = cudaMemcpyAsync(dst[0], src[0], 3 * b, kind, c->st);
+    if (e == cudaErrorInvalidValue) {
+      cudaGetLastError();
+      whole = false;
+    } else {
+      CK(e);
+    }
+  }
+  for (int k = 0; !whole && k < 3; k++) CK(cudaMemcpyAsync(dst[k], src[k], b, kind, c->st));
   CK(cudaStreamSynchronize(c->st));
   return CM3D_NB_OK;
 }
 
+static int put3(Ctx *c, double *dst, const double *x, const double *y, const double *z) {
+  const size_t n = c->n;
+  double *const d[3] = {dst, dst + n, dst + 2 * n};
+  const double *const h[3] = {x, y, z};
+  return copy3(c, d, h, h, cudaMemcpyHostToDevice);
+}
+
 static int get3(Ctx *c, const double *src, double *x, double *y, double *z) {
   const size_t n = c->n;
-  if (y == x + n && z == y + n) {
-    CK(cudaMemcpyAsync(x, src, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
-    return CM3D_NB_OK;
-  }
-  CK(cudaMemcpyAsync(x, src, sizeof(double) * n, cudaMemcpyDeviceToHost, c->st));
-  CK(cudaMemcpyAsync(y, src + n, sizeof(double) * n, cudaMemcpyDeviceToHost, c->st));
-  CK(cudaMemcpyAsync(z, src + 2 * n, sizeof(double) * n, cudaMemcpyDeviceToHost, c->st));
-  CK(cudaStreamSynchronize(c->st));
-  return CM3D_NB_OK;
+  double *const h[3] = {x, y, z};
+  const double *const s[3] = {src, src + n, src + 2 * n}, *const hc[3] = {x, y, z};
+  return copy3(c, h, s, hc, cudaMemcpyDeviceToHost);
 }
 
 int cm3d_nb_set_positions(cm3d_nb_ctx *ctx, const double *px, const double *py, const double *pz) {
