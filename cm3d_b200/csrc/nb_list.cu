@@ -277,8 +277,8 @@ __global__ void k_sorted_init(int n, const SysP *__restrict__ sp, const int *__r
 // 183, 176; 12,288 water atoms 132, 128; 32,000 argon 89, 85; 8 boxes of 32,000
 // 558, 550; 100 of 3000 water atoms 2991, 2931; 31,944 water atoms 411, 411.
 // The FP64 engine, whose builds are as frequent as CM3D's: 32,000 argon atoms
-// 96, 90; 1536 water atoms 151, 149; 5184, 370, 369; but 12,288, 722, 728;
-// 24,000, 1523, 1542).
+// 89, 84; 1536 water atoms 157, 155; 5184, 283, 281; but 12,288, 496, 500;
+// 24,000, 875, 885).
 //
 // A stage reads what other blocks wrote before the barrier; nothing read
 // earlier in the kernel is read again after another block's write, except the
@@ -377,11 +377,9 @@ struct ListK {
 // order.  Returns the pair's full-list entry without j: its list flags
 // (ENT_LJ t, ENT_LJS s, ENT_EL te, ENT_ELS se), near-image bit and cell-shift
 // code, and EXACT_BAD where the code does not exist; 0 for a pair in no list.
-// Not inlined: the few pairs that FP32 cannot decide would otherwise cost
-// every list kernel its registers.
 constexpr uint32_t EXACT_BAD = 1u;
 constexpr uint32_t ENT_FLAGS = ENT_LJ | ENT_EL | ENT_LJS | ENT_ELS;
-__device__ __noinline__ uint32_t exact_entry(const SysP &P, const ListK &K, int i, int j) {
+__device__ __forceinline__ uint32_t exact_test(const SysP &P, const ListK &K, int i, int j) {
   const int n = K.n;
   const double *__restrict__ pos = K.pos;
   const int ti = K.itype[i];
@@ -429,6 +427,11 @@ __device__ __noinline__ uint32_t exact_entry(const SysP &P, const ListK &K, int 
   const int kz = (ci.w - cj.w - (int)mz) * P.nc[2] + (((ci.x >> 20) & 1023) - ((cj.x >> 20) & 1023));
   if (kx < -1 || kx > 1 || ky < -1 || ky > 1 || kz < -1 || kz > 1) return en | 13u << ENT_CODE_SHIFT | EXACT_BAD;
   return en | (uint32_t)((kx + 1) * 9 + (ky + 1) * 3 + (kz + 1)) << ENT_CODE_SHIFT;
+}
+// Not inlined in the full-list kernels: the few pairs that FP32 cannot decide
+// would otherwise cost them their registers.
+__device__ __noinline__ uint32_t exact_entry(const SysP &P, const ListK &K, int i, int j) {
+  return exact_test(P, K, i, j);
 }
 
 // The candidate walk shared by both list kernels.  One warp owns the
@@ -719,8 +722,14 @@ struct ListCaps {
 // list per atom, FILL = true writes them at the scanned offsets, compacted
 // with warp ballots in candidate order (deterministic).  Always built for
 // every system (host-driven builds and the single-system plain engine).
+// Bound by the latency of the candidates' loads, hence by the warps that the
+// registers leave: the FP64 test is in line and three blocks fit an SM, where
+// a call of it took 98 registers and left two; stencil cells wholly out of
+// reach are skipped.  (us per FP64 step of 5184, 12,288 and 24,000 water atoms:
+// called 354, 671, 1274; in line 314, 577, 1057; and with the cells skipped
+// 281, 496, 874.)
 template <bool FILL>
-__global__ void __launch_bounds__(256) k_list_half(
+__global__ void __launch_bounds__(256, 3) k_list_half(
     const __grid_constant__ ListK K, const SysP *__restrict__ sp, const int *__restrict__ sys_of, ListCaps C,
     int *__restrict__ cnt, const long long *__restrict__ off,
     const long long *__restrict__ tot, int2 *__restrict__ l0, int2 *__restrict__ l1, int2 *__restrict__ l2,
@@ -767,7 +776,7 @@ __global__ void __launch_bounds__(256) k_list_half(
     const bool exact = r2f < 0.f;
     bool near;
     uint32_t fl = list_flags(P, K, A, on && !exact, i, mj, r2f, &near);
-    if (on && (exact || near)) fl = exact_entry(P, K, i, j);
+    if (on && (exact || near)) fl = exact_test(P, K, i, j);
     bad |= fl & EXACT_BAD;
     const unsigned b0 = __ballot_sync(0xffffffffu, fl & ENT_LJ), b1 = __ballot_sync(0xffffffffu, fl & ENT_LJS);
     const unsigned b2 = __ballot_sync(0xffffffffu, fl & ENT_EL), b3 = __ballot_sync(0xffffffffu, fl & ENT_ELS);
@@ -782,7 +791,8 @@ __global__ void __launch_bounds__(256) k_list_half(
       p[0] += __popc(b0); p[1] += __popc(b1); p[2] += __popc(b2); p[3] += __popc(b3);
     }
   };
-  walk_candidates(P, K, i, true, qbuf, qr, decide, grid_kind(P), false, make_float3(0.f, 0.f, 0.f), t);
+  const int kind = grid_kind(P);
+  walk_candidates(P, K, i, true, qbuf, qr, decide, kind, kind == G_STENCIL && ortho(P), cell_width(P), t);
   if (FILL) {
     if (bad && lane == 0) atomicAdd((unsigned long long *)(stat + ST_BADSHIFT), 1ull);
   } else if (lane == 0) {
