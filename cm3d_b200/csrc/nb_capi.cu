@@ -187,9 +187,21 @@ static void box_widths(SysP &P, const SysH &H) {
 // 122 with 0.86 A.  The windows beside four copies of the erfc tables now leave
 // room for the full skin in all of these but the 10,125 and 8232.)  In a batch
 // all systems or none run in the compact kernel: there the skin always stops.
-constexpr double LIST_SKIN = 0.2, LIST_SKIN_LEAST = 0.1;
+//
+// A batch's systems with fewer than 3 cells along an axis are walked by a block
+// each in the pair kernel, and from some 500 atoms on that walk, as long as its
+// lists, is the step: they take a skin of LIST_SKIN_COARSE.  (us per step, 0.5 A
+// -- CM3D's --, 1, 1.5 and 2 A: 20 boxes of 1536 water atoms 1371, 1397, 1524,
+// 1690; 60 of them 2026, 1807, 1867, 1946; 8 of 648 790, 822, 877, 896; but 100
+// of 375 592, 585, 583, 575, and 400 of 300 charged atoms 424 and 412 with
+// CM3D's skin and the full one.  One box of 1536 alone, 82, 67, 62, 60.)
+constexpr double LIST_SKIN = 0.2, LIST_SKIN_LEAST = 0.1, LIST_SKIN_COARSE = 0.1;
+constexpr int LIST_COARSE_ATOMS = 512;
 static double list_skin(const SysH &H, double rc_max, bool consistent, double cell_scale, long long slots, bool batch) {
-  double extra = LIST_SKIN * rc_max - H.skin;
+  bool coarse = false;
+  for (int d = 0; d < 3; d++) coarse = coarse || cells_along(H, d, H.rlist_cm, cell_scale) < 3;
+  const bool walked = batch && coarse && H.n > LIST_COARSE_ATOMS;
+  double extra = (walked ? LIST_SKIN_COARSE : LIST_SKIN) * rc_max - H.skin;
   if (!consistent || !(H.skin > 0.0) || !(extra > 0.0)) return 0.0;
   // the most a radius can grow with m cells of it left along direction d
   auto room = [&](int d, int m) { return (1.0 - 1e-9) * box_width(H, d) / (m * cell_scale) - H.rlist_cm; };
