@@ -189,14 +189,15 @@ static void box_widths(SysP &P, const SysH &H) {
 // all systems or none run in the compact kernel: there the skin always stops.
 //
 // A batch's systems with fewer than 3 cells along an axis are walked by a block
-// each in the pair kernel, and from some 500 atoms on that walk, as long as its
+// each in the pair kernel, and from some 1000 atoms on that walk, as long as its
 // lists, is the step: they take a skin of LIST_SKIN_COARSE.  (us per step, 0.5 A
 // -- CM3D's --, 1, 1.5 and 2 A: 20 boxes of 1536 water atoms 1371, 1397, 1524,
-// 1690; 60 of them 2026, 1807, 1867, 1946; 8 of 648 790, 822, 877, 896; but 100
-// of 375 592, 585, 583, 575, and 400 of 300 charged atoms 424 and 412 with
-// CM3D's skin and the full one.  One box of 1536 alone, 82, 67, 62, 60.)
+// 1690; 60 of them 2026, 1807, 1867, 1946; but 100 of 375 592, 585, 583, 575, and
+// 400 of 300 charged atoms 424 and 412 with CM3D's skin and the full one.  Between
+// the two, 8 of 648, 790, 822, 877, 896: these keep the skin that a box has alone,
+// and so its results to the last bit.  One box of 1536 alone, 82, 67, 62, 60.)
 constexpr double LIST_SKIN = 0.2, LIST_SKIN_LEAST = 0.1, LIST_SKIN_COARSE = 0.1;
-constexpr int LIST_COARSE_ATOMS = 512;
+constexpr int LIST_COARSE_ATOMS = 1024;
 static double list_skin(const SysH &H, double rc_max, bool consistent, double cell_scale, long long slots, bool batch) {
   bool coarse = false;
   for (int d = 0; d < 3; d++) coarse = coarse || cells_along(H, d, H.rlist_cm, cell_scale) < 3;

@@ -31,6 +31,7 @@ def lj(natoms, skin_of_cut, charged):
 
 CASES = {
     "water 375, 648, 1536": lambda: [water(5), water(6), water(8)],
+    "water 1029": lambda: [water(7), water(7, 1.0), water(6)],
     "water 1536 at 0.5, 1 and 1.5 A, and 3993": lambda: [water(8), water(8, 1.0), water(8, 1.5), water(11)],
     "charged 510, 512, 514": lambda: [lj(n, 0.06, True) for n in (510, 512, 514)],
     "argon 512, 513, 2048": lambda: [lj(n, 0.06, False) for n in (512, 513, 2048)],
