@@ -461,7 +461,7 @@ constexpr int CODE_EXACT = 31;             // queue code: the FP64 test decides
 constexpr int QUEUE_NEAR = (int)ENT_NEAR;  // queue bit: ENT_NEAR of a small box
 enum { G_EXACT = 0, G_STENCIL = 1, G_IMAGE = 2 };
 
-__device__ __forceinline__ int grid_kind(const SysP &P) {
+__host__ __device__ __forceinline__ int grid_kind(const SysP &P) {
   if (P.nc[0] >= 3 && P.nc[1] >= 3 && P.nc[2] >= 3) return P.smallbox ? G_EXACT : G_STENCIL;
   return P.image_ok ? G_IMAGE : G_EXACT;
 }
@@ -723,13 +723,15 @@ struct ListCaps {
 // with warp ballots in candidate order (deterministic).  Always built for
 // every system (host-driven builds and the single-system plain engine).
 // Bound by the latency of the candidates' loads, hence by the warps that the
-// registers leave: the FP64 test is in line and three blocks fit an SM, where
-// a call of it took 98 registers and left two; stencil cells wholly out of
-// reach are skipped.  (us per FP64 step of 5184, 12,288 and 24,000 water atoms:
-// called 354, 671, 1274; in line 314, 577, 1057; and with the cells skipped
-// 281, 496, 874.)
-template <bool FILL>
-__global__ void __launch_bounds__(256, 3) k_list_half(
+// registers leave.  STENCIL, every system's grid of three and more cells per
+// axis: the FP64 test is in line and three blocks fit an SM, where a call of it
+// takes 98 registers and leaves two; stencil cells wholly out of reach are
+// skipped.  (us per FP64 step of 5184, 12,288 and 24,000 water atoms: called
+// 354, 671, 1274; in line 314, 577, 1057; and with the cells skipped 275, 484,
+// 848.)  In coarser grids, whose few atoms do not fill the SMs, the registers
+// are worth more than the warps (1536 atoms 152; bounded to three blocks, 156).
+template <bool FILL, bool STENCIL>
+__global__ void __launch_bounds__(256, STENCIL ? 3 : 2) k_list_half(
     const __grid_constant__ ListK K, const SysP *__restrict__ sp, const int *__restrict__ sys_of, ListCaps C,
     int *__restrict__ cnt, const long long *__restrict__ off,
     const long long *__restrict__ tot, int2 *__restrict__ l0, int2 *__restrict__ l1, int2 *__restrict__ l2,
@@ -773,10 +775,10 @@ __global__ void __launch_bounds__(256, 3) k_list_half(
     const int2 mj = on ? K.smeta[qbuf[slot]] : make_int2(-1, 0);
     const float r2f = qr[slot];
     const int j = mj.x;
-    const bool exact = r2f < 0.f;
+    const bool exact = !STENCIL && r2f < 0.f;
     bool near;
     uint32_t fl = list_flags(P, K, A, on && !exact, i, mj, r2f, &near);
-    if (on && (exact || near)) fl = exact_test(P, K, i, j);
+    if (on && (exact || near)) fl = STENCIL ? exact_test(P, K, i, j) : exact_entry(P, K, i, j);
     bad |= fl & EXACT_BAD;
     const unsigned b0 = __ballot_sync(0xffffffffu, fl & ENT_LJ), b1 = __ballot_sync(0xffffffffu, fl & ENT_LJS);
     const unsigned b2 = __ballot_sync(0xffffffffu, fl & ENT_EL), b3 = __ballot_sync(0xffffffffu, fl & ENT_ELS);
@@ -791,8 +793,8 @@ __global__ void __launch_bounds__(256, 3) k_list_half(
       p[0] += __popc(b0); p[1] += __popc(b1); p[2] += __popc(b2); p[3] += __popc(b3);
     }
   };
-  const int kind = grid_kind(P);
-  walk_candidates(P, K, i, true, qbuf, qr, decide, kind, kind == G_STENCIL && ortho(P), cell_width(P), t);
+  walk_candidates(P, K, i, true, qbuf, qr, decide, STENCIL ? G_STENCIL : grid_kind(P), STENCIL && ortho(P),
+                  cell_width(P), t);
   if (FILL) {
     if (bad && lane == 0) atomicAdd((unsigned long long *)(stat + ST_BADSHIFT), 1ull);
   } else if (lane == 0) {
@@ -1828,9 +1830,12 @@ int build_lists(Ctx *c, bool device_flag, bool all) {
   }
   if (want_half) {
     // CM3D's lists, by CM3D's radii
+    const bool stencil = std::all_of(c->h_sp.begin(), c->h_sp.end(), [](const SysP &S) { return grid_kind(S) == G_STENCIL; });
+    const auto half_count = stencil ? k_list_half<false, true> : k_list_half<false, false>;
+    const auto half_fill = stencil ? k_list_half<true, true> : k_list_half<true, false>;
     K.rad = c->rad_cm;
     K.own = 0;
-    k_list_half<false><<<grid_for(warps_threads, 256), 256, 0, c->st>>>(
+    half_count<<<grid_for(warps_threads, 256), 256, 0, c->st>>>(
         K, c->sp, c->sys_of, caps(c), c->cnt, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, c->stat, nullptr,
         gate);
     k_scan<int, long long><<<dim3(1, 4), 1024, 0, c->st>>>(c->cnt, c->off, c->ltot, n, gate);
@@ -1845,7 +1850,7 @@ int build_lists(Ctx *c, bool device_flag, bool all) {
         c->hcount[k] = c->h_ltot[k];
       }
     }
-    k_list_half<true><<<grid_for(warps_threads, 256), 256, 0, c->st>>>(
+    half_fill<<<grid_for(warps_threads, 256), 256, 0, c->st>>>(
         K, c->sp, c->sys_of, caps(c), c->cnt, c->off, c->ltot, c->lst[0], c->lst[1], c->lst[2], c->lst[3], c->stat,
         halt, gate);
     c->launches++;
